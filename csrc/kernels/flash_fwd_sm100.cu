@@ -66,7 +66,10 @@ struct Bars {
   uint64_t q_full;
   uint64_t k_full[3], k_empty[3], v_full[2], v_empty[2];
   uint64_t s_full[2], s_empty[2];
-  uint64_t p_full, pv_done;
+  // Two barriers each, by the tile's parity: the scores of tile j + 1 are ready before P(j) is complete, so warps drift a tile apart.  On one barrier a fast
+  // warp's P(j + 1) would be counted as a slow one's P(j), and a warp that waits for P V(n - 1) behind its last tile, while a slow one has yet to deliver
+  // P(n - 2), would take the phase before that for the one it wants.
+  uint64_t p_full[2], pv_done[2];
   uint64_t qa_ready;                   // PT: Q copied to tensor memory (one arrival per softmax warp)
   uint32_t tmem_base;
   int abort_flag;
@@ -128,8 +131,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
       mbar_init(&bars->v_full[i], 1); mbar_init(&bars->v_empty[i], 1);
       mbar_init(&bars->s_full[i], 1); mbar_init(&bars->s_empty[i], 8);
     }
-    mbar_init(&bars->p_full, 8);
-    mbar_init(&bars->pv_done, 1);
+    mbar_init(&bars->p_full[0], 8);
+    mbar_init(&bars->p_full[1], 8);
+    mbar_init(&bars->pv_done[0], 1);
+    mbar_init(&bars->pv_done[1], 1);
     mbar_init(&bars->qa_ready, 8);
     bars->abort_flag = 0;
     fence_barrier_init();
@@ -211,7 +216,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     for (int j = 0; j < n_tiles && ok; ++j) {
       if (j + 1 < n_tiles) { ok = issue_qk(j + 1); if (!ok) break; }
       const int st = j & 1; const uint32_t ph = (j >> 1) & 1;
-      if (!mbar_wait_warp(&bars->p_full, j & 1, abort_flag)) { if (lane == 0) atomicCAS(err, 0, ERR_WAIT_OTHER); ok = false; break; }
+      if (!mbar_wait_warp(&bars->p_full[st], ph, abort_flag)) { if (lane == 0) atomicCAS(err, 0, ERR_WAIT_OTHER); ok = false; break; }
       if (!mbar_wait_warp(&bars->v_full[st], ph, abort_flag)) { if (lane == 0) atomicCAS(err, 0, ERR_WAIT_FULL); ok = false; break; }
       tc_fence_after();
       const uint32_t va = smem_u32(sV + st * C::V_BYTES);
@@ -230,7 +235,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
           }
         }
         umma_commit(&bars->v_empty[st]);
-        umma_commit(&bars->pv_done);
+        umma_commit(&bars->pv_done[st]);
       }
       __syncwarp();
     }
@@ -337,6 +342,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
             }
           }
         }
+        __syncwarp();                                  // the masks above branch by row; what follows takes whole warps
         if constexpr (SIG) {
           const uint32_t pbase = tmem + lane_addr + (st ? C::TMEM_S1 : C::TMEM_S0) + half * (HC / 2);
           // the other thread of the row has its scores in registers before this one overwrites their columns
@@ -352,7 +358,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
           tmem_st_wait();
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&bars->p_full);
+          if (lane == 0) mbar_arrive(&bars->p_full[st]);
           continue;
         }
         {
@@ -377,7 +383,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
       const bool any_need = __any_sync(0xffffffffu, need);
       // PV(j-1) must be complete before the shared P buffer is overwritten or O is rescaled (PT: only the latter)
       if (j > 0 && (!PT || any_need)) {
-        const bool got = mbar_wait(&bars->pv_done, (j - 1) & 1, abort_flag);
+        const bool got = mbar_wait(&bars->pv_done[st ^ 1], ((j - 1) >> 1) & 1, abort_flag);
         if (!__all_sync(0xffffffffu, got)) { atomicCAS(err, 0, ERR_WAIT_OTHER); ok = false; continue; }
         tc_fence_after();
       }
@@ -433,11 +439,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
       if (!PT) fence_proxy_async();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->p_full);
+      if (lane == 0) mbar_arrive(&bars->p_full[st]);
     }
     // epilogue: O / l -> bf16, lse
     if (ok && n_tiles > 0) {
-      const bool got = mbar_wait(&bars->pv_done, (n_tiles - 1) & 1, abort_flag);
+      const bool got = mbar_wait(&bars->pv_done[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1, abort_flag);
       if (!__all_sync(0xffffffffu, got)) { atomicCAS(err, 0, ERR_WAIT_OTHER); ok = false; }
     }
     // the row sum over all columns (both threads of a row reach this barrier: neither branch above skips it)

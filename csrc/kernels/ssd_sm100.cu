@@ -1,295 +1,841 @@
-// Mamba-2 SSD forward scan for sm_100a (chunk 64, state dimension N = 128, head dimension P = 64).
+// Mamba-2 state space scan, forward and backward (head dimension P = 64, state dimension N = 128, chunks of 64 tokens).
 //
-// One CTA walks the chunks of one (batch, pair of heads): two heads of the same B / C group share every key / query
-// operand, so their 64-wide value rows are stacked into the 128 rows (TMEM lanes) of one accumulator.  With a the
-// per-step log decay dt * A of a head, g its running sum inside the chunk, X~ = x dt:
-//     y_i  = e^{g_i} C_i S0 + sum_{j <= i} (C_i . B_j) e^{g_i - g_j} X~_j
-//     S1   = e^{g_L} S0 + sum_j e^{g_L - g_j} X~_j (x) B_j
-// computed transposed (rows = value index p of the two heads):
-//     o1 = S^T C^T ;  o2 = X~^T P_h^T (one product per head, the other head's rows of the operand are zero) ;
-//     dS = (X~ e^{g_L - g})^T B ;  y^T = e^{g} o1 + o2 ;  S^T <- e^{g_L} S^T + dS
-// P_h = (C B^T) o e^{g_i - g_j} (lower triangle) and g arrive from the caller per head.  Same roles and bounded waits
-// as the gated-delta-rule scan: warps 0..3 math (thread = TMEM lane), warp 4 TMA producer, warp 5 MMA issuer.
+// With g_i the running sum of dt A inside a chunk, S the state in front of it and h the head (several heads share one group's B and C):
+//     y_i = e^{g_i} S C_i + sum_{j <= i} (C_i . B_j) e^{g_i - g_j} dt_j x_j + D x_i         S <- e^{g_L} S + sum_j e^{g_L - g_j} dt_j x_j B_j^T
+// The work splits at the state:
+//   ssd_states  one CTA per (batch, head, slice of the state's columns) walks the chunks and leaves the state in front of each of them in memory; run in reverse
+//               with (dy, C, e^{g_i}) in the places of (x, B, dt e^{g_L - g}) it leaves the gradient of the state behind each chunk.  Nothing else is sequential.
+//   ssd_output  y of one chunk and group, head after head: C B^T stays in registers for all of them.
+//   ssd_local   the gradients of one chunk and group, head after head, from the two states.  dC, dB and the score gradients are summed over the heads in
+//               registers, so that the product with B (C) is one per group and not one per head:
+//                 E = dy x^T          M = (C B^T) o e^{g_i - g_j}        W = sum_h E o e^{g_i - g_j} dt_j
+//                 dC = sum_h e^{g_i} (dy S) + W B          dB = sum_h dt_j e^{g_L - g_j} (x dS) + W^T C          dx = dt_j (M^T dy + e^{g_L - g_j} B dS^T) + D dy
+//               and the gradients of the decays from row and column sums of M o E and from the dots of (dy S) with C and (x dS) with B.
+//   ssd_reduce  sums what several CTAs made of one group's dB and dC, and dA and dD over the chunks, in a fixed order.
+// x, B, C and dy enter every product as the bf16 numbers they are.  The forward rounds the state, the weights of a chunk's own tokens and the decayed x to bf16,
+// once each.  The backward keeps all of them in fp32: such an operand goes through the tensor cores as three bf16 terms (24 bits of mantissa), smallest first.
 //
-// Replaces the reference's ported SSD forward kernels ChunkState / StatePassing / ChunkScan
-// (src/dew/nn/kernels/mamba_ssd.py:421-660).
-#include "../common/ptx.cuh"
-#include "../common/tmap.h"
+// The products are narrow (64 rows, 64 to 128 columns, a reduction of 64 to 128) and their fp32 operands change with every head, so they run on mma.sync out of
+// registers, where an operand is scaled and split without passing through memory; 146 GFLOP of them stand in the backward of 2 x 4096 x 64 heads.
+//
+// Replaces the reference's ported SSD kernels ChunkState / StatePassing / ChunkScan (src/dew/nn/kernels/mamba_ssd.py:421-660).
+#include <cstdint>
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include "../common/mma_bf16.cuh"
 
 namespace dewb {
 namespace ssd {
 
-constexpr int ND = 128;           // state dimension (rows of B and C)
-constexpr int PD = 64;            // head dimension
-constexpr int CH = 64;
+using namespace mma16;
+
+constexpr int N = 128, P = 64, L = 64;
 constexpr uint32_t FULL = 0xffffffffu;
-constexpr int THREADS = 192;
-constexpr int TMA_WARP = 4, MMA_WARP = 5;
-constexpr int T16 = CH * 128 * 2;                      // [64 x 128] bf16 tile (two 64-column sub-tiles)
-constexpr int T8 = CH * CH * 2;                        // [64 x 64] bf16 tile
-constexpr int STAGE = 3 * T16 + 2 * T8;                // X~ pair, C, B, P of both heads
-constexpr int OFF_STATE = 2 * STAGE;                   // [128 x 128] bf16 state tile
-constexpr int OFF_VN0 = OFF_STATE + 2 * T16;           // X~^T of head 0 (rows 64..127 zero)
-constexpr int OFF_VN1 = OFF_VN0 + T16;                 // X~^T of head 1 (rows 0..63 zero)
-constexpr int OFF_VD = OFF_VN1 + T16;                  // decayed X~^T of both heads
-constexpr int OFF_G = OFF_VD + T16;                    // g: [stage][head][64]
-constexpr int OFF_BARS = OFF_G + 2 * 2 * CH * 4;
-constexpr int SMEM = OFF_BARS + 256;
-constexpr int F_X = 0, F_C = T16, F_B = 2 * T16, F_P0 = 3 * T16, F_P1 = 3 * T16 + T8;
-static_assert(SMEM <= 232448, "ssd scan exceeds the shared memory of an SM");
+constexpr int SMS = 148;
 
-struct Bars {
-  uint64_t in_full[2], in_empty[2], s_ready, vn_ready, out_full;
-  uint32_t tmem_base;
-  int abort_flag, poisoned;
+// What the kernels read of the call's tensors: element strides between tokens and batch rows; heads (groups) of a token lie P (N) elements apart.
+struct Call {
+  const __nv_bfloat16 *x, *Bm, *Cm, *dy;
+  const float *dt, *A, *D;
+  long long xb, xt, bb, bt, cb, ct;      // dy is contiguous
+  int B, T, H, G, chunks;
 };
-static_assert(sizeof(Bars) <= 256, "Bars must fit its slot");
 
-__device__ __forceinline__ uint32_t swz(int r, int c16) { return static_cast<uint32_t>(r * 128 + ((c16 ^ (r & 7)) << 4)); }
+__device__ __forceinline__ void cp16(void* dst, const void* src, bool real) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(real ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
 
-__device__ __forceinline__ void write_state_row(uint8_t* tile, int v, const float (&S)[ND]) {
+// A tile of 64 rows of CH 16-byte pieces, piece c of row r at (c ^ swizzle(r)): eight rows of one column of pieces lie in eight different bank groups.
+template <int CH>
+__device__ __forceinline__ int piece(int r, int c) { return (r * CH + (CH >= 8 ? c ^ (r & 7) : c ^ ((r >> 1) & 3))) * 16; }
+
+// rows [0, real) from memory, zeros behind them
+template <int CH, int THREADS>
+__device__ __forceinline__ void load_tile(uint8_t* dst, const __nv_bfloat16* src, long long stride, int real) {
 #pragma unroll
-  for (int c16 = 0; c16 < 16; ++c16) {
-    uint4 pk;
-    pk.x = pack_bf16(S[c16 * 8 + 0], S[c16 * 8 + 1]); pk.y = pack_bf16(S[c16 * 8 + 2], S[c16 * 8 + 3]);
-    pk.z = pack_bf16(S[c16 * 8 + 4], S[c16 * 8 + 5]); pk.w = pack_bf16(S[c16 * 8 + 6], S[c16 * 8 + 7]);
-    *reinterpret_cast<uint4*>(tile + (c16 >> 3) * (128 * 128) + swz(v, c16 & 7)) = pk;
+  for (int i = 0; i < L * CH / THREADS; ++i) {
+    const int at = i * THREADS + static_cast<int>(threadIdx.x), r = at / CH, c = at % CH;
+    cp16(dst + piece<CH>(r, c), src + (r < real ? r * stride : 0) + c * 8, r < real);
   }
 }
 
-__global__ void __launch_bounds__(THREADS, 1)
-ssd_scan_fwd_kernel(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtensorMap tc,
-                    const __grid_constant__ CUtensorMap tb, const __grid_constant__ CUtensorMap tp,
-                    const float* __restrict__ gc, const float* __restrict__ initial, __nv_bfloat16* __restrict__ out,
-                    float* __restrict__ final_state, int T, int H, int G, int Tp, int N, int* __restrict__ err) {
-  extern __shared__ __align__(1024) uint8_t smem[];
-  if ((smem_u32(smem) & 1023u) != 0) {
-    if (threadIdx.x == 0) atomicCAS(err, 0, ERR_BAD_ARG);
-    return;
-  }
-  Bars* bars = reinterpret_cast<Bars*>(smem + OFF_BARS);
-  if (threadIdx.x == 0) bars->poisoned = *reinterpret_cast<volatile int*>(err);
-  __syncthreads();
-  if (bars->poisoned != 0) return;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int Hp = H / 2;
-  const int x = blockIdx.x, b = x / Hp, hp = x % Hp;
-  const int h0 = 2 * hp;
-  const int grp = h0 / (H / G);
-  if (tid == 0) {
-    for (int i = 0; i < 2; ++i) { mbar_init(&bars->in_full[i], 1); mbar_init(&bars->in_empty[i], 4); }
-    mbar_init(&bars->s_ready, 4);
-    mbar_init(&bars->vn_ready, 4);
-    mbar_init(&bars->out_full, 1);
-    bars->abort_flag = 0;
-    fence_barrier_init();
-    fence_proxy_async();
-  }
-  if (warp == MMA_WARP) { tmem_alloc(&bars->tmem_base, 256); tmem_relinquish(); }
-  // the halves of the two X~^T operand tiles that belong to the other head stay zero for the whole kernel
-  for (int i = tid; i < 2 * T16 / 16; i += THREADS) reinterpret_cast<uint4*>(smem + OFF_VN0)[i] = make_uint4(0u, 0u, 0u, 0u);
-  fence_proxy_async();
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = bars->tmem_base;
-  volatile int* abort_flag = &bars->abort_flag;
-  uint8_t* sState = smem + OFF_STATE;
-  uint8_t* sVn0 = smem + OFF_VN0;
-  uint8_t* sVn1 = smem + OFF_VN1;
-  uint8_t* sVd = smem + OFF_VD;
-  float* sG = reinterpret_cast<float*>(smem + OFF_G);
-  constexpr int TM_O1 = 0, TM_O2 = 64, TM_DS = 128;
+// Fragments.  A operand (16 rows x 16) of a row-major tile; of its transpose (16 columns x 16 rows).
+template <int CH>
+__device__ __forceinline__ void frag_a(uint32_t (&a)[4], const uint8_t* t, int row, int ks) {
+  const int lane = threadIdx.x & 31, m = lane >> 3;
+  ldsm4(a, smem_addr(t + piece<CH>(row + (m & 1) * 8 + (lane & 7), ks * 2 + (m >> 1))));
+}
+template <int CH>
+__device__ __forceinline__ void frag_a_t(uint32_t (&a)[4], const uint8_t* t, int ks, int col) {      // col: in pieces of 8
+  const int lane = threadIdx.x & 31, m = lane >> 3;
+  ldsm4_t(a, smem_addr(t + piece<CH>(ks * 16 + (m >> 1) * 8 + (lane & 7), col + (m & 1))));
+}
+// B operands of two neighbouring column tiles: reduction along the tile's rows (columns: pieces col, col + 1), or along its columns (columns of the product: rows row ..)
+template <int CH>
+__device__ __forceinline__ void frag_b_t(uint32_t (&b)[4], const uint8_t* t, int ks, int col) {
+  const int lane = threadIdx.x & 31, m = lane >> 3;
+  ldsm4_t(b, smem_addr(t + piece<CH>(ks * 16 + (m & 1) * 8 + (lane & 7), col + (m >> 1))));
+}
+template <int CH>
+__device__ __forceinline__ void frag_b(uint32_t (&b)[4], const uint8_t* t, int row, int ks) {
+  const int lane = threadIdx.x & 31, m = lane >> 3;
+  ldsm4(b, smem_addr(t + piece<CH>(row + (m >> 1) * 8 + (lane & 7), ks * 2 + (m & 1))));
+}
 
-  if (warp == TMA_WARP) {
-    if (lane == 0) {
-      tma_prefetch_desc(&tx); tma_prefetch_desc(&tc); tma_prefetch_desc(&tb); tma_prefetch_desc(&tp);
-      for (int n = 0; n < N; ++n) {
-        const int s = n & 1; const uint32_t ph = (n >> 1) & 1;
-        if (!mbar_wait(&bars->in_empty[s], ph ^ 1, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_EMPTY); break; }
-        uint8_t* st = smem + s * STAGE;
-        uint64_t* bar = &bars->in_full[s];
-        mbar_expect_tx(bar, STAGE + 2 * CH * 4);
+// Two fp32 values as three bf16 pairs, the largest first: 24 bits of mantissa together.
+__device__ __forceinline__ void split3(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  hi = pack2(a, b);
+  const float ra = a - lo_f(hi), rb = b - hi_f(hi);
+  mid = pack2(ra, rb);
+  lo = pack2(ra - lo_f(mid), rb - hi_f(mid));
+}
+
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
+  return v;
+}
+
+// One warp: the running sums of dt A over a chunk, lane l the tokens 2l and 2l + 1.
+__device__ __forceinline__ void running(float dt0, float dt1, float A, float& g0, float& g1) {
+  const int lane = threadIdx.x & 31;
+  const float v0 = dt0 * A, v1 = dt1 * A;
+  float incl = v0 + v1;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const float up = __shfl_up_sync(FULL, incl, o);
+    if (lane >= o) incl += up;
+  }
+  float before = __shfl_up_sync(FULL, incl, 1);
+  if (lane == 0) before = 0.f;
+  g0 = before + v0;
+  g1 = before + (v0 + v1);
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// The walk over the chunks.  Four warps, 16 rows of the state each (S is kept [P, N]); NT column tiles of 8 a CTA.  A call with few (batch, head) pairs is cut
+// along the columns as well, which are independent of each other: one CTA's step is a chain (scale, split, products, decay), so the narrower it is the better
+// while there are SMs for it.
+template <int NT, int TERMS, bool REV, typename Out>
+__global__ void __launch_bounds__(128)
+ssd_states(Call k, const float* __restrict__ initial, Out* __restrict__ states, float* __restrict__ last) {
+  constexpr int CV = NT;                               // 16-byte pieces of a row of B (C)
+  constexpr int U_BYTES = L * P * 2, V_BYTES = L * CV * 16;
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ __align__(16) float weight[2][L], total[2];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & 3, r = lane >> 2;
+  const int b = blockIdx.x / k.H, h = blockIdx.x % k.H, grp = h / (k.H / k.G), col0 = blockIdx.y * NT * 8;
+  const float A = k.A[h];
+  const long long cell = static_cast<long long>(P) * N, at = (warp * 16 + r) * N + col0 + 2 * q;      // this thread's first value of a state
+  const __nv_bfloat16* u = REV ? k.dy + static_cast<long long>(b) * k.T * k.H * P + h * P : k.x + b * k.xb + h * P;
+  const __nv_bfloat16* v = (REV ? k.Cm + b * k.cb : k.Bm + b * k.bb) + grp * N + col0;
+  const long long us = REV ? static_cast<long long>(k.H) * P : k.xt, vs = REV ? k.ct : k.bt;
+  const float* dt = k.dt + static_cast<long long>(b) * k.T * k.H + h;
+
+  float S[NT][4];
+  const float* from = initial == nullptr ? nullptr : initial + blockIdx.x * cell + at;
+#pragma unroll
+  for (int n = 0; n < NT; ++n) {
+    const float2 a = from == nullptr ? make_float2(0.f, 0.f) : *reinterpret_cast<const float2*>(from + n * 8);
+    const float2 c = from == nullptr ? make_float2(0.f, 0.f) : *reinterpret_cast<const float2*>(from + n * 8 + 8 * N);
+    S[n][0] = a.x; S[n][1] = a.y; S[n][2] = c.x; S[n][3] = c.y;
+  }
+  auto chunk = [&](int it) { return REV ? k.chunks - 1 - it : it; };
+  auto fetch = [&](int it) {
+    const int t0 = chunk(it) * L, real = min(L, k.T - t0);
+    uint8_t* st = smem + (it & 1) * (U_BYTES + V_BYTES);
+    load_tile<8, 128>(st, u + t0 * us, us, real);
+    load_tile<CV, 128>(st + U_BYTES, v + t0 * vs, vs, real);
+    cp_commit();
+  };
+  float dt0 = 0.f, dt1 = 0.f;
+  auto fetch_dt = [&](int it) {                        // warp 0
+    const int t = chunk(it) * L + 2 * lane;
+    dt0 = t < k.T ? dt[static_cast<long long>(t) * k.H] : 0.f;
+    dt1 = t + 1 < k.T ? dt[static_cast<long long>(t + 1) * k.H] : 0.f;
+  };
+  auto weigh = [&](int it) {                           // warp 0: e^{g_i}, or dt_j e^{g_L - g_j}
+    float g0, g1;
+    running(dt0, dt1, A, g0, g1);
+    const float gl = __shfl_sync(FULL, g1, 31);
+    weight[it & 1][2 * lane] = REV ? expf(g0) : dt0 * expf(gl - g0);
+    weight[it & 1][2 * lane + 1] = REV ? expf(g1) : dt1 * expf(gl - g1);
+    if (lane == 0) total[it & 1] = expf(gl);
+  };
+  fetch(0);
+  if (warp == 0) { fetch_dt(0); weigh(0); }
+  for (int it = 0; it < k.chunks; ++it) {
+    if (it + 1 < k.chunks) { fetch(it + 1); if (warp == 0) fetch_dt(it + 1); cp_wait<1>(); }
+    else cp_wait<0>();
+    __syncthreads();
+    Out* to = states + (static_cast<long long>(blockIdx.x) * k.chunks + chunk(it)) * cell + at;
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      if constexpr (sizeof(Out) == 4) {
+        *reinterpret_cast<float2*>(to + n * 8) = make_float2(S[n][0], S[n][1]);
+        *reinterpret_cast<float2*>(to + n * 8 + 8 * N) = make_float2(S[n][2], S[n][3]);
+      } else {
+        *reinterpret_cast<uint32_t*>(to + n * 8) = pack2(S[n][0], S[n][1]);
+        *reinterpret_cast<uint32_t*>(to + n * 8 + 8 * N) = pack2(S[n][2], S[n][3]);
+      }
+    }
+    const uint8_t* st = smem + (it & 1) * (U_BYTES + V_BYTES);
+    uint32_t a[TERMS][4][4];
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) {
+      uint32_t w[4];
+      frag_a_t<8>(w, st, ks, warp * 2);
+      const float2 s0 = *reinterpret_cast<const float2*>(&weight[it & 1][ks * 16 + 2 * q]), s1 = *reinterpret_cast<const float2*>(&weight[it & 1][ks * 16 + 8 + 2 * q]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 s = i < 2 ? s0 : s1;
+        if constexpr (TERMS == 3) split3(lo_f(w[i]) * s.x, hi_f(w[i]) * s.y, a[0][ks][i], a[1][ks][i], a[2][ks][i]);
+        else a[0][ks][i] = pack2(lo_f(w[i]) * s.x, hi_f(w[i]) * s.y);
+      }
+    }
+    const float decay = total[it & 1];
+#pragma unroll
+    for (int n = 0; n < NT; n += 2) {
+      uint32_t vb[4][4];
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) frag_b_t<CV>(vb[ks], st + U_BYTES, ks, n);
+      // a chunk's share is summed by itself and joins the state in one rounded step
+      float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int t = TERMS - 1; t >= 0; --t)
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) { mma(c0, a[t][ks], vb[ks][0], vb[ks][1]); mma(c1, a[t][ks], vb[ks][2], vb[ks][3]); }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) { S[n][i] = fmaf(S[n][i], decay, c0[i]); S[n + 1][i] = fmaf(S[n + 1][i], decay, c1[i]); }
+    }
+    if (warp == 0 && it + 1 < k.chunks) weigh(it + 1);
+    __syncthreads();
+  }
+  if (last != nullptr) {
+    float* to = last + blockIdx.x * cell + at;
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      *reinterpret_cast<float2*>(to + n * 8) = make_float2(S[n][0], S[n][1]);
+      *reinterpret_cast<float2*>(to + n * 8 + 8 * N) = make_float2(S[n][2], S[n][3]);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// y of one chunk, one group, `per` of its heads: four warps, 16 tokens each.
+constexpr int OUT_STAGE = L * P * 2 + P * N * 2;
+constexpr int OUT_SMEM = 2 * L * N * 2 + 2 * OUT_STAGE + L * P * 2;
+
+__global__ void __launch_bounds__(128)
+ssd_output(Call k, const __nv_bfloat16* __restrict__ states, __nv_bfloat16* __restrict__ y, int per) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ __align__(16) float sg[2][L], sdt[2][L];
+  uint8_t *tC = smem, *tB = tC + L * N * 2, *stages = tB + L * N * 2, *tY = stages + 2 * OUT_STAGE;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & 3, r = lane >> 2;
+  const int b = blockIdx.x / k.chunks, n = blockIdx.x % k.chunks, grp = blockIdx.y, h0 = grp * (k.H / k.G) + blockIdx.z * per;
+  const int t0 = n * L, real = min(L, k.T - t0), row = warp * 16;
+  auto fetch = [&](int i) {
+    uint8_t* st = stages + (i & 1) * OUT_STAGE;
+    load_tile<8, 128>(st, k.x + b * k.xb + t0 * k.xt + (h0 + i) * P, k.xt, real);
+    load_tile<16, 128>(st + L * P * 2, states + ((static_cast<long long>(b) * k.H + h0 + i) * k.chunks + n) * P * N, N, P);
+    cp_commit();
+  };
+  auto decays = [&](int i) {                           // warp 0
+    const int t = t0 + 2 * lane;
+    const float* dt = k.dt + static_cast<long long>(b) * k.T * k.H + h0 + i;
+    const float a = t < k.T ? dt[static_cast<long long>(t) * k.H] : 0.f, c = t + 1 < k.T ? dt[static_cast<long long>(t + 1) * k.H] : 0.f;
+    float g0, g1;
+    running(a, c, k.A[h0 + i], g0, g1);
+    *reinterpret_cast<float2*>(&sg[i & 1][2 * lane]) = make_float2(g0, g1);
+    *reinterpret_cast<float2*>(&sdt[i & 1][2 * lane]) = make_float2(a, c);
+  };
+  load_tile<16, 128>(tC, k.Cm + b * k.cb + t0 * k.ct + grp * N, k.ct, real);
+  load_tile<16, 128>(tB, k.Bm + b * k.bb + t0 * k.bt + grp * N, k.bt, real);
+  cp_commit();
+  fetch(0);
+  if (warp == 0) decays(0);
+  cp_wait<1>();
+  __syncthreads();
+  float G[8][4];                                       // C B^T of this warp's tokens; column tiles behind them stay unused
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) G[j][i] = 0.f;
+#pragma unroll
+  for (int ks = 0; ks < 8; ++ks) {
+    uint32_t a[4];
+    frag_a<16>(a, tC, row, ks);
+#pragma unroll
+    for (int j = 0; j < 8; j += 2)
+      if (j <= 2 * warp) {
+        uint32_t bb[4];
+        frag_b<16>(bb, tB, j * 8, ks);
+        mma(G[j], a, bb[0], bb[1]);
+        mma(G[j + 1], a, bb[2], bb[3]);
+      }
+  }
+  for (int i = 0; i < per; ++i) {
+    if (i + 1 < per) { fetch(i + 1); if (warp == 0) decays(i + 1); cp_wait<1>(); }
+    else cp_wait<0>();
+    __syncthreads();
+    const uint8_t *tx = stages + (i & 1) * OUT_STAGE, *tS = tx + L * P * 2;
+    const float *g = sg[i & 1], *dt = sdt[i & 1];
+    const float gi0 = g[row + r], gi1 = g[row + r + 8];
+    float acc[8][4];
+#pragma unroll
+    for (int p = 0; p < 8; ++p)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[p][c] = 0.f;
+#pragma unroll
+    for (int ks = 0; ks < 8; ++ks) {
+      uint32_t a[4];
+      frag_a<16>(a, tC, row, ks);
+#pragma unroll
+      for (int p = 0; p < 8; p += 2) {
+        uint32_t bb[4];
+        frag_b<16>(bb, tS, p * 8, ks);
+        mma(acc[p], a, bb[0], bb[1]);
+        mma(acc[p + 1], a, bb[2], bb[3]);
+      }
+    }
+    const float e0 = expf(gi0), e1 = expf(gi1);
+#pragma unroll
+    for (int p = 0; p < 8; ++p) { acc[p][0] *= e0; acc[p][1] *= e0; acc[p][2] *= e1; acc[p][3] *= e1; }
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks)
+      if (ks <= warp) {
+        uint32_t a[4];
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
-          tma_load_4d(st + F_X + t * (CH * 128), &tx, bar, t * 64, hp, n * CH, b);
-          tma_load_4d(st + F_C + t * (CH * 128), &tc, bar, t * 64, grp, n * CH, b);
-          tma_load_4d(st + F_B + t * (CH * 128), &tb, bar, t * 64, grp, n * CH, b);
+          const int j = ks * 16 + t * 8 + 2 * q;
+          const float2 gj = *reinterpret_cast<const float2*>(g + j), d = *reinterpret_cast<const float2*>(dt + j);
+          const float* w = G[ks * 2 + t];
+          const int i0 = row + r, i1 = i0 + 8;
+          a[2 * t] = pack2(j <= i0 ? w[0] * expf(gi0 - gj.x) * d.x : 0.f, j + 1 <= i0 ? w[1] * expf(gi0 - gj.y) * d.y : 0.f);
+          a[2 * t + 1] = pack2(j <= i1 ? w[2] * expf(gi1 - gj.x) * d.x : 0.f, j + 1 <= i1 ? w[3] * expf(gi1 - gj.y) * d.y : 0.f);
         }
-        const long long r0 = (static_cast<long long>(b) * H + h0) * Tp + n * CH;
-        tma_load_2d(st + F_P0, &tp, bar, 0, static_cast<int>(r0));
-        tma_load_2d(st + F_P1, &tp, bar, 0, static_cast<int>(r0 + Tp));
-        bulk_load_1d(sG + (s * 2 + 0) * CH, gc + r0, CH * 4, bar);
-        bulk_load_1d(sG + (s * 2 + 1) * CH, gc + r0 + Tp, CH * 4, bar);
-      }
-    }
-  } else if (warp == MMA_WARP) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_n64 = make_idesc(128, 64, 1, 1, 0, 0);
-      constexpr uint32_t idesc_ds = make_idesc(128, 128, 1, 1, 0, 1);
-      const uint32_t sa = smem_u32(sState), v0a = smem_u32(sVn0), v1a = smem_u32(sVn1), vda = smem_u32(sVd);
-      for (int n = 0; n < N; ++n) {
-        const int s = n & 1; const uint32_t ph = (n >> 1) & 1;
-        const uint32_t st = smem_u32(smem + s * STAGE);
-        if (!mbar_wait(&bars->in_full[s], ph, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_FULL); break; }
-        if (!mbar_wait(&bars->s_ready, n & 1, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_OTHER); break; }
-        tc_fence_after();
 #pragma unroll
-        for (int kk = 0; kk < ND / 16; ++kk) {
-          const uint32_t aoff = (kk >> 2) * (128 * 128) + (kk & 3) * 32, boff = (kk >> 2) * (CH * 128) + (kk & 3) * 32;
-          umma_bf16_ss(tmem + TM_O1, make_sdesc_sw128(sa + aoff, 16, 1024), make_sdesc_sw128(st + F_C + boff, 16, 1024),
-                       idesc_n64, kk > 0 ? 1u : 0u);
-        }
-        if (!mbar_wait(&bars->vn_ready, n & 1, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_OTHER); break; }
-        tc_fence_after();
-#pragma unroll
-        for (int kk = 0; kk < CH / 16; ++kk)
-          umma_bf16_ss(tmem + TM_O2, make_sdesc_sw128(v0a + kk * 32, 16, 1024), make_sdesc_sw128(st + F_P0 + kk * 32, 16, 1024),
-                       idesc_n64, kk > 0 ? 1u : 0u);
-#pragma unroll
-        for (int kk = 0; kk < CH / 16; ++kk)
-          umma_bf16_ss(tmem + TM_O2, make_sdesc_sw128(v1a + kk * 32, 16, 1024), make_sdesc_sw128(st + F_P1 + kk * 32, 16, 1024),
-                       idesc_n64, 1u);
-#pragma unroll
-        for (int kk = 0; kk < CH / 16; ++kk)
-          umma_bf16_ss(tmem + TM_DS, make_sdesc_sw128(vda + kk * 32, 16, 1024),
-                       make_sdesc_sw128(st + F_B + kk * 2048, CH * 128, 1024), idesc_ds, kk > 0 ? 1u : 0u);
-        umma_commit(&bars->out_full);
-      }
-    }
-  } else {
-    const int v = tid;                                   // rows 0..63: head h0, rows 64..127: head h0 + 1
-    const int hh = v >> 6;
-    const uint32_t lane_addr = static_cast<uint32_t>(warp * 32) << 16;
-    float S[ND];
-    if (initial != nullptr) {
-      // initial / final state: [B, H, P, N] fp32; this thread's row is (head h0 + hh, p = v & 63)
-      const float* src = initial + ((static_cast<long long>(b) * H + h0 + hh) * PD + (v & 63)) * ND;
-#pragma unroll
-      for (int d = 0; d < ND; d += 4) {
-        const float4 q4 = *reinterpret_cast<const float4*>(src + d);
-        S[d] = q4.x; S[d + 1] = q4.y; S[d + 2] = q4.z; S[d + 3] = q4.w;
-      }
-    } else {
-#pragma unroll
-      for (int d = 0; d < ND; ++d) S[d] = 0.f;
-    }
-    write_state_row(sState, v, S);
-    fence_proxy_async();
-    tc_fence_before();
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&bars->s_ready);
-    uint8_t* my_vn = hh ? sVn1 : sVn0;
-    bool ok = true;
-    for (int n = 0; n < N && ok; ++n) {
-      const int s = n & 1; const uint32_t ph = (n >> 1) & 1;
-      const uint8_t* st = smem + s * STAGE;
-      const float* gs = sG + (s * 2 + hh) * CH;
-      {
-        const bool got = mbar_wait(&bars->in_full[s], ph, abort_flag);
-        if (!__all_sync(FULL, got)) { if (lane == 0) atomicCAS(err, 0, ERR_WAIT_FULL); ok = false; break; }
-      }
-      const float gl = gs[CH - 1];
-      const uint8_t* xcol = st + F_X + (v >> 6) * (CH * 128) + (v & 7) * 2;
-      const int xc16 = (v & 63) >> 3;
-#pragma unroll
-      for (int j8 = 0; j8 < 8; ++j8) {
-        float vn[8], vd[8];
-#pragma unroll
-        for (int jj = 0; jj < 8; ++jj) {
-          const int j = j8 * 8 + jj;
-          vn[jj] = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(xcol + swz(j, xc16)));
-          vd[jj] = vn[jj] * __expf(gl - gs[j]);
-        }
-        uint4 p0, p1;
-        p0.x = pack_bf16(vn[0], vn[1]); p0.y = pack_bf16(vn[2], vn[3]); p0.z = pack_bf16(vn[4], vn[5]); p0.w = pack_bf16(vn[6], vn[7]);
-        p1.x = pack_bf16(vd[0], vd[1]); p1.y = pack_bf16(vd[2], vd[3]); p1.z = pack_bf16(vd[4], vd[5]); p1.w = pack_bf16(vd[6], vd[7]);
-        *reinterpret_cast<uint4*>(my_vn + swz(v, j8)) = p0;
-        *reinterpret_cast<uint4*>(sVd + swz(v, j8)) = p1;
-      }
-      fence_proxy_async();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->vn_ready);
-      {
-        const bool got = mbar_wait(&bars->out_full, n & 1, abort_flag);
-        if (!__all_sync(FULL, got)) { if (lane == 0) atomicCAS(err, 0, ERR_WAIT_TMEM_FULL); ok = false; break; }
-      }
-      tc_fence_after();
-      // y^T row: out is [B, T, H, P] = [B, T, H / 2, 128] with this thread's column v of pair hp
-      __nv_bfloat16* orow = out + ((static_cast<long long>(b) * T + n * CH) * Hp + hp) * 128 + v;
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint32_t o1[32], o2[32];
-        tmem_ld_32x32b_x32(tmem + lane_addr + TM_O1 + half * 32, o1);
-        tmem_ld_32x32b_x32(tmem + lane_addr + TM_O2 + half * 32, o2);
-        tmem_ld_wait();
-#pragma unroll
-        for (int ii = 0; ii < 32; ++ii) {
-          const int i = half * 32 + ii;
-          const float o = __expf(gs[i]) * __uint_as_float(o1[ii]) + __uint_as_float(o2[ii]);
-          if (n * CH + i < T) orow[static_cast<long long>(i) * Hp * 128] = __float2bfloat16(o);
+        for (int p = 0; p < 8; p += 2) {
+          uint32_t bb[4];
+          frag_b_t<8>(bb, tx, ks, p);
+          mma(acc[p], a, bb[0], bb[1]);
+          mma(acc[p + 1], a, bb[2], bb[3]);
         }
       }
-      const float dl = __expf(gl);
+    const float D = k.D == nullptr ? 0.f : k.D[h0 + i];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        uint32_t d[32];
-        tmem_ld_32x32b_x32(tmem + lane_addr + TM_DS + q * 32, d);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) S[q * 32 + i] = fmaf(S[q * 32 + i], dl, __uint_as_float(d[i]));
-      }
-      write_state_row(sState, v, S);
-      fence_proxy_async();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) { mbar_arrive(&bars->s_ready); mbar_arrive(&bars->in_empty[s]); }
+    for (int p = 0; p < 8; ++p) {
+      const uint32_t x0 = *reinterpret_cast<const uint32_t*>(tx + piece<8>(row + r, p) + q * 4), x1 = *reinterpret_cast<const uint32_t*>(tx + piece<8>(row + r + 8, p) + q * 4);
+      *reinterpret_cast<uint32_t*>(tY + piece<8>(row + r, p) + q * 4) = pack2(fmaf(D, lo_f(x0), acc[p][0]), fmaf(D, hi_f(x0), acc[p][1]));
+      *reinterpret_cast<uint32_t*>(tY + piece<8>(row + r + 8, p) + q * 4) = pack2(fmaf(D, lo_f(x1), acc[p][2]), fmaf(D, hi_f(x1), acc[p][3]));
     }
-    if (ok && final_state != nullptr) {
-      float* dst = final_state + ((static_cast<long long>(b) * H + h0 + hh) * PD + (v & 63)) * ND;
+    __syncwarp();                                      // (a warp stores the rows it made)
 #pragma unroll
-      for (int d = 0; d < ND; d += 4) *reinterpret_cast<float4*>(dst + d) = make_float4(S[d], S[d + 1], S[d + 2], S[d + 3]);
+    for (int s = 0; s < 4; ++s) {
+      const int at = row + s * 4 + (lane >> 3), c = lane & 7;
+      if (at < real)
+        *reinterpret_cast<uint4*>(y + ((static_cast<long long>(b) * k.T + t0 + at) * k.H + h0 + i) * P + c * 8) = *reinterpret_cast<const uint4*>(tY + piece<8>(at, c));
     }
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == MMA_WARP) {
-    __syncwarp();
-    tc_fence_after();
-    tmem_dealloc(tmem, 256);
+    __syncthreads();                                   // the stage is free for the head after the next
   }
 }
 
-static int make_map4(CUtensorMap* m, const void* base, int B, int T, int H, int D, int box_rows) {
-  const uint64_t dims[4] = {static_cast<uint64_t>(D), static_cast<uint64_t>(H), static_cast<uint64_t>(T), static_cast<uint64_t>(B)};
-  const uint64_t strides[3] = {static_cast<uint64_t>(D) * 2, static_cast<uint64_t>(H) * D * 2, static_cast<uint64_t>(T) * H * D * 2};
-  const uint32_t box[4] = {64, 1, static_cast<uint32_t>(box_rows), 1};
-  return make_tmap_nd(m, base, 4, dims, strides, box, 2, true);
+// ---------------------------------------------------------------------------------------------------------------
+// Gradients of one chunk, one group, `per` of its heads: eight warps.  The products over the state's columns give each warp 16 of the 128 columns and all 64
+// tokens, so that every fp32 value of a state is split into its bf16 terms by the one warp that needs it; E and M are made by 16 x 32 pieces.
+constexpr int SLD = N + 4;                             // row of an fp32 state in shared memory: the fragment reads of both orders spread over the banks
+constexpr int LOCAL_STAGE = 2 * L * P * 2 + 2 * P * SLD * 4;
+constexpr int M_BYTES = 10 * 3 * 512;                  // the ten 16 x 16 blocks of M^T with i >= j, three terms each, as A fragments
+struct LocalSums {
+  float rows[4][L];                                    // sum over j < i of M o E dt_j, by the 16 tokens j of a pair of warps
+  float cols[2][L], diag[L], edge[L];                  // sum over i > j of M o E by halves of i; its diagonal; the diagonal of E
+  float dy_state[8][L], x_state[8][L];                 // (dy S) . C and (x dS) . B, by the warps' columns
+  float both[8];                                       // <S, dS>
+  float g[2][L], dt[2][L];
+};
+constexpr int LOCAL_SMEM = 2 * L * N * 2 + 2 * LOCAL_STAGE + M_BYTES + static_cast<int>(sizeof(LocalSums));
+static_assert(LOCAL_SMEM <= 232448, "ssd_local exceeds the shared memory of an SM");
+
+struct Grads {
+  __nv_bfloat16 *dx, *dB, *dC;
+  float *ddt, *partB, *partC, *partA, *partD;          // partB / partC: [splits][B, T, G, N] when a group's heads are split, else null; partA / partD: [B * chunks, H]
+};
+
+// which of the ten blocks of the lower triangle (j tile, i tile >= j tile)
+__device__ __forceinline__ int block_of(int jt, int it) { return jt * 4 - jt * (jt - 1) / 2 + it - jt; }
+
+__global__ void __launch_bounds__(256, 1)
+ssd_local(Call k, const float* __restrict__ states, const float* __restrict__ dstates, Grads out, int per) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  uint8_t *tB = smem, *tC = tB + L * N * 2, *stages = tC + L * N * 2, *tM = stages + 2 * LOCAL_STAGE;
+  LocalSums& sum = *reinterpret_cast<LocalSums*>(tM + M_BYTES);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & 3, r = lane >> 2;
+  const int b = blockIdx.x / k.chunks, n = blockIdx.x % k.chunks, grp = blockIdx.y, h0 = grp * (k.H / k.G) + blockIdx.z * per;
+  const int t0 = n * L, real = min(L, k.T - t0);
+  const int jt = warp >> 1, ih = warp & 1;             // this warp's piece of E^T: tokens j of tile jt, tokens i of half ih
+  const bool lower = ih * 32 + 31 >= jt * 16;          // whether some i >= j is in it
+  const int nc = warp * 16;                            // this warp's columns of the state
+  auto fetch = [&](int i) {
+    uint8_t* st = stages + (i & 1) * LOCAL_STAGE;
+    const int h = h0 + i;
+    load_tile<8, 256>(st, k.x + b * k.xb + t0 * k.xt + h * P, k.xt, real);
+    load_tile<8, 256>(st + L * P * 2, k.dy + ((static_cast<long long>(b) * k.T + t0) * k.H + h) * P, static_cast<long long>(k.H) * P, real);
+    const long long cell = ((static_cast<long long>(b) * k.H + h) * k.chunks + n) * P * N;
+    float* fs = reinterpret_cast<float*>(st + 2 * L * P * 2);
+#pragma unroll
+    for (int s = 0; s < P * N / 4 / 256; ++s) {
+      const int at = s * 256 + static_cast<int>(threadIdx.x), row = at >> 5, c = at & 31;
+      cp16(fs + row * SLD + c * 4, states + cell + row * N + c * 4, true);
+      cp16(fs + (P + row) * SLD + c * 4, dstates + cell + row * N + c * 4, true);
+    }
+    cp_commit();
+  };
+  auto decays = [&](int i) {                           // warp 7
+    const int t = t0 + 2 * lane;
+    const float* dt = k.dt + static_cast<long long>(b) * k.T * k.H + h0 + i;
+    const float a = t < k.T ? dt[static_cast<long long>(t) * k.H] : 0.f, c = t + 1 < k.T ? dt[static_cast<long long>(t + 1) * k.H] : 0.f;
+    float g0, g1;
+    running(a, c, k.A[h0 + i], g0, g1);
+    *reinterpret_cast<float2*>(&sum.g[i & 1][2 * lane]) = make_float2(g0, g1);
+    *reinterpret_cast<float2*>(&sum.dt[i & 1][2 * lane]) = make_float2(a, c);
+  };
+  load_tile<16, 256>(tC, k.Cm + b * k.cb + t0 * k.ct + grp * N, k.ct, real);
+  load_tile<16, 256>(tB, k.Bm + b * k.bb + t0 * k.bt + grp * N, k.bt, real);
+  cp_commit();
+  fetch(0);
+  if (warp == 7) decays(0);
+  for (int i = threadIdx.x; i < 6 * L; i += 256) (i < 4 * L ? &sum.rows[0][0] : &sum.cols[0][0] - 4 * L)[i] = 0.f;      // pieces above the diagonal write none
+  cp_wait<1>();
+  __syncthreads();
+
+  float G[4][4], W[4][4], dC[4][2][4], dB[4][2][4];
+#pragma unroll
+  for (int t = 0; t < 4; ++t)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      G[t][c] = W[t][c] = 0.f;
+      dC[t][0][c] = dC[t][1][c] = dB[t][0][c] = dB[t][1][c] = 0.f;
+    }
+  if (lower) {
+#pragma unroll
+    for (int ks = 0; ks < 8; ++ks) {
+      uint32_t a[4], b0[4], b1[4];
+      frag_a<16>(a, tB, jt * 16, ks);
+      frag_b<16>(b0, tC, ih * 32, ks);
+      frag_b<16>(b1, tC, ih * 32 + 16, ks);
+      mma(G[0], a, b0[0], b0[1]); mma(G[1], a, b0[2], b0[3]);
+      mma(G[2], a, b1[0], b1[1]); mma(G[3], a, b1[2], b1[3]);
+    }
+  }
+
+  for (int i = 0; i < per; ++i) {
+    cp_wait<0>();
+    __syncthreads();                                   // this head has arrived, and nobody reads the one before it any more
+    if (i + 1 < per) { fetch(i + 1); if (warp == 7) decays(i + 1); }
+    const int h = h0 + i;
+    const uint8_t *tx = stages + (i & 1) * LOCAL_STAGE, *ty = tx + L * P * 2;
+    const float *S = reinterpret_cast<const float*>(ty + L * P * 2), *dS = S + P * SLD;
+    const float *g = sum.g[i & 1], *dt = sum.dt[i & 1];
+    const float gl = g[L - 1];
+
+    if (lower) {
+      // ---- E^T = x dy^T of this piece, then M^T, W^T and the sums of M o E
+      float E[4][4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) E[t][c] = 0.f;
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) {
+        uint32_t a[4], b0[4], b1[4];
+        frag_a<8>(a, tx, jt * 16, ks);
+        frag_b<8>(b0, ty, ih * 32, ks);
+        frag_b<8>(b1, ty, ih * 32 + 16, ks);
+        mma(E[0], a, b0[0], b0[1]); mma(E[1], a, b0[2], b0[3]);
+        mma(E[2], a, b1[0], b1[1]); mma(E[3], a, b1[2], b1[3]);
+      }
+      const int j0 = jt * 16 + r, j1 = j0 + 8;
+      const float gj0 = g[j0], gj1 = g[j1], d0 = dt[j0], d1 = dt[j1];
+      float col0 = 0.f, col1 = 0.f;
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const int i0 = ih * 32 + t * 8 + 2 * q;
+        const float2 gi = *reinterpret_cast<const float2*>(g + i0);
+        float m[4], row0 = 0.f, row1 = 0.f;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int ii = i0 + (c & 1), jj = c < 2 ? j0 : j1;
+          const float dec = ii >= jj ? expf((c & 1 ? gi.y : gi.x) - (c < 2 ? gj0 : gj1)) : 0.f, d = c < 2 ? d0 : d1;
+          m[c] = ii >= jj ? G[t][c] * dec : 0.f;
+          const float me = ii >= jj ? m[c] * E[t][c] : 0.f;
+          W[t][c] += ii >= jj ? E[t][c] * dec * d : 0.f;
+          if (ii == jj) { sum.diag[jj] = me; sum.edge[jj] = E[t][c]; }
+          else {
+            if (c < 2) col0 += me; else col1 += me;
+            if (c & 1) row1 += me * d; else row0 += me * d;
+          }
+        }
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) { row0 += __shfl_xor_sync(FULL, row0, o); row1 += __shfl_xor_sync(FULL, row1, o); }
+        if (r == 0) *reinterpret_cast<float2*>(&sum.rows[jt][i0]) = make_float2(row0, row1);
+        // a pair of column tiles is one A fragment of M^T
+        const int it = ih * 2 + (t >> 1);
+        if (it >= jt) {
+          uint32_t hi[2], mid[2], lo[2];
+          split3(m[0], m[1], hi[0], mid[0], lo[0]);
+          split3(m[2], m[3], hi[1], mid[1], lo[1]);
+          uint8_t* to = tM + block_of(jt, it) * 1536 + lane * 16 + (t & 1) * 8;
+          *reinterpret_cast<uint2*>(to) = make_uint2(hi[0], hi[1]);
+          *reinterpret_cast<uint2*>(to + 512) = make_uint2(mid[0], mid[1]);
+          *reinterpret_cast<uint2*>(to + 1024) = make_uint2(lo[0], lo[1]);
+        }
+      }
+      col0 += __shfl_xor_sync(FULL, col0, 1); col0 += __shfl_xor_sync(FULL, col0, 2);
+      col1 += __shfl_xor_sync(FULL, col1, 1); col1 += __shfl_xor_sync(FULL, col1, 2);
+      if (q == 0) { sum.cols[ih][j0] = col0; sum.cols[ih][j1] = col1; }
+    }
+
+    // ---- (dy S) and (x dS): this warp's 16 columns of all tokens
+    float both = 0.f;
+#pragma unroll
+    for (int which = 0; which < 2; ++which) {
+      const float* F = which ? dS : S;
+      uint32_t f[3][4][2][2];
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          const float* at = F + (ks * 16 + 2 * q) * SLD + nc + t * 8 + r;
+          const float v0 = at[0], v1 = at[SLD], v2 = at[8 * SLD], v3 = at[9 * SLD];
+          if (which) {
+            const float* o = S + (ks * 16 + 2 * q) * SLD + nc + t * 8 + r;
+            both += v0 * o[0] + v1 * o[SLD] + v2 * o[8 * SLD] + v3 * o[9 * SLD];
+          }
+          split3(v0, v1, f[0][ks][t][0], f[1][ks][t][0], f[2][ks][t][0]);
+          split3(v2, v3, f[0][ks][t][1], f[1][ks][t][1], f[2][ks][t][1]);
+        }
+      const uint8_t *tu = which ? tx : ty, *tw = which ? tB : tC;
+#pragma unroll
+      for (int mt = 0; mt < 4; ++mt) {
+        uint32_t a[4][4];
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) frag_a<8>(a[ks], tu, mt * 16, ks);
+        float u[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+        for (int term = 2; term >= 0; --term)
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks) {
+            mma(u[0], a[ks], f[term][ks][0][0], f[term][ks][0][1]);
+            mma(u[1], a[ks], f[term][ks][1][0], f[term][ks][1][1]);
+          }
+        const int i0 = mt * 16 + r, i1 = i0 + 8;
+        const float s0 = which ? dt[i0] * expf(gl - g[i0]) : expf(g[i0]), s1 = which ? dt[i1] * expf(gl - g[i1]) : expf(g[i1]);
+        float dot0 = 0.f, dot1 = 0.f;
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          const uint32_t w0 = *reinterpret_cast<const uint32_t*>(tw + piece<16>(i0, warp * 2 + t) + q * 4), w1 = *reinterpret_cast<const uint32_t*>(tw + piece<16>(i1, warp * 2 + t) + q * 4);
+          dot0 += u[t][0] * lo_f(w0) + u[t][1] * hi_f(w0);
+          dot1 += u[t][2] * lo_f(w1) + u[t][3] * hi_f(w1);
+          float(&to)[4] = which ? dB[mt][t] : dC[mt][t];
+          to[0] = fmaf(s0, u[t][0], to[0]); to[1] = fmaf(s0, u[t][1], to[1]);
+          to[2] = fmaf(s1, u[t][2], to[2]); to[3] = fmaf(s1, u[t][3], to[3]);
+        }
+        dot0 += __shfl_xor_sync(FULL, dot0, 1); dot0 += __shfl_xor_sync(FULL, dot0, 2);
+        dot1 += __shfl_xor_sync(FULL, dot1, 1); dot1 += __shfl_xor_sync(FULL, dot1, 2);
+        if (q == 0) {
+          float* to = which ? sum.x_state[warp] : sum.dy_state[warp];
+          to[i0] = dot0; to[i1] = dot1;
+        }
+      }
+    }
+    both = warp_sum(both);
+    if (lane == 0) sum.both[warp] = both;
+
+    // ---- dx: this warp's 8 of the head's 64 columns.  First through the state: B dS^T
+    float X[4][4];
+#pragma unroll
+    for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) X[mt][c] = 0.f;
+#pragma unroll
+    for (int ks = 0; ks < 8; ++ks) {
+      const float* at = dS + (warp * 8 + r) * SLD + ks * 16 + 2 * q;
+      const float2 v0 = *reinterpret_cast<const float2*>(at), v1 = *reinterpret_cast<const float2*>(at + 8);
+      uint32_t f[3][2];
+      split3(v0.x, v0.y, f[0][0], f[1][0], f[2][0]);
+      split3(v1.x, v1.y, f[0][1], f[1][1], f[2][1]);
+#pragma unroll
+      for (int mt = 0; mt < 4; ++mt) {
+        uint32_t a[4];
+        frag_a<16>(a, tB, mt * 16, ks);
+        mma(X[mt], a, f[2][0], f[2][1]);
+        mma(X[mt], a, f[1][0], f[1][1]);
+        mma(X[mt], a, f[0][0], f[0][1]);
+      }
+    }
+#pragma unroll
+    for (int mt = 0; mt < 4; ++mt) {
+      const float s0 = expf(gl - g[mt * 16 + r]), s1 = expf(gl - g[mt * 16 + r + 8]);
+      X[mt][0] *= s0; X[mt][1] *= s0; X[mt][2] *= s1; X[mt][3] *= s1;
+    }
+    __syncthreads();
+    // then through the chunk's own tokens: M^T dy
+    uint32_t yb[2][4];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) ldsm4_t(yb[s], smem_addr(ty + piece<8>(s * 32 + lane, warp)));
+#pragma unroll
+    for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+      for (int it = mt; it < 4; ++it) {
+        const uint8_t* at = tM + block_of(mt, it) * 1536 + lane * 16;
+#pragma unroll
+        for (int term = 2; term >= 0; --term) {
+          // (stored by column tile: rows r and r + 8 of the first, then of the second, which is the fragment's order)
+          const uint4 w = *reinterpret_cast<const uint4*>(at + term * 512);
+          const uint32_t a[4] = {w.x, w.y, w.z, w.w};
+          mma(X[mt], a, yb[it >> 1][(it & 1) * 2], yb[it >> 1][(it & 1) * 2 + 1]);
+        }
+      }
+    const float D = k.D == nullptr ? 0.f : k.D[h];
+#pragma unroll
+    for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int j = mt * 16 + r + half * 8;
+        const uint32_t w = *reinterpret_cast<const uint32_t*>(ty + piece<8>(j, warp) + q * 4);
+        const float d = dt[j];
+        if (j < real)
+          *reinterpret_cast<uint32_t*>(out.dx + ((static_cast<long long>(b) * k.T + t0 + j) * k.H + h) * P + warp * 8 + 2 * q) =
+              pack2(fmaf(D, lo_f(w), d * X[mt][half * 2]), fmaf(D, hi_f(w), d * X[mt][half * 2 + 1]));
+      }
+    if (warp == 0) {
+      // ---- the decays: dg_i from what the token receives less what it gives, its sums to the chunk's end are the gradients of dt A
+      float dg[2], direct[2], given = 0.f, d[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int t = 2 * lane + e;
+        float take = 0.f, give = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) { take += sum.dy_state[w][t]; give += sum.x_state[w][t]; }
+        d[e] = dt[t];
+        give *= expf(gl - g[t]);
+        given += d[e] * give;
+        const float own = sum.cols[0][t] + sum.cols[1][t] + give;
+        dg[e] = ((sum.rows[0][t] + sum.rows[1][t]) + (sum.rows[2][t] + sum.rows[3][t])) + expf(g[t]) * take - d[e] * own;
+        direct[e] = own + sum.diag[t];
+      }
+      given = warp_sum(given);
+      float held = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) held += sum.both[w];
+      if (lane == 31) dg[1] += expf(gl) * held + given;
+      float suffix = dg[0] + dg[1];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float down = __shfl_down_sync(FULL, suffix, o);
+        if (lane + o < 32) suffix += down;
+      }
+      float after = __shfl_down_sync(FULL, suffix, 1);
+      if (lane == 31) after = 0.f;
+      const float da1 = after + dg[1], da0 = after + (dg[0] + dg[1]), A = k.A[h];
+      const int t = 2 * lane;
+      float* to = out.ddt + (static_cast<long long>(b) * k.T + t0) * k.H + h;
+      if (t < real) to[static_cast<long long>(t) * k.H] = fmaf(A, da0, direct[0]);
+      if (t + 1 < real) to[static_cast<long long>(t + 1) * k.H] = fmaf(A, da1, direct[1]);
+      const float sA = warp_sum(d[0] * da0 + d[1] * da1), sD = warp_sum(sum.edge[t] + sum.edge[t + 1]);
+      if (lane == 0) {
+        const long long at = static_cast<long long>(blockIdx.x) * k.H + h;
+        out.partA[at] = sA;
+        out.partD[at] = sD;
+      }
+    }
+  }
+
+  // ---- W B and W^T C, once for all heads: W^T [j][i] in fp32 through the stages' memory
+  __syncthreads();
+  float* tW = reinterpret_cast<float*>(stages);
+  constexpr int WLD = L + 4;
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    float* at = tW + (jt * 16 + r) * WLD + ih * 32 + t * 8 + 2 * q;
+    *reinterpret_cast<float2*>(at) = make_float2(W[t][0], W[t][1]);
+    *reinterpret_cast<float2*>(at + 8 * WLD) = make_float2(W[t][2], W[t][3]);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) {
+      uint32_t f[4];
+      if (ks <= mt) {                                  // dC_i += sum_j W_ij B_j
+        const float* at = tW + (ks * 16 + 2 * q) * WLD + mt * 16 + r;
+        uint32_t a[3][4];
+        split3(at[0], at[WLD], a[0][0], a[1][0], a[2][0]);
+        split3(at[8], at[WLD + 8], a[0][1], a[1][1], a[2][1]);
+        split3(at[8 * WLD], at[9 * WLD], a[0][2], a[1][2], a[2][2]);
+        split3(at[8 * WLD + 8], at[9 * WLD + 8], a[0][3], a[1][3], a[2][3]);
+        frag_b_t<16>(f, tB, ks, warp * 2);
+#pragma unroll
+        for (int term = 2; term >= 0; --term) { mma(dC[mt][0], a[term], f[0], f[1]); mma(dC[mt][1], a[term], f[2], f[3]); }
+      }
+      if (ks >= mt) {                                  // dB_j += sum_i W_ij C_i
+        const float* at = tW + (mt * 16 + r) * WLD + ks * 16 + 2 * q;
+        uint32_t a[3][4];
+        split3(at[0], at[1], a[0][0], a[1][0], a[2][0]);
+        split3(at[8 * WLD], at[8 * WLD + 1], a[0][1], a[1][1], a[2][1]);
+        split3(at[8], at[9], a[0][2], a[1][2], a[2][2]);
+        split3(at[8 * WLD + 8], at[8 * WLD + 9], a[0][3], a[1][3], a[2][3]);
+        frag_b_t<16>(f, tC, ks, warp * 2);
+#pragma unroll
+        for (int term = 2; term >= 0; --term) { mma(dB[mt][0], a[term], f[0], f[1]); mma(dB[mt][1], a[term], f[2], f[3]); }
+      }
+    }
+#pragma unroll
+  for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int t = mt * 16 + r + half * 8;
+      if (t >= real) continue;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const long long at = ((static_cast<long long>(b) * k.T + t0 + t) * k.G + grp) * N + nc + c * 8 + 2 * q;
+        const float b0 = dB[mt][c][half * 2], b1 = dB[mt][c][half * 2 + 1], c0 = dC[mt][c][half * 2], c1 = dC[mt][c][half * 2 + 1];
+        if (out.partB == nullptr) {
+          *reinterpret_cast<uint32_t*>(out.dB + at) = pack2(b0, b1);
+          *reinterpret_cast<uint32_t*>(out.dC + at) = pack2(c0, c1);
+        } else {
+          const long long part = blockIdx.z * (static_cast<long long>(k.B) * k.T * k.G * N);
+          *reinterpret_cast<float2*>(out.partB + part + at) = make_float2(b0, b1);
+          *reinterpret_cast<float2*>(out.partC + part + at) = make_float2(c0, c1);
+        }
+      }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// Blocks [0, H): dA and dD of a head over all chunks; the others: four values of dB and of dC a thread over the splits.
+__global__ void __launch_bounds__(256)
+ssd_reduce(Grads g, float* __restrict__ dA, float* __restrict__ dD, int H, int parts, long long total, int splits) {
+  if (blockIdx.x < H) {
+    __shared__ float sA[8], sD[8];
+    float a = 0.f, d = 0.f;
+    for (int i = threadIdx.x; i < parts; i += 256) { a += g.partA[static_cast<long long>(i) * H + blockIdx.x]; d += g.partD[static_cast<long long>(i) * H + blockIdx.x]; }
+    a = warp_sum(a); d = warp_sum(d);
+    if ((threadIdx.x & 31) == 0) { sA[threadIdx.x >> 5] = a; sD[threadIdx.x >> 5] = d; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      a = d = 0.f;
+      for (int w = 0; w < 8; ++w) { a += sA[w]; d += sD[w]; }
+      dA[blockIdx.x] = a;
+      if (dD != nullptr) dD[blockIdx.x] = d;
+    }
+    return;
+  }
+  const long long at = ((blockIdx.x - H) * 256ll + threadIdx.x) * 4;
+  if (at >= total) return;
+#pragma unroll
+  for (int which = 0; which < 2; ++which) {
+    const float* from = (which ? g.partC : g.partB) + at;
+    float4 s = *reinterpret_cast<const float4*>(from);
+    for (int i = 1; i < splits; ++i) {
+      const float4 v = *reinterpret_cast<const float4*>(from + i * total);
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+    *reinterpret_cast<uint2*>((which ? g.dC : g.dB) + at) = make_uint2(pack2(s.x, s.y), pack2(s.z, s.w));
+  }
+}
+
+template <int NT, int TERMS, bool REV, typename Out>
+static int run_states(const Call& k, const float* initial, Out* states, float* last, cudaStream_t stream) {
+  auto fn = ssd_states<NT, TERMS, REV, Out>;
+  constexpr int bytes = 2 * (L * P * 2 + L * NT * 16);
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  fn<<<dim3(k.B * k.H, 16 / NT), 128, bytes, stream>>>(k, initial, states, last);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// As many columns a CTA as leave every SM one: a chunk's step of a quarter of the columns is a chain not much shorter than that of all of them.
+template <int TERMS, bool REV, typename Out>
+static int walk(const Call& k, const float* initial, Out* states, float* last, cudaStream_t stream) {
+  const int rows = k.B * k.H;
+  if (rows * 2 <= SMS) return run_states<4, TERMS, REV, Out>(k, initial, states, last, stream);
+  if (rows <= SMS) return run_states<8, TERMS, REV, Out>(k, initial, states, last, stream);
+  return run_states<16, TERMS, REV, Out>(k, initial, states, last, stream);
+}
+
+static int check(const Call& k) {
+  if (k.B <= 0 || k.T <= 0 || k.H <= 0 || k.G <= 0 || k.H % k.G != 0 || k.chunks > 65535 || k.G > 65535) return -3;
+  if ((k.xb | k.xt | k.bb | k.bt | k.cb | k.ct) % 8) return -3;
+  if ((reinterpret_cast<uintptr_t>(k.x) | reinterpret_cast<uintptr_t>(k.Bm) | reinterpret_cast<uintptr_t>(k.Cm) | reinterpret_cast<uintptr_t>(k.dy)) & 15) return -3;
+  return 0;
 }
 
 }  // namespace ssd
 }  // namespace dewb
 
-// xdt bf16 [B, T, H, 64] (x * dt), Bm / Cm bf16 [B, T, G, 128], P bf16 [B * H, Tp, 64] (per head, lower triangle of
-// (C B^T) e^{g_i - g_j}), gc fp32 [B * H, Tp] (running sum of dt * A inside each chunk of 64; zero past T), all contiguous;
-// H even, two consecutive heads in one group.  initial / final_state fp32 [B, H, 64, 128] (initial may be null);
-// out bf16 [B, T, H, 64].
-extern "C" int dewb_ssd_scan_fwd(const void* xdt, const void* Bm, const void* Cm, const void* P, const float* gc,
-                                 const float* initial, void* out, float* final_state, int B, int T, int H, int G, int Tp,
-                                 int* err, void* stream_ptr) {
+// In how many parts the backward cuts the heads of a group (the leading size of its partial sums of dB and dC): the power of two that divides them with the
+// shortest last wave, a CTA's start and end counted as a head and a half.
+extern "C" int dewb_ssd_splits(int B, int T, int H, int G) {
+  const int per_group = H / G;
+  const long long base = static_cast<long long>(B) * ((T + dewb::ssd::L - 1) / dewb::ssd::L) * G;
+  int best = 1;
+  double least = 1e30;
+  for (int s = 1; s <= per_group && per_group % s == 0; s *= 2) {
+    const double cost = static_cast<double>((base * s + dewb::ssd::SMS - 1) / dewb::ssd::SMS) * (per_group / s + 1.5);
+    if (cost < least * 0.97) { least = cost; best = s; }
+  }
+  return best;
+}
+
+// x bf16 [B, T, H, 64], Bm / Cm bf16 [B, T, G, 128] with the given strides (batch row, token; in elements, multiples of 8; 16-byte aligned), dt fp32
+// [B, T, H], A [H], D [H] (may be null), initial fp32 [B, H, 64, 128] (may be null) -> y bf16 [B, T, H, 64], last fp32 [B, H, 64, 128]; states: scratch of
+// B * H * ceil(T / 64) * 64 * 128 bf16.  What is not strided is contiguous.
+extern "C" int dewb_ssd_fwd(const void* x, const float* dt, const float* A, const void* Bm, const void* Cm, const float* D, const float* initial, void* states,
+                            void* y, float* last, int B, int T, int H, int G, const long long* strides, void* stream_ptr) {
   using namespace dewb::ssd;
-  if (B <= 0 || T <= 0 || H <= 0 || (H & 1) || G <= 0 || H % G != 0 || ((H / G) & 1) || Tp % CH != 0 || Tp < T) return -3;
-  const int N = (T + CH - 1) / CH;
-  CUtensorMap tx, tc, tb, tp;
-  int r;
-  if ((r = make_map4(&tx, xdt, B, T, H / 2, 128, CH))) return 1000 + r;
-  if ((r = make_map4(&tc, Cm, B, T, G, ND, CH))) return 2000 + r;
-  if ((r = make_map4(&tb, Bm, B, T, G, ND, CH))) return 3000 + r;
-  if ((r = dewb::make_tmap_2d(&tp, P, static_cast<uint64_t>(B) * H * Tp, CH, CH, CH, 64, 2, true))) return 4000 + r;
-  cudaError_t e = cudaFuncSetAttribute(ssd_scan_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-  if (e != cudaSuccess) return static_cast<int>(e);
-  ssd_scan_fwd_kernel<<<B * (H / 2), THREADS, SMEM, reinterpret_cast<cudaStream_t>(stream_ptr)>>>(
-      tx, tc, tb, tp, gc, initial, reinterpret_cast<__nv_bfloat16*>(out), final_state, T, H, G, Tp, N, err);
+  typedef const __nv_bfloat16* in;
+  const Call k{static_cast<in>(x), static_cast<in>(Bm), static_cast<in>(Cm), nullptr, dt, A, D, strides[0], strides[1], strides[2], strides[3], strides[4], strides[5],
+               B, T, H, G, (T + L - 1) / L};
+  int e = check(k);
+  if (e) return e;
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
+  if ((e = walk<1, false, __nv_bfloat16>(k, initial, static_cast<__nv_bfloat16*>(states), last, stream))) return e;
+  int splits = 1;                                      // two CTAs an SM
+  while ((H / G) % (splits * 2) == 0 && static_cast<long long>(B) * k.chunks * G * splits < 2 * SMS) splits *= 2;
+  cudaError_t c = cudaFuncSetAttribute(ssd_output, cudaFuncAttributeMaxDynamicSharedMemorySize, OUT_SMEM);
+  if (c != cudaSuccess) return static_cast<int>(c);
+  ssd_output<<<dim3(B * k.chunks, G, splits), 128, OUT_SMEM, stream>>>(k, static_cast<in>(states), static_cast<__nv_bfloat16*>(y), H / G / splits);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// The gradients of dewb_ssd_fwd's inputs for dy (bf16 [B, T, H, 64], contiguous) and dlast (fp32, gradient of `last`, may be null).  Scratch: states and dstates
+// (fp32, B * H * ceil(T / 64) * 64 * 128 each), partA / partD (B * ceil(T / 64) * H), and with splits = dewb_ssd_splits(...) > 1 partB / partC
+// (splits * B * T * G * 128).  dinitial and dD may be null.
+extern "C" int dewb_ssd_bwd(const void* x, const float* dt, const float* A, const void* Bm, const void* Cm, const float* D, const float* initial, const void* dy,
+                            const float* dlast, float* states, float* dstates, float* partA, float* partD, float* partB, float* partC, void* dx, float* ddt, float* dA,
+                            void* dB, void* dC, float* dD, float* dinitial, int B, int T, int H, int G, const long long* strides, void* stream_ptr) {
+  using namespace dewb::ssd;
+  typedef const __nv_bfloat16* in;
+  typedef __nv_bfloat16* to;
+  const Call k{static_cast<in>(x), static_cast<in>(Bm), static_cast<in>(Cm), static_cast<in>(dy), dt, A, D, strides[0], strides[1], strides[2], strides[3], strides[4],
+               strides[5], B, T, H, G, (T + L - 1) / L};
+  int e = check(k);
+  if (e) return e;
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
+  if ((e = walk<3, false, float>(k, initial, states, nullptr, stream))) return e;
+  if ((e = walk<3, true, float>(k, dlast, dstates, dinitial, stream))) return e;
+  const int splits = dewb_ssd_splits(B, T, H, G);
+  if (splits > 1 && (partB == nullptr || partC == nullptr)) return -3;
+  const Grads g{static_cast<to>(dx), static_cast<to>(dB), static_cast<to>(dC), ddt, splits > 1 ? partB : nullptr, splits > 1 ? partC : nullptr, partA, partD};
+  cudaError_t c = cudaFuncSetAttribute(ssd_local, cudaFuncAttributeMaxDynamicSharedMemorySize, LOCAL_SMEM);
+  if (c != cudaSuccess) return static_cast<int>(c);
+  ssd_local<<<dim3(B * k.chunks, G, splits), 256, LOCAL_SMEM, stream>>>(k, states, dstates, g, H / G / splits);
+  if ((c = cudaGetLastError()) != cudaSuccess) return static_cast<int>(c);
+  const long long total = splits > 1 ? static_cast<long long>(B) * T * G * N : 0;
+  ssd_reduce<<<static_cast<unsigned>(H + (total / 4 + 255) / 256), 256, 0, stream>>>(g, dA, dD, H, B * k.chunks, total, splits);
   return static_cast<int>(cudaGetLastError());
 }

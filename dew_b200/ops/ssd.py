@@ -1,95 +1,129 @@
-"""Mamba-2 SSD on the sm_100a scan kernel (``csrc/kernels/ssd_sm100.cu``): state dimension 128, head dimension 64, heads
-taken in pairs of one B / C group.
+"""Mamba-2 SSD on the sm_100a kernels (``csrc/kernels/ssd_sm100.cu``): state dimension 128, head dimension 64.
 
-Forward: the per-head decayed score blocks ``P_h = (C B^T) o e^{g_i - g_j}`` and the running log decay ``g`` are prepared as
-batched products, then ONE sequential kernel per (batch, head pair) walks the chunks with the state in registers / a bf16
-operand tile (see the kernel's header).  Backward: the loop-free chunked form in PyTorch (``ops.scan.ssd_chunked``) is
-re-evaluated under autograd.  Reference: src/dew/nn/kernels/mamba_ssd.py (ChunkCumsum, BmmChunk, ChunkState, StatePassing,
+Forward: the states between the chunks of 64 tokens (sequential, one CTA per batch row, head and slice of columns), then the outputs of all chunks at once.
+Backward, for bf16 inputs: the states again (nothing but the inputs is kept between the passes) and their gradients by the same walk in reverse, in fp32, then the
+gradients of all chunks at once.  Inputs of other types are rounded to bf16 on the way forward and differentiated as they are: the loop-free chunked form in
+PyTorch (``ops.scan.ssd_chunked``) is re-evaluated under autograd.  Reference: src/dew/nn/kernels/mamba_ssd.py (ChunkCumsum, BmmChunk, ChunkState, StatePassing,
 ChunkScan), src/dew/nn/mixers/mamba2.py:101 ``chunk_ssd``.
 """
 from __future__ import annotations
 
 import ctypes
-from typing import Optional
 
 import torch
 
 from . import library as L
 
 CHUNK = 64
+HEAD, STATE = 64, 128
 
 
 def kernel_available(x: torch.Tensor, Bm: torch.Tensor) -> bool:
     H, P = x.shape[2], x.shape[3]
     G, N = Bm.shape[2], Bm.shape[3]
-    return (x.is_cuda and P == 64 and N == 128 and H % 2 == 0 and H % G == 0 and (H // G) % 2 == 0 and L.exists()
-            and hasattr(L.load(), "dewb_ssd_scan_fwd"))
+    return (x.is_cuda and P == HEAD and N == STATE and H % 2 == 0 and H % G == 0 and (H // G) % 2 == 0 and L.exists()
+            and hasattr(L.load(), "dewb_ssd_fwd"))
 
 
-def prepare(x, dt, A, Bm, Cm):
-    """-> xdt bf16 ``[B,T,H,P]``, Bm / Cm bf16, P bf16 ``[B*H, Tp, 64]``, gc fp32 ``[B*H, Tp]``."""
-    B, T, H, P = x.shape
-    G = Bm.shape[2]
-    Tp = (T + CHUNK - 1) // CHUNK * CHUNK
-    Nc = Tp // CHUNK
-    pad = Tp - T
-    dtf = dt.float()
-    a = torch.nn.functional.pad(dtf * A.float(), (0, 0, 0, pad))                            # [B,Tp,H]
-    gc = a.reshape(B, Nc, CHUNK, H).cumsum(2)                                               # [B,Nc,C,H]
-    xdt = (x.float() * dtf[..., None]).to(torch.bfloat16).contiguous()
-    b16, c16 = Bm.to(torch.bfloat16).contiguous(), Cm.to(torch.bfloat16).contiguous()
-    bc = torch.nn.functional.pad(b16, (0, 0, 0, 0, 0, pad)).reshape(B, Nc, CHUNK, G, -1)
-    cc = torch.nn.functional.pad(c16, (0, 0, 0, 0, 0, pad)).reshape(B, Nc, CHUNK, G, -1)
-    cb = torch.einsum("bcign,bcjgn->bcgij", cc, bc).float()                                 # [B,Nc,G,C,C]
-    g_h = gc.permute(0, 1, 3, 2)                                                            # [B,Nc,H,C]
-    diff = g_h[..., :, None] - g_h[..., None, :]
-    tril = torch.tril(torch.ones(CHUNK, CHUNK, dtype=torch.bool, device=x.device))
-    decay = torch.where(tril, torch.exp(torch.where(tril, diff, torch.zeros_like(diff))), torch.zeros_like(diff))
-    Pm = (cb.repeat_interleave(H // G, 2) * decay).to(torch.bfloat16)                       # [B,Nc,H,C,C]
-    Pm = Pm.permute(0, 2, 1, 3, 4).reshape(B * H, Tp, CHUNK).contiguous()
-    gcf = g_h.permute(0, 2, 1, 3).reshape(B * H, Tp).contiguous()
-    return xdt, b16, c16, Pm, gcf, Tp
+def _rows(t: torch.Tensor) -> torch.Tensor:
+    """``t [B, T, heads, width]`` in bf16 as the kernels take it: a token's heads in one piece, rows on 16-byte boundaries (a view of a wider projection is one)."""
+    t = t.to(torch.bfloat16)
+    inner = t.stride(3) == 1 and (t.shape[2] == 1 or t.stride(2) == t.shape[3])
+    outer = all(n == 1 or s % 8 == 0 for n, s in zip(t.shape[:2], t.stride()))
+    return t if inner and outer and t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
 
 
-def scan_cuda(xdt, b16, c16, Pm, gc, Tp: int, initial_state: Optional[torch.Tensor]):
-    B, T, H, P = xdt.shape
-    G = b16.shape[2]
-    dev = xdt.device
-    out = torch.empty(B, T, H, P, dtype=torch.bfloat16, device=dev)
-    final = torch.empty(B, H, P, b16.shape[3], dtype=torch.float32, device=dev)
-    init = None if initial_state is None else initial_state.float().contiguous()
-    L.ensure_device(xdt)
-    rc = L.load().dewb_ssd_scan_fwd(L.ptr(xdt), L.ptr(b16), L.ptr(c16), L.ptr(Pm), L.ptr(gc), L.ptr(init), L.ptr(out), L.ptr(final),
-                                    ctypes.c_int(B), ctypes.c_int(T), ctypes.c_int(H), ctypes.c_int(G), ctypes.c_int(Tp),
-                                    L.ptr(L.status(dev)), L.stream_ptr())
-    L.check(rc, "ssd_scan_fwd")
-    L.count_launches()
-    return out, final
+def _strides(*tensors: torch.Tensor):
+    """Batch-row and token strides (0 where there is one)."""
+    return (ctypes.c_longlong * (2 * len(tensors)))(*(s if n > 1 else 0 for t in tensors for n, s in zip(t.shape[:2], t.stride())))
+
+
+def _numbers(t, heads: int):
+    """One fp32 number per head."""
+    return None if t is None else t.detach().float().expand(heads).contiguous()
+
+
+def _forward(x, dt, A, Bm, Cm, D, initial):
+    B, T, H, _ = x.shape
+    dev = x.device
+    chunks = -(-T // CHUNK)
+    y = torch.empty(B, T, H, HEAD, dtype=torch.bfloat16, device=dev)
+    last = torch.empty(B, H, HEAD, STATE, dtype=torch.float32, device=dev)
+    states = torch.empty(B, H, chunks, HEAD, STATE, dtype=torch.bfloat16, device=dev)
+    L.ensure_device(x)
+    L.check(L.load().dewb_ssd_fwd(L.ptr(x), L.ptr(dt), L.ptr(A), L.ptr(Bm), L.ptr(Cm), L.ptr(D), L.ptr(initial), L.ptr(states), L.ptr(y), L.ptr(last),
+                                  ctypes.c_int(B), ctypes.c_int(T), ctypes.c_int(H), ctypes.c_int(Bm.shape[2]), _strides(x, Bm, Cm), L.stream_ptr()), "ssd_fwd")
+    L.count_launches(2)
+    return y, last
+
+
+def _backward(x, dt, A, Bm, Cm, D, initial, dy, dlast):
+    """-> dx, ddt, dA, dB, dC, dD, dinitial."""
+    B, T, H, _ = x.shape
+    G, dev = Bm.shape[2], x.device
+    chunks = -(-T // CHUNK)
+    lib = L.load()
+    f32 = dict(dtype=torch.float32, device=dev)
+    splits = lib.dewb_ssd_splits(ctypes.c_int(B), ctypes.c_int(T), ctypes.c_int(H), ctypes.c_int(G))
+    states, dstates = (torch.empty(B, H, chunks, HEAD, STATE, **f32) for _ in range(2))
+    part = torch.empty(2, B * chunks, H, **f32)
+    parts = torch.empty(2, splits, B, T, G, STATE, **f32) if splits > 1 else (None, None)
+    dx = torch.empty(B, T, H, HEAD, dtype=torch.bfloat16, device=dev)
+    dB, dC = (torch.empty(B, T, G, STATE, dtype=torch.bfloat16, device=dev) for _ in range(2))
+    ddt, dA, dD = torch.empty(B, T, H, **f32), torch.empty(H, **f32), None if D is None else torch.empty(H, **f32)
+    dinitial = torch.empty(B, H, HEAD, STATE, **f32)
+    L.ensure_device(x)
+    L.check(lib.dewb_ssd_bwd(L.ptr(x), L.ptr(dt), L.ptr(A), L.ptr(Bm), L.ptr(Cm), L.ptr(D), L.ptr(initial), L.ptr(dy), L.ptr(dlast), L.ptr(states), L.ptr(dstates),
+                             L.ptr(part[0]), L.ptr(part[1]), L.ptr(parts[0]), L.ptr(parts[1]), L.ptr(dx), L.ptr(ddt), L.ptr(dA), L.ptr(dB), L.ptr(dC), L.ptr(dD),
+                             L.ptr(dinitial), ctypes.c_int(B), ctypes.c_int(T), ctypes.c_int(H), ctypes.c_int(G), _strides(x, Bm, Cm), L.stream_ptr()), "ssd_bwd")
+    L.count_launches(4)
+    return dx, ddt, dA, dB, dC, dD, dinitial
 
 
 class _SSD(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, dt, A, Bm, Cm, D, initial_state):
-        ctx.save_for_backward(x, dt, A, Bm, Cm, D, initial_state)
-        xdt, b16, c16, Pm, gc, Tp = prepare(x, dt, A, Bm, Cm)
-        y, S = scan_cuda(xdt, b16, c16, Pm, gc, Tp, initial_state)
-        if D is not None:
-            y = (y.float() + x.float() * D.float()[None, None, :, None]).to(y.dtype)
-        return y.to(x.dtype), S
+        ctx.set_materialize_grads(False)
+        H = x.shape[2]
+        exact = all(t.dtype == torch.bfloat16 for t in (x, Bm, Cm))
+        ctx.exact = exact
+        xb, bb, cb = _rows(x), _rows(Bm), _rows(Cm)
+        ins = (dt.detach().float().contiguous(), _numbers(A, H), bb, cb, _numbers(D, H) if exact else None,
+               None if initial_state is None else initial_state.detach().float().contiguous())
+        y, last = _forward(xb, *ins)
+        ctx.given = tuple(None if t is None else (t.dtype, t.shape) for t in (dt, A, D, initial_state))
+        if exact:
+            ctx.save_for_backward(xb, *ins)
+        else:
+            ctx.save_for_backward(x, dt, A, Bm, Cm, D, initial_state)
+            if D is not None:
+                y = (y.float() + x.float() * D.float()[None, None, :, None]).to(y.dtype)
+        return y.to(x.dtype), last
 
     @staticmethod
-    def backward(ctx, dy, dS):
-        from .scan import ssd_chunked
+    def backward(ctx, dy, dlast):
         saved = ctx.saved_tensors
-        with torch.enable_grad():
-            leaves = [None if t is None else t.detach().requires_grad_(t.is_floating_point()) for t in saved]
-            y, S = ssd_chunked(*leaves)
-            need = [(t, i) for i, t in enumerate(leaves) if t is not None and ctx.needs_input_grad[i]]
-            grads = torch.autograd.grad((y, S), [t for t, _ in need], (dy.to(y.dtype), dS.to(S.dtype)), allow_unused=True)
-        out = [None] * 7
-        for (t, i), g in zip(need, grads):
-            out[i] = g
-        return tuple(out)
+        x = saved[0]
+        dy = torch.zeros(x.shape, dtype=x.dtype, device=x.device) if dy is None else dy
+        if not ctx.exact:
+            from .scan import ssd_chunked
+            with torch.enable_grad():
+                leaves = [None if t is None else t.detach().requires_grad_(t.is_floating_point()) for t in saved]
+                y, S = ssd_chunked(*leaves)
+                need = [(t, i) for i, t in enumerate(leaves) if t is not None and ctx.needs_input_grad[i]]
+                dlast = torch.zeros_like(S) if dlast is None else dlast
+                grads = torch.autograd.grad((y, S), [t for t, _ in need], (dy.to(y.dtype), dlast.to(S.dtype)), allow_unused=True)
+            out = [None] * 7
+            for (t, i), g in zip(need, grads):
+                out[i] = g
+            return tuple(out)
+        dy = dy.to(torch.bfloat16).contiguous()
+        if dy.data_ptr() % 16:
+            dy = dy.clone()
+        dx, ddt, dA, dB, dC, dD, dinitial = _backward(*saved, dy, None if dlast is None else dlast.float().contiguous())
+        fit = lambda g, given: None if given is None else g.sum_to_size(given[1]).to(given[0])
+        dt_, A_, D_, initial_ = ctx.given
+        return dx, fit(ddt, dt_), fit(dA, A_), dB, dC, fit(dD, D_), fit(dinitial, initial_)
 
 
 def ssd(x, dt, A, Bm, Cm, D=None, initial_state=None):

@@ -232,7 +232,7 @@ def bench_gdn(out, peaks, flush, iters=10, shapes=None):
 
 
 def bench_ssd(out, peaks, flush, iters=10, shapes=None):
-    """Mamba-2 SSD forward: the scan kernel against the loop-free chunked form in PyTorch."""
+    """Mamba-2 SSD forward and backward: the kernels against the loop-free chunked form in PyTorch (forward)."""
     from ..ops import scan
     for B, T, H, G in shapes or [(1, 4096, 64, 1), (2, 8192, 32, 1)]:
         x = torch.randn(B, T, H, 64, device="cuda").to(torch.bfloat16)
@@ -241,13 +241,13 @@ def bench_ssd(out, peaks, flush, iters=10, shapes=None):
         Bm = (torch.randn(B, T, G, 128, device="cuda") / 8).to(torch.bfloat16)
         Cm = (torch.randn(B, T, G, 128, device="cuda") / 8).to(torch.bfloat16)
         with torch.no_grad():
-            from ..ops import ssd as K
             t_k = device_time(lambda: scan.ssd(x, dt, A, Bm, Cm), iters=iters, flush=flush)
-            prep = K.prepare(x, dt, A, Bm, Cm)
-            t_s = device_time(lambda: K.scan_cuda(*prep, None), iters=iters, flush=flush)
             t_t = device_time(lambda: scan.ssd_chunked(x, dt, A, Bm, Cm), iters=max(2, iters // 3), flush=flush)
+        leaves = [t.requires_grad_() for t in (x, dt, A, Bm, Cm)]
+        dy = torch.randn_like(x)
+        t_b = device_time(lambda: torch.autograd.grad(scan.ssd(*leaves)[0], leaves, dy), iters=iters, flush=flush)
         L.check_status()
-        _row(out, kernel="ssd", B=B, T=T, H=H, G=G, fwd_ms=t_k.median_ms, scan_kernel_ms=t_s.median_ms, torch_chunked_ms=t_t.median_ms)
+        _row(out, kernel="ssd", B=B, T=T, H=H, G=G, fwd_ms=t_k.median_ms, fwd_bwd_ms=t_b.median_ms, torch_chunked_ms=t_t.median_ms)
 
 
 def bench_sampling(out, peaks, flush, iters=10):

@@ -26,13 +26,16 @@ NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--use_fast_math", "-Xcompiler",
               "--expt-relaxed-constexpr"]
 
 # Files whose 32-bit arithmetic has to hold up on its own (decoders that run in fp32): compiled without fast math.
-EXACT_MATH = ("residual_streams", "paged_attention", "latent_attention", "decayed_recurrence", "gated_recurrence", "gated_chunks", "token_mix", "moe_serve", "ssd_sm100")
+EXACT_MATH = ("residual_streams", "paged_attention", "latent_attention", "decayed_recurrence", "gated_recurrence", "gated_chunks", "token_mix", "moe_serve")
+
+# The same for kernels of training, which a program that only decodes does not build: gradients that are kept in fp32.
+EXACT_TRAINING = ("ssd_sm100",)
 
 # Subsets of the library a program can build alone, as ``libdewb_<part>.so``: a process that only decodes needs neither the training nor
 # the multi-GPU kernels.
 PARTS = {
     "decoder": ("elementwise", "decode_attention", "decode_attention_tma", "flash_fwd_sm100", "gemm_sm100", "gemm_pair_sm100")
-    + tuple(name for name in EXACT_MATH if name != "ssd_sm100"),
+    + EXACT_MATH,
 }
 
 
@@ -58,7 +61,7 @@ def _digest(path: Path) -> str:
 
 
 def _flags(src: Path) -> List[str]:
-    return [f for f in NVCC_FLAGS if f != "--use_fast_math"] if src.stem in EXACT_MATH else NVCC_FLAGS
+    return [f for f in NVCC_FLAGS if f != "--use_fast_math"] if src.stem in EXACT_MATH + EXACT_TRAINING else NVCC_FLAGS
 
 
 def _compile(src: Path, verbose: bool) -> Path:

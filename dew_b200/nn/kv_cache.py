@@ -413,7 +413,7 @@ class KVStore:
     def can_decode_packed(self, qkv: torch.Tensor, Hq: int, softcap: float = 0.0) -> bool:
         return (qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.is_contiguous() and self.kind == 0 and self.row_ids is None
                 and qkv.shape[0] == self.rows and self.head_dim == 128 and self.page_size % 64 == 0 and not softcap
-                and Hq // self.kv_heads <= 8 and os.environ.get("DEWB_DECODE", "stream") == "stream"
+                and Hq // self.kv_heads <= 8 and L.env("DEWB_DECODE", "stream") == "stream"
                 and hasattr(L.load(), "dewb_rope_append"))
 
     MIN_TILES = 4            # fewest 64-key tiles one CTA of the balanced decode kernel takes (bounds the parts a row is cut into)
@@ -426,9 +426,9 @@ class KVStore:
         longest = min(self.max_len, window + visible.keep if window else self.max_len, visible.chunk or self.max_len)
         max_tiles = -(-longest // 64) + 1 + int(visible.keep > 0)         # (+ 1: a window, or kept first keys, that straddle a tile boundary)
         # (factors and sigmoid weights are built for the balanced form)
-        persist = visible.gain is not None or visible.sigmoid is not None or (R <= 1024 and os.environ.get("DEWB_DECODE_PERSIST", "1") == "1")
+        persist = visible.gain is not None or visible.sigmoid is not None or (R <= 1024 and L.env("DEWB_DECODE_PERSIST", "1") == "1")
         if persist:
-            min_tiles = int(os.environ.get("DEWB_DECODE_MIN_TILES", self.MIN_TILES))
+            min_tiles = int(L.env("DEWB_DECODE_MIN_TILES", self.MIN_TILES))
             splits = (max_tiles - 1) // min_tiles + 2
         else:
             share = 8                                                     # tiles a CTA takes
@@ -439,19 +439,20 @@ class KVStore:
         pm, pl, pa = self._partials(n, D, q.device)
         if getattr(self, "_arrivals", None) is None or self._arrivals.numel() < R * kv_heads:
             self._arrivals = torch.zeros(R * kv_heads, dtype=torch.int32, device=q.device)
-        common = (L.ptr(q), L.ptr(self.k[layer]), L.ptr(self.v[layer]), ctypes.c_longlong(self.pages * self.page_size),
-                  L.ptr(self.page_table if table is None else table), L.ptr(lens32), L.ptr(pm), L.ptr(pl), L.ptr(pa), L.ptr(self._arrivals), L.ptr(sinks32),
-                  L.ptr(out), ctypes.c_int(R), ctypes.c_int(Hq), ctypes.c_int(kv_heads), ctypes.c_int(self.page_size),
-                  ctypes.c_int(self.max_pages), ctypes.c_int(splits))
+        at = lambda t: 0 if t is None else t.data_ptr()
         if persist:
             if getattr(self, "_ctas", None) is None:
                 self._ctas = 2 * torch.cuda.get_device_properties(q.device).multi_processor_count
-            L.check(lib.dewb_paged_decode_persist(*common, ctypes.c_int(min_tiles), ctypes.c_float(scale),
-                                                  ctypes.c_int(window or 0), ctypes.c_int(visible.keep), ctypes.c_int(visible.chunk or 0),
-                                                ctypes.c_float(visible.softcap), L.ptr(visible.gain), L.ptr(visible.sigmoid), ctypes.c_longlong(q_row_stride),
-                                                ctypes.c_int(self._ctas),
-                                                  L.ptr(L.status(q.device)), L.stream_ptr()), "paged_decode_persist")
+            L.check(lib.dewb_paged_decode_persist(at(q), at(self.k[layer]), at(self.v[layer]), self.pages * self.page_size, at(self.page_table if table is None else table),
+                                                  at(lens32), at(pm), at(pl), at(pa), at(self._arrivals), at(sinks32), at(out), R, Hq, kv_heads, self.page_size,
+                                                  self.max_pages, splits, min_tiles, scale, window or 0, visible.keep, visible.chunk or 0, visible.softcap,
+                                                  at(visible.gain), at(visible.sigmoid), q_row_stride, self._ctas, at(L.status(q.device)), L.stream()),
+                    "paged_decode_persist")
         else:
+            common = (L.ptr(q), L.ptr(self.k[layer]), L.ptr(self.v[layer]), ctypes.c_longlong(self.pages * self.page_size),
+                      L.ptr(self.page_table if table is None else table), L.ptr(lens32), L.ptr(pm), L.ptr(pl), L.ptr(pa), L.ptr(self._arrivals), L.ptr(sinks32),
+                      L.ptr(out), ctypes.c_int(R), ctypes.c_int(Hq), ctypes.c_int(kv_heads), ctypes.c_int(self.page_size),
+                      ctypes.c_int(self.max_pages), ctypes.c_int(splits))
             L.check(lib.dewb_paged_decode_fused(*common, ctypes.c_int(share), ctypes.c_float(scale),
                                                 ctypes.c_int(window or 0), ctypes.c_int(visible.keep), ctypes.c_int(visible.chunk or 0),
                                                 ctypes.c_float(visible.softcap), ctypes.c_longlong(q_row_stride),
@@ -465,10 +466,9 @@ class KVStore:
         lib = L.load()
         R, H, D = qkv.shape
         pos32, lens32 = self._step_ints(positions)
-        L.check(lib.dewb_rope_append(L.ptr(qkv), L.ptr(cos), L.ptr(sin), L.ptr(pos32), ctypes.c_int(R), ctypes.c_int(Hq),
-                                     ctypes.c_int(self.kv_heads), ctypes.c_int(D), ctypes.c_int(cos.shape[0] if cos is not None else 0),
-                                     L.ptr(self.k[layer]), L.ptr(self.v[layer]), L.ptr(self.page_table), ctypes.c_int(self.page_size),
-                                     ctypes.c_int(self.max_pages), L.stream_ptr()), "rope_append")
+        at = lambda t: 0 if t is None else t.data_ptr()
+        L.check(lib.dewb_rope_append(at(qkv), at(cos), at(sin), at(pos32), R, Hq, self.kv_heads, D, cos.shape[0] if cos is not None else 0, at(self.k[layer]),
+                                     at(self.v[layer]), at(self.page_table), self.page_size, self.max_pages, L.stream()), "rope_append")
         out = torch.empty((R, Hq, D), dtype=qkv.dtype, device=qkv.device)
         sk = getattr(self, "_sinks32", None)
         if sinks is not None and (sk is None or sk[0] is not sinks):

@@ -133,15 +133,23 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         return r if bias is None else r.add_(bias.to(r.dtype))
     if bias is not None and (accumulate or out is not None and out.dtype != torch.bfloat16 or out_dtype != torch.bfloat16):
         raise ValueError("gemm: a bias joins a fresh bf16 output only")
-    if out is None:
+    fresh = out is None
+    kind = out_dtype if fresh else out.dtype
+    plain = not a_mn and not b_mn and kind == torch.bfloat16 and (fresh or not accumulate) and alpha == 1.0
+    tiles = ((M + 127) // 128) * ((N + 255) // 256)
+    cell = ("decode",) if (M <= 128 and plain and bias is None) else (("skinny",) if tiles < 24 else None)
+    if (fresh and cell is not None and kernel is None and _GEMM.declared.get(cell) == "cublas" and alpha == 1.0 and a.dtype == b.dtype == kind
+            and not _GEMM.forced_by_environment() and not (torch.is_grad_enabled() and (a.requires_grad or b.requires_grad))):
+        # a small product that its measured cell sends to the library arm: nothing about it needs looking up
+        _GEMM._record("cublas", {}, None, cell)
+        A, Bt = a.t() if a_mn else a, b if b_mn else b.t()
+        return torch.mm(A, Bt) if bias is None else torch.addmm(bias.to(kind), A, Bt)
+    if fresh:
         out = torch.empty((M, N), dtype=out_dtype, device=a.device)
         accumulate = False
     case = dict(dtype=a.dtype if a.dtype == b.dtype else None, lda=a.stride(0), ldb=b.stride(0), ldd=out.stride(0),
                 aligned=(a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0),
-                inner_contig=(a.stride(1) == 1 and b.stride(1) == 1 and out.stride(1) == 1), M=M, N=N, K=K,
-                plain=(not a_mn and not b_mn and out.dtype == torch.bfloat16 and not accumulate and alpha == 1.0))
-    tiles = ((M + 127) // 128) * ((N + 255) // 256)
-    cell = ("decode",) if (M <= 128 and case["plain"] and bias is None) else (("skinny",) if tiles < 24 else None)
+                inner_contig=(a.stride(1) == 1 and b.stride(1) == 1 and out.stride(1) == 1), M=M, N=N, K=K, plain=plain)
     if bias is not None:
         case["plain"] = False                                    # (the weight-streaming kernel has no bias epilogue)
     if kernel is None and cell is None and tiles >= 148 and _pair_built() and all(case[x] % 8 == 0 for x in ("lda", "ldb", "ldd")) and case["aligned"]:
@@ -211,14 +219,19 @@ def grad_accumulates(p) -> bool:
     return True
 
 
+def _linear(x, weight, bias):
+    """``x`` contiguous; the bias joins in the product's epilogue."""
+    if x.dim() == 2:
+        return gemm(x, weight, bias=bias)
+    return gemm(x.view(-1, x.shape[-1]), weight, bias=bias).view(*x.shape[:-1], weight.shape[0])
+
+
 class _Linear(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias):
         ctx.save_for_backward(x, weight)
         ctx.has_bias = bias is not None
-        x2 = x.reshape(-1, x.shape[-1])
-        y = gemm(x2, weight, bias=bias)                          # the bias joins in the product's epilogue
-        return y.reshape(*x.shape[:-1], weight.shape[0])
+        return _linear(x, weight, bias)
 
     @staticmethod
     def backward(ctx, dy):
@@ -248,6 +261,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
         return F.linear(x, weight.to(x.dtype) if weight.dtype != x.dtype else weight, bias)
     if not x.is_contiguous():
         x = x.contiguous()
+    if L.unrecorded(x, weight, bias):
+        return _linear(x, weight, bias)
     return _Linear.apply(x, weight, bias)
 
 
@@ -308,30 +323,33 @@ def _bwd_scratch(rows: int, d: int, device) -> torch.Tensor:
     return torch.empty((blocks, d), dtype=torch.float32, device=device)
 
 
+def _rms_norm(x, other, w, eps, mode):
+    """Contiguous ``x``, ``other`` -> y, h (mode 1) or None, the rows' 1 / rms, and the weights as the kernel took them."""
+    d = x.shape[-1]
+    rows = x.numel() // d if d else 0
+    y = torch.empty_like(x)
+    h = torch.empty_like(x) if mode == 1 else None
+    rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
+    wb = w if w.dtype == torch.bfloat16 else w.to(torch.bfloat16)
+    rc = L.load().dewb_rmsnorm_fwd(x.data_ptr(), 0 if other is None else other.data_ptr(), wb.data_ptr(), y.data_ptr(), 0 if h is None else h.data_ptr(), rstd.data_ptr(),
+                                   rows, d, eps, mode, L.stream())
+    if rc:
+        L.check(rc, "rmsnorm_fwd")
+    L.count_launches()
+    return y, h, rstd, wb
+
+
 class _RMSNorm(torch.autograd.Function):
     """mode 0 plain, 1 stream (x + branch, emits both), 2 gated (norm(x) * w * silu(z))."""
 
     @staticmethod
     def forward(ctx, x, other, w, eps, mode):
-        lib = L.load()
         d = x.shape[-1]
-        x2 = x.reshape(-1, d)
-        rows = x2.shape[0]
-        o2 = other.reshape(-1, d) if other is not None else None
-        y = torch.empty_like(x2)
-        h = torch.empty_like(x2) if mode == 1 else None
-        rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
-        wb = w if w.dtype == torch.bfloat16 else w.to(torch.bfloat16)
-        L.check(lib.dewb_rmsnorm_fwd(L.ptr(x2), L.ptr(o2), L.ptr(wb), L.ptr(y), L.ptr(h), L.ptr(rstd), c_ll(rows),
-                                     c_int(d), c_float(eps), c_int(mode), L.stream_ptr()), "rmsnorm_fwd")
-        L.count_launches()
+        y, h, rstd, wb = _rms_norm(x, other, w, eps, mode)
         ctx.mode, ctx.shape = mode, x.shape
-        ctx.save_for_backward(h if mode == 1 else x2, wb, rstd, o2 if mode == 2 else None)
+        ctx.save_for_backward((h if mode == 1 else x).view(-1, d), wb, rstd, other.view(-1, d) if mode == 2 else None)
         ctx.w_dtype = w.dtype
-        if mode == 1:
-            ctx.mark_non_differentiable()
-            return y.reshape(x.shape), h.reshape(x.shape)
-        return y.reshape(x.shape)
+        return (y, h) if mode == 1 else y
 
     @staticmethod
     def backward(ctx, dy, dh=None):
@@ -364,14 +382,16 @@ def _norm_cuda_ok(x, w):
 
 def rms_norm(x: torch.Tensor, w: torch.Tensor, eps: float = 1e-6) -> torch.Tensor:
     if L.use_cuda(x) and _norm_cuda_ok(x, w):
-        return _RMSNorm.apply(x.contiguous(), None, w, eps, 0)
+        x = x.contiguous()
+        return _rms_norm(x, None, w, eps, 0)[0] if L.unrecorded(x, w) else _RMSNorm.apply(x, None, w, eps, 0)
     return rms_norm_reference(x, w, eps)
 
 
 def stream_rms_norm(x: torch.Tensor, branch: torch.Tensor, w: torch.Tensor, eps: float = 1e-6):
     """Residual-stream norm: ``h = x + branch``; returns ``(norm(h) * w, h)`` from one pass."""
     if L.use_cuda(x) and _norm_cuda_ok(x, w):
-        return _RMSNorm.apply(x.contiguous(), branch.contiguous(), w, eps, 1)
+        x, branch = x.contiguous(), branch.contiguous()
+        return _rms_norm(x, branch, w, eps, 1)[:2] if L.unrecorded(x, branch, w) else _RMSNorm.apply(x, branch, w, eps, 1)
     h = (x.float() + branch.float()).to(x.dtype)
     return rms_norm_reference(h, w, eps), h
 
@@ -379,7 +399,8 @@ def stream_rms_norm(x: torch.Tensor, branch: torch.Tensor, w: torch.Tensor, eps:
 def gated_rms_norm(x: torch.Tensor, z: torch.Tensor, w: torch.Tensor, eps: float = 1e-6) -> torch.Tensor:
     """``norm(x) * w * silu(z)`` (the output gate of gated-delta-net / Mamba-2 blocks)."""
     if L.use_cuda(x) and _norm_cuda_ok(x, w):
-        return _RMSNorm.apply(x.contiguous(), z.contiguous(), w, eps, 2)
+        x, z = x.contiguous(), z.contiguous()
+        return _rms_norm(x, z, w, eps, 2)[0] if L.unrecorded(x, z, w) else _RMSNorm.apply(x, z, w, eps, 2)
     return (rms_norm_reference(x, w, eps).float() * F.silu(z.float())).to(x.dtype)
 
 
@@ -387,21 +408,23 @@ def gated_rms_norm(x: torch.Tensor, z: torch.Tensor, w: torch.Tensor, eps: float
 # SwiGLU
 
 
+def _swiglu(gu):
+    F2 = gu.shape[-1]
+    Fh = F2 // 2
+    out = torch.empty(*gu.shape[:-1], Fh, dtype=gu.dtype, device=gu.device)
+    rc = L.load().dewb_swiglu_fwd(gu.data_ptr(), gu.data_ptr() + Fh * 2, out.data_ptr(), gu.numel() // F2, Fh, F2, L.stream())
+    if rc:
+        L.check(rc, "swiglu_fwd")
+    L.count_launches()
+    return out
+
+
 class _PackedSwiGLU(torch.autograd.Function):
     @staticmethod
     def forward(ctx, gu):
-        lib = L.load()
-        F2 = gu.shape[-1]
-        Fh = F2 // 2
-        g2 = gu.reshape(-1, F2)
-        rows = g2.shape[0]
-        out = torch.empty((rows, Fh), dtype=gu.dtype, device=gu.device)
-        L.check(lib.dewb_swiglu_fwd(L.ptr(g2), ctypes.c_void_p(g2.data_ptr() + Fh * 2), L.ptr(out), c_ll(rows),
-                                    c_int(Fh), c_ll(F2), L.stream_ptr()), "swiglu_fwd")
-        L.count_launches()
-        ctx.save_for_backward(g2)
+        ctx.save_for_backward(gu.view(-1, gu.shape[-1]))
         ctx.shape = gu.shape
-        return out.reshape(*gu.shape[:-1], Fh)
+        return _swiglu(gu)
 
     @staticmethod
     def backward(ctx, dy):
@@ -423,7 +446,8 @@ def packed_swiglu(gu: torch.Tensor) -> torch.Tensor:
     """``silu(gu[..., :F]) * gu[..., F:]`` on the output of a fused gate|up projection."""
     Fh = gu.shape[-1] // 2
     if L.use_cuda(gu) and gu.dtype == torch.bfloat16 and Fh % 8 == 0:
-        return _PackedSwiGLU.apply(gu.contiguous())
+        gu = gu.contiguous()
+        return _swiglu(gu) if L.unrecorded(gu) else _PackedSwiGLU.apply(gu)
     g, u = gu[..., :Fh], gu[..., Fh:]
     return (F.silu(g.float()) * u.float()).to(gu.dtype)
 
@@ -552,21 +576,27 @@ def rope_reference(x, cos, sin, positions=None, rot_heads=None):
     return out.to(x.dtype)
 
 
+def _rotate(x, cos, sin, positions, rot_heads):
+    """-> the rotated copy and the int32 positions it was rotated by (None: the row's own)."""
+    H, D = x.shape[-2], x.shape[-1]
+    out = x.clone()
+    pos = None
+    if positions is not None:
+        pos = positions.reshape(-1).to(torch.int32).contiguous()
+    elif out.dim() == 4 and out.shape[0] > 1:
+        pos = torch.arange(out.shape[1], device=x.device, dtype=torch.int32).repeat(out.shape[0])
+    rc = L.load().dewb_rope(out.data_ptr(), cos.data_ptr(), sin.data_ptr(), 0 if pos is None else pos.data_ptr(), out.numel() // (H * D), H, rot_heads, D, cos.shape[0], 1.0,
+                            L.stream())
+    if rc:
+        L.check(rc, "rope")
+    L.count_launches()
+    return out, pos
+
+
 class _Rope(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, cos, sin, positions, rot_heads):
-        lib = L.load()
-        H, D = x.shape[-2], x.shape[-1]
-        out = x.clone()
-        tokens = out.numel() // (H * D)
-        pos = None
-        if positions is not None:
-            pos = positions.reshape(-1).to(torch.int32).contiguous()
-        elif out.dim() == 4 and out.shape[0] > 1:
-            pos = torch.arange(out.shape[1], device=x.device, dtype=torch.int32).repeat(out.shape[0])
-        L.check(lib.dewb_rope(L.ptr(out), L.ptr(cos), L.ptr(sin), L.ptr(pos), c_ll(tokens), c_int(H), c_int(rot_heads),
-                              c_int(D), c_int(cos.shape[0]), c_float(1.0), L.stream_ptr()), "rope")
-        L.count_launches()
+        out, pos = _rotate(x, cos, sin, positions, rot_heads)
         ctx.save_for_backward(cos, sin, pos)
         ctx.rot_heads = rot_heads
         return out
@@ -591,7 +621,8 @@ def rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, positions: Optio
     H, D = x.shape[-2], x.shape[-1]
     rh = H if rot_heads is None else rot_heads
     if L.use_cuda(x) and x.dtype == torch.bfloat16 and D % 16 == 0:
-        return _Rope.apply(x.contiguous(), cos, sin, positions, rh)
+        x = x.contiguous()
+        return _rotate(x, cos, sin, positions, rh)[0] if L.unrecorded(x, cos, sin) else _Rope.apply(x, cos, sin, positions, rh)
     return rope_reference(x, cos.to(x.device), sin.to(x.device), positions, rh)
 
 

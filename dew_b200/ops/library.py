@@ -50,8 +50,43 @@ def load(build_if_missing: bool = False) -> ctypes.CDLL:
             build.build(verbose=False)
         else:
             raise LibraryMissing(f"{_LIB_PATH} is not built; run `python -m dew_b200.ops.build`")
-    _LIB = ctypes.CDLL(str(_LIB_PATH))
+    _LIB = _declare(ctypes.CDLL(str(_LIB_PATH)))
     return _LIB
+
+
+# Argument types of the launchers that small steps call most: p a pointer, l a 64-bit and i a 32-bit integer, f a float.  A declared launcher takes Python numbers
+# as they are; the others are given ctypes objects by their callers.
+_SIGNATURES = {
+    "dewb_rmsnorm_fwd": "pppppp" + "lifi" + "p",
+    "dewb_swiglu_fwd": "ppp" + "lil" + "p",
+    "dewb_rope": "pppp" + "liiiif" + "p",
+    "dewb_rope_append": "pppp" + "iiiii" + "ppp" + "ii" + "p",
+    "dewb_paged_decode_persist": "ppp" + "l" + "pppppppp" + "iiiiiii" + "f" + "iii" + "f" + "pp" + "l" + "i" + "pp",
+}
+_TYPES = {"p": ctypes.c_void_p, "l": ctypes.c_longlong, "i": ctypes.c_int, "f": ctypes.c_float}
+
+
+def _declare(lib: ctypes.CDLL) -> ctypes.CDLL:
+    for name, kinds in _SIGNATURES.items():
+        if hasattr(lib, name):
+            getattr(lib, name).argtypes = [_TYPES[k] for k in kinds]
+    return lib
+
+
+_ENV = getattr(os.environ, "_data", None)          # the environment as the bytes it is kept in
+_ENCODED: Dict[str, object] = {}
+
+
+def env(name: str, default: Optional[str] = None) -> Optional[str]:
+    """``os.environ.get`` for names that every call looks up: ``os.environ`` encodes the name and raises an exception inside for each one that is not set, which
+    takes longer than a launch."""
+    if _ENV is None:
+        return os.environ.get(name, default)
+    key = _ENCODED.get(name)
+    if key is None:
+        key = _ENCODED[name] = os.environ.encodekey(name)
+    value = _ENV.get(key)
+    return default if value is None else os.environ.decodevalue(value)
 
 
 def load_part(part: str) -> ctypes.CDLL:
@@ -66,14 +101,27 @@ def load_part(part: str) -> ctypes.CDLL:
 
 def use_cuda(*tensors: torch.Tensor) -> bool:
     """True when the op must run on the CUDA library (all tensors on a GPU)."""
-    t = next((x for x in tensors if isinstance(x, torch.Tensor)), None)
-    if t is None or not t.is_cuda:
+    for t in tensors:
+        if isinstance(t, torch.Tensor):
+            break
+    else:
         return False
-    if os.environ.get("DEWB_FORCE_REFERENCE") == "1":
+    if not t.is_cuda or env("DEWB_FORCE_REFERENCE") == "1":
         return False
-    load()  # raises LibraryMissing on a GPU box without the build
+    if _LIB is None:
+        load()  # raises LibraryMissing on a GPU box without the build
     ensure_device(t)
     return True
+
+
+def unrecorded(*tensors: Optional[torch.Tensor]) -> bool:
+    """Whether a call on these tensors leaves no trace in autograd, forward-mode differentiation, a functorch transform or a trace, so that its launches may run
+    without an autograd node around them (the node alone takes as long as two launches)."""
+    if torch.is_grad_enabled():
+        for t in tensors:
+            if t is not None and t.requires_grad:
+                return False
+    return (torch.autograd.forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active() and torch._C._get_tracing_state() is None)
 
 
 _TLS = threading.local()
@@ -82,14 +130,21 @@ _TLS = threading.local()
 def ensure_device(t: torch.Tensor) -> None:
     """Make ``t``'s device current for the library's own CUDA runtime on this thread (autograd runs backward on
     worker threads where nothing has selected a device yet)."""
-    idx = t.device.index if t.device.index is not None else torch.cuda.current_device()
+    idx = t.get_device()
+    if idx < 0:
+        idx = torch.cuda.current_device()
     if getattr(_TLS, "device", None) != idx:
         check(load().dewb_set_device(ctypes.c_int(idx)), "set_device")
         _TLS.device = idx
 
 
+def stream() -> int:
+    """The current stream of the current device."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
 def stream_ptr() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(stream())
 
 
 def ptr(t: Optional[torch.Tensor]) -> ctypes.c_void_p:

@@ -7,9 +7,10 @@ src/dew/nn/kernels/selection.py:1-60,113-300, restated for one backend: the sm_1
 """
 from __future__ import annotations
 
-import os
 from dataclasses import dataclass, field
 from typing import Any, Callable, Dict, List, Optional, Sequence, Tuple
+
+from . import library as L
 
 
 class KernelRefused(RuntimeError):
@@ -50,8 +51,14 @@ class Op:
     declared: Dict[Tuple, str] = field(default_factory=dict)   # cell key -> kernel name chosen by measurement
     routes: Dict[str, Dict[str, Any]] = field(default_factory=dict)   # kernel name -> call counts and refusal codes seen
 
+    def forced_by_environment(self) -> Optional[str]:
+        return L.env(self._switch)
+
+    def __post_init__(self):
+        self._switch = f"DEWB_KERNEL_{self.name.upper()}"
+
     def select(self, case: Dict[str, Any], forced: Optional[str] = None, cell: Optional[Tuple] = None) -> str:
-        forced = forced or os.environ.get(f"DEWB_KERNEL_{self.name.upper()}")
+        forced = forced or self.forced_by_environment()
         reasons: Dict[str, List[str]] = {}
         order = list(self.kernels)
         if cell is not None and cell in self.declared:

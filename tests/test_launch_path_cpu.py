@@ -1,0 +1,46 @@
+"""What lets a call leave out its autograd node, and the environment as every call reads it."""
+import os
+
+import pytest
+import torch
+import torch.autograd.forward_ad as fwd
+
+from dew_b200.ops import library as L
+
+
+def test_only_calls_that_nothing_records_leave_out_their_node():
+    x, w = torch.ones(2), torch.ones(2, requires_grad=True)
+    assert L.unrecorded(x) and L.unrecorded(x, None) and not L.unrecorded(x, w)
+    with torch.no_grad():
+        assert L.unrecorded(x, w)
+        with fwd.dual_level():
+            assert not L.unrecorded(x)
+        seen = []
+        torch.func.vmap(lambda t: (seen.append(L.unrecorded(t)), t)[1])(x)
+        torch.func.grad(lambda t: (seen.append(L.unrecorded(t)), t.sum())[1])(x)
+        torch.jit.trace(lambda t: (seen.append(L.unrecorded(t)), t * 2)[1], (x,), check_trace=False)
+        assert seen == [False] * 3
+        assert L.unrecorded(x)
+
+
+def test_environment_is_read_as_it_is_now(monkeypatch):
+    monkeypatch.delenv("DEWB_SOME_SWITCH", raising=False)
+    assert L.env("DEWB_SOME_SWITCH") is None and L.env("DEWB_SOME_SWITCH", "7") == "7"
+    monkeypatch.setenv("DEWB_SOME_SWITCH", "1")
+    assert L.env("DEWB_SOME_SWITCH") == os.environ["DEWB_SOME_SWITCH"] == "1"
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (5, 40, 24), (128, 256, 64)])
+def test_small_products_with_and_without_a_node(M, N, K):
+    from dew_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x, w, b = (torch.randn(*s, generator=g, device="cuda").bfloat16() for s in ((M, K), (N, K), (N,)))
+    truth = x.double() @ w.double().t() + b.double()
+    with torch.no_grad():
+        plain = ops.linear(x, w, b)
+    recorded = ops.linear(x, w.clone().requires_grad_(), b)
+    assert torch.equal(plain, recorded)
+    # one rounding of an fp32 sum to bf16
+    assert float((plain.double() - truth).norm() / truth.norm()) < 3e-3
+    assert torch.equal(ops.linear(x, w), ops.gemm(x, w, out=torch.empty(M, N, device="cuda", dtype=torch.bfloat16)))

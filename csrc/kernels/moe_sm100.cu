@@ -336,6 +336,37 @@ moe_pull_kernel(Peers src, const float* __restrict__ w, const int* __restrict__ 
   if (world > 1) last_block_signals(counter, flags, slot_pulled, rank, world, seq);
 }
 
+// The gradient of a pair's routing weight: <dy of its token, its row>.  One warp a pair; bound by reading the rows once.
+__global__ void __launch_bounds__(256)
+moe_pair_dots_kernel(const bf16* __restrict__ gathered, const bf16* __restrict__ dy, float* __restrict__ out, int pairs, int k, int d) {
+  const int lane = threadIdx.x & 31, p = (blockIdx.x * 256 + threadIdx.x) >> 5;
+  if (p >= pairs) return;
+  const uint4* a = reinterpret_cast<const uint4*>(gathered + static_cast<long long>(p) * d);
+  const uint4* b = reinterpret_cast<const uint4*>(dy + static_cast<long long>(p / k) * d);
+  float s0 = 0.f, s1 = 0.f;
+#pragma unroll 4
+  for (int i = lane; i < d / 8; i += 32) {
+    float x[8], y[8];
+    unpack8(a[i], x);
+    unpack8(b[i], y);
+#pragma unroll
+    for (int c = 0; c < 8; c += 2) { s0 = fmaf(x[c], y[c], s0); s1 = fmaf(x[c + 1], y[c + 1], s1); }
+  }
+  s0 = warp_sum(s0 + s1);
+  if (lane == 0) out[p] = s0;
+}
+
+// Zeroes the rows between an expert's last one and the next expert's first: at most 127 each, a warp a row.
+__global__ void __launch_bounds__(256)
+moe_zero_pads_kernel(bf16* __restrict__ rows, const int* __restrict__ offsets, const int* __restrict__ counts, int rows_cap, int d, const int* __restrict__ err) {
+  if (status_poisoned(err)) return;
+  const int e = blockIdx.x, lane = threadIdx.x & 31, end = min(offsets[e + 1], rows_cap);
+  for (int r = offsets[e] + counts[e] + static_cast<int>(blockIdx.y * 8 + (threadIdx.x >> 5)); r < end; r += gridDim.y * 8) {
+    if (r < 0) return;
+    for (int i = lane; i < d / 8; i += 32) reinterpret_cast<uint4*>(rows + static_cast<long long>(r) * d)[i] = make_uint4(0u, 0u, 0u, 0u);
+  }
+}
+
 static inline int warp_grid(int T) {
   long long b = (static_cast<long long>(T) * 32 + 255) / 256;
   if (b < 1) b = 1;
@@ -412,5 +443,22 @@ extern "C" int dewb_moe_pull(const unsigned long long* src_ptrs, const float* w,
       make_peers(src_ptrs, world), w, dest_rank, dest_pos, reinterpret_cast<bf16*>(out), reinterpret_cast<bf16*>(gathered),
       make_peers(flag_ptrs, world), reinterpret_cast<const uint32_t*>(my_flags), slot_ready, slot_pulled, seq, limit_ns,
       counter, T, d, k, rank, world, err);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// gathered [pairs, d] bf16, dy [pairs / k, d] bf16 -> out [pairs] fp32: their dot products, pair p with row p / k.
+extern "C" int dewb_moe_pair_dots(const void* gathered, const void* dy, float* out, int pairs, int k, int d, void* stream) {
+  if (d % 8 != 0 || k <= 0 || ((reinterpret_cast<uintptr_t>(gathered) | reinterpret_cast<uintptr_t>(dy)) & 15)) return -3;
+  if (pairs <= 0) return 0;
+  moe_pair_dots_kernel<<<(pairs + 7) / 8, 256, 0, STREAM(stream)>>>(reinterpret_cast<const bf16*>(gathered), reinterpret_cast<const bf16*>(dy), out, pairs, k, d);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// rows [rows_cap, d] bf16 of `experts` groups (offsets [experts + 1], counts [experts], as dewb_moe_plan writes them): zeros behind each group's last row.  Does
+// nothing once the status word says that an earlier kernel gave up (the plan was not written then).
+extern "C" int dewb_moe_zero_pads(void* rows, const int* offsets, const int* counts, int experts, int rows_cap, int d, const int* err, void* stream) {
+  if (d % 8 != 0 || (reinterpret_cast<uintptr_t>(rows) & 15)) return -3;
+  if (experts <= 0) return 0;
+  moe_zero_pads_kernel<<<dim3(experts, 4), 256, 0, STREAM(stream)>>>(reinterpret_cast<bf16*>(rows), offsets, counts, rows_cap, d, err);
   return static_cast<int>(cudaGetLastError());
 }

@@ -73,6 +73,20 @@ def quantize_mx(x: torch.Tensor, sf_rows: Optional[int] = None) -> Tuple[torch.T
     return q, packed.view(torch.int32).reshape(K // 128, sf_rows)
 
 
+def quantize_mx_t(x: torch.Tensor, sf_rows: int) -> Tuple[torch.Tensor, torch.Tensor]:
+    """``x [G, N, K]`` bf16 (N a multiple of 128) -> ``quantize_mx`` of its transpose ``[G * K, N]``, without the transpose in memory where the kernel takes the
+    sizes (whole tiles of 64 columns, contiguous)."""
+    G_, N, K = x.shape
+    if (L.use_cuda(x) and x.dtype == torch.bfloat16 and N % 128 == 0 and K % 64 == 0 and G_ < 65536 and x.is_contiguous() and x.data_ptr() % 16 == 0
+            and hasattr(L.load(), "dewb_quantize_mx_t")):
+        q = torch.empty((G_ * K, N), dtype=torch.float8_e4m3fn, device=x.device)
+        sf = torch.zeros((N // 128, sf_rows), dtype=torch.int32, device=x.device)
+        L.check(L.load().dewb_quantize_mx_t(L.ptr(x), L.ptr(q), L.ptr(sf), c_int(G_), c_int(N), c_int(K), c_ll(sf_rows), L.stream_ptr()), "quantize_mx_t")
+        L.count_launches()
+        return q, sf
+    return quantize_mx(x.transpose(1, 2).contiguous().reshape(G_ * K, N), sf_rows=sf_rows)
+
+
 def gemm_mx(aq, sfa, bq, sfb, tile_group: Optional[torch.Tensor] = None, groups: int = 1, out: Optional[torch.Tensor] = None,
             zero_skipped: bool = True) -> torch.Tensor:
     """``[M, K] x [groups * N, K]^T -> [M, N]`` bf16.  With ``tile_group`` the rows of ``aq`` are expert-sorted and each 128-row
@@ -142,7 +156,7 @@ def _quantized_weight(w: torch.Tensor, transposed: bool, ident: int = 0):
         if hit is not None and hit[0] == stamp:
             return hit[1], hit[2]
     if transposed:
-        q, sc = quantize_mx(w.transpose(1, 2).contiguous().reshape(G_ * K, N), sf_rows=_pad128(G_ * K + TILE_N))
+        q, sc = quantize_mx_t(w, _pad128(G_ * K + TILE_N))
     else:
         q, sc = quantize_mx(w.reshape(G_ * N, K), sf_rows=_pad128(G_ * N + TILE_N))
     if _CACHE_ON[0]:

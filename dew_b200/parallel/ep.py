@@ -115,9 +115,8 @@ class TokenExchange:
         self.rows_cap, self.features = need, features
         make = (lambda n, dt: _LocalBuffer(n, dt, device)) if self.world == 1 else \
             (lambda n, dt: SymmetricBuffer(n, dt, device, self.group, zero=True))
-        # (one row more than the plan addresses: the target of the padding-zeroing writes that have nothing to zero)
-        self.recv, self.out = make((need + 1) * features, torch.bfloat16), make(need * features, torch.bfloat16)
-        self.recv_back = make((need + 1) * features, torch.bfloat16) if self.lean else None
+        self.recv, self.out = make(need * features, torch.bfloat16), make(need * features, torch.bfloat16)
+        self.recv_back = make(need * features, torch.bfloat16) if self.lean else None
         if self.counts is None:
             self.counts, self.flags = make(max(64, self.experts), torch.int32), make(64, torch.int32)
             self.counter = torch.zeros(4, dtype=torch.int32, device=device)
@@ -160,12 +159,6 @@ class TokenExchange:
         L.count_launches(2)
         layout = G.GroupLayout(None, local_counts, offsets, tile_group, self.rows_cap)
         plan = ExchangePlan(dest_rank, dest_pos, layout, info, T, k)
-        if self.lean:
-            # rows [offset + count, next offset) of every local expert: the (at most 127) alignment rows nobody pushes; a fixed-size
-            # index (entries with nothing to zero point at the spare row) keeps this free of data-dependent shapes
-            j = torch.arange(127, device=dev, dtype=torch.int64)[None, :]
-            first = (offsets[:-1] + local_counts).long()[:, None] + j
-            plan.pad_rows = torch.where(first < offsets[1:].long()[:, None], first, self.rows_cap).reshape(-1)
         return plan
 
     def push(self, x: torch.Tensor, plan: ExchangePlan, pair_scale: Optional[torch.Tensor] = None, backward: bool = False) -> torch.Tensor:
@@ -189,7 +182,10 @@ class TokenExchange:
         self._wait(self.SLOT_PUSHED, self.seq)
         if not self.lean:
             return buf.tensor[: self.rows_cap * d].view(self.rows_cap, d).clone()
-        buf.tensor.view(self.rows_cap + 1, d).index_fill_(0, plan.pad_rows, 0)
+        # the (at most 127) rows behind each expert's last one, which nobody pushes
+        L.check(L.load().dewb_moe_zero_pads(L.ptr(buf.tensor), L.ptr(plan.layout.offsets), L.ptr(plan.layout.counts), ctypes.c_int(self.per), ctypes.c_int(self.rows_cap),
+                                            ctypes.c_int(d), L.ptr(L.status(x.device)), L.stream_ptr()), "moe_zero_pads")
+        L.count_launches()
         # a tensor of its own over the buffer's memory, not a view: autograd saves it for the weight gradient, and the buffer's next
         # use (the following microbatch's push, after this microbatch's backward) must not read as an in-place change of a saved view
         base = buf.tensor
@@ -263,7 +259,16 @@ class _PullRows(torch.autograd.Function):
         d_rows = ctx.exchange.push(dy, plan, pair_scale=weights.reshape(-1), backward=True)
         dw = None
         if gathered is not None:
-            dw = (gathered.view(plan.tokens, plan.top_k, -1).float() * dy.float().unsqueeze(1)).sum(-1).to(weights.dtype)
+            if plan.top_k == 1:
+                # a token's only weight, where the weights are normalised, is 1 whatever its score: what reaches the router is the rounding of this sum alone, and
+                # stays what PyTorch's order of summation makes of it
+                dw = (gathered.view(plan.tokens, 1, -1).float() * dy.float().unsqueeze(1)).sum(-1)
+            else:
+                dw = torch.empty(plan.tokens, plan.top_k, dtype=torch.float32, device=dy.device)
+                L.check(L.load().dewb_moe_pair_dots(L.ptr(gathered), L.ptr(dy), L.ptr(dw), ctypes.c_int(dw.numel()), ctypes.c_int(plan.top_k), ctypes.c_int(dy.shape[1]),
+                                                    L.stream_ptr()), "moe_pair_dots")
+                L.count_launches()
+            dw = dw.to(weights.dtype)
         return d_rows, dw, None, None
 
 

@@ -66,8 +66,24 @@ _GEMM.kernels = [
         Requirement("inner", lambda c: c["inner_contig"], "the contiguous dimension must have stride 1"),
     ], receipt="tcgen05 weight-streaming kernel, K split over a thread-block cluster and summed through distributed shared "
                "memory, csrc/kernels/gemm_skinny_sm100.cu"),
+    Kernel("sm100_rows", [
+        Requirement("built", lambda c: hasattr(L.load(), "dewb_gemm_rows_bf16"), "the few-row kernel is not in this build of libdewb.so"),
+        Requirement("rows", lambda c: c["M"] <= 4, "at most four rows"),
+        Requirement("plain", lambda c: c.get("k_major", False), "K-major operands, fresh bf16 output, alpha = 1"),
+        Requirement("dtype", lambda c: c["dtype"] == torch.bfloat16, "operands must be bf16"),
+        Requirement("ld", lambda c: c["lda"] % 8 == 0 and c["ldb"] % 8 == 0 and c["K"] % 8 == 0, "row strides and K must be multiples of 8 elements"),
+        Requirement("align", lambda c: c["aligned"], "base pointers must be 16-byte aligned"),
+        Requirement("inner", lambda c: c["inner_contig"], "the contiguous dimension must have stride 1"),
+    ], receipt="few rows against streamed weights on the CUDA cores, csrc/kernels/gemm_rows.cu"),
     Kernel("cublas", [], receipt="library arm (torch.matmul)"),
 ]
+
+
+def _few_rows(M: int, N: int, K: int) -> bool:
+    """Where the few-row kernel is ahead of the library's (microseconds inside a graph, weights not in cache: one row by 2048 x 1024 3.1 against 4.9, 1024 x 2816
+    6.7 against 9.0, 5632 x 1024 4.7 against 5.1, 6144 x 4096 12.3 against 11.2; four rows by 2048 x 1024 4.3 against 4.5, 1024 x 2816 8.6 against 8.0): the weights
+    arrive in a few microseconds, and at three or four rows in half of those, beyond which the products of the CUDA cores show."""
+    return 1 <= M <= 4 and N * K <= (6 << 20 if M <= 2 else 2 << 20)
 
 
 def _skinny_built() -> bool:
@@ -141,6 +157,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     if (fresh and cell is not None and kernel is None and _GEMM.declared.get(cell) == "cublas" and alpha == 1.0 and a.dtype == b.dtype == kind
             and not _GEMM.forced_by_environment() and not (torch.is_grad_enabled() and (a.requires_grad or b.requires_grad))):
         # a small product that its measured cell sends to the library arm: nothing about it needs looking up
+        if (_few_rows(M, N, K) and not a_mn and not b_mn and kind == torch.bfloat16 and K % 8 == 0 and a.stride(1) == b.stride(1) == 1 and a.stride(0) % 8 == 0
+                and b.stride(0) % 8 == 0 and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0 and N > 0 and _rows_built()):
+            return _gemm_rows(a, b, bias)
         _GEMM._record("cublas", {}, None, cell)
         A, Bt = a.t() if a_mn else a, b if b_mn else b.t()
         return torch.mm(A, Bt) if bias is None else torch.addmm(bias.to(kind), A, Bt)
@@ -149,7 +168,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         accumulate = False
     case = dict(dtype=a.dtype if a.dtype == b.dtype else None, lda=a.stride(0), ldb=b.stride(0), ldd=out.stride(0),
                 aligned=(a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0),
-                inner_contig=(a.stride(1) == 1 and b.stride(1) == 1 and out.stride(1) == 1), M=M, N=N, K=K, plain=plain)
+                inner_contig=(a.stride(1) == 1 and b.stride(1) == 1 and out.stride(1) == 1), M=M, N=N, K=K, plain=plain, k_major=plain and fresh)
     if bias is not None:
         case["plain"] = False                                    # (the weight-streaming kernel has no bias epilogue)
     if kernel is None and cell is None and tiles >= 148 and _pair_built() and all(case[x] % 8 == 0 for x in ("lda", "ldb", "ldd")) and case["aligned"]:
@@ -164,6 +183,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         else:
             kernel = first
     which = _GEMM.select(case, forced=kernel, cell=cell)
+    if which == "sm100_rows":
+        return _gemm_rows(a, b, bias)
     if which == "cublas":
         r = _gemm_reference_cuda(a, b, a_mn, b_mn, alpha, out, accumulate)
         return r if bias is None else r.add_(bias.to(r.dtype))
@@ -191,6 +212,22 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             c_ll(b.stride(0)), c_ll(out.stride(0)), c_int(int(a_mn)), c_int(int(b_mn)), c_int(epi),
             c_float(alpha), L.ptr(L.status(a.device)), c_int(max_ctas), L.stream_ptr())
     L.check(rc, which)
+    L.count_launches()
+    return out
+
+
+def _rows_built() -> bool:
+    return hasattr(L.load(), "dewb_gemm_rows_bf16")
+
+
+def _gemm_rows(a, b, bias):
+    M, N, K = a.shape[0], b.shape[0], a.shape[1]
+    _GEMM._record("sm100_rows", {}, None, None)
+    out = torch.empty((M, N), dtype=torch.bfloat16, device=a.device)
+    bb = None if bias is None else bias.to(torch.bfloat16).contiguous()
+    rc = L.load().dewb_gemm_rows_bf16(a.data_ptr(), b.data_ptr(), 0 if bb is None else bb.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), N, L.stream())
+    if rc:
+        L.check(rc, "sm100_rows")
     L.count_launches()
     return out
 

@@ -58,6 +58,8 @@ def load(build_if_missing: bool = False) -> ctypes.CDLL:
 # as they are; the others are given ctypes objects by their callers.
 _SIGNATURES = {
     "dewb_rmsnorm_fwd": "pppppp" + "lifi" + "p",
+    "dewb_ada_fwd": "ppppp" + "l" + "ppp" + "lii" + "f" + "p",
+    "dewb_gemm_rows_bf16": "pppp" + "iii" + "lll" + "p",
     "dewb_swiglu_fwd": "ppp" + "lil" + "p",
     "dewb_rope": "pppp" + "liiiif" + "p",
     "dewb_rope_append": "pppp" + "iiiii" + "ppp" + "ii" + "p",

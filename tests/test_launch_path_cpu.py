@@ -31,7 +31,9 @@ def test_environment_is_read_as_it_is_now(monkeypatch):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (5, 40, 24), (128, 256, 64)])
+# one to four rows take the few-row kernel up to its line (2 and 6 M weights), K's pieces short of and past its unrolled steps
+@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (1, 1, 264), (2, 37, 1032), (3, 2400, 256), (4, 4096, 512), (4, 4104, 512), (1, 6144, 1024), (2, 6152, 1024), (5, 40, 24),
+                                   (128, 256, 64)])
 def test_small_products_with_and_without_a_node(M, N, K):
     from dew_b200 import ops
     g = torch.Generator(device="cuda").manual_seed(M)
@@ -41,6 +43,9 @@ def test_small_products_with_and_without_a_node(M, N, K):
         plain = ops.linear(x, w, b)
     recorded = ops.linear(x, w.clone().requires_grad_(), b)
     assert torch.equal(plain, recorded)
-    # one rounding of an fp32 sum to bf16
-    assert float((plain.double() - truth).norm() / truth.norm()) < 3e-3
-    assert torch.equal(ops.linear(x, w), ops.gemm(x, w, out=torch.empty(M, N, device="cuda", dtype=torch.bfloat16)))
+    # one rounding of an fp32 sum to bf16: half a unit of eight bits at the most, where a single value is the whole result
+    assert float((plain.double() - truth).norm() / truth.norm()) < 2.0 ** -8
+    want = x.double() @ w.double().t()
+    wide = torch.randn(M, K + 16, generator=g, device="cuda").bfloat16()[:, 8:K + 8]          # rows of a wider tensor
+    for a, t in ((x, want), (wide, wide.double() @ w.double().t())):
+        assert float((ops.gemm(a, w).double() - t).norm() / t.norm()) < 2.0 ** -8

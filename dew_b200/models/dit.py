@@ -12,7 +12,8 @@ from typing import Any, Mapping, Optional, Sequence
 import torch
 import torch.nn as nn
 
-from ..nn.dit import ConditioningEmbed, ModulatedBlock, PatchEmbedding, PatchSequenceOutput, sincos_2d
+from ..nn.dit import ConditioningEmbed, ModulatedBlock, PatchEmbedding, PatchSequenceOutput
+from ..ops.ada import sincos_grid
 from ..utils.registry import register
 
 
@@ -39,7 +40,7 @@ class SimpleDiT(nn.Module):
         gh, gw = H // self.patch_size, W // self.patch_size
         dt = self.embed.proj.weight.dtype
         tokens = self.embed(x.to(dt))
-        tokens = tokens + sincos_2d(gh, gw, self.emb_features, tokens.device).to(dt)[None]
+        tokens = tokens + sincos_grid(gh, gw, self.emb_features, tokens.device, dt)[None]
         c = self.conditioning(temb, conditions.get("text"), conditions.get("label"), duration, conditions.get("guidance"))
         routed = None
         for i, block in enumerate(self.blocks):

@@ -104,10 +104,12 @@ class SelfAttention(nn.Module):
             best = torch.maximum(best, s.amax((0, 3, 4)).reshape(H))
         self.qk_max = best if self.qk_max is None else torch.maximum(self.qk_max, best)
 
-    def project(self, x, cos=None, sin=None, positions=None):
+    def project(self, x, cos=None, sin=None, positions=None, qkv=None):
+        """``qkv``: the packed projection, where the caller has it already."""
         B, S, _ = x.shape
         H, Hkv, D = self.num_heads, self.num_kv_heads, self.head_dim
-        qkv = self.qkv_proj(x).view(B, S, H + 2 * Hkv, D)
+        if qkv is None:
+            qkv = self.qkv_proj(x).view(B, S, H + 2 * Hkv, D)
         if self.q_norm is not None and self.qk_norm_full:
             q = self.q_norm(qkv[:, :, :H].reshape(B, S, H * D)).view(B, S, H, D)
             k = self.k_norm(qkv[:, :, H:H + Hkv].reshape(B, S, Hkv * D)).view(B, S, Hkv, D)
@@ -163,22 +165,25 @@ class SelfAttention(nn.Module):
                 or self.weighting != "softmax" or self.head_temperature is not None:
             return self._general(x, positions, segment_ids, cache, layer)
         cos, sin = self._tables(cos, sin)
-        if (cache is None and x.is_cuda and cos is not None and self.head_transform is None and self.gate_proj is None and self.q_norm is None and self.window is None and not self.softcap
+        qkv = None
+        if (cache is None and x.is_cuda and self.head_transform is None and self.gate_proj is None and self.q_norm is None and self.window is None and not self.softcap
                 and self.sinks is None and segment_ids is None and not self.track_qk_max and self.q_gain is None):
             from ..ops.attn import packed_attention
             H, Hkv, D = self.num_heads, self.num_kv_heads, self.head_dim
-            o = packed_attention(self.qkv_proj(x).view(B, S, H + 2 * Hkv, D), cos, sin, positions, H, Hkv, self.causal)
+            qkv = self.qkv_proj(x).view(B, S, H + 2 * Hkv, D)
+            o = packed_attention(qkv, cos, sin, positions, H, Hkv, self.causal)
             if o is not None:
                 return self.o_proj(o.reshape(B, S, H * D))
         if (cache is not None and S == 1 and self.q_norm is None and self.q_gain is None and positions is not None and cos is not None
                 and self.head_transform is None and self.gate_proj is None and hasattr(cache, "decode_packed")):
             # decode step: rotation, cache append and attention straight from the packed projection (no slices, no copies)
             H, Hkv, D = self.num_heads, self.num_kv_heads, self.head_dim
-            qkv = self.qkv_proj(x).view(B, H + 2 * Hkv, D)
-            if cache.can_decode_packed(qkv, H, self.softcap):
-                o = cache.decode_packed(layer, qkv, cos, sin, positions.reshape(-1), H, window=self.window, sinks=self.sinks)
+            qkv = self.qkv_proj(x).view(B, S, H + 2 * Hkv, D)
+            heads = qkv.view(B, H + 2 * Hkv, D)
+            if cache.can_decode_packed(heads, H, self.softcap):
+                o = cache.decode_packed(layer, heads, cos, sin, positions.reshape(-1), H, window=self.window, sinks=self.sinks)
                 return self.o_proj(o.reshape(B, 1, H * D))
-        q, k, v = self.project(x, cos, sin, positions)
+        q, k, v = self.project(x, cos, sin, positions, qkv)
         if self.track_qk_max and cache is None and self.training:
             self._record_qk_max(q, k)
         if cache is None and hasattr(segment_ids, "visible"):

@@ -13,7 +13,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from .. import ops
+from ..ops import ada
 from .attention import SelfAttention
 from .layers import LayerNorm, Linear, sinusoidal
 from .mlp import GeluMLP
@@ -82,8 +82,13 @@ class ConditioningEmbed(nn.Module):
         return c
 
 
-def modulate(x, shift, scale):
-    return x * (1 + scale.unsqueeze(1)) + shift.unsqueeze(1)
+modulate = ada.modulate
+
+
+def _bare(norm: nn.Module) -> bool:
+    """Whether calling ``norm`` is the layer norm without weights and nothing else, so that it may run inside the kernel of what surrounds it."""
+    return type(norm) is LayerNorm and norm.weight is None and norm.bias is None and not (norm._forward_hooks or norm._forward_pre_hooks or norm._backward_hooks
+                                                                                         or norm._backward_pre_hooks)
 
 
 class ModulatedBlock(nn.Module):
@@ -101,9 +106,12 @@ class ModulatedBlock(nn.Module):
     def forward(self, x, c):
         m = self.ada_proj(F.silu(c) if self.adaln_silu else c)
         s1, sc1, g1, s2, sc2, g2 = m.chunk(6, -1)
-        x = x + g1.unsqueeze(1) * self.attn(modulate(self.norm1(x), s1, sc1))
-        x = x + g2.unsqueeze(1) * self.mlp(modulate(self.norm2(x), s2, sc2))
-        return x
+        if not (_bare(self.norm1) and _bare(self.norm2)):
+            x = x + g1.unsqueeze(1) * self.attn(modulate(self.norm1(x), s1, sc1))
+            return x + g2.unsqueeze(1) * self.mlp(modulate(self.norm2(x), s2, sc2))
+        a = self.attn(ada.ada_norm(x, s1, sc1, self.norm1.eps))
+        y, x = ada.gated_ada_norm(x, a, g1, s2, sc2, self.norm2.eps)
+        return ada.gated_add(x, self.mlp(y), g2)
 
 
 class PatchSequenceOutput(nn.Module):
@@ -118,7 +126,7 @@ class PatchSequenceOutput(nn.Module):
 
     def forward(self, x, c, grid):
         shift, scale = self.ada_proj(F.silu(c)).chunk(2, -1)
-        x = self.out(modulate(self.norm(x), shift, scale)).float()
+        x = self.out(ada.ada_norm(x, shift, scale, self.norm.eps) if _bare(self.norm) else modulate(self.norm(x), shift, scale)).float()
         B = x.shape[0]
         gh, gw = grid
         p, C = self.patch_size, self.out_channels

@@ -1,0 +1,129 @@
+"""Modulated layer norms and gated residuals of diffusion transformers (``csrc/kernels/ada_norm.cu``), and the fixed position table of a patch grid.
+
+``h = x + gate * branch`` and ``y = norm(h) * (1 + scale) + shift`` over tokens ``[B, n, d]`` with one shift, scale and gate ``[B, d]`` per image: one kernel each
+way on a GPU in bf16, the plain expressions elsewhere.  Parity: ``modulate`` and the gated residuals of src/dew/nn/dit.py:572-727.
+"""
+from __future__ import annotations
+
+import ctypes
+from typing import Optional, Tuple
+
+import torch
+import torch.nn.functional as F
+
+from . import library as L
+
+c_ll, c_int = ctypes.c_longlong, ctypes.c_int
+MAX_WIDTH = 2048
+
+
+def modulate(x, shift, scale):
+    return x * (1 + scale.unsqueeze(1)) + shift.unsqueeze(1)
+
+
+def _usable(x: torch.Tensor, branch: Optional[torch.Tensor], *mods: torch.Tensor) -> bool:
+    """Rows of one width in whole 16-byte pieces, and per image one row of every modulation, all at one stride (slices of one projection)."""
+    if not (x.dim() == 3 and x.dtype == torch.bfloat16 and L.use_cuda(x) and hasattr(L.load(), "dewb_ada_fwd")):
+        return False
+    B, n, d = x.shape
+    if d % 8 or d > MAX_WIDTH or not 0 < B < 65536 or n == 0 or (branch is not None and (branch.shape != x.shape or branch.dtype != x.dtype or branch.device != x.device)):
+        return False
+    stride = mods[0].stride(0)
+    return stride % 8 == 0 and all(m.shape == (B, d) and m.dtype == x.dtype and m.device == x.device and m.stride(1) == 1 and m.stride(0) == stride
+                                   and m.data_ptr() % 16 == 0 for m in mods)
+
+
+def _rows(t: torch.Tensor) -> torch.Tensor:
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+def _forward(x, branch, gate, shift, scale, eps):
+    """-> y, h, stats (None where there is no norm; h is x where there is no branch)."""
+    B, n, d = x.shape
+    norm = shift is not None
+    h = x if branch is None else torch.empty_like(x)
+    y = torch.empty_like(x) if norm else None
+    stats = torch.empty(B * n, 2, dtype=torch.float32, device=x.device) if norm else None
+    at = lambda t: 0 if t is None else t.data_ptr()
+    L.check(L.load().dewb_ada_fwd(at(x), at(branch), at(shift), at(scale), at(gate), (gate if shift is None else shift).stride(0), 0 if branch is None else at(h), at(y), at(stats),
+                                  B * n, n, d, eps, L.stream()), "ada_fwd")
+    L.count_launches()
+    return y, h, stats
+
+
+class _Ada(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, branch, gate, shift, scale, eps):
+        ctx.set_materialize_grads(False)
+        y, h, stats = _forward(x, branch, gate, shift, scale, eps)
+        ctx.save_for_backward(h, branch, gate, scale, stats)
+        if branch is None:
+            return y
+        return h if shift is None else (y, h)
+
+    @staticmethod
+    def backward(ctx, *grads):
+        h, branch, gate, scale, stats = ctx.saved_tensors
+        norm = scale is not None
+        dy, dh = (grads[0], None) if branch is None else (None, grads[0]) if not norm else grads
+        if norm and dy is None:
+            dy = torch.zeros_like(h)
+        dy, dh = (None if t is None else _rows(t.to(h.dtype)) for t in (dy, dh))
+        B, n, d = h.shape
+        lib = L.load()
+        slab = lib.dewb_ada_slab(c_int(B), c_int(n))
+        sets = 2 * norm + (branch is not None)
+        L.ensure_device(h)
+        part = torch.empty(B, -(-n // slab), sets, d, dtype=torch.float32, device=h.device)
+        dmod = torch.empty(B, sets, d, dtype=h.dtype, device=h.device)
+        dx = torch.empty_like(h) if norm else dh
+        dbranch = None if branch is None else torch.empty_like(h)
+        L.check(lib.dewb_ada_bwd(L.ptr(dy), L.ptr(dh), L.ptr(h), L.ptr(branch), L.ptr(scale), L.ptr(gate), c_ll((gate if scale is None else scale).stride(0)), L.ptr(stats), L.ptr(dx),
+                                 L.ptr(dbranch), L.ptr(part), L.ptr(dmod), c_int(B), c_int(n), c_int(d), c_int(slab), L.stream_ptr()), "ada_bwd")
+        L.count_launches(2)
+        return dx, dbranch, None if branch is None else dmod[:, 2 * norm], dmod[:, 0] if norm else None, dmod[:, 1] if norm else None, None
+
+
+def _run(x, branch, gate, shift, scale, eps):
+    x, branch = _rows(x), None if branch is None else _rows(branch)
+    if L.unrecorded(x, branch, gate, shift, scale):
+        y, h, _ = _forward(x, branch, gate, shift, scale, eps)
+        return y if branch is None else h if shift is None else (y, h)
+    return _Ada.apply(x, branch, gate, shift, scale, eps)
+
+
+def ada_norm(x: torch.Tensor, shift: torch.Tensor, scale: torch.Tensor, eps: float = 1e-6) -> torch.Tensor:
+    """``norm(x) * (1 + scale) + shift`` with the layer norm without weights."""
+    if _usable(x, None, shift, scale):
+        return _run(x, None, None, shift, scale, eps)
+    return modulate(F.layer_norm(x, (x.shape[-1],), None, None, eps), shift, scale)
+
+
+def gated_ada_norm(x: torch.Tensor, branch: torch.Tensor, gate: torch.Tensor, shift: torch.Tensor, scale: torch.Tensor, eps: float = 1e-6) -> Tuple[torch.Tensor, torch.Tensor]:
+    """``h = x + gate * branch``; -> (``norm(h) * (1 + scale) + shift``, ``h``)."""
+    if _usable(x, branch, shift, scale, gate):
+        return _run(x, branch, gate, shift, scale, eps)
+    h = x + gate.unsqueeze(1) * branch
+    return modulate(F.layer_norm(h, (h.shape[-1],), None, None, eps), shift, scale), h
+
+
+def gated_add(x: torch.Tensor, branch: torch.Tensor, gate: torch.Tensor) -> torch.Tensor:
+    """``x + gate * branch``."""
+    if _usable(x, branch, gate):
+        return _run(x, branch, gate, None, None, 0.0)
+    return x + gate.unsqueeze(1) * branch
+
+
+def sincos_grid(h: int, w: int, dim: int, device, dtype) -> torch.Tensor:
+    """``[h * w, dim]``: the fixed 2-D sine-cosine signal of ``nn.dit.sincos_2d``, made by one kernel where a GPU wants it in bf16."""
+    from ..nn.dit import sincos_2d
+    device = torch.device(device)
+    if device.type == "cuda" and dtype == torch.bfloat16 and dim % 4 == 0 and h > 0 and w > 0 and h * w * dim < 1 << 31 and L.env("DEWB_FORCE_REFERENCE") != "1" \
+            and hasattr(L.load(), "dewb_sincos_grid"):
+        out = torch.empty(h * w, dim, dtype=dtype, device=device)
+        L.ensure_device(out)
+        L.check(L.load().dewb_sincos_grid(L.ptr(out), c_int(h), c_int(w), c_int(dim), L.stream_ptr()), "sincos_grid")
+        L.count_launches()
+        return out
+    return sincos_2d(h, w, dim, device).to(dtype)

@@ -29,7 +29,7 @@ NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--use_fast_math", "-Xcompiler",
 EXACT_MATH = ("residual_streams", "paged_attention", "latent_attention", "decayed_recurrence", "gated_recurrence", "gated_chunks", "token_mix", "moe_serve")
 
 # The same for kernels of training, which a program that only decodes does not build: gradients that are kept in fp32.
-EXACT_TRAINING = ("ssd_sm100",)
+EXACT_TRAINING = ("ssd_sm100", "ada_norm")
 
 # Subsets of the library a program can build alone, as ``libdewb_<part>.so``: a process that only decodes needs neither the training nor
 # the multi-GPU kernels.

@@ -125,6 +125,22 @@ def flash_sm100(q, k, v, causal: bool, scale: float, window=None, softcap: float
     return flash_fwd(q, k, v, causal, scale, need_lse=False, var=var)[0]
 
 
+def _packed(qkv, cos, sin, positions, Hq: int, Hkv: int, causal: bool, scale: float, need_lse: bool):
+    """Rotates ``qkv`` in place (not where ``cos`` is None) and attends; -> out, lse, the positions the rotation took."""
+    B, S, H, D = qkv.shape
+    pos = None
+    if cos is not None:
+        if positions is not None:
+            pos = positions.reshape(-1).to(torch.int32).contiguous()
+        elif B > 1:
+            pos = torch.arange(S, device=qkv.device, dtype=torch.int32).repeat(B)
+        L.check(L.load().dewb_rope(L.ptr(qkv), L.ptr(cos), L.ptr(sin), L.ptr(pos), c_ll(B * S), c_int(H), c_int(Hq + Hkv),
+                                   c_int(D), c_int(cos.shape[0]), c_float(1.0), L.stream_ptr()), "rope")
+        L.count_launches()      # written through the raw pointer: autograd neither sees nor needs to see the change
+    out, lse = flash_fwd(qkv[:, :, :Hq], qkv[:, :, Hq:Hq + Hkv], qkv[:, :, Hq + Hkv:], causal, scale, need_lse)
+    return out, lse, pos
+
+
 class _PackedRopeFlash(torch.autograd.Function):
     """RoPE + flash attention over one packed projection ``qkv [B, S, Hq + 2 Hkv, D]``.
 
@@ -134,18 +150,7 @@ class _PackedRopeFlash(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, qkv, cos, sin, positions, Hq, Hkv, causal, scale):
-        B, S, H, D = qkv.shape
-        pos = None
-        if cos is not None:
-            if positions is not None:
-                pos = positions.reshape(-1).to(torch.int32).contiguous()
-            elif B > 1:
-                pos = torch.arange(S, device=qkv.device, dtype=torch.int32).repeat(B)
-            L.check(L.load().dewb_rope(L.ptr(qkv), L.ptr(cos), L.ptr(sin), L.ptr(pos), c_ll(B * S), c_int(H), c_int(Hq + Hkv),
-                                       c_int(D), c_int(cos.shape[0]), c_float(1.0), L.stream_ptr()), "rope")
-            L.count_launches()      # written through the raw pointer: autograd neither sees nor needs to see the change
-        q, k, v = qkv[:, :, :Hq], qkv[:, :, Hq:Hq + Hkv], qkv[:, :, Hq + Hkv:]
-        out, lse = flash_fwd(q, k, v, causal, scale)
+        out, lse, pos = _packed(qkv, cos, sin, positions, Hq, Hkv, causal, scale, True)
         ctx.save_for_backward(qkv, out, lse, cos, sin, pos)
         ctx.meta = (Hq, Hkv, causal, scale)
         return out
@@ -167,4 +172,6 @@ class _PackedRopeFlash(torch.autograd.Function):
 
 def packed_rope_flash(qkv, cos, sin, positions, Hq: int, Hkv: int, causal: bool, scale: float):
     """``qkv`` must be a fresh contiguous bf16 tensor nobody else reads: it is rotated in place."""
+    if L.unrecorded(qkv):
+        return _packed(qkv, cos, sin, positions, Hq, Hkv, causal, scale, False)[0]
     return _PackedRopeFlash.apply(qkv, cos, sin, positions, Hq, Hkv, causal, scale)

@@ -352,6 +352,26 @@ __device__ __forceinline__ float fast_exp2(float x) {
 __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
 
+// v[i] = alpha * v[i] + bias[i] for 32 neighbouring output columns, of which `cols` exist; the bias row comes in 16-byte pieces where it starts on such a boundary
+__device__ __forceinline__ void scale_and_bias(uint32_t (&v)[32], float alpha, const __nv_bfloat16* __restrict__ bias, int cols) {
+  if (cols >= 32 && (reinterpret_cast<uintptr_t>(bias) & 15) == 0) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint4 b = reinterpret_cast<const uint4*>(bias)[j];
+      const uint32_t w[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        v[j * 8 + 2 * i] = __float_as_uint(fmaf(alpha, __uint_as_float(v[j * 8 + 2 * i]), bf16_lo(w[i])));
+        v[j * 8 + 2 * i + 1] = __float_as_uint(fmaf(alpha, __uint_as_float(v[j * 8 + 2 * i + 1]), bf16_hi(w[i])));
+      }
+    }
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < 32; ++i)
+    if (i < cols) v[i] = __float_as_uint(fmaf(alpha, __uint_as_float(v[i]), __bfloat162float(bias[i])));
+}
+
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

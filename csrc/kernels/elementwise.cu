@@ -529,15 +529,63 @@ rmsnorm_dw_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const
   }
 }
 
-// out[col] (+)= sum_r partial[r, col]; one thread per column, coalesced over columns
-__global__ void colsum_kernel(const float* __restrict__ partial, int nrows, int d, float* __restrict__ out_f32,
-                              bf16* __restrict__ out_bf16, int accumulate) {
-  const int col = blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= d) return;
+// out[col] (+)= sum_r partial[r, col].  A block takes 32 columns; its eight warps share the rows, each with COLSUM_UNROLL loads in flight, and meet in shared memory.
+// (One thread per column walked 296 rows one load after another: 14 us for 2048 columns.)
+constexpr int COLSUM_UNROLL = 8;
+__global__ void __launch_bounds__(256)
+colsum_kernel(const float* __restrict__ partial, int nrows, int d, float* __restrict__ out_f32, bf16* __restrict__ out_bf16, int accumulate) {
+  __shared__ float red[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, col = blockIdx.x * 32 + lane;
   float s = 0.f;
-  for (int r = 0; r < nrows; ++r) s += partial[static_cast<long long>(r) * d + col];
+  for (int r0 = warp; r0 < nrows; r0 += 8 * COLSUM_UNROLL) {
+    float v[COLSUM_UNROLL];
+#pragma unroll
+    for (int u = 0; u < COLSUM_UNROLL; ++u) {
+      const int r = r0 + u * 8;
+      v[u] = r < nrows && col < d ? partial[static_cast<long long>(r) * d + col] : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < COLSUM_UNROLL; ++u) s += v[u];
+  }
+  red[warp][lane] = s;
+  __syncthreads();
+  if (warp != 0 || col >= d) return;
+  s = ((red[0][lane] + red[1][lane]) + (red[2][lane] + red[3][lane])) + ((red[4][lane] + red[5][lane]) + (red[6][lane] + red[7][lane]));
   if (out_f32 != nullptr) out_f32[col] = accumulate ? out_f32[col] + s : s;
   if (out_bf16 != nullptr) out_bf16[col] = __float2bfloat16(accumulate ? __bfloat162float(out_bf16[col]) + s : s);
+}
+
+// Column sums of a bf16 matrix over slabs of its rows (the gradient of a bias): part[slab, col].  Bound by the read of x; a warp takes 256 columns, the eight warps
+// of a block every eighth row of its slab, four rows in flight.
+__global__ void __launch_bounds__(256)
+colsum_bf16_kernel(const bf16* __restrict__ x, float* __restrict__ part, long long rows, int d, long long ldx, int slab) {
+  __shared__ float red[8][256];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, col = blockIdx.x * 256 + lane * 8;
+  const long long end = min(rows, (blockIdx.y + 1ll) * slab);
+  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (col < d) {
+    for (long long r0 = blockIdx.y * static_cast<long long>(slab) + warp; r0 < end; r0 += 32) {
+      uint4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = r0 + u * 8 < end ? *reinterpret_cast<const uint4*>(x + (r0 + u * 8) * ldx + col) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        float f[8];
+        unpack8(v[u], f);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) s[c] += f[c];
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 8; ++c) red[warp][lane * 8 + c] = s[c];
+  __syncthreads();
+  const int mine = blockIdx.x * 256 + threadIdx.x;
+  if (mine >= d) return;
+  float t = 0.f;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) t += red[w][threadIdx.x];
+  part[static_cast<long long>(blockIdx.y) * d + mine] = t;
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -916,7 +964,7 @@ extern "C" int dewb_rmsnorm_bwd(const void* dy, const void* x, const void* w, co
     dim3 g((nvec + 31) / 32, splits);
     if (z != nullptr) rmsnorm_dw_kernel<true><<<g, 256, 0, STREAM(stream)>>>((const bf16*)dy, (const bf16*)x, rstd, (const bf16*)z, dw_partial, rows, d);
     else rmsnorm_dw_kernel<false><<<g, 256, 0, STREAM(stream)>>>((const bf16*)dy, (const bf16*)x, rstd, nullptr, dw_partial, rows, d);
-    colsum_kernel<<<(d + 255) / 256, 256, 0, STREAM(stream)>>>(dw_partial, splits, d, dw_f32, (bf16*)dw_bf16, accumulate);
+    colsum_kernel<<<(d + 31) / 32, 256, 0, STREAM(stream)>>>(dw_partial, splits, d, dw_f32, (bf16*)dw_bf16, accumulate);
     return LAST_ERR();
   }
   if (z != nullptr)
@@ -927,7 +975,7 @@ extern "C" int dewb_rmsnorm_bwd(const void* dy, const void* x, const void* w, co
     rmsnorm_bwd_kernel<false><<<blocks, NORM_THREADS, 0, STREAM(stream)>>>(
         (const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd, (const bf16*)dres, nullptr, (bf16*)dx, nullptr,
         dw_partial, rows, d);
-  colsum_kernel<<<(d + 255) / 256, 256, 0, STREAM(stream)>>>(dw_partial, blocks, d, dw_f32, (bf16*)dw_bf16, accumulate);
+  colsum_kernel<<<(d + 31) / 32, 256, 0, STREAM(stream)>>>(dw_partial, blocks, d, dw_f32, (bf16*)dw_bf16, accumulate);
   return LAST_ERR();
 }
 
@@ -1079,7 +1127,7 @@ static int noalloc_body(const void* dy, const void* x, const void* w, const floa
   if (splits > max_useful) splits = static_cast<int>(max_useful);
   dim3 g((nvec + 31) / 32, splits);
   rmsnorm_dw_kernel<false><<<g, 256, 0, STREAM(stream)>>>((const bf16*)dy, (const bf16*)x, rstd, nullptr, partial, rows, d);
-  colsum_kernel<<<(d + 255) / 256, 256, 0, STREAM(stream)>>>(partial, splits, d, dw_f32, (bf16*)dw_bf16, accumulate);
+  colsum_kernel<<<(d + 31) / 32, 256, 0, STREAM(stream)>>>(partial, splits, d, dw_f32, (bf16*)dw_bf16, accumulate);
   return LAST_ERR();
 }
 
@@ -1095,4 +1143,23 @@ extern "C" int dewb_rmsnorm_bwd_noalloc(const void* dy, const void* x, const voi
   NoallocDeviceScope scope(device);
   if (scope.err != cudaSuccess) return static_cast<int>(scope.err);
   return noalloc_body(dy, x, w, rstd, dres, dx, dw_f32, dw_bf16, accumulate, rows, d, device, stream);
+}
+
+// Slabs that dewb_colsum_bf16 cuts `rows` rows of d columns into (the rows of its scratch).
+extern "C" int dewb_colsum_slabs(long long rows, int d) {
+  const long long across = (d + 255) / 256, most = (rows + 63) / 64;
+  long long slabs = (148 * 4 + across - 1) / across;
+  if (slabs > most) slabs = most;
+  return static_cast<int>(slabs < 1 ? 1 : slabs);
+}
+
+// out [d] bf16 = the column sums of x [rows, d] bf16 (row stride ldx; d and ldx multiples of 8, 16-byte aligned); part: fp32 scratch [slabs, d].
+extern "C" int dewb_colsum_bf16(const void* x, float* part, void* out, long long rows, int d, long long ldx, void* stream) {
+  if (d <= 0 || d % 8 || ldx % 8 || rows <= 0 || (reinterpret_cast<uintptr_t>(x) & 15)) return -3;
+  const int slabs = dewb_colsum_slabs(rows, d);
+  const long long slab = (rows + slabs - 1) / slabs;
+  if (slab > 0x7fffffff) return -3;
+  colsum_bf16_kernel<<<dim3((d + 255) / 256, slabs), 256, 0, STREAM(stream)>>>((const bf16*)x, part, rows, d, ldx, static_cast<int>(slab));
+  colsum_kernel<<<(d + 31) / 32, 256, 0, STREAM(stream)>>>(part, slabs, d, nullptr, (bf16*)out, 0);
+  return LAST_ERR();
 }

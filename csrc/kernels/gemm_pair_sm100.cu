@@ -10,8 +10,9 @@
 //               credited to the leader CTA's "full" barrier (no multicast: every load lands in the issuing CTA only)
 //   warp 1      MMA issuer (leader CTA only): tcgen05.mma.cta_group::2 256x256x16; tcgen05.commit to the "empty"
 //               barrier of BOTH CTAs frees a stage; commit to both CTAs' "accumulator full" barriers ends a tile
-//   warps 2..5  epilogue (both CTAs): tcgen05.ld the CTA's own accumulator half, convert, store; the leader's MMA
-//               warp learns from both CTAs' epilogues (remote mbarrier arrive) that an accumulator is free again
+//   warps 2..9  epilogue (both CTAs): tcgen05.ld the CTA's own accumulator half, convert, store; the leader's MMA
+//               warp learns from both CTAs' epilogues (remote mbarrier arrive) that an accumulator is free again.  Two warps share a quarter of the rows and
+//               take half of the columns each: at short reductions a tile's products take less than one warp's way through 256 columns (K = 768: 6100 cycles)
 //
 // Operand layouts as in the single-CTA kernel (K-major or MN-major per operand), so forward, input gradient and weight
 // gradient of a linear layer read their operands in place.
@@ -36,7 +37,8 @@ constexpr int B_BYTES = HALF_N * BK * 2;    // 16 KiB
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int ACC_COLS = BN;
 constexpr int TMEM_COLS = 2 * ACC_COLS;     // both accumulators
-constexpr int THREADS = 192;
+constexpr int EPI_WARPS = 8;
+constexpr int THREADS = 64 + 32 * EPI_WARPS;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
 
 enum Epilogue : int { EPI_BF16 = 0, EPI_F32 = 1, EPI_F32_ACC = 2, EPI_BF16_ACC = 3 };
@@ -45,7 +47,7 @@ struct Shared {
   uint64_t full[STAGES];       // used in the leader: both CTAs' loads of a stage have landed
   uint64_t empty[STAGES];      // in each CTA: the pair MMAs that read the stage have completed
   uint64_t tmem_full[2];       // in each CTA: the accumulator is complete
-  uint64_t tmem_empty[2];      // used in the leader: both CTAs' epilogues have drained the accumulator (8 warps)
+  uint64_t tmem_empty[2];      // used in the leader: both CTAs' epilogues have drained the accumulator (EPI_WARPS warps each)
   uint32_t tmem_base;
   int abort_flag;
   int poisoned;
@@ -70,11 +72,8 @@ __device__ __forceinline__ void store_chunk(const uint32_t (&r_in)[32], void* Dp
   // scale, then the bias (one bf16 value per output column); the stores below see the finished values
   uint32_t r[32];
 #pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    float v = alpha_in * __uint_as_float(r_in[i]);
-    if (bias != nullptr && col + i < N) v += __bfloat162float(bias[col + i]);
-    r[i] = __float_as_uint(v);
-  }
+  for (int i = 0; i < 32; ++i) r[i] = bias != nullptr ? r_in[i] : __float_as_uint(alpha_in * __uint_as_float(r_in[i]));
+  if (bias != nullptr) scale_and_bias(r, alpha_in, bias + col, N - col);
   constexpr float alpha = 1.f;
   if (EPI == EPI_BF16 || EPI == EPI_BF16_ACC) {
     __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(Dptr) + static_cast<long long>(row) * ldd + col;
@@ -155,7 +154,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&sh->full[s], 1); mbar_init(&sh->empty[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&sh->tmem_full[a], 1); mbar_init(&sh->tmem_empty[a], 8); }
+    for (int a = 0; a < 2; ++a) { mbar_init(&sh->tmem_full[a], 1); mbar_init(&sh->tmem_empty[a], 2 * EPI_WARPS); }
     sh->abort_flag = 0;
     // an earlier launch reported a timed-out wait: do no work (decided for the pair as a whole, below)
     sh->poisoned = *reinterpret_cast<volatile int*>(err);
@@ -258,8 +257,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue (warps 2..5, both CTAs)
+    // ------------------------------------------------------------------ epilogue (warps 2..9, both CTAs)
     const int q = warp & 3;                 // TMEM lane quarter this warp may read
+    const int first = (warp - 2) / 4 * (BN / 64);      // its first chunk of 32 columns
     int acc = 0; uint32_t acc_phase = 0;
     bool ok = true;
     for (int t = pair; t < num_tiles && ok; t += num_pairs) {
@@ -271,12 +271,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       tc_fence_after();
       const uint32_t taddr = tmem_base + acc * ACC_COLS + (static_cast<uint32_t>(q * 32) << 16);
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32b_x32(taddr + c * 32, r);
+      for (int c = first; c < first + BN / 64; c += 2) {
+        uint32_t r0[32], r1[32];
+        tmem_ld_32x32b_x32(taddr + c * 32, r0);
+        tmem_ld_32x32b_x32(taddr + c * 32 + 32, r1);
         tmem_ld_wait();
         const int col = n0 + c * 32;
-        if (row < M && col < N) store_chunk<EPI>(r, Dptr, row, col, N, ldd, alpha, bias);
+        if (row < M && col < N) store_chunk<EPI>(r0, Dptr, row, col, N, ldd, alpha, bias);
+        if (row < M && col + 32 < N) store_chunk<EPI>(r1, Dptr, row, col + 32, N, ldd, alpha, bias);
       }
       tc_fence_before();
       __syncwarp();

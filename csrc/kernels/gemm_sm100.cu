@@ -1,9 +1,13 @@
 // Dense bf16 GEMM for sm_100a: D[M,N] = A[M,K] * B[N,K]^T with fp32 accumulation in tensor memory.
 //
-// One persistent CTA per SM, 192 threads in three roles:
+// One persistent CTA per SM, 320 threads in three roles:
 //   warp 0      TMA producer   : cp.async.bulk.tensor tiles of A and B into a 4-stage shared-memory ring
 //   warp 1      MMA issuer     : one elected lane issues tcgen05.mma (128x256x16) into one of two TMEM accumulators
-//   warps 2..5  epilogue       : tcgen05.ld the finished accumulator, convert, store; overlaps the next tile's MMAs
+//   warps 2..9  epilogue       : tcgen05.ld the finished accumulator, convert, store; overlaps the next tile's MMAs.  Two warps share a quarter of the rows
+//                                and take half of the columns each
+//
+// Weight gradients whose outputs have few tiles (768 x 2304 of 16384 tokens: 54) split the reduction: every split's partial product goes to fp32 scratch and a
+// small kernel adds them in order.
 //
 // Operand layouts. "K-major" means the reduction index is contiguous in global memory; "MN-major" means the
 // M (for A) or N (for B) index is contiguous. The three combinations cover a linear layer's forward
@@ -26,7 +30,8 @@ constexpr int B_BYTES = BN * BK * 2;   // 32 KiB
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int ACC_COLS = BN;           // fp32 columns per accumulator
 constexpr int TMEM_COLS = 2 * ACC_COLS;  // 512: both accumulators
-constexpr int THREADS = 192;
+constexpr int EPI_WARPS = 8;
+constexpr int THREADS = 64 + 32 * EPI_WARPS;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
 
 enum Epilogue : int { EPI_BF16 = 0, EPI_F32 = 1, EPI_F32_ACC = 2, EPI_BF16_ACC = 3 };
@@ -49,6 +54,8 @@ struct Shared {
 //           each 128-row tile (< 0: the tile holds no rows)
 //   mode 2  grouped reduction D_g = A[rows of g]^T-style product over the rows of g (weight gradient); the reduction
 //           runs over rows [group_offsets[g], group_offsets[g+1]) and D stacks the groups, `d_group_stride` apart
+//   mode 3  split reduction   D_g = the product over reduction indices [g, g + 1) * `b_rows_per_group` (a multiple of BK); D stacks the
+//           splits, `d_group_stride` apart
 struct GroupArgs {
   const int* tile_group;
   const int* group_offsets;
@@ -85,11 +92,12 @@ __device__ __forceinline__ Tile decode_tile(int t, int tiles_m, int tiles_n, int
   Tile ti;
   int m_blk, n_blk;
   ti.b_row0 = 0; ti.k_begin = 0; ti.k_iters = (K + bk - 1) / bk; ti.d_off = 0; ti.skip = false;
-  if (ga.mode == 2) {
+  if (ga.mode >= 2) {
     const int per = tiles_m * tiles_n;
     const int g = t / per;
     tile_coords(t - g * per, tiles_m, tiles_n, m_blk, n_blk);
-    const int r0 = ga.group_offsets[g], r1 = ga.group_offsets[g + 1];
+    const int r0 = ga.mode == 3 ? g * ga.b_rows_per_group : ga.group_offsets[g];
+    const int r1 = ga.mode == 3 ? min(K, r0 + ga.b_rows_per_group) : ga.group_offsets[g + 1];
     ti.k_begin = r0;
     ti.k_iters = (r1 - r0 + BK - 1) / BK;
     ti.d_off = static_cast<long long>(g) * ga.d_group_stride;
@@ -130,11 +138,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   const int lane = threadIdx.x & 31;
   const int tiles_m = (M + BM - 1) / BM;
   const int tiles_n = (N + BN - 1) / BN;
-  const int num_tiles = tiles_m * tiles_n * (ga.mode == 2 ? ga.groups : 1);
+  const int num_tiles = tiles_m * tiles_n * (ga.mode >= 2 ? ga.groups : 1);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&sh->full[s], 1); mbar_init(&sh->empty[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&sh->tmem_full[a], 1); mbar_init(&sh->tmem_empty[a], 4); }
+    for (int a = 0; a < 2; ++a) { mbar_init(&sh->tmem_full[a], 1); mbar_init(&sh->tmem_empty[a], EPI_WARPS); }
     sh->abort_flag = 0;
     fence_barrier_init();
     fence_proxy_async();
@@ -227,8 +235,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue (warps 2..5)
+    // ------------------------------------------------------------------ epilogue (warps 2..9)
     const int q = warp & 3;                 // TMEM lane quarter this warp may read
+    const int first = (warp - 2) / 4 * (BN / 64);      // its first chunk of 32 columns
     int acc = 0; uint32_t acc_phase = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
@@ -239,7 +248,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       if (ti.k_iters == 0) {
         // an empty group: its product is zero (nothing to add when accumulating)
         if ((EPI == EPI_BF16 || EPI == EPI_F32) && row < M) {
-          for (int c = 0; c < BN && n0 + c < N; ++c) {
+          for (int c = first * 32; c < first * 32 + BN / 2 && n0 + c < N; ++c) {
             if (EPI == EPI_BF16) reinterpret_cast<__nv_bfloat16*>(Dptr)[ti.d_off + static_cast<long long>(row) * ldd + n0 + c] = __float2bfloat16(0.f);
             else reinterpret_cast<float*>(Dptr)[ti.d_off + static_cast<long long>(row) * ldd + n0 + c] = 0.f;
           }
@@ -250,7 +259,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       tc_fence_after();
       const uint32_t taddr = tmem_base + acc * ACC_COLS + (static_cast<uint32_t>(q * 32) << 16);
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
+      for (int c = first; c < first + BN / 64; ++c) {
         uint32_t r[32];
         tmem_ld_32x32b_x32(taddr + c * 32, r);
         tmem_ld_wait();
@@ -266,9 +275,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         float al = alpha;
         if (ga.bias != nullptr && row < M && col < N) {
           // scale, then the bias: the stores below see the finished values
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (col + i < N) r[i] = __float_as_uint(alpha * __uint_as_float(r[i]) + __bfloat162float(ga.bias[col + i]));
+          scale_and_bias(r, alpha, ga.bias + col, N - col);
           al = 1.f;
         }
         if (row < M && col < N) {
@@ -354,7 +361,7 @@ static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, void* D, int
     if (e != cudaSuccess) return static_cast<int>(e);
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * (ga.mode == 2 ? ga.groups : 1);
+  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * (ga.mode >= 2 ? ga.groups : 1);
   const int grid = tiles < sms ? tiles : sms;
   kern<<<grid, THREADS, SMEM_BYTES, stream>>>(ta, tb, D, M, N, K, ldd, alpha, ga, err);
   return static_cast<int>(cudaGetLastError());
@@ -389,6 +396,30 @@ static int dispatch(int a_mn, int b_mn, int epi, const CUtensorMap& ta, const CU
   if (!a_mn && b_mn) return launch_epi<false, true>(epi, ta, tb, D, M, N, K, ldd, alpha, ga, err, sms, stream);
   if (a_mn && !b_mn) return launch_epi<true, false>(epi, ta, tb, D, M, N, K, ldd, alpha, ga, err, sms, stream);
   return launch_epi<true, true>(epi, ta, tb, D, M, N, K, ldd, alpha, ga, err, sms, stream);
+}
+
+// part [splits, M, N] fp32 -> D [M, N] (row stride ldd): the sum over the splits as bf16 (epi 0) or fp32 (1), or added to what is there in fp32 (2) or bf16 (3)
+__global__ void __launch_bounds__(256)
+split_sum_kernel(const float* __restrict__ part, void* __restrict__ D, int M, int N, long long ldd, int splits, float alpha, int epi, const int* __restrict__ err) {
+  if (*reinterpret_cast<const volatile int*>(err) != 0) return;
+  const long long total = static_cast<long long>(M) * N, at = (blockIdx.x * 256ll + threadIdx.x) * 4;
+  if (at >= total) return;
+  float4 s = *reinterpret_cast<const float4*>(part + at);
+  for (int k = 1; k < splits; ++k) {
+    const float4 v = *reinterpret_cast<const float4*>(part + k * total + at);
+    s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+  }
+  s.x *= alpha; s.y *= alpha; s.z *= alpha; s.w *= alpha;
+  const long long to = at / N * ldd + at % N;
+  if (epi == EPI_F32 || epi == EPI_F32_ACC) {
+    float4* d = reinterpret_cast<float4*>(reinterpret_cast<float*>(D) + to);
+    if (epi == EPI_F32_ACC) { const float4 o = *d; s.x += o.x; s.y += o.y; s.z += o.z; s.w += o.w; }
+    *d = s;
+  } else {
+    uint2* d = reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(D) + to);
+    if (epi == EPI_BF16_ACC) { const uint2 o = *d; s.x += bf16_lo(o.x); s.y += bf16_hi(o.x); s.z += bf16_lo(o.y); s.w += bf16_hi(o.y); }
+    *d = make_uint2(pack_bf16(s.x, s.y), pack_bf16(s.z, s.w));
+  }
 }
 
 }  // namespace gemm
@@ -447,6 +478,33 @@ extern "C" int dewb_gemm_bf16_bias(const void* A, const void* B, void* D, const 
   const int rc = dewb_gemm_bf16(A, B, D, M, N, K, lda, ldb, ldd, a_mn, b_mn, epi, alpha, err, max_ctas, stream_ptr);
   g_dense_bias = nullptr;
   return rc;
+}
+
+// The same product with its reduction in `splits` parts of `per` (a multiple of 64; splits * per >= K, every part with something in it): scratch holds
+// splits * M * N floats.  N and ldd multiples of 4, D and scratch 16-byte aligned.
+extern "C" int dewb_gemm_bf16_split(const void* A, const void* B, void* D, float* scratch, int M, int N, int K, int splits, int per, long long lda, long long ldb,
+                                    long long ldd, int a_mn, int b_mn, int epi, float alpha, int* err, void* stream_ptr) {
+  using namespace dewb;
+  using namespace dewb::gemm;
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || (N % 4) || (ldd % 4) ||
+      (reinterpret_cast<uintptr_t>(D) & 15) || (reinterpret_cast<uintptr_t>(scratch) & 15) || splits < 1 || per % BK || per <= 0 ||
+      static_cast<long long>(splits) * per < K || static_cast<long long>(splits - 1) * per >= K || epi < 0 || epi > 3)
+    return -3;
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
+  CUtensorMap ta, tb;
+  int r;
+  if (!a_mn) r = make_tmap_2d(&ta, A, M, K, lda, BM, BK, 2, true);
+  else       r = make_tmap_2d(&ta, A, K, M, lda, BK, 64, 2, true);
+  if (r) return 1000 + r;
+  if (!b_mn) r = make_tmap_2d(&tb, B, N, K, ldb, BN, BK, 2, true);
+  else       r = make_tmap_2d(&tb, B, K, N, ldb, BK, 64, 2, true);
+  if (r) return 2000 + r;
+  GroupArgs ga{nullptr, nullptr, 3, per, splits, static_cast<long long>(M) * N, nullptr, nullptr, nullptr};
+  if ((r = dispatch(a_mn, b_mn, EPI_F32, ta, tb, scratch, M, N, K, N, 1.f, ga, err, sm_count(), stream))) return r;
+  const long long total = static_cast<long long>(M) * N;
+  split_sum_kernel<<<static_cast<unsigned>((total / 4 + 255) / 256), 256, 0, stream>>>(scratch, D, M, N, ldd, splits, alpha, epi, err);
+  return static_cast<int>(cudaGetLastError());
 }
 
 // Grouped rows (mixture-of-experts forward and input gradient):

@@ -130,6 +130,23 @@ _GEMM.declared[("decode",)] = os.environ.get("DEWB_DECODE_GEMM", "cublas")
 _SKINNY_PDL = int(os.environ.get("DEWB_SKINNY_PDL", "1"))
 
 
+def reduction_splits(M: int, N: int, K: int, sms: int = 148) -> int:
+    """Parts the reduction of a product with few output tiles is cut into: the fewest that come close to the shortest last wave of (tile, part) pairs, each at least
+    1024 long (a part costs its fp32 partial product, written and read once).  1: no cut - one wave or more of tiles, a short reduction, or nothing to gain."""
+    tiles = -(-M // 128) * -(-N // 256)
+    if tiles * 2 > sms:
+        return 1
+    best, least = 1, 1.0
+    for s in range(2, min(8, K // 1024) + 1):
+        per = -(-K // s // 64) * 64
+        if (s - 1) * per >= K:
+            continue
+        wave = -(-tiles * s // sms) / s
+        if wave < 0.85 * least:
+            best, least = s, wave
+    return best
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False,
          out: Optional[torch.Tensor] = None, out_dtype: torch.dtype = torch.bfloat16, accumulate: bool = False,
          alpha: float = 1.0, max_ctas: int = 0, kernel: Optional[str] = None, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -207,6 +224,16 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         L.check(rc, which)
         L.count_launches()
         return out
+    if which == "sm100_tcgen05" and max_ctas == 0:
+        splits = reduction_splits(M, N, K)
+        if splits > 1 and N % 4 == 0 and hasattr(lib, "dewb_gemm_bf16_split"):
+            scratch = torch.empty(splits, M, N, dtype=torch.float32, device=a.device)
+            rc = lib.dewb_gemm_bf16_split(L.ptr(a), L.ptr(b), L.ptr(out), L.ptr(scratch), c_int(M), c_int(N), c_int(K), c_int(splits), c_int(-(-K // splits // 64) * 64),
+                                          c_ll(a.stride(0)), c_ll(b.stride(0)), c_ll(out.stride(0)), c_int(int(a_mn)), c_int(int(b_mn)), c_int(epi), c_float(alpha),
+                                          L.ptr(L.status(a.device)), L.stream_ptr())
+            L.check(rc, which)
+            L.count_launches(2)
+            return out
     fn = lib.dewb_gemm_pair_bf16 if which == "sm100_pair" else lib.dewb_gemm_bf16
     rc = fn(L.ptr(a), L.ptr(b), L.ptr(out), c_int(M), c_int(N), c_int(K), c_ll(a.stride(0)),
             c_ll(b.stride(0)), c_ll(out.stride(0)), c_int(int(a_mn)), c_int(int(b_mn)), c_int(epi),
@@ -256,6 +283,20 @@ def grad_accumulates(p) -> bool:
     return True
 
 
+def _column_sums(dy):
+    """``dy.sum(0)`` of a bf16 matrix (a bias' gradient)."""
+    rows, d = dy.shape
+    if not (L.use_cuda(dy) and dy.dtype == torch.bfloat16 and rows >= 256 and d % 8 == 0 and d > 0 and dy.stride(1) == 1 and dy.stride(0) % 8 == 0 and dy.data_ptr() % 16 == 0
+            and hasattr(L.load(), "dewb_colsum_bf16")):
+        return dy.sum(0)
+    lib = L.load()
+    part = torch.empty(lib.dewb_colsum_slabs(c_ll(rows), c_int(d)), d, dtype=torch.float32, device=dy.device)
+    out = torch.empty(d, dtype=torch.bfloat16, device=dy.device)
+    L.check(lib.dewb_colsum_bf16(L.ptr(dy), L.ptr(part), L.ptr(out), c_ll(rows), c_int(d), c_ll(dy.stride(0)), L.stream_ptr()), "colsum_bf16")
+    L.count_launches(2)
+    return out
+
+
 def _linear(x, weight, bias):
     """``x`` contiguous; the bias joins in the product's epilogue."""
     if x.dim() == 2:
@@ -288,7 +329,7 @@ class _Linear(torch.autograd.Function):
             else:
                 dw = gemm(dy2, x2, a_mn=True, b_mn=True)                   # dY^T[N,M] @ x[M,K]
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = dy2.sum(0)
+            db = _column_sums(dy2)
         return dx, dw, db
 
 

@@ -8,6 +8,7 @@
 //              see it through the saved log-sum-exp)
 //   gain     : each head's scores times a number of its own, in front of the cap (forward only)
 //   sig      : every visible key weighs sigmoid(score + sig[head]), and nothing is divided by the sum of the weights (forward only)
+//   first    : rows behind one another in one sequence, each from a multiple of the key tile on: the first key tile that a query tile sees (forward only; causal)
 //   segments : packed documents - a query sees a key only if both carry the same segment id; ids are non-decreasing
 //              along the sequence (0 = padding, allowed after the last document), which is what lets whole tiles be skipped
 #pragma once
@@ -26,6 +27,7 @@ struct Variant {
   int keep;
   const float* gain;       // [Hq] or null
   const float* sig;        // [Hq] or null
+  const int* first;        // [query tiles] or null
 };
 
 // tanh to fp32 accuracy relative to 1 (scores under a cap are fp32 quantities): 1 - 2 / (1 + e^2x)
@@ -37,6 +39,7 @@ __device__ __forceinline__ int first_key_tile(const Variant& v, int b, int q0, i
   int lo = 0;
   if (v.window > 0) lo = max(0, (q0 + off - v.window + 1) / bn);
   if (v.chunk > 0) lo = max(lo, (q0 + off) / v.chunk * v.chunk / bn);
+  if (v.first != nullptr) lo = max(lo, v.first[q0 / bn]);
   if (v.q_seg != nullptr && v.k_seg != nullptr) {
     const int first = v.q_seg[static_cast<long long>(b) * S + min(q0, S - 1)];
     const int* ks = v.k_seg + static_cast<long long>(b) * T;

@@ -812,7 +812,7 @@ extern "C" int dewb_flash_bwd_var(const void* dO, const void* q, const void* k, 
       dos[0], dos[1], dos[2], os[0], os[1], os[2], wide);
   const float* lse2 = delta + static_cast<long long>(B) * Hq * S;
   // the sink logits reach the backward through the saved log-sum-exp alone
-  const Variant var{window, softcap, nullptr, q_seg, k_seg};
+  const Variant var{window, softcap, nullptr, q_seg, k_seg, 0, 0, nullptr, nullptr, nullptr};
   const bool any = window > 0 || softcap > 0.f || q_seg != nullptr;
 #define DEWB_BWD_GO(DD, CC, VV) launch_bwd<DD, CC, VV>(dO, q, k, v, lse, lse2, delta, dq, dk, dv, B, S, T, Hq, Hkv, qs, ks, vs, os, dos, dqs, dks, dvs, scale, var, err, stream)
   if (D == 128) {

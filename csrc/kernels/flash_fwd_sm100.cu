@@ -558,12 +558,13 @@ extern "C" int dewb_flash_set_variant(int variant) {
 // out [B,S,Hq,D] with its own strides; lse [B,Hq,S] fp32 (natural log), may be null.
 // Variants (each off at 0 / null): `gain` [Hq] fp32 factors of the heads' scores, `sig` [Hq] fp32: sigmoid weights (causal, without lse and sinks), `window` keys visible behind each query, `keep` first keys visible beside a window, `chunk` positions a query sees no key from outside of, `softcap`, `sinks` [Hq] fp32, `q_seg` [B,S] /
 // `k_seg` [B,T] int32 segment ids of packed documents (non-decreasing along the sequence, rows 16-byte aligned: S, T % 4 == 0).
-extern "C" int dewb_flash_fwd_var(const void* q, const void* k, const void* v, void* out, float* lse, int B, int S, int T,
+// `first` (see dewb_flash_fwd_rows) may be null
+static int flash_fwd_any(const void* q, const void* k, const void* v, void* out, float* lse, int B, int S, int T,
                                   int Hq, int Hkv, int D, long long q_sb, long long q_ss, long long q_sh, long long k_sb,
                                   long long k_ss, long long k_sh, long long v_sb, long long v_ss, long long v_sh,
                                   long long o_sb, long long o_ss, long long o_sh, float scale, int causal, int window,
                                   int keep, int chunk, float softcap, const float* sinks, const int* q_seg, const int* k_seg, const float* gain,
-                                  const float* sig, int* err, void* stream_ptr) {
+                                  const float* sig, const int* first, int* err, void* stream_ptr) {
   using namespace dewb::attnfwd;
   if (D != 128 && D != 64) return -3;
   if (Hq % Hkv != 0) return -3;
@@ -581,9 +582,9 @@ extern "C" int dewb_flash_fwd_var(const void* q, const void* k, const void* v, v
   if ((r = make_qkv_map(&tv, v, B, T, Hkv, D, v_sb, v_ss, v_sh))) return 3000 + r;
   const float scale_log2 = scale * 1.4426950408889634f;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
-  const Variant var{window, softcap, sinks, q_seg, k_seg, chunk, keep, gain, sig};
+  const Variant var{window, softcap, sinks, q_seg, k_seg, chunk, keep, gain, sig, first};
   const Parts parts{D / 64, D, nullptr, 0};
-  const bool any = window > 0 || chunk > 0 || softcap > 0.f || sinks != nullptr || q_seg != nullptr || gain != nullptr || sig != nullptr;
+  const bool any = window > 0 || chunk > 0 || softcap > 0.f || sinks != nullptr || q_seg != nullptr || gain != nullptr || sig != nullptr || first != nullptr;
 #define DEWB_FLASH_GO(DD, CC, PP, VV) launch<DD, DD, CC, PP, VV>(tq, tk, tv, tq, tk, out, lse, B, S, T, Hq, Hkv, o_sb, o_ss, o_sh, scale_log2, var, parts, err, stream)
   const bool pt = g_variant != 0;
   if (sig != nullptr) {
@@ -603,6 +604,28 @@ extern "C" int dewb_flash_fwd_var(const void* q, const void* k, const void* v, v
   if (causal) return pt ? DEWB_FLASH_GO(64, true, true, false) : DEWB_FLASH_GO(64, true, false, false);
   return pt ? DEWB_FLASH_GO(64, false, true, false) : DEWB_FLASH_GO(64, false, false, false);
 #undef DEWB_FLASH_GO
+}
+
+extern "C" int dewb_flash_fwd_var(const void* q, const void* k, const void* v, void* out, float* lse, int B, int S, int T,
+                                  int Hq, int Hkv, int D, long long q_sb, long long q_ss, long long q_sh, long long k_sb,
+                                  long long k_ss, long long k_sh, long long v_sb, long long v_ss, long long v_sh,
+                                  long long o_sb, long long o_ss, long long o_sh, float scale, int causal, int window,
+                                  int keep, int chunk, float softcap, const float* sinks, const int* q_seg, const int* k_seg, const float* gain,
+                                  const float* sig, int* err, void* stream_ptr) {
+  return flash_fwd_any(q, k, v, out, lse, B, S, T, Hq, Hkv, D, q_sb, q_ss, q_sh, k_sb, k_ss, k_sh, v_sb, v_ss, v_sh, o_sb, o_ss, o_sh, scale, causal, window, keep, chunk,
+                       softcap, sinks, q_seg, k_seg, gain, sig, nullptr, err, stream_ptr);
+}
+
+// Causal attention of several rows that lie behind one another in one sequence of S tokens (S a multiple of 128), each row from a multiple of 128 on: a query of
+// tile t (128 queries) sees no key from before tile first[t] (int32 [S / 128]), the first tile of its row.  Every key tile in between belongs to the row, so nothing
+// is masked but the diagonal.  q, k, v, out [S, heads, D] with their (token, head) strides; window, softcap and sinks as above.
+extern "C" int dewb_flash_fwd_rows(const void* q, const void* k, const void* v, void* out, int S, int Hq, int Hkv, int D, long long q_ss, long long q_sh, long long k_ss,
+                                   long long k_sh, long long v_ss, long long v_sh, long long o_ss, long long o_sh, float scale, int window, float softcap,
+                                   const float* sinks, const int* first, int* err, void* stream_ptr) {
+  if (S % 128 || first == nullptr) return -3;
+  if (S <= 0) return 0;
+  return flash_fwd_any(q, k, v, out, nullptr, 1, S, S, Hq, Hkv, D, q_ss * S, q_ss, q_sh, k_ss * S, k_ss, k_sh, v_ss * S, v_ss, v_sh, o_ss * S, o_ss, o_sh, scale, 1, window, 0, 0,
+                       softcap, sinks, nullptr, nullptr, nullptr, nullptr, first, err, stream_ptr);
 }
 
 extern "C" int dewb_flash_fwd(const void* q, const void* k, const void* v, void* out, float* lse, int B, int S, int T,
@@ -638,7 +661,7 @@ extern "C" int dewb_flash_fwd_parts(const void* q, const void* k, const void* k2
   if ((r = make_qkv_map(&tk2, k2, B, T, 1, db, k2_sb, k2_ss, k2_ss))) return 2500 + r;
   if ((r = make_qkv_map(&tv, v, B, T, H, dv, v_sb, v_ss, v_sh))) return 3000 + r;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
-  const Variant var{0, 0.f, nullptr, nullptr, nullptr, 0, 0, nullptr, nullptr};
+  const Variant var{0, 0.f, nullptr, nullptr, nullptr, 0, 0, nullptr, nullptr, nullptr};
   const Parts parts{first, dv, static_cast<const __nv_bfloat16*>(gate), gate_stride};
   const long long oss = static_cast<long long>(H) * dv, osb = oss * S;
 #define DEWB_PARTS_GO(KK, VV) launch<KK, VV, true, true, false>(tq, tk, tv, tq2, tk2, out, nullptr, B, S, T, H, H, osb, oss, dv, \

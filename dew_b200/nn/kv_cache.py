@@ -365,6 +365,10 @@ class KVStore:
     def write(self, layer: int, k: torch.Tensor, v: torch.Tensor, positions: torch.Tensor) -> None:
         """Store ``k, v [R, S, Hkv, D]`` at ``positions [R, S]`` (negative positions are skipped)."""
         R, S = positions.shape
+        if k.dim() == 4 and k.shape[:2] == v.shape[:2] == (R, S) and k.stride(0) == S * k.stride(1) and v.stride(0) == S * v.stride(1):
+            rows = None if self.row_ids is None else self.row_ids.to(torch.int32)
+            if self._scatter(layer, k[0], v[0], positions, rows, S):
+                return
         rows = self._rows(R)[:, None].expand(R, S).reshape(-1)
         flat = positions.reshape(-1)
         live = flat >= 0
@@ -379,6 +383,23 @@ class KVStore:
             self.v_scale[layer].reshape(-1, self.kv_heads)[slots] = vs
         else:
             kp[slots], vp[slots] = kk.to(kp.dtype), vv.to(vp.dtype)
+
+    def _scatter(self, layer: int, k: torch.Tensor, v: torch.Tensor, positions: torch.Tensor, rows: Optional[torch.Tensor], per_row: int) -> bool:
+        """Tokens ``k, v [*, Hkv, D]`` (one after another at one stride; as many as there are positions) into their pages by one kernel: token t goes to store row
+        ``rows[t // per_row]`` (None: the index itself).  False where the kernel does not take the types or the layout."""
+        n, width = positions.numel(), self.kv_heads * self.head_dim
+        fits = lambda t: (t.dtype == torch.bfloat16 and t.shape[1:] == (self.kv_heads, self.head_dim) and t.stride(2) == 1 and (self.kv_heads == 1 or t.stride(1) == self.head_dim)
+                          and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0)
+        if not (self.slots is None and self.kind == 0 and self.dtype == torch.bfloat16 and n < 1 << 31 and width % 8 == 0 and k.is_cuda and L.use_cuda(k) and fits(k) and fits(v)
+                and hasattr(L.load(), "dewb_kv_scatter")):
+            return False
+        pos32 = positions.reshape(-1).to(torch.int32)
+        L.check(L.load().dewb_kv_scatter(L.ptr(k), L.ptr(v), ctypes.c_longlong(k.stride(0)), ctypes.c_longlong(v.stride(0)), L.ptr(self.k[layer]), L.ptr(self.v[layer]),
+                                         L.ptr(self.page_table), L.ptr(rows), L.ptr(pos32), ctypes.c_int(n), ctypes.c_int(per_row), ctypes.c_int(width),
+                                         ctypes.c_int(self.page_size), ctypes.c_int(self.max_pages), ctypes.c_int(self.rows), ctypes.c_int(self.pages), L.stream_ptr()),
+                "kv_scatter")
+        L.count_launches()
+        return True
 
     def append(self, layer: int, k: torch.Tensor, v: torch.Tensor, positions: torch.Tensor) -> None:
         """One token per row: ``k, v [R, Hkv, D]`` written at ``positions [R]``."""
@@ -571,6 +592,63 @@ class KVStore:
         kc, vc = self.gather(layer, total, dtype=q.dtype)
         # bottom-right aligned causal attention of the chunk against everything cached so far (rows share `start`)
         return ops.attention_reference(q, kc, vc, causal=causal, window=window, softcap=softcap, sinks=sinks)
+
+
+class PackedRows:
+    """Stands where the cache would while whole prompts enter it behind one another as ONE row of tokens without the padding between them: each prompt from a multiple
+    of ``TILE`` tokens on (the flash kernel's tile), so that its attention is cut at tiles and its products have nothing else to skip.  The first tokens of rows of
+    ``store``; bf16 heads of 64 or 128."""
+    TILE = 128
+
+    def __init__(self, store: KVStore, lengths: Sequence[int]):
+        dev = store.device
+        whole = [-(-n // self.TILE) * self.TILE for n in lengths]
+        starts = [0]
+        for n in whole:
+            starts.append(starts[-1] + n)
+        self.store, self.total = store, starts[-1]
+        # (row, position) of every token, one row of the packed form; positions below 0 fill a prompt up to whole tiles
+        host = torch.full((2, self.total), -1, dtype=torch.int32)
+        first = torch.empty(self.total // self.TILE, dtype=torch.int32)
+        for r, (n, s, e) in enumerate(zip(lengths, starts, starts[1:])):
+            host[0, s:e] = r
+            host[1, s:s + n] = torch.arange(n, dtype=torch.int32)
+            first[s // self.TILE:e // self.TILE] = s // self.TILE
+        self.rows, pos32 = host.to(dev)
+        self.first, self.positions = first.to(dev), pos32.long()[None]
+        self.last = torch.tensor([s + n - 1 for s, n in zip(starts, lengths)], device=dev)
+
+    @staticmethod
+    def takes(store: KVStore, model, lengths: Sequence[int], width: int) -> bool:
+        """Whether the model's layers are attention over this store alone and nothing in them looks at a token's neighbours by index, the kernels take its heads, and
+        enough padding goes: one row's worth of tiles in eight."""
+        from ..models.causal_transformer import CausalTransformer
+        from .attention import SelfAttention
+        if not (store.slots is None and store.kind == 0 and store.dtype == torch.bfloat16 and store.device.type == "cuda" and store.row_ids is None and store.head_dim in (64, 128)
+                and len(lengths) == store.rows and type(model) is CausalTransformer and L.env("DEWB_FORCE_REFERENCE") != "1" and L.env("DEWB_KERNEL_ATTENTION") is None
+                and hasattr(L.load(), "dewb_flash_fwd_rows")):
+            return False
+        cfg = model.config
+        if (cfg.fp32_stack or cfg.loop is not None or cfg.hyper_connections > 1 or cfg.altup > 1 or cfg.depth_residual_block or not cfg.causal or model.engrams is not None
+                or getattr(model, "tp", None) is not None or min(lengths) < 1 or max(lengths) > width):
+            return False
+        for layer in model.layers:
+            m = layer.mixer
+            if type(m) is not SelfAttention or layer.cross is not None or layer.streams is not None or m.num_heads % m.num_kv_heads or m.num_kv_heads != store.kv_heads \
+                    or m.head_dim != store.head_dim or (layer.sparse and getattr(layer.mlp, "mix", None) is not None and layer.mlp.mix.capacity_factor is not None):
+                return False
+        tiles = sum(-(-n // PackedRows.TILE) for n in lengths)
+        return 8 * tiles <= 7 * len(lengths) * -(-width // PackedRows.TILE)
+
+    def attend(self, layer: int, q, k, v, positions, causal=True, window=None, softcap=0.0, sinks=None):
+        from ..ops.flash import Variants, flash_fwd_rows
+        q, k, v = q[0], k[0], v[0]
+        if not self.store._scatter(layer, k, v, self.positions, self.rows, 1):
+            k, v = k.contiguous(), v.contiguous()
+            if not self.store._scatter(layer, k, v, self.positions, self.rows, 1):
+                raise L.KernelError("the packed prompt's keys and values do not fit the pages' layout")
+        at = lambda t: t if t.stride(2) == 1 and t.stride(0) % 8 == 0 and t.stride(1) % 8 == 0 and t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
+        return flash_fwd_rows(at(q), at(k), at(v), q.shape[-1] ** -0.5, self.first, Variants(window, softcap, sinks))[None]
 
 
 class Uncached:

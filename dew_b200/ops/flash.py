@@ -57,6 +57,21 @@ def flash_fwd(q, k, v, causal: bool, scale: float, need_lse: bool = True, var: V
     return out, lse
 
 
+def flash_fwd_rows(q, k, v, scale: float, first: torch.Tensor, var: Variants = NONE):
+    """Causal attention of rows that lie behind one another, ``q [S, Hq, D]``, ``k, v [S, Hkv, D]``, each row from a multiple of 128 tokens on; ``first`` int32
+    ``[S / 128]``: the first 128-token tile of every tile's row.  Window, soft cap and sinks of ``var``."""
+    S, Hq, D = q.shape
+    out = torch.empty((S, Hq, D), dtype=q.dtype, device=q.device)
+    st = []
+    for t in (q, k, v, out):
+        assert t.stride(2) == 1
+        st += [c_ll(t.stride(0)), c_ll(t.stride(1))]
+    L.check(L.load().dewb_flash_fwd_rows(L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(out), c_int(S), c_int(Hq), c_int(k.shape[1]), c_int(D), *st, c_float(scale), c_int(var.window),
+                                         c_float(var.softcap), L.ptr(var.sinks), L.ptr(first), L.ptr(L.status(q.device)), L.stream_ptr()), "flash_fwd_rows")
+    L.count_launches()
+    return out
+
+
 def bwd_available() -> bool:
     try:
         return hasattr(L.load(), "dewb_flash_bwd")

@@ -13,7 +13,7 @@ from typing import Any, Callable, List, Optional, Sequence, Tuple
 
 import torch
 
-from ..nn.kv_cache import KVCache, KVStore
+from ..nn.kv_cache import KVCache, KVStore, PackedRows
 from ..utils import keys as K
 
 
@@ -198,12 +198,25 @@ class RowBatch:
     def prefill(self, tokens: torch.Tensor, lengths: torch.Tensor) -> torch.Tensor:
         """The prompts ``[rows, S]`` (right-padded), from their first token; returns last-position logits ``[rows, V]``."""
         R, S = tokens.shape
+        if self.splits_head and self.device.type == "cuda" and self.store.slots is None and S > PackedRows.TILE and not torch.cuda.is_current_stream_capturing():
+            counts = lengths.tolist()
+            if PackedRows.takes(self.store, self.model, counts, S):
+                return self._prefill_packed(tokens, counts)
         if self.store.slots is not None and self.device.type == "cuda" and 1 < S and S % 128:
             tokens = torch.nn.functional.pad(tokens, (0, 128 - S % 128))          # whole tiles for the flash kernel
         pos = torch.arange(tokens.shape[1], device=tokens.device)[None].expand(R, -1)
         pos = torch.where(pos < lengths[:, None], pos, torch.full_like(pos, -1))
         return self.forward(tokens, pos, (0, S) if self.store.slots is not None else None,
                             (torch.arange(R, device=tokens.device), (lengths - 1).clamp_min(0)))
+
+    def _prefill_packed(self, tokens: torch.Tensor, counts: List[int]) -> torch.Tensor:
+        """The prompts behind one another, without the padding to the longest."""
+        rows = PackedRows(self.store, counts)
+        pos = rows.positions
+        ids = tokens[rows.rows.long(), pos[0].clamp_min(0)][None]                 # (what fills a prompt up to whole tiles repeats its first token; nobody sees it)
+        with torch.no_grad():
+            hidden = self.call(ids, positions=pos, cache=rows, return_hidden=True)
+            return self.model.logits(hidden[0].index_select(0, rows.last))
 
     def feed(self, pieces: Sequence[Sequence[int]], want: Optional[Sequence[Sequence[int]]] = None) -> Optional[torch.Tensor]:
         """The next tokens of every row (an empty piece: the row rests); returns the logits at ``want`` (places within each piece, row by

@@ -116,25 +116,82 @@ __device__ __forceinline__ void running(float dt0, float dt1, float A, float& g0
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// The walk over the chunks.  Four warps, 16 rows of the state each (S is kept [P, N]); NT column tiles of 8 a CTA.  A call with few (batch, head) pairs is cut
-// along the columns as well, which are independent of each other: one CTA's step is a chain (scale, split, products, decay), so the narrower it is the better
-// while there are SMs for it.
-template <int NT, int TERMS, bool REV, typename Out>
-__global__ void __launch_bounds__(128)
-ssd_states(Call k, const float* __restrict__ initial, Out* __restrict__ states, float* __restrict__ last) {
+// The walk over the chunks, forward (blockIdx.z 0) and in reverse (1) side by side.  Four warps, 16 rows of the state each (S is kept [P, N]); NT column tiles of 8 a
+// CTA.  The columns are independent of each other, and one CTA's step is a chain (scale, split, products, decay), so a call with few (batch, head) pairs is cut
+// along them.  A fifth warp fetches the tiles two chunks ahead, a sixth makes the weights one ahead, so that a step has one barrier and nothing of either in its chain.
+// (With both in the computing warps and a launch for each direction, 2 x 4096 tokens of 64 heads took 306 us both ways instead of 241, and 124 us for the forward pass instead of 88.)
+constexpr int WALK_STAGES = 3, WALK_THREADS = 192;
+template <int NT, int TERMS, typename Out>
+__global__ void __launch_bounds__(WALK_THREADS, NT <= 8 ? 2 : 1)
+ssd_states(Call k, const float* __restrict__ initial, Out* __restrict__ states, float* __restrict__ last, const float* __restrict__ rev_initial, Out* __restrict__ rev_states,
+           float* __restrict__ rev_last) {
   constexpr int CV = NT;                               // 16-byte pieces of a row of B (C)
   constexpr int U_BYTES = L * P * 2, V_BYTES = L * CV * 16;
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ __align__(16) float weight[2][L], total[2];
+  const bool rev = blockIdx.z != 0;
+  if (rev) { initial = rev_initial; states = rev_states; last = rev_last; }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & 3, r = lane >> 2;
   const int b = blockIdx.x / k.H, h = blockIdx.x % k.H, grp = h / (k.H / k.G), col0 = blockIdx.y * NT * 8;
-  const float A = k.A[h];
+  auto chunk = [&](int it) { return rev ? k.chunks - 1 - it : it; };
+  if (warp == 4) {
+    const __nv_bfloat16* u = rev ? k.dy + static_cast<long long>(b) * k.T * k.H * P + h * P : k.x + b * k.xb + h * P;
+    const __nv_bfloat16* v = (rev ? k.Cm + b * k.cb : k.Bm + b * k.bb) + grp * N + col0;
+    const long long us = rev ? static_cast<long long>(k.H) * P : k.xt, vs = rev ? k.ct : k.bt;
+    auto fetch = [&](int it) {
+      if (it < k.chunks) {
+        const int t0 = chunk(it) * L, real = min(L, k.T - t0);
+        uint8_t* st = smem + (it % WALK_STAGES) * (U_BYTES + V_BYTES);
+#pragma unroll 4
+        for (int i = 0; i < L * 8 / 32; ++i) {
+          const int row = i * 4 + (lane >> 3), c = lane & 7;
+          cp16(st + piece<8>(row, c), u + (t0 + (row < real ? row : 0)) * us + c * 8, row < real);
+        }
+#pragma unroll 4
+        for (int i = 0; i < L * CV / 32; ++i) {
+          const int row = (i * 32 + lane) / CV, c = (i * 32 + lane) % CV;
+          cp16(st + U_BYTES + piece<CV>(row, c), v + (t0 + (row < real ? row : 0)) * vs + c * 8, row < real);
+        }
+      }
+      cp_commit();                                     // (a group for every chunk, empty behind the last)
+    };
+    fetch(0);
+    fetch(1);
+    for (int it = 0; it < k.chunks; ++it) {
+      cp_wait<1>();
+      __syncthreads();                                 // chunk `it` is there, and chunk it - 1's stage is free
+      fetch(it + 2);
+    }
+    return;
+  }
+  if (warp == 5) {
+    const float A = k.A[h];
+    const float* dt = k.dt + static_cast<long long>(b) * k.T * k.H + h;
+    float next0, next1;
+    auto fetch = [&](int it) {
+      const int t = it < k.chunks ? chunk(it) * L + 2 * lane : k.T;
+      next0 = t < k.T ? dt[static_cast<long long>(t) * k.H] : 0.f;
+      next1 = t + 1 < k.T ? dt[static_cast<long long>(t + 1) * k.H] : 0.f;
+    };
+    auto weigh = [&](int it) {                         // e^{g_i}, or dt_j e^{g_L - g_j}
+      const float dt0 = next0, dt1 = next1;
+      fetch(it + 1);
+      float g0, g1;
+      running(dt0, dt1, A, g0, g1);
+      const float gl = __shfl_sync(FULL, g1, 31);
+      weight[it & 1][2 * lane] = rev ? expf(g0) : dt0 * expf(gl - g0);
+      weight[it & 1][2 * lane + 1] = rev ? expf(g1) : dt1 * expf(gl - g1);
+      if (lane == 0) total[it & 1] = expf(gl);
+    };
+    fetch(0);
+    weigh(0);
+    for (int it = 0; it < k.chunks; ++it) {
+      __syncthreads();
+      if (it + 1 < k.chunks) weigh(it + 1);            // (the other half: chunk it reads its own)
+    }
+    return;
+  }
   const long long cell = static_cast<long long>(P) * N, at = (warp * 16 + r) * N + col0 + 2 * q;      // this thread's first value of a state
-  const __nv_bfloat16* u = REV ? k.dy + static_cast<long long>(b) * k.T * k.H * P + h * P : k.x + b * k.xb + h * P;
-  const __nv_bfloat16* v = (REV ? k.Cm + b * k.cb : k.Bm + b * k.bb) + grp * N + col0;
-  const long long us = REV ? static_cast<long long>(k.H) * P : k.xt, vs = REV ? k.ct : k.bt;
-  const float* dt = k.dt + static_cast<long long>(b) * k.T * k.H + h;
-
   float S[NT][4];
   const float* from = initial == nullptr ? nullptr : initial + blockIdx.x * cell + at;
 #pragma unroll
@@ -143,33 +200,7 @@ ssd_states(Call k, const float* __restrict__ initial, Out* __restrict__ states, 
     const float2 c = from == nullptr ? make_float2(0.f, 0.f) : *reinterpret_cast<const float2*>(from + n * 8 + 8 * N);
     S[n][0] = a.x; S[n][1] = a.y; S[n][2] = c.x; S[n][3] = c.y;
   }
-  auto chunk = [&](int it) { return REV ? k.chunks - 1 - it : it; };
-  auto fetch = [&](int it) {
-    const int t0 = chunk(it) * L, real = min(L, k.T - t0);
-    uint8_t* st = smem + (it & 1) * (U_BYTES + V_BYTES);
-    load_tile<8, 128>(st, u + t0 * us, us, real);
-    load_tile<CV, 128>(st + U_BYTES, v + t0 * vs, vs, real);
-    cp_commit();
-  };
-  float dt0 = 0.f, dt1 = 0.f;
-  auto fetch_dt = [&](int it) {                        // warp 0
-    const int t = chunk(it) * L + 2 * lane;
-    dt0 = t < k.T ? dt[static_cast<long long>(t) * k.H] : 0.f;
-    dt1 = t + 1 < k.T ? dt[static_cast<long long>(t + 1) * k.H] : 0.f;
-  };
-  auto weigh = [&](int it) {                           // warp 0: e^{g_i}, or dt_j e^{g_L - g_j}
-    float g0, g1;
-    running(dt0, dt1, A, g0, g1);
-    const float gl = __shfl_sync(FULL, g1, 31);
-    weight[it & 1][2 * lane] = REV ? expf(g0) : dt0 * expf(gl - g0);
-    weight[it & 1][2 * lane + 1] = REV ? expf(g1) : dt1 * expf(gl - g1);
-    if (lane == 0) total[it & 1] = expf(gl);
-  };
-  fetch(0);
-  if (warp == 0) { fetch_dt(0); weigh(0); }
   for (int it = 0; it < k.chunks; ++it) {
-    if (it + 1 < k.chunks) { fetch(it + 1); if (warp == 0) fetch_dt(it + 1); cp_wait<1>(); }
-    else cp_wait<0>();
     __syncthreads();
     Out* to = states + (static_cast<long long>(blockIdx.x) * k.chunks + chunk(it)) * cell + at;
 #pragma unroll
@@ -182,7 +213,7 @@ ssd_states(Call k, const float* __restrict__ initial, Out* __restrict__ states, 
         *reinterpret_cast<uint32_t*>(to + n * 8 + 8 * N) = pack2(S[n][2], S[n][3]);
       }
     }
-    const uint8_t* st = smem + (it & 1) * (U_BYTES + V_BYTES);
+    const uint8_t* st = smem + (it % WALK_STAGES) * (U_BYTES + V_BYTES);
     uint32_t a[TERMS][4][4];
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) {
@@ -211,8 +242,6 @@ ssd_states(Call k, const float* __restrict__ initial, Out* __restrict__ states, 
 #pragma unroll
       for (int i = 0; i < 4; ++i) { S[n][i] = fmaf(S[n][i], decay, c0[i]); S[n + 1][i] = fmaf(S[n + 1][i], decay, c1[i]); }
     }
-    if (warp == 0 && it + 1 < k.chunks) weigh(it + 1);
-    __syncthreads();
   }
   if (last != nullptr) {
     float* to = last + blockIdx.x * cell + at;
@@ -344,17 +373,19 @@ ssd_output(Call k, const __nv_bfloat16* __restrict__ states, __nv_bfloat16* __re
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Gradients of one chunk, one group, `per` of its heads: eight warps.  The products over the state's columns give each warp 16 of the 128 columns and all 64
-// tokens, so that every fp32 value of a state is split into its bf16 terms by the one warp that needs it; E and M are made by 16 x 32 pieces.
+// Gradients of one chunk, one group, `per` of its heads: sixteen warps, four a scheduler (with eight of twice the work each, the tensor pipe was busy for 30 % of the
+// time and the rest went to waits: 610 us for 2 x 4096 tokens of 64 heads instead of 585).  The products over the state's columns give each warp 8 of the 128 columns and all
+// 64 tokens, so that every fp32 value of a state is split into its bf16 terms by the one warp that needs it; E and M are made by 16 x 16 pieces.
+constexpr int LOCAL_WARPS = 16, LOCAL_THREADS = 32 * LOCAL_WARPS;
 constexpr int SLD = N + 4;                             // row of an fp32 state in shared memory: the fragment reads of both orders spread over the banks
 constexpr int LOCAL_STAGE = 2 * L * P * 2 + 2 * P * SLD * 4;
 constexpr int M_BYTES = 10 * 3 * 512;                  // the ten 16 x 16 blocks of M^T with i >= j, three terms each, as A fragments
 struct LocalSums {
-  float rows[4][L];                                    // sum over j < i of M o E dt_j, by the 16 tokens j of a pair of warps
-  float cols[2][L], diag[L], edge[L];                  // sum over i > j of M o E by halves of i; its diagonal; the diagonal of E
-  float dy_state[8][L], x_state[8][L];                 // (dy S) . C and (x dS) . B, by the warps' columns
-  float both[8];                                       // <S, dS>
-  float g[2][L], dt[2][L];
+  float rows[4][L];                                    // sum over j < i of M o E dt_j, by the tile of j
+  float cols[4][L], diag[L], edge[L];                  // sum over i > j of M o E, by the tile of i; its diagonal; the diagonal of E
+  float dy_state[LOCAL_WARPS][L], x_state[LOCAL_WARPS][L];      // (dy S) . C and (x dS) . B, by the warps' columns
+  float both[LOCAL_WARPS];                             // <S, dS>
+  float g[2][L], dt[2][L], head[2][L], tail[2][L];     // of this head and the next: g, dt, e^g, e^{g_L - g}
 };
 constexpr int LOCAL_SMEM = 2 * L * N * 2 + 2 * LOCAL_STAGE + M_BYTES + static_cast<int>(sizeof(LocalSums));
 static_assert(LOCAL_SMEM <= 232448, "ssd_local exceeds the shared memory of an SM");
@@ -367,7 +398,7 @@ struct Grads {
 // which of the ten blocks of the lower triangle (j tile, i tile >= j tile)
 __device__ __forceinline__ int block_of(int jt, int it) { return jt * 4 - jt * (jt - 1) / 2 + it - jt; }
 
-__global__ void __launch_bounds__(256, 1)
+__global__ void __launch_bounds__(LOCAL_THREADS, 1)
 ssd_local(Call k, const float* __restrict__ states, const float* __restrict__ dstates, Grads out, int per) {
   extern __shared__ __align__(128) uint8_t smem[];
   uint8_t *tB = smem, *tC = tB + L * N * 2, *stages = tC + L * N * 2, *tM = stages + 2 * LOCAL_STAGE;
@@ -375,94 +406,90 @@ ssd_local(Call k, const float* __restrict__ states, const float* __restrict__ ds
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & 3, r = lane >> 2;
   const int b = blockIdx.x / k.chunks, n = blockIdx.x % k.chunks, grp = blockIdx.y, h0 = grp * (k.H / k.G) + blockIdx.z * per;
   const int t0 = n * L, real = min(L, k.T - t0);
-  const int jt = warp >> 1, ih = warp & 1;             // this warp's piece of E^T: tokens j of tile jt, tokens i of half ih
-  const bool lower = ih * 32 + 31 >= jt * 16;          // whether some i >= j is in it
-  const int nc = warp * 16;                            // this warp's columns of the state
+  const int jt = warp >> 2, it = warp & 3;             // this warp's piece of E^T: tokens j of tile jt, tokens i of tile it
+  const bool lower = it >= jt;                         // whether some i >= j is in it
+  const int pt = warp & 7, side = warp >> 3;           // its piece of dx: columns 8 pt .. of the head, tokens of the tiles 0 and 3 or 1 and 2
   auto fetch = [&](int i) {
     uint8_t* st = stages + (i & 1) * LOCAL_STAGE;
     const int h = h0 + i;
-    load_tile<8, 256>(st, k.x + b * k.xb + t0 * k.xt + h * P, k.xt, real);
-    load_tile<8, 256>(st + L * P * 2, k.dy + ((static_cast<long long>(b) * k.T + t0) * k.H + h) * P, static_cast<long long>(k.H) * P, real);
+    load_tile<8, LOCAL_THREADS>(st, k.x + b * k.xb + t0 * k.xt + h * P, k.xt, real);
+    load_tile<8, LOCAL_THREADS>(st + L * P * 2, k.dy + ((static_cast<long long>(b) * k.T + t0) * k.H + h) * P, static_cast<long long>(k.H) * P, real);
     const long long cell = ((static_cast<long long>(b) * k.H + h) * k.chunks + n) * P * N;
     float* fs = reinterpret_cast<float*>(st + 2 * L * P * 2);
 #pragma unroll
-    for (int s = 0; s < P * N / 4 / 256; ++s) {
-      const int at = s * 256 + static_cast<int>(threadIdx.x), row = at >> 5, c = at & 31;
+    for (int s = 0; s < P * N / 4 / LOCAL_THREADS; ++s) {
+      const int at = s * LOCAL_THREADS + static_cast<int>(threadIdx.x), row = at >> 5, c = at & 31;
       cp16(fs + row * SLD + c * 4, states + cell + row * N + c * 4, true);
       cp16(fs + (P + row) * SLD + c * 4, dstates + cell + row * N + c * 4, true);
     }
     cp_commit();
   };
-  auto decays = [&](int i) {                           // warp 7
+  auto decays = [&](int i) {                           // the last warp
     const int t = t0 + 2 * lane;
     const float* dt = k.dt + static_cast<long long>(b) * k.T * k.H + h0 + i;
     const float a = t < k.T ? dt[static_cast<long long>(t) * k.H] : 0.f, c = t + 1 < k.T ? dt[static_cast<long long>(t + 1) * k.H] : 0.f;
     float g0, g1;
     running(a, c, k.A[h0 + i], g0, g1);
+    const float gl = __shfl_sync(FULL, g1, 31);
     *reinterpret_cast<float2*>(&sum.g[i & 1][2 * lane]) = make_float2(g0, g1);
     *reinterpret_cast<float2*>(&sum.dt[i & 1][2 * lane]) = make_float2(a, c);
+    *reinterpret_cast<float2*>(&sum.head[i & 1][2 * lane]) = make_float2(expf(g0), expf(g1));
+    *reinterpret_cast<float2*>(&sum.tail[i & 1][2 * lane]) = make_float2(expf(gl - g0), expf(gl - g1));
   };
-  load_tile<16, 256>(tC, k.Cm + b * k.cb + t0 * k.ct + grp * N, k.ct, real);
-  load_tile<16, 256>(tB, k.Bm + b * k.bb + t0 * k.bt + grp * N, k.bt, real);
+  load_tile<16, LOCAL_THREADS>(tC, k.Cm + b * k.cb + t0 * k.ct + grp * N, k.ct, real);
+  load_tile<16, LOCAL_THREADS>(tB, k.Bm + b * k.bb + t0 * k.bt + grp * N, k.bt, real);
   cp_commit();
   fetch(0);
-  if (warp == 7) decays(0);
-  for (int i = threadIdx.x; i < 6 * L; i += 256) (i < 4 * L ? &sum.rows[0][0] : &sum.cols[0][0] - 4 * L)[i] = 0.f;      // pieces above the diagonal write none
+  if (warp == LOCAL_WARPS - 1) decays(0);
+  if (threadIdx.x < 8 * L) (threadIdx.x < 4 * L ? &sum.rows[0][0] : &sum.cols[0][0] - 4 * L)[threadIdx.x] = 0.f;      // pieces above the diagonal write none
   cp_wait<1>();
   __syncthreads();
 
-  float G[4][4], W[4][4], dC[4][2][4], dB[4][2][4];
+  float G[2][4], W[2][4], dC[4][4], dB[4][4];
 #pragma unroll
-  for (int t = 0; t < 4; ++t)
+  for (int c = 0; c < 4; ++c) {
+    G[0][c] = G[1][c] = W[0][c] = W[1][c] = 0.f;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      G[t][c] = W[t][c] = 0.f;
-      dC[t][0][c] = dC[t][1][c] = dB[t][0][c] = dB[t][1][c] = 0.f;
-    }
+    for (int t = 0; t < 4; ++t) dC[t][c] = dB[t][c] = 0.f;
+  }
   if (lower) {
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks) {
-      uint32_t a[4], b0[4], b1[4];
+      uint32_t a[4], c[4];
       frag_a<16>(a, tB, jt * 16, ks);
-      frag_b<16>(b0, tC, ih * 32, ks);
-      frag_b<16>(b1, tC, ih * 32 + 16, ks);
-      mma(G[0], a, b0[0], b0[1]); mma(G[1], a, b0[2], b0[3]);
-      mma(G[2], a, b1[0], b1[1]); mma(G[3], a, b1[2], b1[3]);
+      frag_b<16>(c, tC, it * 16, ks);
+      mma(G[0], a, c[0], c[1]);
+      mma(G[1], a, c[2], c[3]);
     }
   }
 
   for (int i = 0; i < per; ++i) {
     cp_wait<0>();
     __syncthreads();                                   // this head has arrived, and nobody reads the one before it any more
-    if (i + 1 < per) { fetch(i + 1); if (warp == 7) decays(i + 1); }
+    if (i + 1 < per) { fetch(i + 1); if (warp == LOCAL_WARPS - 1) decays(i + 1); }
     const int h = h0 + i;
     const uint8_t *tx = stages + (i & 1) * LOCAL_STAGE, *ty = tx + L * P * 2;
     const float *S = reinterpret_cast<const float*>(ty + L * P * 2), *dS = S + P * SLD;
-    const float *g = sum.g[i & 1], *dt = sum.dt[i & 1];
-    const float gl = g[L - 1];
+    const float *g = sum.g[i & 1], *dt = sum.dt[i & 1], *head = sum.head[i & 1], *tail = sum.tail[i & 1];
 
     if (lower) {
       // ---- E^T = x dy^T of this piece, then M^T, W^T and the sums of M o E
-      float E[4][4];
-#pragma unroll
-      for (int t = 0; t < 4; ++t)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) E[t][c] = 0.f;
+      float E[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks) {
-        uint32_t a[4], b0[4], b1[4];
+        uint32_t a[4], c[4];
         frag_a<8>(a, tx, jt * 16, ks);
-        frag_b<8>(b0, ty, ih * 32, ks);
-        frag_b<8>(b1, ty, ih * 32 + 16, ks);
-        mma(E[0], a, b0[0], b0[1]); mma(E[1], a, b0[2], b0[3]);
-        mma(E[2], a, b1[0], b1[1]); mma(E[3], a, b1[2], b1[3]);
+        frag_b<8>(c, ty, it * 16, ks);
+        mma(E[0], a, c[0], c[1]);
+        mma(E[1], a, c[2], c[3]);
       }
       const int j0 = jt * 16 + r, j1 = j0 + 8;
       const float gj0 = g[j0], gj1 = g[j1], d0 = dt[j0], d1 = dt[j1];
       float col0 = 0.f, col1 = 0.f;
+      uint8_t* to = tM + block_of(jt, it) * 1536 + lane * 16;
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const int i0 = ih * 32 + t * 8 + 2 * q;
+      for (int t = 0; t < 2; ++t) {
+        const int i0 = it * 16 + t * 8 + 2 * q;
         const float2 gi = *reinterpret_cast<const float2*>(g + i0);
         float m[4], row0 = 0.f, row1 = 0.f;
 #pragma unroll
@@ -481,135 +508,125 @@ ssd_local(Call k, const float* __restrict__ states, const float* __restrict__ ds
 #pragma unroll
         for (int o = 4; o < 32; o <<= 1) { row0 += __shfl_xor_sync(FULL, row0, o); row1 += __shfl_xor_sync(FULL, row1, o); }
         if (r == 0) *reinterpret_cast<float2*>(&sum.rows[jt][i0]) = make_float2(row0, row1);
-        // a pair of column tiles is one A fragment of M^T
-        const int it = ih * 2 + (t >> 1);
-        if (it >= jt) {
-          uint32_t hi[2], mid[2], lo[2];
-          split3(m[0], m[1], hi[0], mid[0], lo[0]);
-          split3(m[2], m[3], hi[1], mid[1], lo[1]);
-          uint8_t* to = tM + block_of(jt, it) * 1536 + lane * 16 + (t & 1) * 8;
-          *reinterpret_cast<uint2*>(to) = make_uint2(hi[0], hi[1]);
-          *reinterpret_cast<uint2*>(to + 512) = make_uint2(mid[0], mid[1]);
-          *reinterpret_cast<uint2*>(to + 1024) = make_uint2(lo[0], lo[1]);
-        }
+        // the pair of column tiles is one A fragment of M^T
+        uint32_t hi[2], mid[2], lo[2];
+        split3(m[0], m[1], hi[0], mid[0], lo[0]);
+        split3(m[2], m[3], hi[1], mid[1], lo[1]);
+        *reinterpret_cast<uint2*>(to + t * 8) = make_uint2(hi[0], hi[1]);
+        *reinterpret_cast<uint2*>(to + 512 + t * 8) = make_uint2(mid[0], mid[1]);
+        *reinterpret_cast<uint2*>(to + 1024 + t * 8) = make_uint2(lo[0], lo[1]);
       }
       col0 += __shfl_xor_sync(FULL, col0, 1); col0 += __shfl_xor_sync(FULL, col0, 2);
       col1 += __shfl_xor_sync(FULL, col1, 1); col1 += __shfl_xor_sync(FULL, col1, 2);
-      if (q == 0) { sum.cols[ih][j0] = col0; sum.cols[ih][j1] = col1; }
+      if (q == 0) { sum.cols[it][j0] = col0; sum.cols[it][j1] = col1; }
     }
 
-    // ---- (dy S) and (x dS): this warp's 16 columns of all tokens
+    // ---- (dy S) and (x dS): this warp's 8 columns of all tokens
     float both = 0.f;
 #pragma unroll
     for (int which = 0; which < 2; ++which) {
-      const float* F = which ? dS : S;
-      uint32_t f[3][4][2][2];
+      const float* F = (which ? dS : S) + 2 * q * SLD + warp * 8 + r;
+      uint32_t f[3][4][2];
 #pragma unroll
-      for (int ks = 0; ks < 4; ++ks)
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          const float* at = F + (ks * 16 + 2 * q) * SLD + nc + t * 8 + r;
-          const float v0 = at[0], v1 = at[SLD], v2 = at[8 * SLD], v3 = at[9 * SLD];
-          if (which) {
-            const float* o = S + (ks * 16 + 2 * q) * SLD + nc + t * 8 + r;
-            both += v0 * o[0] + v1 * o[SLD] + v2 * o[8 * SLD] + v3 * o[9 * SLD];
-          }
-          split3(v0, v1, f[0][ks][t][0], f[1][ks][t][0], f[2][ks][t][0]);
-          split3(v2, v3, f[0][ks][t][1], f[1][ks][t][1], f[2][ks][t][1]);
+      for (int ks = 0; ks < 4; ++ks) {
+        const float* at = F + ks * 16 * SLD;
+        const float v0 = at[0], v1 = at[SLD], v2 = at[8 * SLD], v3 = at[9 * SLD];
+        if (which) {
+          const float* o = at - P * SLD;
+          both += v0 * o[0] + v1 * o[SLD] + v2 * o[8 * SLD] + v3 * o[9 * SLD];
         }
+        split3(v0, v1, f[0][ks][0], f[1][ks][0], f[2][ks][0]);
+        split3(v2, v3, f[0][ks][1], f[1][ks][1], f[2][ks][1]);
+      }
       const uint8_t *tu = which ? tx : ty, *tw = which ? tB : tC;
 #pragma unroll
       for (int mt = 0; mt < 4; ++mt) {
+        // two sums side by side, so that a product need not wait for the one before it
+        float u[4] = {0.f, 0.f, 0.f, 0.f}, u2[4] = {0.f, 0.f, 0.f, 0.f};
         uint32_t a[4][4];
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) frag_a<8>(a[ks], tu, mt * 16, ks);
-        float u[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
         for (int term = 2; term >= 0; --term)
 #pragma unroll
-          for (int ks = 0; ks < 4; ++ks) {
-            mma(u[0], a[ks], f[term][ks][0][0], f[term][ks][0][1]);
-            mma(u[1], a[ks], f[term][ks][1][0], f[term][ks][1][1]);
+          for (int ks = 0; ks < 4; ks += 2) {
+            mma(u, a[ks], f[term][ks][0], f[term][ks][1]);
+            mma(u2, a[ks + 1], f[term][ks + 1][0], f[term][ks + 1][1]);
           }
-        const int i0 = mt * 16 + r, i1 = i0 + 8;
-        const float s0 = which ? dt[i0] * expf(gl - g[i0]) : expf(g[i0]), s1 = which ? dt[i1] * expf(gl - g[i1]) : expf(g[i1]);
-        float dot0 = 0.f, dot1 = 0.f;
 #pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          const uint32_t w0 = *reinterpret_cast<const uint32_t*>(tw + piece<16>(i0, warp * 2 + t) + q * 4), w1 = *reinterpret_cast<const uint32_t*>(tw + piece<16>(i1, warp * 2 + t) + q * 4);
-          dot0 += u[t][0] * lo_f(w0) + u[t][1] * hi_f(w0);
-          dot1 += u[t][2] * lo_f(w1) + u[t][3] * hi_f(w1);
-          float(&to)[4] = which ? dB[mt][t] : dC[mt][t];
-          to[0] = fmaf(s0, u[t][0], to[0]); to[1] = fmaf(s0, u[t][1], to[1]);
-          to[2] = fmaf(s1, u[t][2], to[2]); to[3] = fmaf(s1, u[t][3], to[3]);
-        }
+        for (int c = 0; c < 4; ++c) u[c] += u2[c];
+        const int i0 = mt * 16 + r, i1 = i0 + 8;
+        const float s0 = which ? dt[i0] * tail[i0] : head[i0], s1 = which ? dt[i1] * tail[i1] : head[i1];
+        const uint32_t w0 = *reinterpret_cast<const uint32_t*>(tw + piece<16>(i0, warp) + q * 4), w1 = *reinterpret_cast<const uint32_t*>(tw + piece<16>(i1, warp) + q * 4);
+        float dot0 = u[0] * lo_f(w0) + u[1] * hi_f(w0), dot1 = u[2] * lo_f(w1) + u[3] * hi_f(w1);
+        float(&to)[4] = which ? dB[mt] : dC[mt];
+        to[0] = fmaf(s0, u[0], to[0]); to[1] = fmaf(s0, u[1], to[1]);
+        to[2] = fmaf(s1, u[2], to[2]); to[3] = fmaf(s1, u[3], to[3]);
         dot0 += __shfl_xor_sync(FULL, dot0, 1); dot0 += __shfl_xor_sync(FULL, dot0, 2);
         dot1 += __shfl_xor_sync(FULL, dot1, 1); dot1 += __shfl_xor_sync(FULL, dot1, 2);
         if (q == 0) {
-          float* to = which ? sum.x_state[warp] : sum.dy_state[warp];
-          to[i0] = dot0; to[i1] = dot1;
+          float* at = which ? sum.x_state[warp] : sum.dy_state[warp];
+          at[i0] = dot0; at[i1] = dot1;
         }
       }
     }
     both = warp_sum(both);
     if (lane == 0) sum.both[warp] = both;
 
-    // ---- dx: this warp's 8 of the head's 64 columns.  First through the state: B dS^T
-    float X[4][4];
-#pragma unroll
-    for (int mt = 0; mt < 4; ++mt)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) X[mt][c] = 0.f;
+    // ---- dx of this warp's piece.  First through the state: B dS^T
+    float X[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks) {
-      const float* at = dS + (warp * 8 + r) * SLD + ks * 16 + 2 * q;
+      const float* at = dS + (pt * 8 + r) * SLD + ks * 16 + 2 * q;
       const float2 v0 = *reinterpret_cast<const float2*>(at), v1 = *reinterpret_cast<const float2*>(at + 8);
       uint32_t f[3][2];
       split3(v0.x, v0.y, f[0][0], f[1][0], f[2][0]);
       split3(v1.x, v1.y, f[0][1], f[1][1], f[2][1]);
+      uint32_t a[2][4];
 #pragma unroll
-      for (int mt = 0; mt < 4; ++mt) {
-        uint32_t a[4];
-        frag_a<16>(a, tB, mt * 16, ks);
-        mma(X[mt], a, f[2][0], f[2][1]);
-        mma(X[mt], a, f[1][0], f[1][1]);
-        mma(X[mt], a, f[0][0], f[0][1]);
-      }
+      for (int m = 0; m < 2; ++m) frag_a<16>(a[m], tB, (m ? 3 - side : side) * 16, ks);
+#pragma unroll
+      for (int term = 2; term >= 0; --term)
+#pragma unroll
+        for (int m = 0; m < 2; ++m) mma(X[m], a[m], f[term][0], f[term][1]);
     }
 #pragma unroll
-    for (int mt = 0; mt < 4; ++mt) {
-      const float s0 = expf(gl - g[mt * 16 + r]), s1 = expf(gl - g[mt * 16 + r + 8]);
-      X[mt][0] *= s0; X[mt][1] *= s0; X[mt][2] *= s1; X[mt][3] *= s1;
+    for (int m = 0; m < 2; ++m) {
+      const int j = (m ? 3 - side : side) * 16 + r;
+      X[m][0] *= tail[j]; X[m][1] *= tail[j]; X[m][2] *= tail[j + 8]; X[m][3] *= tail[j + 8];
     }
     __syncthreads();
     // then through the chunk's own tokens: M^T dy
     uint32_t yb[2][4];
 #pragma unroll
-    for (int s = 0; s < 2; ++s) ldsm4_t(yb[s], smem_addr(ty + piece<8>(s * 32 + lane, warp)));
+    for (int s = 0; s < 2; ++s) ldsm4_t(yb[s], smem_addr(ty + piece<8>(s * 32 + lane, pt)));
 #pragma unroll
-    for (int mt = 0; mt < 4; ++mt)
+    for (int m = 0; m < 2; ++m) {
+      const int mt = m ? 3 - side : side;
 #pragma unroll
-      for (int it = mt; it < 4; ++it) {
-        const uint8_t* at = tM + block_of(mt, it) * 1536 + lane * 16;
+      for (int ks = 0; ks < 4; ++ks) {
+        if (ks < mt) continue;
+        const uint8_t* at = tM + block_of(mt, ks) * 1536 + lane * 16;
 #pragma unroll
         for (int term = 2; term >= 0; --term) {
           // (stored by column tile: rows r and r + 8 of the first, then of the second, which is the fragment's order)
           const uint4 w = *reinterpret_cast<const uint4*>(at + term * 512);
           const uint32_t a[4] = {w.x, w.y, w.z, w.w};
-          mma(X[mt], a, yb[it >> 1][(it & 1) * 2], yb[it >> 1][(it & 1) * 2 + 1]);
+          mma(X[m], a, yb[ks >> 1][(ks & 1) * 2], yb[ks >> 1][(ks & 1) * 2 + 1]);
         }
       }
+    }
     const float D = k.D == nullptr ? 0.f : k.D[h];
 #pragma unroll
-    for (int mt = 0; mt < 4; ++mt)
+    for (int m = 0; m < 2; ++m)
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
-        const int j = mt * 16 + r + half * 8;
-        const uint32_t w = *reinterpret_cast<const uint32_t*>(ty + piece<8>(j, warp) + q * 4);
+        const int j = (m ? 3 - side : side) * 16 + r + half * 8;
+        const uint32_t w = *reinterpret_cast<const uint32_t*>(ty + piece<8>(j, pt) + q * 4);
         const float d = dt[j];
         if (j < real)
-          *reinterpret_cast<uint32_t*>(out.dx + ((static_cast<long long>(b) * k.T + t0 + j) * k.H + h) * P + warp * 8 + 2 * q) =
-              pack2(fmaf(D, lo_f(w), d * X[mt][half * 2]), fmaf(D, hi_f(w), d * X[mt][half * 2 + 1]));
+          *reinterpret_cast<uint32_t*>(out.dx + ((static_cast<long long>(b) * k.T + t0 + j) * k.H + h) * P + pt * 8 + 2 * q) =
+              pack2(fmaf(D, lo_f(w), d * X[m][half * 2]), fmaf(D, hi_f(w), d * X[m][half * 2 + 1]));
       }
     if (warp == 0) {
       // ---- the decays: dg_i from what the token receives less what it gives, its sums to the chunk's end are the gradients of dt A
@@ -619,19 +636,19 @@ ssd_local(Call k, const float* __restrict__ states, const float* __restrict__ ds
         const int t = 2 * lane + e;
         float take = 0.f, give = 0.f;
 #pragma unroll
-        for (int w = 0; w < 8; ++w) { take += sum.dy_state[w][t]; give += sum.x_state[w][t]; }
+        for (int w = 0; w < LOCAL_WARPS; ++w) { take += sum.dy_state[w][t]; give += sum.x_state[w][t]; }
         d[e] = dt[t];
-        give *= expf(gl - g[t]);
+        give *= tail[t];
         given += d[e] * give;
-        const float own = sum.cols[0][t] + sum.cols[1][t] + give;
-        dg[e] = ((sum.rows[0][t] + sum.rows[1][t]) + (sum.rows[2][t] + sum.rows[3][t])) + expf(g[t]) * take - d[e] * own;
+        const float own = ((sum.cols[0][t] + sum.cols[1][t]) + (sum.cols[2][t] + sum.cols[3][t])) + give;
+        dg[e] = ((sum.rows[0][t] + sum.rows[1][t]) + (sum.rows[2][t] + sum.rows[3][t])) + head[t] * take - d[e] * own;
         direct[e] = own + sum.diag[t];
       }
       given = warp_sum(given);
       float held = 0.f;
 #pragma unroll
-      for (int w = 0; w < 8; ++w) held += sum.both[w];
-      if (lane == 31) dg[1] += expf(gl) * held + given;
+      for (int w = 0; w < LOCAL_WARPS; ++w) held += sum.both[w];
+      if (lane == 31) dg[1] += head[L - 1] * held + given;
       float suffix = dg[0] + dg[1];
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -659,17 +676,22 @@ ssd_local(Call k, const float* __restrict__ states, const float* __restrict__ ds
   float* tW = reinterpret_cast<float*>(stages);
   constexpr int WLD = L + 4;
 #pragma unroll
-  for (int t = 0; t < 4; ++t) {
-    float* at = tW + (jt * 16 + r) * WLD + ih * 32 + t * 8 + 2 * q;
+  for (int t = 0; t < 2; ++t) {
+    float* at = tW + (jt * 16 + r) * WLD + it * 16 + t * 8 + 2 * q;
     *reinterpret_cast<float2*>(at) = make_float2(W[t][0], W[t][1]);
     *reinterpret_cast<float2*>(at + 8 * WLD) = make_float2(W[t][2], W[t][3]);
   }
   __syncthreads();
+  uint32_t fB[2][4], fC[2][4];
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    ldsm4_t(fB[s], smem_addr(tB + piece<16>(s * 32 + lane, warp)));
+    ldsm4_t(fC[s], smem_addr(tC + piece<16>(s * 32 + lane, warp)));
+  }
 #pragma unroll
   for (int mt = 0; mt < 4; ++mt)
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) {
-      uint32_t f[4];
       if (ks <= mt) {                                  // dC_i += sum_j W_ij B_j
         const float* at = tW + (ks * 16 + 2 * q) * WLD + mt * 16 + r;
         uint32_t a[3][4];
@@ -677,9 +699,8 @@ ssd_local(Call k, const float* __restrict__ states, const float* __restrict__ ds
         split3(at[8], at[WLD + 8], a[0][1], a[1][1], a[2][1]);
         split3(at[8 * WLD], at[9 * WLD], a[0][2], a[1][2], a[2][2]);
         split3(at[8 * WLD + 8], at[9 * WLD + 8], a[0][3], a[1][3], a[2][3]);
-        frag_b_t<16>(f, tB, ks, warp * 2);
 #pragma unroll
-        for (int term = 2; term >= 0; --term) { mma(dC[mt][0], a[term], f[0], f[1]); mma(dC[mt][1], a[term], f[2], f[3]); }
+        for (int term = 2; term >= 0; --term) mma(dC[mt], a[term], fB[ks >> 1][(ks & 1) * 2], fB[ks >> 1][(ks & 1) * 2 + 1]);
       }
       if (ks >= mt) {                                  // dB_j += sum_i W_ij C_i
         const float* at = tW + (mt * 16 + r) * WLD + ks * 16 + 2 * q;
@@ -688,9 +709,8 @@ ssd_local(Call k, const float* __restrict__ states, const float* __restrict__ ds
         split3(at[8 * WLD], at[8 * WLD + 1], a[0][1], a[1][1], a[2][1]);
         split3(at[8], at[9], a[0][2], a[1][2], a[2][2]);
         split3(at[8 * WLD + 8], at[8 * WLD + 9], a[0][3], a[1][3], a[2][3]);
-        frag_b_t<16>(f, tC, ks, warp * 2);
 #pragma unroll
-        for (int term = 2; term >= 0; --term) { mma(dB[mt][0], a[term], f[0], f[1]); mma(dB[mt][1], a[term], f[2], f[3]); }
+        for (int term = 2; term >= 0; --term) mma(dB[mt], a[term], fC[ks >> 1][(ks & 1) * 2], fC[ks >> 1][(ks & 1) * 2 + 1]);
       }
     }
 #pragma unroll
@@ -699,18 +719,15 @@ ssd_local(Call k, const float* __restrict__ states, const float* __restrict__ ds
     for (int half = 0; half < 2; ++half) {
       const int t = mt * 16 + r + half * 8;
       if (t >= real) continue;
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const long long at = ((static_cast<long long>(b) * k.T + t0 + t) * k.G + grp) * N + nc + c * 8 + 2 * q;
-        const float b0 = dB[mt][c][half * 2], b1 = dB[mt][c][half * 2 + 1], c0 = dC[mt][c][half * 2], c1 = dC[mt][c][half * 2 + 1];
-        if (out.partB == nullptr) {
-          *reinterpret_cast<uint32_t*>(out.dB + at) = pack2(b0, b1);
-          *reinterpret_cast<uint32_t*>(out.dC + at) = pack2(c0, c1);
-        } else {
-          const long long part = blockIdx.z * (static_cast<long long>(k.B) * k.T * k.G * N);
-          *reinterpret_cast<float2*>(out.partB + part + at) = make_float2(b0, b1);
-          *reinterpret_cast<float2*>(out.partC + part + at) = make_float2(c0, c1);
-        }
+      const long long at = ((static_cast<long long>(b) * k.T + t0 + t) * k.G + grp) * N + warp * 8 + 2 * q;
+      const float b0 = dB[mt][half * 2], b1 = dB[mt][half * 2 + 1], c0 = dC[mt][half * 2], c1 = dC[mt][half * 2 + 1];
+      if (out.partB == nullptr) {
+        *reinterpret_cast<uint32_t*>(out.dB + at) = pack2(b0, b1);
+        *reinterpret_cast<uint32_t*>(out.dC + at) = pack2(c0, c1);
+      } else {
+        const long long part = blockIdx.z * (static_cast<long long>(k.B) * k.T * k.G * N);
+        *reinterpret_cast<float2*>(out.partB + part + at) = make_float2(b0, b1);
+        *reinterpret_cast<float2*>(out.partC + part + at) = make_float2(c0, c1);
       }
     }
 }
@@ -748,23 +765,26 @@ ssd_reduce(Grads g, float* __restrict__ dA, float* __restrict__ dD, int H, int p
   }
 }
 
-template <int NT, int TERMS, bool REV, typename Out>
-static int run_states(const Call& k, const float* initial, Out* states, float* last, cudaStream_t stream) {
-  auto fn = ssd_states<NT, TERMS, REV, Out>;
-  constexpr int bytes = 2 * (L * P * 2 + L * NT * 16);
+template <typename Out>
+struct Walk { const float* initial; Out* states; float* last; };
+
+template <int NT, int TERMS, typename Out>
+static int run_states(const Call& k, const Walk<Out>& forward, const Walk<Out>* reverse, cudaStream_t stream) {
+  auto fn = ssd_states<NT, TERMS, Out>;
+  constexpr int bytes = WALK_STAGES * (L * P * 2 + L * NT * 16);
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e != cudaSuccess) return static_cast<int>(e);
-  fn<<<dim3(k.B * k.H, 16 / NT), 128, bytes, stream>>>(k, initial, states, last);
+  const Walk<Out> none{nullptr, nullptr, nullptr}, &back = reverse == nullptr ? none : *reverse;
+  fn<<<dim3(k.B * k.H, 16 / NT, reverse == nullptr ? 1 : 2), WALK_THREADS, bytes, stream>>>(k, forward.initial, forward.states, forward.last, back.initial, back.states, back.last);
   return static_cast<int>(cudaGetLastError());
 }
 
-// As many columns a CTA as leave every SM one: a chunk's step of a quarter of the columns is a chain not much shorter than that of all of them.
-template <int TERMS, bool REV, typename Out>
-static int walk(const Call& k, const float* initial, Out* states, float* last, cudaStream_t stream) {
-  const int rows = k.B * k.H;
-  if (rows * 2 <= SMS) return run_states<4, TERMS, REV, Out>(k, initial, states, last, stream);
-  if (rows <= SMS) return run_states<8, TERMS, REV, Out>(k, initial, states, last, stream);
-  return run_states<16, TERMS, REV, Out>(k, initial, states, last, stream);
+// A quarter of the columns a CTA while that leaves every SM no more than two of them, else half (two more resident CTAs hide what a step's chain waits for, and a
+// step of half the columns scales and splits half as often as two of a quarter).
+template <int TERMS, typename Out>
+static int walk(const Call& k, const Walk<Out>& forward, const Walk<Out>* reverse, cudaStream_t stream) {
+  const int rows = k.B * k.H * (reverse == nullptr ? 1 : 2);
+  return rows * 4 <= 2 * SMS ? run_states<4, TERMS, Out>(k, forward, reverse, stream) : run_states<8, TERMS, Out>(k, forward, reverse, stream);
 }
 
 static int check(const Call& k) {
@@ -803,7 +823,8 @@ extern "C" int dewb_ssd_fwd(const void* x, const float* dt, const float* A, cons
   int e = check(k);
   if (e) return e;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
-  if ((e = walk<1, false, __nv_bfloat16>(k, initial, static_cast<__nv_bfloat16*>(states), last, stream))) return e;
+  const Walk<__nv_bfloat16> forward{initial, static_cast<__nv_bfloat16*>(states), last};
+  if ((e = walk<1, __nv_bfloat16>(k, forward, nullptr, stream))) return e;
   int splits = 1;                                      // two CTAs an SM
   while ((H / G) % (splits * 2) == 0 && static_cast<long long>(B) * k.chunks * G * splits < 2 * SMS) splits *= 2;
   cudaError_t c = cudaFuncSetAttribute(ssd_output, cudaFuncAttributeMaxDynamicSharedMemorySize, OUT_SMEM);
@@ -826,14 +847,14 @@ extern "C" int dewb_ssd_bwd(const void* x, const float* dt, const float* A, cons
   int e = check(k);
   if (e) return e;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
-  if ((e = walk<3, false, float>(k, initial, states, nullptr, stream))) return e;
-  if ((e = walk<3, true, float>(k, dlast, dstates, dinitial, stream))) return e;
+  const Walk<float> forward{initial, states, nullptr}, reverse{dlast, dstates, dinitial};
+  if ((e = walk<3, float>(k, forward, &reverse, stream))) return e;
   const int splits = dewb_ssd_splits(B, T, H, G);
   if (splits > 1 && (partB == nullptr || partC == nullptr)) return -3;
   const Grads g{static_cast<to>(dx), static_cast<to>(dB), static_cast<to>(dC), ddt, splits > 1 ? partB : nullptr, splits > 1 ? partC : nullptr, partA, partD};
   cudaError_t c = cudaFuncSetAttribute(ssd_local, cudaFuncAttributeMaxDynamicSharedMemorySize, LOCAL_SMEM);
   if (c != cudaSuccess) return static_cast<int>(c);
-  ssd_local<<<dim3(B * k.chunks, G, splits), 256, LOCAL_SMEM, stream>>>(k, states, dstates, g, H / G / splits);
+  ssd_local<<<dim3(B * k.chunks, G, splits), LOCAL_THREADS, LOCAL_SMEM, stream>>>(k, states, dstates, g, H / G / splits);
   if ((c = cudaGetLastError()) != cudaSuccess) return static_cast<int>(c);
   const long long total = splits > 1 ? static_cast<long long>(B) * T * G * N : 0;
   ssd_reduce<<<static_cast<unsigned>(H + (total / 4 + 255) / 256), 256, 0, stream>>>(g, dA, dD, H, B * k.chunks, total, splits);

@@ -269,7 +269,7 @@ def scan_fwd_cuda(q, k, gc, W, U, P, scale: float, initial_state, save_states: b
     rep = H // q.shape[2]
     N = (T + CHUNK - 1) // CHUNK
     dev = q.device
-    o = torch.empty(B, T, H, HEAD_DIM, dtype=torch.bfloat16, device=dev)
+    o = None if save_vn else torch.empty(B, T, H, HEAD_DIM, dtype=torch.bfloat16, device=dev)      # the backward's walk has no use for it
     final = torch.empty(X, HEAD_DIM, HEAD_DIM, dtype=torch.float32, device=dev)
     states = torch.empty(X, N, HEAD_DIM, HEAD_DIM, dtype=torch.bfloat16, device=dev) if save_states else None
     vn = None

@@ -23,7 +23,7 @@
 // A CTA fills an SM's shared memory, so neither kernel is bound by a unit but by the chain inside a CTA: loads, products, a row of each block a thread, sums.  The
 // state kernel therefore gives the sums over the features that need no solve to four warps of their own, which also fetch the second chunk and issue its products
 // while the first is being solved; the pair kernel has sixteen warps, four a row, and orders its loads so that the second batch flies while the first is multiplied.
-// Measured at 2 x 8192 tokens of 16 heads, with eight warps in turn and now: state 1133 -> 811 us, pair 1054 -> 229 us.
+// Measured at 2 x 8192 tokens of 16 heads, with eight warps in turn and now: state 1133 -> 405 us, pair 1054 -> 229 us.
 #include "../common/ptx.cuh"
 #include "../common/tmap.h"
 
@@ -56,11 +56,11 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// v[k] holds this lane's term for token k (32 tokens); on return lane l holds the sum over the warp of token l's terms.
-// 31 shuffles for 32 sums (a butterfly that halves the token set at every step) instead of 5 per sum.
-__device__ __forceinline__ float reduce_scatter32(float (&v)[32], int lane) {
+// v[k] holds this lane's term for token k (16 tokens); on return lanes l and l + 16 hold the sum over the warp of token l's terms.
+// 16 shuffles for 16 sums (a butterfly that halves the token set at every step) instead of 5 per sum.
+__device__ __forceinline__ float reduce_scatter16(float (&v)[16], int lane) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
+  for (int o = 8; o > 0; o >>= 1) {
     const bool upper = (lane & o) != 0;
 #pragma unroll
     for (int k = 0; k < o; ++k) {
@@ -69,7 +69,7 @@ __device__ __forceinline__ float reduce_scatter32(float (&v)[32], int lane) {
       v[k] = keep + __shfl_xor_sync(FULL, send, o);
     }
   }
-  return v[0];
+  return v[0] + __shfl_xor_sync(FULL, v[0], 16);
 }
 
 // Four 8 x 8 pieces of bf16, plain and transposed, by the rows' addresses.
@@ -240,9 +240,7 @@ gdn_bwd_state_kernel(const __grid_constant__ CUtensorMap tk, const __grid_consta
     products(0);
   }
   if (warp < 8) {
-    // token row i: A[i][j] = beta_i (k_i . k_j) e^{g_i - g_j} (j < i), stored transposed: sAT[c][j][i], each row of the
-    // transpose rotated by four floats per row so that the solve's broadcast float4 reads stay aligned and these
-    // column-wise stores stay free of bank conflicts.  Half a row a thread.
+    // token row i: A[i][j] = beta_i (k_i . k_j) e^{g_i - g_j} (j < i), stored transposed: sAT[c][j][i].  Half a row a thread.
     const int i = f, c = i >> 6, il = i & 63, j0 = (warp >> 2) * 32;
     const bool got = mbar_wait(bar_kk, 0, abort_flag);
     if (__all_sync(FULL, got)) {
@@ -255,7 +253,7 @@ gdn_bwd_state_kernel(const __grid_constant__ CUtensorMap tk, const __grid_consta
 #pragma unroll
       for (int jj = 0; jj < 32; ++jj) {
         const int j = j0 + jj;
-        at[j * CH + ((il + 4 * j) & 63)] = j < il ? bi * __uint_as_float(v[jj]) * __expf(gi - tail->g[c * 64 + j]) : 0.f;
+        at[j * CH + il] = j < il ? bi * __uint_as_float(v[jj]) * __expf(gi - tail->g[c * 64 + j]) : 0.f;
       }
     } else if (lane == 0) {
       atomicCAS(err, 0, ERR_WAIT_TMEM_FULL);
@@ -276,118 +274,133 @@ gdn_bwd_state_kernel(const __grid_constant__ CUtensorMap tk, const __grid_consta
     const uint32_t from = tmem + TM_SET + c * TM_LEN + lane_addr;
     const long long trow = static_cast<long long>(x) * Tp + n * CH;
     if (warp < 8) {
-      float xs[CH];
+      // y[16 p ..]: the right-hand sides of the 16 rows of block 3 - p, and of block rb - p once the blocks behind rb are solved
+      float y[CH];
       if (warp < 4) {
         if (ok) {
-          uint32_t v0[32], v1[32];
-          tmem_ld_32x32b_x32(from + TM_DW, v0);
-          tmem_ld_32x32b_x32(from + TM_DW + 32, v1);
-          tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < CH; ++j) xs[j] = -__uint_as_float(j < 32 ? v0[j & 31] : v1[j & 31]);
+          for (int p = 0; p < 4; ++p) {
+            uint32_t v0[16];
+            tmem_ld_32x32b_x16(from + TM_DW + (3 - p) * 16, v0);
+            tmem_ld_wait();
+#pragma unroll
+            for (int ii = 0; ii < 16; ++ii) y[p * 16 + ii] = -__uint_as_float(v0[ii]);
+          }
         }
       } else {
         if (ok) {
 #pragma unroll
-          for (int j = 0; j < CH; ++j) xs[j] = tile_get(sdVn, CH, j, f);
+          for (int k = 0; k < CH; ++k) y[k] = tile_get(sdVn, CH, (3 - (k >> 4)) * 16 + (k & 15), f);
         }
       }
       if (c + 1 < chunks) asm volatile("bar.arrive 3, 384;" ::: "memory");        // past this chunk's waits, and the tile of dVn is free
-      if (ok) {
-        // back substitution: x_i = r_i - sum_{j > i} A[j][i] x_j  (xs holds r, then x)
-        const float* at = sAT + c * (CH * CH);
+      bool got = true;
+      if (warp >= 4) {
+        got = __all_sync(FULL, mbar_wait(bar_v, c, abort_flag));
+        if (!got && lane == 0) atomicCAS(err, 0, ERR_WAIT_FULL);
+      }
+      if (ok && got) {
+        // Back substitution x_i = r_i - sum_{j > i} A[j][i] x_j by blocks of 16 rows, what follows from a block's x in the same turn, so that one loop of 16 rows is all
+        // the code there is: unrolled over the 64 rows, code of more than 100 KB went by once a chunk and the warps waited for it (no instruction for half of all cycles: 790 us instead of 405)
+        const float gl = tail->g[c * 64 + 63];
+#pragma unroll 1
+        for (int rb = 3; rb >= 0; --rb) {
+          const float* at = sAT + c * (CH * CH) + rb * 16 * CH + rb * 16;
 #pragma unroll
-        for (int i = CH - 2; i >= 0; --i) {
-          float acc = xs[i], acc1 = 0.f;                   // two chains: half the dependent latency per row
-          const float4* arow = reinterpret_cast<const float4*>(at + i * CH);
+          for (int i = 14; i >= 0; --i) {
+            float acc = y[i], acc1 = 0.f;                  // two chains: half the dependent latency per row
 #pragma unroll
-          for (int j4 = (i + 1) >> 2; j4 < 16; ++j4) {
-            const float4 av = arow[(j4 + i) & 15];
-            if (j4 * 4 + 0 > i) acc = fmaf(-av.x, xs[j4 * 4 + 0], acc);
-            if (j4 * 4 + 1 > i) acc1 = fmaf(-av.y, xs[j4 * 4 + 1], acc1);
-            if (j4 * 4 + 2 > i) acc = fmaf(-av.z, xs[j4 * 4 + 2], acc);
-            if (j4 * 4 + 3 > i) acc1 = fmaf(-av.w, xs[j4 * 4 + 3], acc1);
+            for (int j4 = (i + 1) >> 2; j4 < 4; ++j4) {
+              const float4 av = *reinterpret_cast<const float4*>(at + i * CH + j4 * 4);
+              if (j4 * 4 + 0 > i) acc = fmaf(-av.x, y[j4 * 4 + 0], acc);
+              if (j4 * 4 + 1 > i) acc1 = fmaf(-av.y, y[j4 * 4 + 1], acc1);
+              if (j4 * 4 + 2 > i) acc = fmaf(-av.z, y[j4 * 4 + 2], acc);
+              if (j4 * 4 + 3 > i) acc1 = fmaf(-av.w, y[j4 * 4 + 3], acc1);
+            }
+            y[i] = acc + acc1;
           }
-          xs[i] = acc + acc1;
+          const int j0 = rb * 16, r0 = c * 64 + j0, t1 = n * CH + j0;
+          float p1[16];
+          if (warp < 4) {
+            // dKt column; dk_part = e^{g_L - g} dKd + beta e^g dKt; its sum over the key index
+            uint32_t v0[16];
+            tmem_ld_32x32b_x16(from + TM_DKD + j0, v0);
+            tmem_ld_wait();
+            __nv_bfloat16* to = dKt + (trow + j0) * HD + f;
+            float* part = dk_part + ((static_cast<long long>(b) * T + t1) * H + h) * HD + f;
+#pragma unroll
+            for (int jj = 0; jj < 16; ++jj) {
+              const float dkd = __expf(gl - tail->g[r0 + jj]) * __uint_as_float(v0[jj]);
+              to[jj * HD] = __float2bfloat16(y[jj]);
+              if (t1 + jj < T) part[static_cast<long long>(jj) * H * HD] = dkd + tail->beta[r0 + jj] * tail->eg[r0 + jj] * y[jj];
+              p1[jj] = y[jj] * tile_get(sK, PT, r0 + jj, f);
+            }
+            const float sum = reduce_scatter16(p1, lane);
+            if (lane < 16) tail->sum_k[warp][r0 + lane] = sum;
+          } else {
+            __nv_bfloat16 *to = dVt + (trow + j0) * HD + f, *out = dv + ((static_cast<long long>(b) * T + t1) * H + h) * HD + f;
+#pragma unroll
+            for (int jj = 0; jj < 16; ++jj) {
+              to[jj * HD] = __float2bfloat16(y[jj]);
+              if (t1 + jj < T) out[static_cast<long long>(jj) * H * HD] = __float2bfloat16(tail->beta[r0 + jj] * y[jj]);
+              p1[jj] = y[jj] * tile_get(sV, CH, j0 + jj, f);
+            }
+            const float sum = reduce_scatter16(p1, lane);
+            if (lane < 16) tail->sum_v[warp & 3][r0 + lane] = sum;
+          }
+          // the rows above take this block's share
+#pragma unroll
+          for (int p = 1; p < 4; ++p) {
+            if (p > rb) break;
+#pragma unroll
+            for (int ii = 0; ii < 16; ++ii) {
+              float acc = y[p * 16 + ii];
+#pragma unroll
+              for (int j4 = 0; j4 < 4; ++j4) {
+                const float4 av = *reinterpret_cast<const float4*>(at + (ii - p * 16) * CH + j4 * 4);
+                acc = fmaf(-av.x, y[j4 * 4 + 0], acc);
+                acc = fmaf(-av.y, y[j4 * 4 + 1], acc);
+                acc = fmaf(-av.z, y[j4 * 4 + 2], acc);
+                acc = fmaf(-av.w, y[j4 * 4 + 3], acc);
+              }
+              y[p * 16 + ii] = acc;
+            }
+          }
+#pragma unroll
+          for (int k = 0; k < CH - 16; ++k) y[k] = y[k + 16];
         }
       }
-      if (warp < 4) {
-        if (ok) {
-          // dKt column; dk_part = e^{g_L - g} dKd + beta e^g dKt; its sum over the key index
-          const float gl = tail->g[c * 64 + 63];
-#pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            uint32_t v0[32];
-            tmem_ld_32x32b_x32(from + TM_DKD + half * 32, v0);
-            tmem_ld_wait();
-            float p1[32];
-#pragma unroll
-            for (int jj = 0; jj < 32; ++jj) {
-              const int j = half * 32 + jj, r = c * 64 + j;
-              const float dkd = __expf(gl - tail->g[r]) * __uint_as_float(v0[jj]);
-              dKt[(trow + j) * HD + f] = __float2bfloat16(xs[j]);
-              const int t = n * CH + j;
-              if (t < T) dk_part[((static_cast<long long>(b) * T + t) * H + h) * HD + f] = dkd + tail->beta[r] * tail->eg[r] * xs[j];
-              p1[jj] = xs[j] * tile_get(sK, PT, r, f);
-            }
-            tail->sum_k[warp][c * 64 + half * 32 + lane] = reduce_scatter32(p1, lane);
-          }
-        }
-      } else {
-        const bool got = __all_sync(FULL, mbar_wait(bar_v, c, abort_flag));
-        if (!got && lane == 0) atomicCAS(err, 0, ERR_WAIT_FULL);
-        if (ok && got) {
-#pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            float p1[32];
-#pragma unroll
-            for (int jj = 0; jj < 32; ++jj) {
-              const int j = half * 32 + jj, r = c * 64 + j;
-              dVt[(trow + j) * HD + f] = __float2bfloat16(xs[j]);
-              const int t = n * CH + j;
-              if (t < T) dv[((static_cast<long long>(b) * T + t) * H + h) * HD + f] = __float2bfloat16(tail->beta[r] * xs[j]);
-              p1[jj] = xs[j] * tile_get(sV, CH, j, f);
-            }
-            tail->sum_v[warp & 3][c * 64 + half * 32 + lane] = reduce_scatter32(p1, lane);
-          }
-        }
-        if (c + 1 < chunks) {
-          asm volatile("bar.sync 4, 128;" ::: "memory");
-          if (tid == 128 && tail->abort_flag == 0) fetch_v(n + 1);
-          __syncwarp();
-        }
+      if (warp >= 4 && c + 1 < chunks) {
+        asm volatile("bar.sync 4, 128;" ::: "memory");
+        if (tid == 128 && tail->abort_flag == 0) fetch_v(n + 1);
+        __syncwarp();
       }
     } else {
       if (ok) {
         const float gl = tail->g[c * 64 + 63];
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          uint32_t v0[32];
-          float p1[32];
-          tmem_ld_32x32b_x32(from + TM_X1 + half * 32, v0);
+#pragma unroll 1
+        for (int j0 = 0; j0 < CH; j0 += 16) {
+          const int r0 = c * 64 + j0, t1 = n * CH + j0;
+          uint32_t v0[16], v1[16];
+          float p1[16], p2[16];
+          tmem_ld_32x32b_x16(from + TM_X1 + j0, v0);
+          tmem_ld_32x32b_x16(from + TM_DKD + j0, v1);
           tmem_ld_wait();
+          float* part = dq_part + ((static_cast<long long>(b) * T + t1) * H + h) * HD + f;
 #pragma unroll
-          for (int jj = 0; jj < 32; ++jj) {
-            const int j = half * 32 + jj, r = c * 64 + j;
-            const float dq1 = scale * tail->eg[r] * __uint_as_float(v0[jj]);
-            const int t = n * CH + j;
-            if (t < T) dq_part[((static_cast<long long>(b) * T + t) * H + h) * HD + f] = dq1;
-            p1[jj] = dq1 * tile_get(sQ, CH, j, f);
+          for (int jj = 0; jj < 16; ++jj) {
+            const float dq1 = scale * tail->eg[r0 + jj] * __uint_as_float(v0[jj]);
+            if (t1 + jj < T) part[static_cast<long long>(jj) * H * HD] = dq1;
+            p1[jj] = dq1 * tile_get(sQ, CH, j0 + jj, f);
+            p2[jj] = __expf(gl - tail->g[r0 + jj]) * __uint_as_float(v1[jj]) * tile_get(sK, PT, r0 + jj, f);
           }
-          tail->sum_q[warp & 3][c * 64 + half * 32 + lane] = reduce_scatter32(p1, lane);
-          tmem_ld_32x32b_x32(from + TM_DKD + half * 32, v0);
-          tmem_ld_wait();
-#pragma unroll
-          for (int jj = 0; jj < 32; ++jj) {
-            const int r = c * 64 + half * 32 + jj;
-            p1[jj] = __expf(gl - tail->g[r]) * __uint_as_float(v0[jj]) * tile_get(sK, PT, r, f);
-          }
-          tail->sum_kd[warp & 3][c * 64 + half * 32 + lane] = reduce_scatter32(p1, lane);
+          const float s1 = reduce_scatter16(p1, lane), s2 = reduce_scatter16(p2, lane);
+          if (lane < 16) { tail->sum_q[warp & 3][r0 + lane] = s1; tail->sum_kd[warp & 3][r0 + lane] = s2; }
         }
         // <dS1, S0>: 8 x 8 pieces of dS1 against pieces of the transposed state, transposed on the way to the registers.  A warp has 32 rows of dS1.
         float acc = 0.f;
         const int m = lane >> 3, r8 = lane & 7;
-#pragma unroll 4
+#pragma unroll 2
         for (int i = 0; i < 16; ++i) {                     // 32 keys by 8 values
           uint32_t a[4], s4[4];
           const int key = (warp & 3) * 32 + m * 8;

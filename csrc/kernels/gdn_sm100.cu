@@ -157,51 +157,44 @@ gdn_prepare_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   }
   // the other lanes of the issuing thread's warp park here instead of spinning on the barrier beside it
   if (warp == 0) __syncwarp();
-  if (warp < 4) {
-    // thread = token row i of the 128; its chunk's 64 columns of both score matrices
-    const int i = tid, c = i >> 6, il = i & 63;
+  {
+    // (half a row a thread of all eight warps: 213 -> 203 us for 2 x 8192 tokens of 16 heads; four warps did whole rows while four waited)
+    // token row i of the 128, and 32 of its chunk's 64 columns of both score matrices (half of its row of Q) a thread
+    const int i = tid & 127, c = i >> 6, il = i & 63, part = warp >> 2, j0 = part * 32;
     const bool got = mbar_wait(&tail->bar_mma, 0, abort_flag);
     if (!__all_sync(FULL, got)) { if (lane == 0) atomicCAS(err, 0, ERR_WAIT_TMEM_FULL); ok = false; }
-    const uint32_t lane_addr = static_cast<uint32_t>(warp * 32) << 16;
+    const uint32_t from = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + c * 64 + j0;
     const float gi = tail->g[i], bi = tail->beta[i];
     const long long row = static_cast<long long>(x) * Tp + t0 + i;
-    float a[CH];
+    float a[32];
     if (ok) {
       tc_fence_after();
-      uint32_t v0[32], v1[32];
-      // P row: scale * (q_i . k_j) * e^{g_i - g_j} for j <= i
-      tmem_ld_32x32b_x32(tmem + lane_addr + 128 + c * 64, v0);
-      tmem_ld_32x32b_x32(tmem + lane_addr + 128 + c * 64 + 32, v1);
+      uint32_t vp[32], va[32];
+      tmem_ld_32x32b_x32(from + 128, vp);
+      tmem_ld_32x32b_x32(from, va);
       tmem_ld_wait();
-      uint4* prow = reinterpret_cast<uint4*>(P + row * CH);
+      // P row: scale * (q_i . k_j) * e^{g_i - g_j} for j <= i;  A row: beta_i * (k_i . k_j) * e^{g_i - g_j} for j < i
+      uint4* prow = reinterpret_cast<uint4*>(P + row * CH + j0);
 #pragma unroll
-      for (int j8 = 0; j8 < 8; ++j8) {
+      for (int j8 = 0; j8 < 4; ++j8) {
         float p[8];
 #pragma unroll
         for (int jj = 0; jj < 8; ++jj) {
-          const int j = j8 * 8 + jj;
-          const float s = __uint_as_float(j < 32 ? v0[j & 31] : v1[j & 31]);
-          p[jj] = (j <= il) ? scale * s * __expf(gi - tail->g[c * 64 + j]) : 0.f;
+          const int at = j8 * 8 + jj, j = j0 + at;
+          const float decay = j <= il ? __expf(gi - tail->g[c * 64 + j]) : 0.f;
+          p[jj] = j <= il ? scale * __uint_as_float(vp[at]) * decay : 0.f;
+          a[at] = j < il ? bi * __uint_as_float(va[at]) * decay : 0.f;
         }
         uint4 pk;
         pk.x = pack_bf16(p[0], p[1]); pk.y = pack_bf16(p[2], p[3]); pk.z = pack_bf16(p[4], p[5]); pk.w = pack_bf16(p[6], p[7]);
         prow[j8] = pk;
       }
-      // A row: beta_i * (k_i . k_j) * e^{g_i - g_j} for j < i
-      tmem_ld_32x32b_x32(tmem + lane_addr + c * 64, v0);
-      tmem_ld_32x32b_x32(tmem + lane_addr + c * 64 + 32, v1);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < CH; ++j) {
-        const float s = __uint_as_float(j < 32 ? v0[j & 31] : v1[j & 31]);
-        a[j] = (j < il) ? bi * s * __expf(gi - tail->g[c * 64 + j]) : 0.f;
-      }
       if (Qg != nullptr) {
         const float m = scale * tail->eg[i];
-        uint4* qrow = reinterpret_cast<uint4*>(Qg + row * HD);
+        uint4* qrow = reinterpret_cast<uint4*>(Qg + row * HD + part * 64);
 #pragma unroll
-        for (int c16 = 0; c16 < 16; ++c16) {
-          const uint4 in = *reinterpret_cast<const uint4*>(sQ + (c16 >> 3) * (PT * 128) + swz(i, c16 & 7));
+        for (int c16 = 0; c16 < 8; ++c16) {
+          const uint4 in = *reinterpret_cast<const uint4*>(sQ + part * (PT * 128) + swz(i, c16));
           uint4 o;
           o.x = pack_bf16(bf16_lo(in.x) * m, bf16_hi(in.x) * m); o.y = pack_bf16(bf16_lo(in.y) * m, bf16_hi(in.y) * m);
           o.z = pack_bf16(bf16_lo(in.z) * m, bf16_hi(in.z) * m); o.w = pack_bf16(bf16_lo(in.w) * m, bf16_hi(in.w) * m);
@@ -209,15 +202,15 @@ gdn_prepare_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
         }
       }
     }
-    // every row of Q has been read (by the tensor core and by its thread) before A overwrites the tile
-    named_barrier_sync(1, 128);
+    // every row of Q has been read (by the tensor core and by its threads) before A overwrites the tile
+    __syncthreads();
     if (ok) {
       // row i of chunk c at sA[c][il][.], its columns rotated by 4 * il so that neither these stores nor the broadcast
       // reads of the solve meet a bank conflict
       float4* arow = reinterpret_cast<float4*>(sA + c * (CH * CH) + il * CH);
 #pragma unroll
-      for (int j4 = 0; j4 < 16; ++j4)
-        arow[(j4 + il) & 15] = make_float4(a[j4 * 4], a[j4 * 4 + 1], a[j4 * 4 + 2], a[j4 * 4 + 3]);
+      for (int j4 = 0; j4 < 8; ++j4)
+        arow[(part * 8 + j4 + il) & 15] = make_float4(a[j4 * 4], a[j4 * 4 + 1], a[j4 * 4 + 2], a[j4 * 4 + 3]);
     }
     tc_fence_before();
   }

@@ -111,7 +111,7 @@ def use_cuda(*tensors: torch.Tensor) -> bool:
     if not t.is_cuda or env("DEWB_FORCE_REFERENCE") == "1":
         return False
     if _LIB is None:
-        load()  # raises LibraryMissing on a GPU box without the build
+        load()  # raises LibraryMissing on a machine with a GPU and no build
     ensure_device(t)
     return True
 

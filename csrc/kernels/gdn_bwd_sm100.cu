@@ -45,11 +45,6 @@ __device__ __forceinline__ float tile_get(const uint8_t* tile, int rows, int r, 
   const uint8_t* p = tile + (c >> 6) * (rows * 128) + swz(r, (c & 63) >> 3) + (c & 7) * 2;
   return __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(p));
 }
-__device__ __forceinline__ void tile_put(uint8_t* tile, int rows, int r, int c, float v) {
-  uint8_t* p = tile + (c >> 6) * (rows * 128) + swz(r, (c & 63) >> 3) + (c & 7) * 2;
-  *reinterpret_cast<__nv_bfloat16*>(p) = __float2bfloat16(v);
-}
-
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);

@@ -39,10 +39,6 @@ constexpr int CH = 64;            // chunk length
 constexpr int PT = 128;           // tokens per prepare CTA
 constexpr uint32_t FULL = 0xffffffffu;
 
-__device__ __forceinline__ void named_barrier_sync(int id, int threads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-
 // Byte offset of the 16-byte piece `c16` (8 bf16) of row `r` inside a 128-byte-swizzled tile whose rows are 128 bytes.
 __device__ __forceinline__ uint32_t swz(int r, int c16) { return static_cast<uint32_t>(r * 128 + ((c16 ^ (r & 7)) << 4)); }
 

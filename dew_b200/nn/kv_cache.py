@@ -421,14 +421,17 @@ class KVStore:
     # ------------------------------------------------------------------ the fused decode step
     def _step_ints(self, positions: torch.Tensor):
         """(positions, lengths) of a decode step as int32, computed once per step: every layer of a forward passes the same
-        positions tensor, so the conversions and the ``where`` run for the first layer only."""
-        key = (positions.data_ptr(), positions._version, tuple(positions.shape), torch.cuda.is_current_stream_capturing() if positions.is_cuda else False)
+        positions, so the conversions and the ``where`` run for the first layer only.  The positions' storage is held beside the
+        copies: while it is, no other tensor can stand at its address with the same version."""
+        storage = positions.untyped_storage()
+        key = (storage._cdata, positions.storage_offset(), positions._version, positions.dtype, tuple(positions.shape), positions.stride(),
+               torch.cuda.is_current_stream_capturing() if positions.is_cuda else False)
         cached = getattr(self, "_ints", None)
         if cached is not None and cached[0] == key:
             return cached[1], cached[2]
         pos32 = positions.to(torch.int32).contiguous()
         lens32 = torch.where(pos32 >= 0, pos32 + 1, torch.zeros_like(pos32))
-        self._ints = (key, pos32, lens32)
+        self._ints = (key, pos32, lens32, storage)
         return pos32, lens32
 
     def can_decode_packed(self, qkv: torch.Tensor, Hq: int, softcap: float = 0.0) -> bool:

@@ -494,10 +494,8 @@ class KVStore:
         L.check(lib.dewb_rope_append(at(qkv), at(cos), at(sin), at(pos32), R, Hq, self.kv_heads, D, cos.shape[0] if cos is not None else 0, at(self.k[layer]),
                                      at(self.v[layer]), at(self.page_table), self.page_size, self.max_pages, L.stream()), "rope_append")
         out = torch.empty((R, Hq, D), dtype=qkv.dtype, device=qkv.device)
-        sk = getattr(self, "_sinks32", None)
-        if sinks is not None and (sk is None or sk[0] is not sinks):
-            self._sinks32 = sk = (sinks, sinks.detach().float().contiguous())
-        self._fused_decode(lib, layer, qkv, H * D, lens32, R, Hq, D, window, sk[1] if sinks is not None else None, out)
+        sinks32 = None if sinks is None else sinks.detach().float().contiguous()      # referenced until the launch is enqueued
+        self._fused_decode(lib, layer, qkv, H * D, lens32, R, Hq, D, window, sinks32, out)
         L.count_launches(1)
         return out
 

@@ -1,8 +1,11 @@
 """The paged cache: the integers of a decode step."""
+from types import SimpleNamespace
+
 import pytest
 import torch
 
 from dew_b200.nn.kv_cache import KVCache, KVStore
+from dew_b200.ops import library as L
 
 
 def test_a_step_reads_its_own_positions():
@@ -18,3 +21,15 @@ def test_a_step_reads_its_own_positions():
     assert store._step_ints(positions.reshape(-1))[0] is first[0]
     positions.add_(1)
     assert [t.tolist() for t in store._step_ints(positions.reshape(-1))] == [[4, 0], [5, 1]]
+
+
+def test_a_decode_step_reads_the_sinks_as_they_are_now(monkeypatch):
+    store, seen = KVStore(KVCache(), 1, 2, 64, 1, 64, device="cpu"), []
+    monkeypatch.setattr(L, "load", lambda *a: SimpleNamespace(dewb_rope_append=lambda *a: 0))
+    monkeypatch.setattr(L, "stream", lambda: 0)
+    monkeypatch.setattr(store, "_fused_decode", lambda lib, layer, q, stride, lens, R, Hq, D, window, sinks, out: seen.append(sinks.tolist()))
+    sinks = torch.tensor([1.0, 2.0], dtype=torch.bfloat16)
+    for _ in range(2):
+        store.decode_packed(0, torch.zeros(2, 4, 64), None, None, torch.tensor([0, 1]), 2, sinks=sinks)
+        sinks.mul_(2)                                                          # an update of the parameter in place
+    assert seen == [[1.0, 2.0], [2.0, 4.0]]

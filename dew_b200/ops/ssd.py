@@ -38,9 +38,17 @@ def _strides(*tensors: torch.Tensor):
     return (ctypes.c_longlong * (2 * len(tensors)))(*(s if n > 1 else 0 for t in tensors for n, s in zip(t.shape[:2], t.stride())))
 
 
-def _numbers(t, heads: int):
-    """One fp32 number per head."""
-    return None if t is None else t.detach().float().expand(heads).contiguous()
+def _sized(x, dt, A, Bm, Cm, D, initial):
+    """dt ``[B, T, H]``, A and D ``[H]``, the initial state ``[B, H, 64, 128]``: in fp32, in these sizes, on ``x``'s device, as the kernels index them (what broadcasts
+    to them is expanded; what does not is refused here, as are B and C of other sizes)."""
+    B, T, H = x.shape[:3]
+    if Bm.shape != Cm.shape or Bm.shape[:2] != x.shape[:2]:
+        raise ValueError(f"ssd: x {tuple(x.shape)}, B {tuple(Bm.shape)} and C {tuple(Cm.shape)} do not belong together")
+    for t in (dt, A, Bm, Cm, D, initial):
+        if t is not None and t.dim() and t.device != x.device:
+            raise ValueError(f"ssd: operands on {t.device} and on {x.device}")
+    fp32 = lambda t, *size: None if t is None else t.detach().to(x.device).float().expand(size).contiguous()
+    return fp32(dt, B, T, H), fp32(A, H), fp32(D, H), fp32(initial, B, H, HEAD, STATE)
 
 
 def _forward(x, dt, A, Bm, Cm, D, initial):
@@ -84,12 +92,11 @@ class _SSD(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, dt, A, Bm, Cm, D, initial_state):
         ctx.set_materialize_grads(False)
-        H = x.shape[2]
         exact = all(t.dtype == torch.bfloat16 for t in (x, Bm, Cm))
         ctx.exact = exact
+        dt32, A32, D32, initial32 = _sized(x, dt, A, Bm, Cm, D, initial_state)
         xb, bb, cb = _rows(x), _rows(Bm), _rows(Cm)
-        ins = (dt.detach().float().contiguous(), _numbers(A, H), bb, cb, _numbers(D, H) if exact else None,
-               None if initial_state is None else initial_state.detach().float().contiguous())
+        ins = (dt32, A32, bb, cb, D32 if exact else None, initial32)
         y, last = _forward(xb, *ins)
         ctx.given = tuple(None if t is None else (t.dtype, t.shape) for t in (dt, A, D, initial_state))
         if exact:
@@ -129,4 +136,6 @@ class _SSD(torch.autograd.Function):
 def ssd(x, dt, A, Bm, Cm, D=None, initial_state=None):
     """x ``[B,T,H,64]``, dt ``[B,T,H]`` (after softplus), A ``[H]``, B / C ``[B,T,G,128]`` -> (y ``[B,T,H,64]``, state
     ``[B,H,64,128]`` fp32)."""
+    if A.dim() > 1 and A.numel() == A.shape[-1]:
+        A = A.reshape(-1)
     return _SSD.apply(x, dt, A, Bm, Cm, D, initial_state)

@@ -74,6 +74,7 @@ _GEMM.kernels = [
         Requirement("ld", lambda c: c["lda"] % 8 == 0 and c["ldb"] % 8 == 0 and c["K"] % 8 == 0, "row strides and K must be multiples of 8 elements"),
         Requirement("align", lambda c: c["aligned"], "base pointers must be 16-byte aligned"),
         Requirement("inner", lambda c: c["inner_contig"], "the contiguous dimension must have stride 1"),
+        Requirement("operands", lambda c: c.get("row_operands", False), "operands on one device and, if any, a bias of one number per output column"),
     ], receipt="few rows against streamed weights on the CUDA cores, csrc/kernels/gemm_rows.cu"),
     Kernel("cublas", [], receipt="library arm (torch.matmul)"),
 ]
@@ -174,8 +175,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     if (fresh and cell is not None and kernel is None and _GEMM.declared.get(cell) == "cublas" and alpha == 1.0 and a.dtype == b.dtype == kind
             and not _GEMM.forced_by_environment() and not (torch.is_grad_enabled() and (a.requires_grad or b.requires_grad))):
         # a small product that its measured cell sends to the library arm: nothing about it needs looking up
-        if (_few_rows(M, N, K) and not a_mn and not b_mn and kind == torch.bfloat16 and K % 8 == 0 and a.stride(1) == b.stride(1) == 1 and a.stride(0) % 8 == 0
-                and b.stride(0) % 8 == 0 and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0 and N > 0 and _rows_built()):
+        if _few_rows(M, N, K) and not a_mn and not b_mn and kind == torch.bfloat16 and _rows_take(a, b, bias):
             return _gemm_rows(a, b, bias)
         _GEMM._record("cublas", {}, None, cell)
         A, Bt = a.t() if a_mn else a, b if b_mn else b.t()
@@ -185,7 +185,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         accumulate = False
     case = dict(dtype=a.dtype if a.dtype == b.dtype else None, lda=a.stride(0), ldb=b.stride(0), ldd=out.stride(0),
                 aligned=(a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0),
-                inner_contig=(a.stride(1) == 1 and b.stride(1) == 1 and out.stride(1) == 1), M=M, N=N, K=K, plain=plain, k_major=plain and fresh)
+                inner_contig=(a.stride(1) == 1 and b.stride(1) == 1 and out.stride(1) == 1), M=M, N=N, K=K, plain=plain, k_major=plain and fresh, row_operands=_row_operands(a, b, bias))
     if bias is not None:
         case["plain"] = False                                    # (the weight-streaming kernel has no bias epilogue)
     if kernel is None and cell is None and tiles >= 148 and _pair_built() and all(case[x] % 8 == 0 for x in ("lda", "ldb", "ldd")) and case["aligned"]:
@@ -243,8 +243,14 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     return out
 
 
-def _rows_built() -> bool:
-    return hasattr(L.load(), "dewb_gemm_rows_bf16")
+def _row_operands(a, b, bias) -> bool:
+    """Operands that the few-row kernel may read as ``[M, K]``, ``[N, K]`` and ``[N]``: a bias that would broadcast, or would not fit, is the library arm's."""
+    return a.device == b.device and (bias is None or bias.shape == b.shape[:1] and bias.device == a.device)
+
+
+def _rows_take(a, b, bias) -> bool:
+    return (a.shape[1] % 8 == 0 and b.shape[0] > 0 and a.stride(1) == b.stride(1) == 1 and a.stride(0) % 8 == 0 and b.stride(0) % 8 == 0 and a.data_ptr() % 16 == 0
+            and b.data_ptr() % 16 == 0 and _row_operands(a, b, bias) and hasattr(L.load(), "dewb_gemm_rows_bf16"))
 
 
 def _gemm_rows(a, b, bias):

@@ -1,4 +1,5 @@
 """Which small products the few-row kernel is given: on the CPU, with the kernel's launcher replaced by a list of its calls."""
+import contextlib
 from types import SimpleNamespace
 
 import pytest
@@ -42,8 +43,10 @@ def test_a_bias_of_another_shape_is_broadcast_or_refused(launched):
     assert not launched
 
 
-def test_a_weight_on_another_device_is_left_to_the_library_arm(launched):
+def test_operands_on_another_device_are_left_to_the_library_arm(launched):
     x, w, b = _operands()
-    Fn.gemm(x, w.to("meta"), bias=b)                   # (PyTorch refuses a weight on the host beside rows on a GPU, and takes one without memory)
-    Fn.gemm(x, w, bias=b.to("meta"))
+    for operands in ((w.to("meta"), None), (w, b.to("meta")), (w.to("meta"), b)):
+        with contextlib.suppress(RuntimeError):        # (what it refuses, it refuses on the host)
+            Fn.gemm(x, operands[0], bias=operands[1])
     assert not launched
+

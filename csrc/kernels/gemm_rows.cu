@@ -2,8 +2,9 @@
 //
 // Bound by the read of w.  A warp makes COLS columns of all rows: its lanes walk K in 16-byte pieces, COLS x DEPTH of them in flight, and the pieces of x come from
 // the first-level cache, where all the warps of an SM share them.  No tensor core: at four rows the products of a weight piece take less than its arrival, and a
-// tensor-core tile would compute 124 rows of nothing.  COLS is the largest of 4, 2, 1 that still gives every SM four warps, since a warp's time is the latency of its
-// chain of loads for matrices this small.
+// tensor-core tile would compute 124 rows of nothing.  COLS is the largest of 4, 2, 1 that still gives every SM sixteen warps: more columns share the pieces of x, but
+// for matrices this small a warp's time is the latency of its chain of loads.  One row by 12288 x 512, COLS 1, 2, 4: 4.9, 5.0, 3.9 us; by 8192 x 256: 3.1, 2.7, 2.6; by
+// 3072 x 2048: 5.6, 6.3, 7.0.  Three and four rows are taken up to 4096 columns, where it is 1.
 #include <cstdint>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -73,9 +74,13 @@ rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict
 template <int M>
 static int go(const void* x, const void* w, const void* bias, void* y, int N, int K, long long ldx, long long ldw, long long ldy, cudaStream_t stream) {
   typedef const __nv_bfloat16* in;
-  const int cols = N >= 148 * WARPS * 4 * 4 ? 4 : N >= 148 * WARPS * 4 * 2 ? 2 : 1;
+  int cols = 1;
+  auto fn = rows_kernel<M, 1>;
+  if constexpr (M <= 2) {
+    cols = N >= 148 * WARPS * 4 * 4 ? 4 : N >= 148 * WARPS * 4 * 2 ? 2 : 1;
+    fn = cols == 4 ? rows_kernel<M, 4> : cols == 2 ? rows_kernel<M, 2> : rows_kernel<M, 1>;
+  }
   const unsigned blocks = static_cast<unsigned>((N + cols * WARPS - 1) / (cols * WARPS));
-  auto fn = cols == 4 ? rows_kernel<M, 4> : cols == 2 ? rows_kernel<M, 2> : rows_kernel<M, 1>;
   fn<<<blocks, WARPS * 32, 0, stream>>>(static_cast<in>(x), static_cast<in>(w), static_cast<in>(bias), static_cast<__nv_bfloat16*>(y), N, K, ldx, ldw, ldy);
   return static_cast<int>(cudaGetLastError());
 }

@@ -81,10 +81,18 @@ _GEMM.kernels = [
 
 
 def _few_rows(M: int, N: int, K: int) -> bool:
-    """Where the few-row kernel is ahead of the library's (microseconds inside a graph, weights not in cache: one row by 2048 x 1024 3.1 against 4.9, 1024 x 2816
-    6.7 against 9.0, 5632 x 1024 4.7 against 5.1, 6144 x 4096 12.3 against 11.2; four rows by 2048 x 1024 4.3 against 4.5, 1024 x 2816 8.6 against 8.0): the weights
-    arrive in a few microseconds, and at three or four rows in half of those, beyond which the products of the CUDA cores show."""
-    return 1 <= M <= 4 and N * K <= (6 << 20 if M <= 2 else 2 << 20)
+    """Where the few-row kernel is ahead of the library's (microseconds inside a graph, weights not in cache, kernel against library).  Up to a few megabytes of
+    weights: one row by 2048 x 1024 3.4 against 5.1, by 3072 x 2048 5.6 against 8.1, by 12288 x 512 3.9 against 4.8, by 6144 x 4096 12.3 against 11.2; at three or four
+    rows the products of the CUDA cores show sooner (four by 2048 x 1024 4.4 against 4.5, by 8192 x 256 3.5 against 3.3).  A warp walks a whole reduction, so long
+    ones are ahead only while the library does not split them (one row by 64 x 8192 5.8 against 11.8, by 384 x 8192 13.1 against 12.5, by 64 x 16384 17.7 against
+    13.8; four rows by 64 x 4096 5.2 against 6.9, by 512 x 2048 5.7 against 4.7); short ones leave it most of its time for the sums over a warp's lanes, which counts
+    once there are many columns (two rows by 4096 x 64 2.1 against 2.3, by 8192 x 128 2.6 against 2.5, by 16384 x 64 3.1 against 2.4)."""
+    if not 1 <= M <= 4:
+        return False
+    pair = M <= 2
+    if K > (4096 if pair else 1024):
+        return K <= 8192 and N * K <= (1 << 20 if pair else 1 << 18)
+    return N <= (12288 if pair else 4096) and N * K <= (6 << 20 if pair else 2 << 20) and (K >= 256 or N <= (4096 if pair else 2048))
 
 
 def _skinny_built() -> bool:

@@ -50,3 +50,25 @@ def test_operands_on_another_device_are_left_to_the_library_arm(launched):
             Fn.gemm(x, operands[0], bias=operands[1])
     assert not launched
 
+
+# the library arm keeps what it does faster: long reductions (it splits them), many columns of short ones, more than a few megabytes
+@pytest.mark.parametrize("M,N,K", [(1, 8, 262144), (2, 64, 16384), (1, 384, 8192), (4, 512, 2048), (3, 256, 4096), (2, 65536, 16), (2, 8192, 128), (4, 8192, 256), (1, 32000, 1024), (5, 8, 8)])
+def test_products_that_the_library_arm_does_faster_stay_there(launched, M, N, K):
+    assert not Fn._few_rows(M, N, K)
+
+
+def test_the_few_row_kernel_keeps_what_it_does_faster():
+    assert all(Fn._few_rows(*s) for s in [(1, 8, 8), (1, 2048, 1024), (2, 3072, 2048), (1, 12288, 512), (2, 64, 8192), (4, 32, 8192), (4, 2048, 1024), (3, 4096, 256), (2, 1536, 4096)])
+
+
+@pytest.mark.gpu
+# one, two and four columns a warp, at the last and first sizes of each; the longest reduction; three and four rows
+@pytest.mark.parametrize("M,N,K", [(1, 4735, 256), (2, 4736, 264), (1, 9471, 256), (2, 9473, 264), (2, 12288, 512), (2, 9, 8192), (3, 4095, 256), (4, 31, 8192)])
+def test_few_rows_against_64_bits(M, N, K):
+    from dew_b200.ops.selection import route_report
+    x, w, b = (t.cuda() for t in _operands(M, N, K))
+    route_report(reset=True)
+    y = Fn.gemm(x, w, bias=b)
+    assert route_report()["gemm"]["sm100_rows"]["calls"] == 1
+    want = x.double() @ w.double().t() + b.double()
+    assert float((y.double() - want).norm() / want.norm()) < 2.0 ** -8                # one rounding of an fp32 sum to bf16

@@ -68,7 +68,7 @@ _GEMM.kernels = [
                "memory, csrc/kernels/gemm_skinny_sm100.cu"),
     Kernel("sm100_rows", [
         Requirement("built", lambda c: hasattr(L.load(), "dewb_gemm_rows_bf16"), "the few-row kernel is not in this build of libdewb.so"),
-        Requirement("rows", lambda c: c["M"] <= 4, "at most four rows"),
+        Requirement("size", lambda c: _few_rows(c["M"], c["N"], c["K"]), "at most four rows, of sizes that the library arm does no faster"),
         Requirement("plain", lambda c: c.get("k_major", False), "K-major operands, fresh bf16 output, alpha = 1"),
         Requirement("dtype", lambda c: c["dtype"] == torch.bfloat16, "operands must be bf16"),
         Requirement("ld", lambda c: c["lda"] % 8 == 0 and c["ldb"] % 8 == 0 and c["K"] % 8 == 0, "row strides and K must be multiples of 8 elements"),
@@ -136,6 +136,9 @@ _GEMM.declared[("skinny",)] = "cublas"
 # 6.6-7.6 us a call, this library's cluster split-K kernel 14.4 us - so the cell names the library arm; DEWB_DECODE_GEMM=sm100_skinny
 # selects the weight-streaming kernel (and with it the SwiGLU epilogue of `linear_swiglu`).
 _GEMM.declared[("decode",)] = os.environ.get("DEWB_DECODE_GEMM", "cublas")
+# One to four rows of a few megabytes of weights, with or without a bias (`_few_rows`).  A DEWB_DECODE_GEMM that is set names the kernel of these too.
+if "DEWB_DECODE_GEMM" not in os.environ:
+    _GEMM.declared[("rows",)] = "sm100_rows"
 _SKINNY_PDL = int(os.environ.get("DEWB_SKINNY_PDL", "1"))
 
 
@@ -180,14 +183,16 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     plain = not a_mn and not b_mn and kind == torch.bfloat16 and (fresh or not accumulate) and alpha == 1.0
     tiles = ((M + 127) // 128) * ((N + 255) // 256)
     cell = ("decode",) if (M <= 128 and plain and bias is None) else (("skinny",) if tiles < 24 else None)
-    if (fresh and cell is not None and kernel is None and _GEMM.declared.get(cell) == "cublas" and alpha == 1.0 and a.dtype == b.dtype == kind
-            and not _GEMM.forced_by_environment() and not (torch.is_grad_enabled() and (a.requires_grad or b.requires_grad))):
-        # a small product that its measured cell sends to the library arm: nothing about it needs looking up
-        if _few_rows(M, N, K) and not a_mn and not b_mn and kind == torch.bfloat16 and _rows_take(a, b, bias):
+    if (fresh and cell is not None and kernel is None and alpha == 1.0 and a.dtype == b.dtype == kind and not _GEMM.forced_by_environment()
+            and not (torch.is_grad_enabled() and (a.requires_grad or b.requires_grad))):
+        # a small product whose measured cell is the few-row kernel's or the library arm's: nothing about it needs looking up
+        if plain and _few_rows(M, N, K) and _GEMM.declared.get(("rows",)) == "sm100_rows" and _rows_take(a, b, bias):
+            _GEMM._record("sm100_rows", {}, None, ("rows",))
             return _gemm_rows(a, b, bias)
-        _GEMM._record("cublas", {}, None, cell)
-        A, Bt = a.t() if a_mn else a, b if b_mn else b.t()
-        return torch.mm(A, Bt) if bias is None else torch.addmm(bias.to(kind), A, Bt)
+        if _GEMM.declared.get(cell) == "cublas":
+            _GEMM._record("cublas", {}, None, cell)
+            A, Bt = a.t() if a_mn else a, b if b_mn else b.t()
+            return torch.mm(A, Bt) if bias is None else torch.addmm(bias.to(kind), A, Bt)
     if fresh:
         out = torch.empty((M, N), dtype=out_dtype, device=a.device)
         accumulate = False
@@ -263,7 +268,6 @@ def _rows_take(a, b, bias) -> bool:
 
 def _gemm_rows(a, b, bias):
     M, N, K = a.shape[0], b.shape[0], a.shape[1]
-    _GEMM._record("sm100_rows", {}, None, None)
     out = torch.empty((M, N), dtype=torch.bfloat16, device=a.device)
     bb = None if bias is None else bias.to(torch.bfloat16).contiguous()
     rc = L.load().dewb_gemm_rows_bf16(a.data_ptr(), b.data_ptr(), 0 if bb is None else bb.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), N, L.stream())

@@ -1,5 +1,8 @@
 """Which small products the few-row kernel is given: on the CPU, with the kernel's launcher replaced by a list of its calls."""
 import contextlib
+import os
+import subprocess
+import sys
 from types import SimpleNamespace
 
 import pytest
@@ -59,6 +62,28 @@ def test_products_that_the_library_arm_does_faster_stay_there(launched, M, N, K)
 
 def test_the_few_row_kernel_keeps_what_it_does_faster():
     assert all(Fn._few_rows(*s) for s in [(1, 8, 8), (1, 2048, 1024), (2, 3072, 2048), (1, 12288, 512), (2, 64, 8192), (4, 32, 8192), (4, 2048, 1024), (3, 4096, 256), (2, 1536, 4096)])
+
+
+def test_the_measured_cell_is_the_kernels_own(launched, monkeypatch):
+    from dew_b200.ops.selection import route_report
+    x, w, b = _operands()
+    route_report(reset=True)
+    Fn.gemm(x, w, bias=b)
+    assert route_report()["gemm"] == {"sm100_rows": {"calls": 1, "forced": 0, "declared_cell": 1, "after_refusals": {}}}
+    # an explicit DEWB_DECODE_GEMM leaves no cell of the few-row kernel, and its entry refuses what the library arm does faster
+    monkeypatch.delitem(Fn._GEMM.declared, ("rows",))
+    Fn.gemm(x, w, bias=b)
+    assert len(launched) == 1
+    entry = next(k for k in Fn._GEMM.kernels if k.name == "sm100_rows")
+    case = dict(M=2, K=64, lda=64, ldb=64, ldd=40, aligned=True, inner_contig=True, dtype=torch.bfloat16, plain=True, k_major=True, row_operands=True)
+    assert not entry.refusals(dict(case, N=36)) and entry.refusals(dict(case, N=36004)) and entry.refusals(dict(case, N=36, row_operands=False))
+
+
+def test_an_explicit_choice_of_the_decode_kernel_holds_for_few_rows():
+    code = "from dew_b200.ops import functional as F; print(sorted(F._GEMM.declared.items()))"
+    out = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, DEWB_DECODE_GEMM="cublas"), capture_output=True, text=True, check=True,
+                         cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__)))).stdout
+    assert "('decode',), 'cublas'" in out and "rows" not in out
 
 
 @pytest.mark.gpu

@@ -365,7 +365,7 @@ class KVStore:
     def write(self, layer: int, k: torch.Tensor, v: torch.Tensor, positions: torch.Tensor) -> None:
         """Store ``k, v [R, S, Hkv, D]`` at ``positions [R, S]`` (negative positions are skipped)."""
         R, S = positions.shape
-        if k.dim() == 4 and k.shape[:2] == v.shape[:2] == (R, S) and k.stride(0) == S * k.stride(1) and v.stride(0) == S * v.stride(1):
+        if R and k.dim() == 4 and k.shape[:2] == v.shape[:2] == (R, S) and k.stride(0) == S * k.stride(1) and v.stride(0) == S * v.stride(1):
             rows = None if self.row_ids is None else self.row_ids.to(torch.int32)
             if self._scatter(layer, k[0], v[0], positions, rows, S):
                 return

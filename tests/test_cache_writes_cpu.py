@@ -1,4 +1,4 @@
-"""The paged cache: the integers of a decode step."""
+"""The paged cache: the integers of a decode step, and writes of many tokens."""
 from types import SimpleNamespace
 
 import pytest
@@ -33,3 +33,11 @@ def test_a_decode_step_reads_the_sinks_as_they_are_now(monkeypatch):
         store.decode_packed(0, torch.zeros(2, 4, 64), None, None, torch.tensor([0, 1]), 2, sinks=sinks)
         sinks.mul_(2)                                                          # an update of the parameter in place
     assert seen == [[1.0, 2.0], [2.0, 4.0]]
+
+
+def test_no_rows_write_nothing():
+    store = KVStore(KVCache(), 1, 2, 16, 1, 8, device="cpu")
+    for S in (0, 3):
+        store.write(0, torch.ones(0, S, 1, 8), torch.ones(0, S, 1, 8), torch.zeros(0, S, dtype=torch.long))
+    store.write(0, torch.ones(2, 0, 1, 8), torch.ones(2, 0, 1, 8), torch.zeros(2, 0, dtype=torch.long))
+    assert not store.k.any()

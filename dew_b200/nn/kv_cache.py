@@ -365,9 +365,10 @@ class KVStore:
     def write(self, layer: int, k: torch.Tensor, v: torch.Tensor, positions: torch.Tensor) -> None:
         """Store ``k, v [R, S, Hkv, D]`` at ``positions [R, S]`` (negative positions are skipped)."""
         R, S = positions.shape
-        if R and k.dim() == 4 and k.shape[:2] == v.shape[:2] == (R, S) and k.stride(0) == S * k.stride(1) and v.stride(0) == S * v.stride(1):
-            rows = None if self.row_ids is None else self.row_ids.to(torch.int32)
-            if self._scatter(layer, k[0], v[0], positions, rows, S):
+        ids = self.row_ids
+        if (R and k.dim() == 4 and k.shape[:2] == v.shape[:2] == (R, S) and k.stride(0) == S * k.stride(1) and v.stride(0) == S * v.stride(1)
+                and (ids is None or ids.shape == (R,))):
+            if self._scatter(layer, k[0], v[0], positions, None if ids is None else ids.to(torch.int32), S):
                 return
         rows = self._rows(R)[:, None].expand(R, S).reshape(-1)
         flat = positions.reshape(-1)
@@ -391,7 +392,7 @@ class KVStore:
         fits = lambda t: (t.dtype == torch.bfloat16 and t.shape[1:] == (self.kv_heads, self.head_dim) and t.stride(2) == 1 and (self.kv_heads == 1 or t.stride(1) == self.head_dim)
                           and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0)
         if not (self.slots is None and self.kind == 0 and self.dtype == torch.bfloat16 and n < 1 << 31 and width % 8 == 0 and k.is_cuda and L.use_cuda(k) and fits(k) and fits(v)
-                and hasattr(L.load(), "dewb_kv_scatter")):
+                and self.k.device == k.device == v.device == positions.device and (rows is None or rows.device == k.device) and hasattr(L.load(), "dewb_kv_scatter")):
             return False
         pos32 = positions.reshape(-1).to(torch.int32)
         L.check(L.load().dewb_kv_scatter(L.ptr(k), L.ptr(v), ctypes.c_longlong(k.stride(0)), ctypes.c_longlong(v.stride(0)), L.ptr(self.k[layer]), L.ptr(self.v[layer]),

@@ -41,3 +41,36 @@ def test_no_rows_write_nothing():
         store.write(0, torch.ones(0, S, 1, 8), torch.ones(0, S, 1, 8), torch.zeros(0, S, dtype=torch.long))
     store.write(0, torch.ones(2, 0, 1, 8), torch.ones(2, 0, 1, 8), torch.zeros(2, 0, dtype=torch.long))
     assert not store.k.any()
+
+
+def test_rows_that_were_not_selected_for_the_call_are_refused(monkeypatch):
+    store, scattered = KVStore(KVCache(), 1, 3, 16, 1, 8, dtype=torch.bfloat16, device="cpu"), []
+    monkeypatch.setattr(store, "_scatter", lambda layer, k, v, positions, rows, per_row: scattered.append(rows) or True)
+    k, positions = torch.ones(2, 4, 1, 8, dtype=torch.bfloat16), torch.arange(4)[None].repeat(2, 1)
+    # the scatter reads one store row per row of the call: other numbers are broadcast or refused by the indexed write
+    store.select(torch.tensor([1])).write(0, k, k, positions)
+    assert not scattered and bool(store.k[0, 1, :4].all()) and not store.k[0, 0].any()
+    with pytest.raises(RuntimeError):
+        store.select(torch.tensor([0, 1, 2])).write(0, k, k, positions)
+    store.select(torch.tensor([2, 0])).write(0, k, k, positions)
+    store.select(None).write(0, k, k, positions)
+    assert [None if r is None else r.tolist() for r in scattered] == [[2, 0], None]
+
+
+class _OnGpu:
+    """What the scatter asks a tensor of, as one of a GPU would answer."""
+
+    def __init__(self, shape, device, dtype=torch.bfloat16):
+        t = torch.zeros(shape, dtype=dtype)
+        self.t, self.device, self.dtype, self.shape, self.is_cuda = t, torch.device(device), dtype, t.shape, True
+        self.stride, self.data_ptr, self.numel = t.stride, lambda: 0, t.numel
+
+
+def test_the_scatter_reads_one_device(monkeypatch):
+    store, launched = KVStore(KVCache(), 1, 3, 16, 1, 8, dtype=torch.bfloat16, device="cpu"), []
+    monkeypatch.setattr(L, "use_cuda", lambda *t: True)
+    monkeypatch.setattr(L, "load", lambda *a: SimpleNamespace(dewb_kv_scatter=lambda *a: launched.append(a)))
+    store.k = SimpleNamespace(device=torch.device("cuda:0"))
+    k, other, host = _OnGpu((2, 1, 8), "cuda:0"), _OnGpu((2, 1, 8), "cuda:1"), torch.zeros(2, dtype=torch.int32)
+    assert not store._scatter(0, k, k, host, None, 1) and not store._scatter(0, k, other, host, None, 1) and not store._scatter(0, other, other, host, None, 1)
+    assert not launched

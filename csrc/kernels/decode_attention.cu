@@ -18,6 +18,7 @@
 
 #include "../common/attn_variant.cuh"
 #include "../common/key_range.cuh"
+#include "../common/ptx.cuh"
 
 namespace dewb {
 namespace decode {
@@ -418,38 +419,44 @@ extern "C" int dewb_rope_append(void* qkv, const float* cosb, const float* sinb,
   return static_cast<int>(cudaGetLastError());
 }
 
-// positions[row] = slot to write (the row's current length), or < 0 to skip the row.
 // Keys and values [tokens, Hkv * D] bf16 (rows k_stride / v_stride elements apart) into their pages: token t belongs to store row rows[t / per_row] (t / per_row itself
-// where rows is null) at positions[t]; positions below 0, and what lies outside the table, are skipped.  A warp a token, bound by the copy.
+// where rows is null) at positions[t]; positions below 0 are skipped (padding).  A row or position outside the table, or a page outside the pool, is an error that the
+// status word reports; nothing is written for it.  A warp a token, bound by the copy.
 __global__ void __launch_bounds__(256)
 kv_scatter_kernel(const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v, long long k_stride, long long v_stride, __nv_bfloat16* __restrict__ kpool,
                   __nv_bfloat16* __restrict__ vpool, const int* __restrict__ page_table, const int* __restrict__ rows, const int* __restrict__ positions, int tokens, int per_row,
-                  int pieces, int page_size, int max_pages, int store_rows, int pages) {
+                  int pieces, int page_size, int max_pages, int store_rows, int pages, int* __restrict__ err) {
   const int t = (blockIdx.x * 256 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (t >= tokens) return;
   const int pos = positions[t], at = t / per_row, row = rows == nullptr ? at : rows[at];
-  if (pos < 0 || row < 0 || row >= store_rows || pos / page_size >= max_pages) return;
-  const int page = page_table[static_cast<long long>(row) * max_pages + pos / page_size];
-  if (page < 0 || page >= pages) return;
+  if (pos < 0) return;
+  const bool inside = row >= 0 && row < store_rows && pos / page_size < max_pages;
+  const int page = inside ? page_table[static_cast<long long>(row) * max_pages + pos / page_size] : -1;
+  if (page < 0 || page >= pages) {
+    if (lane == 0) atomicCAS(err, 0, static_cast<int>(dewb::ERR_BAD_ARG));
+    return;
+  }
   const long long to = (static_cast<long long>(page) * page_size + pos % page_size) * pieces;
   const uint4 *ks = reinterpret_cast<const uint4*>(k + t * k_stride), *vs = reinterpret_cast<const uint4*>(v + t * v_stride);
   uint4 *kd = reinterpret_cast<uint4*>(kpool) + to, *vd = reinterpret_cast<uint4*>(vpool) + to;
   for (int i = lane; i < pieces; i += 32) { kd[i] = ks[i]; vd[i] = vs[i]; }
 }
 
-// width = Hkv * D and the strides multiples of 8, everything 16-byte aligned; pools of `pages` pages of page_size tokens; page_table [store_rows, max_pages].
+// width = Hkv * D and the strides multiples of 8, everything 16-byte aligned; pools of `pages` pages of page_size tokens; page_table [store_rows, max_pages]; err: the
+// device's status word.
 extern "C" int dewb_kv_scatter(const void* k, const void* v, long long k_stride, long long v_stride, void* kpool, void* vpool, const int* page_table, const int* rows,
-                               const int* positions, int tokens, int per_row, int width, int page_size, int max_pages, int store_rows, int pages, void* stream_ptr) {
+                               const int* positions, int tokens, int per_row, int width, int page_size, int max_pages, int store_rows, int pages, int* err, void* stream_ptr) {
   if (width % 8 || k_stride % 8 || v_stride % 8 || per_row <= 0 || page_size <= 0 ||
       ((reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(kpool) | reinterpret_cast<uintptr_t>(vpool)) & 15))
     return -3;
   if (tokens <= 0) return 0;
   kv_scatter_kernel<<<(tokens + 7) / 8, 256, 0, reinterpret_cast<cudaStream_t>(stream_ptr)>>>(
       reinterpret_cast<const __nv_bfloat16*>(k), reinterpret_cast<const __nv_bfloat16*>(v), k_stride, v_stride, reinterpret_cast<__nv_bfloat16*>(kpool),
-      reinterpret_cast<__nv_bfloat16*>(vpool), page_table, rows, positions, tokens, per_row, width / 8, page_size, max_pages, store_rows, pages);
+      reinterpret_cast<__nv_bfloat16*>(vpool), page_table, rows, positions, tokens, per_row, width / 8, page_size, max_pages, store_rows, pages, err);
   return static_cast<int>(cudaGetLastError());
 }
 
+// positions[row] = slot to write (the row's current length), or < 0 to skip the row.
 extern "C" int dewb_kv_append(const void* k_new, const void* v_new, void* kpool, void* vpool, float* kscale,
                               float* vscale, const int* page_table, const int* positions, int rows, int Hkv, int D,
                               int page_size, int max_pages, int kv_kind, void* stream_ptr) {

@@ -397,8 +397,8 @@ class KVStore:
         pos32 = positions.reshape(-1).to(torch.int32)
         L.check(L.load().dewb_kv_scatter(L.ptr(k), L.ptr(v), ctypes.c_longlong(k.stride(0)), ctypes.c_longlong(v.stride(0)), L.ptr(self.k[layer]), L.ptr(self.v[layer]),
                                          L.ptr(self.page_table), L.ptr(rows), L.ptr(pos32), ctypes.c_int(n), ctypes.c_int(per_row), ctypes.c_int(width),
-                                         ctypes.c_int(self.page_size), ctypes.c_int(self.max_pages), ctypes.c_int(self.rows), ctypes.c_int(self.pages), L.stream_ptr()),
-                "kv_scatter")
+                                         ctypes.c_int(self.page_size), ctypes.c_int(self.max_pages), ctypes.c_int(self.rows), ctypes.c_int(self.pages),
+                                         L.ptr(L.status(k.device)), L.stream_ptr()), "kv_scatter")
         L.count_launches()
         return True
 

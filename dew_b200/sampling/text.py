@@ -198,6 +198,9 @@ class RowBatch:
     def prefill(self, tokens: torch.Tensor, lengths: torch.Tensor) -> torch.Tensor:
         """The prompts ``[rows, S]`` (right-padded), from their first token; returns last-position logits ``[rows, V]``."""
         R, S = tokens.shape
+        room = self.store.max_pages * self.store.page_size
+        if S > room and int(lengths.max()) > room:
+            raise ValueError(f"a prompt of {int(lengths.max())} tokens does not fit rows of {room}")
         if self.splits_head and self.device.type == "cuda" and self.store.slots is None and S > PackedRows.TILE and not torch.cuda.is_current_stream_capturing():
             counts = lengths.tolist()
             if PackedRows.takes(self.store, self.model, counts, S):

@@ -74,3 +74,35 @@ def test_the_scatter_reads_one_device(monkeypatch):
     k, other, host = _OnGpu((2, 1, 8), "cuda:0"), _OnGpu((2, 1, 8), "cuda:1"), torch.zeros(2, dtype=torch.int32)
     assert not store._scatter(0, k, k, host, None, 1) and not store._scatter(0, k, other, host, None, 1) and not store._scatter(0, other, other, host, None, 1)
     assert not launched
+
+
+def _decoder(**where):
+    from dew_b200.models import CausalTransformer
+    return CausalTransformer(vocab_size=31, emb_features=32, num_layers=1, num_heads=2, head_dim=16, mlp_features=32, max_seq_len=64, qk_norm=False, **where).eval()
+
+
+def test_a_prompt_longer_than_its_row_is_refused_on_the_host():
+    from dew_b200.sampling.text import RowBatch
+    batch, tokens = RowBatch(_decoder(), 2, 16), torch.zeros(2, 20, dtype=torch.long)
+    with pytest.raises(ValueError, match="17 tokens"):
+        batch.prefill(tokens, torch.tensor([3, 17]))
+    assert batch.prefill(tokens, torch.tensor([3, 16])).shape == (2, 31)      # (the padding alone reaches past the rows)
+
+
+@pytest.mark.gpu
+# a position behind the row's last page; a row that the store does not have
+@pytest.mark.parametrize("place,row", [(32, 0), (1 << 30, 0), (3, 2)])
+def test_what_lies_outside_the_pages_is_reported_and_not_written(place, row):
+    store = KVStore(KVCache(page_size=16), 1, 2, 32, 2, 64, device="cuda")
+    k = torch.randn(2, 6, 2, 64, generator=torch.Generator().manual_seed(0)).cuda().bfloat16()
+    positions = torch.arange(6, device="cuda")[None].repeat(2, 1)
+    positions[1] = -1
+    positions[1, 5] = place
+    rows = torch.tensor([1, row], dtype=torch.int32, device="cuda")
+    L.check_status()
+    assert store._scatter(0, k[0], k[0], positions, rows, 6)
+    with pytest.raises(L.KernelError):
+        L.check_status()
+    want = torch.zeros_like(store.k)
+    want[0, 2, :6] = k[0]
+    assert torch.equal(store.k, want) and torch.equal(store.v, want)

@@ -622,8 +622,8 @@ class PackedRows:
 
     @staticmethod
     def takes(store: KVStore, model, lengths: Sequence[int], width: int) -> bool:
-        """Whether the model's layers are attention over this store alone and nothing in them looks at a token's neighbours by index, the kernels take its heads, and
-        enough padding goes: one row's worth of tiles in eight."""
+        """Whether the model's layers are attention over this store alone and nothing in them looks at a token's neighbours by index or at other ranks, the kernels take
+        its heads, and enough padding goes: one row's worth of tiles in eight."""
         from ..models.causal_transformer import CausalTransformer
         from .attention import SelfAttention
         if not (store.slots is None and store.kind == 0 and store.dtype == torch.bfloat16 and store.device.type == "cuda" and store.row_ids is None and store.head_dim in (64, 128)
@@ -636,6 +636,8 @@ class PackedRows:
             return False
         for layer in model.layers:
             m = layer.mixer
+            if layer.sparse and getattr(getattr(layer.mlp, "ep", None), "world", 1) > 1:      # (its ranks exchange buffers of one size: as many tokens on each)
+                return False
             if type(m) is not SelfAttention or layer.cross is not None or layer.streams is not None or m.num_heads % m.num_kv_heads or m.num_kv_heads != store.kv_heads \
                     or m.head_dim != store.head_dim or (layer.sparse and getattr(layer.mlp, "mix", None) is not None and layer.mlp.mix.capacity_factor is not None):
                 return False

@@ -18,6 +18,8 @@ from typing import Dict, List, Optional, Sequence
 import torch
 import torch.nn as nn
 
+from ..utils.hooks import moves_weights
+
 
 def _signature(layer: nn.Module):
     return tuple((n, tuple(p.shape), p.dtype) for n, p in layer.named_parameters())
@@ -62,8 +64,8 @@ class HostBanks:
         self.copies = 0
         self._handles = []
         for i, layer in enumerate(self.layers):
-            self._handles.append(layer.register_forward_pre_hook(lambda m, a, i=i: self._enter(i)))
-            self._handles.append(layer.register_forward_hook(lambda m, a, out, i=i: self._leave(i)))
+            self._handles.append(layer.register_forward_pre_hook(moves_weights(lambda m, a, i=i: self._enter(i))))
+            self._handles.append(layer.register_forward_hook(moves_weights(lambda m, a, out, i=i: self._leave(i))))
         for i in range(slots):
             self._fetch(i, first=True)
 

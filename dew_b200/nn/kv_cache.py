@@ -623,8 +623,9 @@ class PackedRows:
     @staticmethod
     def takes(store: KVStore, model, lengths: Sequence[int], width: int) -> bool:
         """Whether the model's layers are attention over this store alone and nothing in them looks at a token's neighbours by index or at other ranks, the kernels take
-        its heads, and enough padding goes: one row's worth of tiles in eight."""
+        its heads, no hook may see that its calls are given one row of tokens, and enough padding goes: one row's worth of tiles in eight."""
         from ..models.causal_transformer import CausalTransformer
+        from ..utils.hooks import watched
         from .attention import SelfAttention
         if not (store.slots is None and store.kind == 0 and store.dtype == torch.bfloat16 and store.device.type == "cuda" and store.row_ids is None and store.head_dim in (64, 128)
                 and len(lengths) == store.rows and type(model) is CausalTransformer and L.env("DEWB_FORCE_REFERENCE") != "1" and L.env("DEWB_KERNEL_ATTENTION") is None
@@ -642,7 +643,7 @@ class PackedRows:
                     or m.head_dim != store.head_dim or (layer.sparse and getattr(layer.mlp, "mix", None) is not None and layer.mlp.mix.capacity_factor is not None):
                 return False
         tiles = sum(-(-n // PackedRows.TILE) for n in lengths)
-        return 8 * tiles <= 7 * len(lengths) * -(-width // PackedRows.TILE)
+        return 8 * tiles <= 7 * len(lengths) * -(-width // PackedRows.TILE) and not watched(model)
 
     def attend(self, layer: int, q, k, v, positions, causal=True, window=None, softcap=0.0, sinks=None):
         from ..ops.flash import Variants, flash_fwd_rows

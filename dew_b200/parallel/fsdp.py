@@ -36,6 +36,7 @@ from ..objectives.base import Aux, Step, pool
 from ..ops import library as L
 from ..training.state import TrainState
 from ..utils import keys as K
+from ..utils.hooks import moves_weights
 from ..utils.trees import flatten, module_path_to_tree_path, unflatten
 from .symm import SymmetricBuffer
 
@@ -302,7 +303,7 @@ class FSDPEngine:
                     return tuple(new_args), kwargs
             # the first unit's inputs (token ids) carry no gradient: it is finalised after backward returns
             return None
-        return hook
+        return moves_weights(hook)
 
     # ------------------------------------------------------------------ state
     def fresh_state(self, key: int) -> TrainState:

@@ -35,3 +35,21 @@ def test_experts_of_several_ranks_keep_the_padded_form(takes):
     for world, packed in ((1, True), (2, False)):
         model.layers[-1].mlp.ep = SimpleNamespace(world=world)
         assert takes(model) == packed
+
+
+def test_a_watched_decoder_keeps_the_padded_form(takes):
+    from dew_b200.nn.inspection import ActivationWatch
+    from dew_b200.utils.hooks import moves_weights
+    model = _decoder()
+    with ActivationWatch(model, ["layers.1.mlp"]):
+        assert not takes(model)
+    assert takes(model)
+    look = lambda *args: None
+    for register in (model.register_forward_hook, model.layers[0].mixer.register_forward_pre_hook, torch.nn.modules.module.register_module_forward_hook,
+                     torch.nn.modules.module.register_module_forward_pre_hook):
+        handle = register(look)
+        assert not takes(model)
+        handle.remove()
+    # a hook that brings a layer's weights sees nothing of its tokens
+    model.layers[0].register_forward_pre_hook(moves_weights(lambda *args: None))
+    assert takes(model)

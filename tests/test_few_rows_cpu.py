@@ -92,8 +92,10 @@ def test_an_explicit_choice_of_the_decode_kernel_holds_for_few_rows():
 def test_few_rows_against_64_bits(M, N, K):
     from dew_b200.ops.selection import route_report
     x, w, b = (t.cuda() for t in _operands(M, N, K))
+    if N >= 6144:                                      # (with a bias the dense kernel's epilogue takes them)
+        b = None
     route_report(reset=True)
     y = Fn.gemm(x, w, bias=b)
     assert route_report()["gemm"]["sm100_rows"]["calls"] == 1
-    want = x.double() @ w.double().t() + b.double()
+    want = x.double() @ w.double().t() + (0 if b is None else b.double())
     assert float((y.double() - want).norm() / want.norm()) < 2.0 ** -8                # one rounding of an fp32 sum to bf16

@@ -621,19 +621,19 @@ class PackedRows:
         self.last = torch.tensor([s + n - 1 for s, n in zip(starts, lengths)], device=dev)
 
     @staticmethod
-    def takes(store: KVStore, model, lengths: Sequence[int], width: int) -> bool:
+    def suits(store: KVStore, model) -> bool:
         """Whether the model's layers are attention over this store alone and nothing in them looks at a token's neighbours by index or at other ranks, the kernels take
-        its heads, no hook may see that its calls are given one row of tokens, and enough padding goes: one row's worth of tiles in eight."""
+        its heads, and no hook may see that its calls are given one row of tokens."""
         from ..models.causal_transformer import CausalTransformer
         from ..utils.hooks import watched
         from .attention import SelfAttention
         if not (store.slots is None and store.kind == 0 and store.dtype == torch.bfloat16 and store.device.type == "cuda" and store.row_ids is None and store.head_dim in (64, 128)
-                and len(lengths) == store.rows and type(model) is CausalTransformer and L.env("DEWB_FORCE_REFERENCE") != "1" and L.env("DEWB_KERNEL_ATTENTION") is None
+                and type(model) is CausalTransformer and L.env("DEWB_FORCE_REFERENCE") != "1" and L.env("DEWB_KERNEL_ATTENTION") is None
                 and hasattr(L.load(), "dewb_flash_fwd_rows")):
             return False
         cfg = model.config
         if (cfg.fp32_stack or cfg.loop is not None or cfg.hyper_connections > 1 or cfg.altup > 1 or cfg.depth_residual_block or not cfg.causal or model.engrams is not None
-                or getattr(model, "tp", None) is not None or min(lengths) < 1 or max(lengths) > width):
+                or getattr(model, "tp", None) is not None):
             return False
         for layer in model.layers:
             m = layer.mixer
@@ -642,8 +642,19 @@ class PackedRows:
             if type(m) is not SelfAttention or layer.cross is not None or layer.streams is not None or m.num_heads % m.num_kv_heads or m.num_kv_heads != store.kv_heads \
                     or m.head_dim != store.head_dim or (layer.sparse and getattr(layer.mlp, "mix", None) is not None and layer.mlp.mix.capacity_factor is not None):
                 return False
+        return not watched(model)
+
+    @staticmethod
+    def pays(store: KVStore, lengths: Sequence[int], width: int) -> bool:
+        """Whether these are whole rows of the store's and enough padding goes, of ``width`` tokens a row: one row's worth of tiles in eight."""
+        if len(lengths) != store.rows or min(lengths) < 1 or max(lengths) > width:
+            return False
         tiles = sum(-(-n // PackedRows.TILE) for n in lengths)
-        return 8 * tiles <= 7 * len(lengths) * -(-width // PackedRows.TILE) and not watched(model)
+        return 8 * tiles <= 7 * len(lengths) * -(-width // PackedRows.TILE)
+
+    @staticmethod
+    def takes(store: KVStore, model, lengths: Sequence[int], width: int) -> bool:
+        return PackedRows.pays(store, lengths, width) and PackedRows.suits(store, model)
 
     def attend(self, layer: int, q, k, v, positions, causal=True, window=None, softcap=0.0, sinks=None):
         from ..ops.flash import Variants, flash_fwd_rows

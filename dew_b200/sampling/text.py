@@ -201,9 +201,10 @@ class RowBatch:
         room = self.store.max_pages * self.store.page_size
         if S > room and int(lengths.max()) > room:
             raise ValueError(f"a prompt of {int(lengths.max())} tokens does not fit rows of {room}")
-        if self.splits_head and self.device.type == "cuda" and self.store.slots is None and S > PackedRows.TILE and not torch.cuda.is_current_stream_capturing():
-            counts = lengths.tolist()
-            if PackedRows.takes(self.store, self.model, counts, S):
+        if (self.splits_head and self.device.type == "cuda" and self.store.slots is None and S > PackedRows.TILE and not torch.cuda.is_current_stream_capturing()
+                and PackedRows.suits(self.store, self.model)):
+            counts = lengths.tolist()                        # (the lengths are read from the device only where they decide something)
+            if PackedRows.pays(self.store, counts, S):
                 return self._prefill_packed(tokens, counts)
         if self.store.slots is not None and self.device.type == "cuda" and 1 < S and S % 128:
             tokens = torch.nn.functional.pad(tokens, (0, 128 - S % 128))          # whole tiles for the flash kernel

@@ -53,3 +53,16 @@ def test_a_watched_decoder_keeps_the_padded_form(takes):
     # a hook that brings a layer's weights sees nothing of its tokens
     model.layers[0].register_forward_pre_hook(moves_weights(lambda *args: None))
     assert takes(model)
+
+
+def test_lengths_are_read_only_where_they_decide(monkeypatch):
+    from dew_b200.sampling.text import RowBatch
+
+    class Lengths(torch.Tensor):
+        def tolist(self):
+            raise AssertionError("read from the device")
+
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    batch = RowBatch(CausalTransformer(vocab_size=31, emb_features=32, num_layers=1, num_heads=2, head_dim=16, mlp_features=32, max_seq_len=200, qk_norm=False).eval(), 2, 200)
+    batch.device = torch.device("cuda")                                        # (its store is on the host and its heads are narrow: never packed)
+    assert batch.prefill(torch.zeros(2, 150, dtype=torch.long), torch.tensor([3, 150]).as_subclass(Lengths)).shape == (2, 31)

@@ -14,6 +14,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ..ops import ada
+from ..utils.hooks import runs_alone
 from .attention import SelfAttention
 from .layers import LayerNorm, Linear, sinusoidal
 from .mlp import GeluMLP
@@ -87,8 +88,7 @@ modulate = ada.modulate
 
 def _bare(norm: nn.Module) -> bool:
     """Whether calling ``norm`` is the layer norm without weights and nothing else, so that it may run inside the kernel of what surrounds it."""
-    return type(norm) is LayerNorm and norm.weight is None and norm.bias is None and not (norm._forward_hooks or norm._forward_pre_hooks or norm._backward_hooks
-                                                                                         or norm._backward_pre_hooks)
+    return type(norm) is LayerNorm and norm.weight is None and norm.bias is None and runs_alone(norm)
 
 
 class ModulatedBlock(nn.Module):

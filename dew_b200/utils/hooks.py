@@ -1,4 +1,4 @@
-"""Whether a module's hooks would notice that its call is made in another form."""
+"""Whether anybody would notice that a module's call is made in another form, or not at all."""
 from __future__ import annotations
 
 from torch.nn.modules import module as _all
@@ -27,3 +27,10 @@ def _watched(module) -> bool:
         if child is not None and _watched(child):
             return True
     return False
+
+
+def runs_alone(module) -> bool:
+    """Whether calling ``module`` is running its class's ``forward`` and nothing else: no hook of its own or of all modules, in either direction, and no ``forward``
+    set on the instance."""
+    return not ("forward" in module.__dict__ or module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks
+                or _all._global_forward_hooks or _all._global_forward_pre_hooks or _all._global_backward_hooks or _all._global_backward_pre_hooks)

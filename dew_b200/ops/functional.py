@@ -302,9 +302,9 @@ def grad_accumulates(p) -> bool:
 
 
 def _column_sums(dy):
-    """``dy.sum(0)`` of a bf16 matrix (a bias' gradient)."""
+    """``dy.sum(0)`` of a bf16 matrix (a bias' gradient).  The kernel leaves no graph: where the gradient is differentiated again, PyTorch sums."""
     rows, d = dy.shape
-    if not (L.use_cuda(dy) and dy.dtype == torch.bfloat16 and rows >= 256 and d % 8 == 0 and d > 0 and dy.stride(1) == 1 and dy.stride(0) % 8 == 0 and dy.data_ptr() % 16 == 0
+    if (torch.is_grad_enabled() and dy.requires_grad) or not (L.use_cuda(dy) and dy.dtype == torch.bfloat16 and rows >= 256 and d % 8 == 0 and d > 0 and dy.stride(1) == 1 and dy.stride(0) % 8 == 0 and dy.data_ptr() % 16 == 0
             and hasattr(L.load(), "dewb_colsum_bf16")):
         return dy.sum(0)
     lib = L.load()

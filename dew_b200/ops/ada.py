@@ -52,12 +52,31 @@ def _forward(x, branch, gate, shift, scale, eps):
     return y, h, stats
 
 
+def _gradients(h, branch, gate, scale, eps, dy, dh):
+    """What the backward kernel computes, as expressions that can be differentiated again: -> gradients of x, branch, gate, shift, scale."""
+    wide = torch.promote_types(h.dtype, torch.float32)
+    row = lambda t: t.to(wide).unsqueeze(1)
+    g = torch.zeros((), dtype=wide, device=h.device) if dh is None else dh.to(wide)
+    dbranch = dgate = dshift = dscale = None
+    if scale is not None:
+        u = h.to(wide) - h.to(wide).mean(-1, keepdim=True)
+        rstd = torch.rsqrt(u.square().mean(-1, keepdim=True) + eps)
+        u, v = u * rstd, dy.to(wide)
+        a = v * (1 + row(scale))
+        g = g + rstd * (a - a.mean(-1, keepdim=True) - u * (a * u).mean(-1, keepdim=True))
+        dshift, dscale = v.sum(1), (v * u).sum(1)
+    if branch is not None:
+        dbranch, dgate = row(gate) * g, (branch.to(wide) * g).sum(1)
+    return tuple(None if t is None else t.to(h.dtype) for t in (g, dbranch, dgate, dshift, dscale))
+
+
 class _Ada(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, branch, gate, shift, scale, eps):
         ctx.set_materialize_grads(False)
         y, h, stats = _forward(x, branch, gate, shift, scale, eps)
         ctx.save_for_backward(h, branch, gate, scale, stats)
+        ctx.eps = eps
         if branch is None:
             return y
         return h if shift is None else (y, h)
@@ -69,6 +88,8 @@ class _Ada(torch.autograd.Function):
         dy, dh = (grads[0], None) if branch is None else (None, grads[0]) if not norm else grads
         if norm and dy is None:
             dy = torch.zeros_like(h)
+        if torch.is_grad_enabled():                          # (create_graph: the kernel's results would have no history)
+            return (*_gradients(h, branch, gate, scale, ctx.eps, dy, dh), None)
         dy, dh = (None if t is None else _rows(t.to(h.dtype)) for t in (dy, dh))
         B, n, d = h.shape
         lib = L.load()

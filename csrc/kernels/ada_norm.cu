@@ -263,7 +263,7 @@ extern "C" int dewb_ada_fwd(const void* x, const void* branch, const void* shift
 // Tokens of an image that one block of the backward takes (the slabs of `part`): about two blocks an SM, at least a row for every warp.
 extern "C" int dewb_ada_slab(int B, int n) {
   int slab = n;
-  while (slab > 8 && static_cast<long long>(B) * ((n + slab - 1) / slab) < 2 * 148) slab = (slab + 1) / 2;
+  while (slab > 8 && static_cast<long long>(B) * ((n + slab - 1) / slab) < 2 * 148) slab = slab > 15 ? (slab + 1) / 2 : 8;      // (never below 8: 9 tokens are one block of eight rows and one of one, not five and four)
   return slab;
 }
 

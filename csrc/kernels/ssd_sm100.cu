@@ -788,7 +788,9 @@ static int walk(const Call& k, const Walk<Out>& forward, const Walk<Out>* revers
 }
 
 static int check(const Call& k) {
-  if (k.B <= 0 || k.T <= 0 || k.H <= 0 || k.G <= 0 || k.H % k.G != 0 || k.chunks > 65535 || k.G > 65535) return -3;
+  if (k.B <= 0 || k.T <= 0 || k.H <= 0 || k.G <= 0 || k.H % k.G != 0 || k.G > 65535) return -3;
+  // (batch rows by chunks, and by heads, lie along the grid's first dimension)
+  if (static_cast<long long>(k.B) * k.chunks > 0x7fffffff || static_cast<long long>(k.B) * k.H > 0x7fffffff) return -3;
   if ((k.xb | k.xt | k.bb | k.bt | k.cb | k.ct) % 8) return -3;
   if ((reinterpret_cast<uintptr_t>(k.x) | reinterpret_cast<uintptr_t>(k.Bm) | reinterpret_cast<uintptr_t>(k.Cm) | reinterpret_cast<uintptr_t>(k.dy)) & 15) return -3;
   return 0;

@@ -182,10 +182,10 @@ class SparseMLP(nn.Module):
             y = self.ep.dispatch_compute_combine(self, x2, w, ids)
         elif x2.is_cuda and x2.dtype == torch.bfloat16 and mix.experts <= 256 and mix.top_k <= 16 and self.use_kernels:
             # one rank: the same device-planned dispatch / combine kernels, with this rank as its own only peer
-            from ..parallel.ep import TokenExchange, exchange_experts
+            from ..parallel.ep import TokenExchange, constant_weights, exchange_experts
             if self._exchange is None:
                 self._exchange = TokenExchange(mix.experts, _SELF_GROUP)
-            y = exchange_experts(self._exchange, self.experts, x2, w, ids)
+            y = exchange_experts(self._exchange, self.experts, x2, w, ids, constant_weights(mix))
         else:
             layout = G.group_layout(ids, mix.experts)
             xs = G.permute(x2, layout, mix.top_k)

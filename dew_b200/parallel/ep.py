@@ -245,8 +245,8 @@ class _PullRows(torch.autograd.Function):
     """Combine; its backward dispatches ``w[t, j] * dy[t]`` to the owners and takes ``dw[t, j] = <dy[t], row(t, j)>``."""
 
     @staticmethod
-    def forward(ctx, rows, weights, exchange, plan):
-        ctx.exchange, ctx.plan = exchange, plan
+    def forward(ctx, rows, weights, exchange, plan, constant=False):
+        ctx.exchange, ctx.plan, ctx.constant = exchange, plan, constant
         out, gathered = exchange.pull(rows, plan, weights, keep_rows=weights.requires_grad)
         ctx.save_for_backward(weights, gathered)
         return out
@@ -259,21 +259,25 @@ class _PullRows(torch.autograd.Function):
         d_rows = ctx.exchange.push(dy, plan, pair_scale=weights.reshape(-1), backward=True)
         dw = None
         if gathered is not None:
-            if plan.top_k == 1:
-                # a token's only weight, where the weights are normalised, is 1 whatever its score: what reaches the router is the rounding of this sum alone, and
-                # stays what PyTorch's order of summation makes of it
-                dw = (gathered.view(plan.tokens, 1, -1).float() * dy.float().unsqueeze(1)).sum(-1)
+            if ctx.constant:
+                # the weight is 1 times a constant whatever the router says: its gradient cancels down to the rounding of this sum, which stays PyTorch's
+                dw = (gathered.view(plan.tokens, plan.top_k, -1).float() * dy.float().unsqueeze(1)).sum(-1)
             else:
                 dw = torch.empty(plan.tokens, plan.top_k, dtype=torch.float32, device=dy.device)
                 L.check(L.load().dewb_moe_pair_dots(L.ptr(gathered), L.ptr(dy), L.ptr(dw), ctypes.c_int(dw.numel()), ctypes.c_int(plan.top_k), ctypes.c_int(dy.shape[1]),
                                                     L.stream_ptr()), "moe_pair_dots")
                 L.count_launches()
             dw = dw.to(weights.dtype)
-        return d_rows, dw, None, None
+        return d_rows, dw, None, None, None
 
 
-def exchange_experts(exchange: TokenExchange, experts, x2: torch.Tensor, weights: torch.Tensor, ids: torch.Tensor) -> torch.Tensor:
-    """plan -> dispatch -> grouped expert MLP on the received rows -> combine, all on this library's kernels."""
+def constant_weights(mix) -> bool:
+    """Whether a token's routing weight does not depend on its scores: the only one, and normalised."""
+    return mix.top_k == 1 and (bool(mix.norm_topk_prob) or mix.score_function == "top_softmax")
+
+
+def exchange_experts(exchange: TokenExchange, experts, x2: torch.Tensor, weights: torch.Tensor, ids: torch.Tensor, constant: bool = False) -> torch.Tensor:
+    """plan -> dispatch -> grouped expert MLP on the received rows -> combine, all on this library's kernels.  ``constant``: see ``constant_weights``."""
     plan = exchange.plan(ids, x2.shape[1])
     exchange.last_info = plan.info            # device tensor {rows received, overflowed, busiest owner's rows, pairs dropped}: read it after the step
     if getattr(exchange, "totals", None) is None:
@@ -286,7 +290,7 @@ def exchange_experts(exchange: TokenExchange, experts, x2: torch.Tensor, weights
         out_rows = experts(rows, plan.layout, out=exchange.claim_out(x2.shape[1]) if exchange.write_in_place else None, lean=True)
     else:
         out_rows = experts(rows, plan.layout)
-    return _PullRows.apply(out_rows, weights.float(), exchange, plan)
+    return _PullRows.apply(out_rows, weights.float(), exchange, plan, constant)
 
 
 class _GatherExperts(torch.autograd.Function):
@@ -369,7 +373,7 @@ class ExpertParallel:
             # device-planned exchange over peer memory (TokenExchange); the path below is the NCCL / gloo form of the same protocol
             if self.exchange is None:
                 self.exchange = TokenExchange(mlp.mix.experts, self.group, self.capacity_factor)
-            return exchange_experts(self.exchange, mlp.experts, x2, weights, ids)
+            return exchange_experts(self.exchange, mlp.experts, x2, weights, ids, constant_weights(mlp.mix))
         W, E = self.world, mlp.mix.experts
         per = E // W
         T, k = ids.shape

@@ -29,6 +29,7 @@ def test_forward_and_gradients(B, n, d, form):
         shift, scale, gate = m.chunk(3, -1)
         if dt != torch.bfloat16:
             h = x if form == "norm" else x + gate.unsqueeze(1) * branch
+            h = h + (h.detach().bfloat16().to(dt) - h.detach())                # (the stream carries h in bf16: what is normalised is what it carries)
             y = (h - h.mean(-1, keepdim=True)) * torch.rsqrt(h.var(-1, unbiased=False, keepdim=True) + 1e-6) * (1 + scale.unsqueeze(1)) + shift.unsqueeze(1)
             return (y,) if form == "norm" else (h,) if form == "gate" else (y, h)
         if form == "norm":
@@ -44,12 +45,12 @@ def test_forward_and_gradients(B, n, d, form):
         outs.append(out)
         grads.append(torch.autograd.grad([o for o, _ in kept], leaves, [p for _, p in kept], allow_unused=True))
     L.check_status()
-    # one rounding of each result to bf16; y and its gradients read h as it was rounded
+    # one rounding of each result to bf16 (2^-9 of each value); h as it was rounded is the reference's as well, but beside a rounding boundary the fp32 sum may take the other side
     for a, b in zip(*outs):
         assert rel_err(a, b) < 4e-3
-    for a, b in zip(*grads):
-        assert (a is None) == (b is None) or float(b.abs().max()) == 0
-        if a is not None and b is not None and d > 8:
+    for i, (a, b) in enumerate(zip(*grads)):
+        assert (a is None) == (b is None) == (form == "norm" and i == 1)                  # (no branch in that form)
+        if a is not None:
             assert rel_err(a, b) < 6e-3
     with torch.no_grad():
         assert all(torch.equal(a, b) for a, b in zip(run(x, branch, m, torch.bfloat16), outs[0]))

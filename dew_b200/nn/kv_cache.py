@@ -391,7 +391,7 @@ class KVStore:
         n, width = positions.numel(), self.kv_heads * self.head_dim
         fits = lambda t: (t.dtype == torch.bfloat16 and t.shape[1:] == (self.kv_heads, self.head_dim) and t.stride(2) == 1 and (self.kv_heads == 1 or t.stride(1) == self.head_dim)
                           and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0)
-        if not (self.slots is None and self.kind == 0 and self.dtype == torch.bfloat16 and n < 1 << 31 and width % 8 == 0 and k.is_cuda and L.use_cuda(k) and fits(k) and fits(v)
+        if not (self.slots is None and self.kind == 0 and self.dtype == torch.bfloat16 and n < 1 << 27 and width % 8 == 0 and k.is_cuda and L.use_cuda(k) and fits(k) and fits(v)
                 and self.k.device == k.device == v.device == positions.device and (rows is None or rows.device == k.device) and hasattr(L.load(), "dewb_kv_scatter")):
             return False
         pos32 = positions.reshape(-1).to(torch.int32)

@@ -73,6 +73,12 @@ def test_the_scatter_reads_one_device(monkeypatch):
     store.k = SimpleNamespace(device=torch.device("cuda:0"))
     k, other, host = _OnGpu((2, 1, 8), "cuda:0"), _OnGpu((2, 1, 8), "cuda:1"), torch.zeros(2, dtype=torch.int32)
     assert not store._scatter(0, k, k, host, None, 1) and not store._scatter(0, k, other, host, None, 1) and not store._scatter(0, other, other, host, None, 1)
+    # a warp a token, found by a 32-bit thread number
+    positions = SimpleNamespace(numel=lambda: 1 << 27, device=torch.device("cuda:0"), reshape=lambda *s: torch.zeros(1))
+    monkeypatch.setattr(L, "status", lambda *a: None)
+    monkeypatch.setattr(L, "stream_ptr", lambda: None)
+    store.k = store.v = type("Pool", (), {"device": torch.device("cuda:0"), "__getitem__": lambda self, i: None})()
+    assert not store._scatter(0, k, k, positions, None, 1)
     assert not launched
 
 

@@ -82,4 +82,4 @@ def test_modulated_norms_are_differentiated_twice(form):
     L.check_status()
     # a rounding of h, of each first gradient and of each second one, which reads both
     for a, b in zip(got[0] + got[1], want[0] + want[1]):
-        assert float((a.double() - b).norm()) < 2e-2 * float(b.norm())
+        assert float((a.double() - b).norm()) <= 2e-2 * float(b.norm())                  # (both are zero where nothing is reached)

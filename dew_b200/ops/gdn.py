@@ -1,4 +1,4 @@
-"""Gated delta rule on the sm_100a kernels (``csrc/kernels/gdn_sm100.cu``): three launches per forward or backward.
+"""Gated delta rule on the sm_100a kernels (``csrc/kernels/gdn_sm100.cu``, ``gdn_bwd_sm100.cu``): two launches forward, five backward.
 
 ``prepare``   chunk-parallel, one CTA per 128 tokens of one (batch, head): within-chunk cumulative log decay, ``K K^T`` and
               ``Q K^T`` on the tensor cores, the strictly lower system ``(I + A) [W | U] = [beta e^g K | beta V]`` solved by
@@ -8,9 +8,10 @@
 ``scan_bwd``  the same walk in reverse for the state gradient: ``dVn = P^T dO + e^{g_L - g} K dS``;
               ``dS <- e^{g_L} dS + (e^g Q)^T dO - W^T dVn``; it leaves every chunk's exit-state gradient in memory.
 
-The remaining gradients are local to a chunk once its entry state and exit-state gradient are known; they are taken by
-differentiating the chunk-local formula, batched over all chunks (``_chunk_local``).  Every stage has a PyTorch
-restatement here (``*_reference``) that serves as the oracle for the kernels and as the CPU path.
+The remaining gradients are local to a chunk once its entry state and exit-state gradient are known: two kernels, all chunks at once
+(``gdn_bwd_state_kernel``, ``gdn_bwd_pair_kernel``).  Only the inputs are kept between the passes, so the backward prepares and walks
+forward again.  Every stage has a PyTorch restatement here (``*_reference``; ``_chunk_local`` for the last) that serves as the oracle
+for the kernels and as the CPU path.
 
 Replaces src/dew/nn/kernels/fla_gdn.py (``KktSolve``, ``RecomputeWU``, ``ChunkFwdH``, ``ChunkFwdO``, ``ChunkBwdDhu``) and the
 recurrence template's chunked forward (src/dew/nn/kernels/templates/recurrence/chunk_forward.py).

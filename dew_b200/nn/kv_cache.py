@@ -265,7 +265,7 @@ class KVStore:
         bank = self.__dict__.setdefault("_per_head", {})
         key = (t.data_ptr(), t._version)
         if (slot, name) not in bank or bank[slot, name][0] != key:
-            bank[slot, name] = (key, t.detach().float().contiguous())
+            bank[slot, name] = (key, t.detach().float().contiguous(), t)          # (held: no other tensor can stand at its address)
         return bank[slot, name][1]
 
     def _decode_slot(self, slot: int, packed: torch.Tensor, heads: P.Heads, c: Call, scale: float, visible: P.Visible = P.PLAIN) -> torch.Tensor:

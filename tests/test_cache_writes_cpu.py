@@ -23,6 +23,14 @@ def test_a_step_reads_its_own_positions():
     assert [t.tolist() for t in store._step_ints(positions.reshape(-1))] == [[4, 0], [5, 1]]
 
 
+def test_a_layers_numbers_per_head_are_its_own():
+    store = KVStore(KVCache(), 1, 2, 64, 1, 64, device="cpu")
+    for i in range(20):                                                        # temporaries of one size, as above
+        assert float(store._fp32_of(0, "sinks", torch.full((1000,), i, dtype=torch.bfloat16))[0]) == i
+    kept = torch.ones(4)
+    assert store._fp32_of(0, "gain", kept) is store._fp32_of(0, "gain", kept)
+
+
 def test_a_decode_step_reads_the_sinks_as_they_are_now(monkeypatch):
     store, seen = KVStore(KVCache(), 1, 2, 64, 1, 64, device="cpu"), []
     monkeypatch.setattr(L, "load", lambda *a: SimpleNamespace(dewb_rope_append=lambda *a: 0))

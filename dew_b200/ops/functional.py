@@ -198,7 +198,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         accumulate = False
     case = dict(dtype=a.dtype if a.dtype == b.dtype else None, lda=a.stride(0), ldb=b.stride(0), ldd=out.stride(0),
                 aligned=(a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0),
-                inner_contig=(a.stride(1) == 1 and b.stride(1) == 1 and out.stride(1) == 1), M=M, N=N, K=K, plain=plain, k_major=plain and fresh, row_operands=_row_operands(a, b, bias))
+                inner_contig=(a.stride(1) == 1 and b.stride(1) == 1 and out.stride(1) == 1), M=M, N=N, K=K, plain=plain, k_major=plain and fresh,
+                row_operands=_row_operands(a, b, bias))
     if bias is not None:
         case["plain"] = False                                    # (the weight-streaming kernel has no bias epilogue)
     if kernel is None and cell is None and tiles >= 148 and _pair_built() and all(case[x] % 8 == 0 for x in ("lda", "ldb", "ldd")) and case["aligned"]:
@@ -304,7 +305,9 @@ def grad_accumulates(p) -> bool:
 def _column_sums(dy):
     """``dy.sum(0)`` of a bf16 matrix (a bias' gradient).  The kernel leaves no graph: where the gradient is differentiated again, PyTorch sums."""
     rows, d = dy.shape
-    if (torch.is_grad_enabled() and dy.requires_grad) or not (L.use_cuda(dy) and dy.dtype == torch.bfloat16 and rows >= 256 and d % 8 == 0 and d > 0 and dy.stride(1) == 1 and dy.stride(0) % 8 == 0 and dy.data_ptr() % 16 == 0
+    if torch.is_grad_enabled() and dy.requires_grad:
+        return dy.sum(0)
+    if not (L.use_cuda(dy) and dy.dtype == torch.bfloat16 and rows >= 256 and d % 8 == 0 and d > 0 and dy.stride(1) == 1 and dy.stride(0) % 8 == 0 and dy.data_ptr() % 16 == 0
             and hasattr(L.load(), "dewb_colsum_bf16")):
         return dy.sum(0)
     lib = L.load()

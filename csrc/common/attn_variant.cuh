@@ -53,6 +53,26 @@ __device__ __forceinline__ int first_key_tile(const Variant& v, int b, int q0, i
   return min(lo, n_tiles);
 }
 
+// The same, found by a whole warp: 32 tiles of packed documents a turn.
+__device__ __forceinline__ int first_key_tile_of_warp(const Variant& v, int b, int q0, int S, int T, int bn, int n_tiles, int lane) {
+  const int off = T - S;
+  int lo = 0;
+  if (v.window > 0) lo = max(0, (q0 + off - v.window + 1) / bn);
+  if (v.chunk > 0) lo = max(lo, (q0 + off) / v.chunk * v.chunk / bn);
+  if (v.first != nullptr) lo = max(lo, v.first[q0 / bn]);
+  if (v.q_seg != nullptr && v.k_seg != nullptr) {
+    const int first = v.q_seg[static_cast<long long>(b) * S + min(q0, S - 1)];
+    const int* ks = v.k_seg + static_cast<long long>(b) * T;
+    for (; lo < n_tiles; lo += 32) {
+      const int t = lo + lane;
+      const int last = t < n_tiles ? ks[min(t * bn + bn - 1, T - 1)] : 0;
+      const unsigned stop = __ballot_sync(0xffffffffu, last == 0 || last >= first);
+      if (stop != 0) { lo += __ffs(stop) - 1; break; }
+    }
+  }
+  return min(lo, n_tiles);
+}
+
 // One past the last query block (of `bq` rows) that can see any key of the tile [kv0, kv0 + bkv).
 __device__ __forceinline__ int end_query_block(const Variant& v, int b, int kv0, int bkv, int S, int T, int bq) {
   const int off = T - S;

@@ -352,6 +352,29 @@ __device__ __forceinline__ float fast_exp2(float x) {
 __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
 
+// Two fp32 values in a register pair, one instruction for both.
+__device__ __forceinline__ uint64_t pair_of(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpair(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
 // v[i] = alpha * v[i] + bias[i] for 32 neighbouring output columns, of which `cols` exist; the bias row comes in 16-byte pieces where it starts on such a boundary
 __device__ __forceinline__ void scale_and_bias(uint32_t (&v)[32], float alpha, const __nv_bfloat16* __restrict__ bias, int cols) {
   if (cols >= 32 && (reinterpret_cast<uintptr_t>(bias) & 15) == 0) {
@@ -371,6 +394,12 @@ __device__ __forceinline__ void scale_and_bias(uint32_t (&v)[32], float alpha, c
   for (int i = 0; i < 32; ++i)
     if (i < cols) v[i] = __float_as_uint(fmaf(alpha, __uint_as_float(v[i]), __bfloat162float(bias[i])));
 }
+
+// Registers moved between the warpgroups of a block, each call by a whole warpgroup; the sum must stay within what the block was launched with.
+template <int N>
+__device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

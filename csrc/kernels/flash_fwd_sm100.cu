@@ -1,4 +1,7 @@
-// Flash attention forward for sm_100a (bf16, causal or full, GQA): queries and keys up to 64, 128 or 192 wide, values up to 64 or 128.
+// Flash attention forward for sm_100a (bf16, causal or full, GQA), one query tile a CTA, and the entry points of every forward.
+//
+// Queries and keys of one width, 64 or 128, with values as wide, go to the kernel with two query tiles a CTA (flash_fwd_pair_sm100.cu); this file's kernel serves
+// queries and keys up to 64, 128 or 192 wide beside values up to 64 or 128, and the form of the plain kernels that passes P through shared memory.
 //
 // Queries and keys may come in two parts of their own widths (latent attention: an unrotated part per head, a rotated part whose keys all heads
 // share); each part fills whole 64-column sub-tiles of the operand, the columns past its width read as zeros.  `gate` multiplies the output by a
@@ -23,6 +26,10 @@
 #include "../common/attn_variant.cuh"
 
 namespace dewb {
+namespace attnpair {      // flash_fwd_pair_sm100.cu
+int run(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, void* out, float* lse, int B, int S, int T, int Hq, int Hkv, int D, long long osb, long long oss,
+        long long osh, float scale_log2, int causal, const attn::Variant& var, int* err, cudaStream_t stream);
+}
 namespace attnfwd {
 
 constexpr int BM = 128;        // query rows per CTA
@@ -35,7 +42,7 @@ __device__ __forceinline__ void named_barrier_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-using attn::Variant;
+using attn::Variant;      // (of the entry points)
 
 // DK: width of a query / key row in shared memory, DV: of a value row
 template <int DK, int DV>
@@ -74,7 +81,6 @@ struct Bars {
   uint32_t tmem_base;
   int abort_flag;
   int poisoned;
-  int j_lo;                            // first key tile this query tile sees (variants only), the kept first ones aside
   float xmax[2][2][BM];   // [tile parity][column half][row]: partial row maxima exchanged between the two halves; the
                           // parity the last tile did not use carries the partial row sums at the end
 };
@@ -85,14 +91,13 @@ static_assert(sizeof(Bars) <= 2560, "Bars must fit the space Cfg::SMEM leaves af
 // probabilities (tcgen05.st) and the P V product reads its A operand from there, so P never crosses shared memory (no
 // 32 KB store + 32 KB operand fetch per tile) and the softmax of the next tile need not wait for the product to drain
 // a shared buffer.  PT = false is the shared-memory form (P in the 128-byte-swizzled K-major layout).
-// SIG: the weights are sigmoids (Variant::sig): no maxima, no sums, nothing to rescale.
-template <int DK, int DV, bool CAUSAL, bool PT, bool VAR, bool SIG>
+template <int DK, int DV, bool CAUSAL, bool PT>
 __global__ void __launch_bounds__(THREADS, 1)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                  const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tq2, const __grid_constant__ CUtensorMap tk2,
                  __nv_bfloat16* __restrict__ out, float* __restrict__ lse,
                  int S, int T, int Hq, int Hkv, long long o_stride_b, long long o_stride_s, long long o_stride_h,
-                 float scale_log2, Variant var, Parts parts, int* __restrict__ err) {
+                 float scale_log2, Parts parts, int* __restrict__ err) {
   using C = Cfg<DK, DV>;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // The tiles fill 224 KiB, so this kernel has no static shared memory and no alignment slack: the dynamic window must
@@ -124,7 +129,6 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
   const int n_all = CAUSAL ? min((q0 + BM + (T - S) + BN - 1) / BN, (T + BN - 1) / BN) : (T + BN - 1) / BN;
 
   if (threadIdx.x == 0) {
-    if (VAR) bars->j_lo = attn::first_key_tile(var, b, q0, S, T, BN, n_all);
     mbar_init(&bars->q_full, 1);
     for (int i = 0; i < C::KSTAGES; ++i) { mbar_init(&bars->k_full[i], 1); mbar_init(&bars->k_empty[i], 1); }
     for (int i = 0; i < 2; ++i) {
@@ -147,11 +151,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
   volatile int* abort_flag = &bars->abort_flag;
-  // every role walks the kept first tiles, then the key tiles j_lo .. n_all - 1; rings, phases and "first tile" tests count the walk
-  const int j_lo = VAR ? bars->j_lo : 0;
-  const int n_kept = VAR ? min(j_lo, (var.keep + BN - 1) / BN) : 0;
-  const int n_tiles = n_kept + n_all - j_lo;
-  auto tile_of = [&](int j) { return VAR ? (j < n_kept ? j : j_lo + j - n_kept) : j; };
+  const int n_tiles = n_all;
 
   if (warp == TMA_WARP) {
     // ------------------------------------------------------------------ TMA producer
@@ -165,7 +165,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
         const int st = j & 1; const uint32_t ph = (j >> 1) & 1;
         const int ks = j % C::KSTAGES; const uint32_t kph = (j / C::KSTAGES) & 1;
         if (!mbar_wait(&bars->k_empty[ks], kph ^ 1, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_EMPTY); ok = false; break; }
-        const int key0 = tile_of(j) * BN;
+        const int key0 = j * BN;
         mbar_expect_tx(&bars->k_full[ks], C::K_BYTES);
 #pragma unroll
         for (int t = 0; t < C::SUB; ++t) {
@@ -247,8 +247,6 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     const uint32_t lane_addr = static_cast<uint32_t>(q4 * 32) << 16;
     float m_used = -INFINITY, l = 0.f;
     bool ok = true;
-    if (VAR && var.gain != nullptr) scale_log2 *= var.gain[h];
-    const float sig2 = SIG ? var.sig[h] * 1.4426950408889634f : 0.f;
     if (PT) {
       // this thread's half of its query row, from the swizzled shared tile to tensor memory: lane = row, 32-bit column w
       // = features 2w, 2w + 1 (the layout of a tensor-memory A operand)
@@ -298,69 +296,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
         tc_fence_before();
         __syncwarp();
         if (!PT && lane == 0) mbar_arrive(&bars->s_empty[st]);   // the score buffer may be overwritten by tile j + 2
-        const int k0 = tile_of(j) * BN + half * HC;
+        const int k0 = j * BN + half * HC;
         const int limit = CAUSAL ? (q0 + r + (T - S)) : (T - 1);   // last visible key index for this row
-        if (VAR && var.softcap > 0.f) {
-          // cap * tanh(score / cap), kept in the log2 domain: scale_log2 = scale * log2(e)
-          const float inv_cap = 1.f / (var.softcap * 1.4426950408889634f), cap2 = var.softcap * 1.4426950408889634f;
-#pragma unroll
-          for (int i = 0; i < HC; ++i) s[i] = cap2 * attn::soft_tanh(s[i] * inv_cap);
-        }
         if (k0 + HC - 1 > limit || k0 + HC > T) {
 #pragma unroll
           for (int i = 0; i < HC; ++i) if (k0 + i > limit || k0 + i >= T) s[i] = -INFINITY;
         }
-        if (VAR) {
-          if (var.window > 0 || var.chunk > 0) {
-            const int at = q0 + r + (T - S);
-            int first = var.window > 0 ? at - var.window + 1 : 0;   // first visible key of this row
-            if (var.chunk > 0) first = max(first, at / var.chunk * var.chunk);
-            if (k0 < first) {
-#pragma unroll
-              for (int i = 0; i < HC; ++i) if (k0 + i < first && k0 + i >= var.keep) s[i] = -INFINITY;
-            }
-          }
-          if (var.q_seg != nullptr && k0 < T) {
-            const int row_q = min(q0 + r, S - 1);
-            const int mine = var.q_seg[static_cast<long long>(b) * S + row_q];
-            const int* ks = var.k_seg + static_cast<long long>(b) * T + k0;
-            // ids are non-decreasing: the whole half-tile matches iff its ends do
-            const int e0 = ks[0], e1 = ks[min(HC - 1, T - 1 - k0)];
-            if (e0 != mine || e1 != mine) {
-#pragma unroll
-              for (int i = 0; i < HC; i += 4) {
-                if (k0 + i + 3 < T) {
-                  const int4 id = *reinterpret_cast<const int4*>(ks + i);
-                  if (id.x != mine) s[i] = -INFINITY;
-                  if (id.y != mine) s[i + 1] = -INFINITY;
-                  if (id.z != mine) s[i + 2] = -INFINITY;
-                  if (id.w != mine) s[i + 3] = -INFINITY;
-                } else {
-                  for (int q = 0; q < 4; ++q) if (k0 + i + q < T && ks[i + q] != mine) s[i + q] = -INFINITY;
-                }
-              }
-            }
-          }
-        }
         __syncwarp();                                  // the masks above branch by row; what follows takes whole warps
-        if constexpr (SIG) {
-          const uint32_t pbase = tmem + lane_addr + (st ? C::TMEM_S1 : C::TMEM_S0) + half * (HC / 2);
-          // the other thread of the row has its scores in registers before this one overwrites their columns
-          named_barrier_sync(1 + q4, 64);
-#pragma unroll
-          for (int c = 0; c < HC / 32; ++c) {
-            uint32_t pk[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-              pk[i] = pack_bf16(__fdividef(1.f, 1.f + fast_exp2(-(s[c * 32 + 2 * i] + sig2))), __fdividef(1.f, 1.f + fast_exp2(-(s[c * 32 + 2 * i + 1] + sig2))));
-            tmem_st_32x32b_x16(pbase + c * 16, pk);
-          }
-          tmem_st_wait();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bars->p_full[st]);
-          continue;
-        }
         {
           // four independent chains, not one of 64 dependent maxima
           float m0 = s[0], m1 = s[1], m2 = s[2], m3 = s[3];
@@ -368,10 +310,6 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
           for (int i = 4; i < HC; i += 4) { m0 = fmaxf(m0, s[i]); m1 = fmaxf(m1, s[i + 1]); m2 = fmaxf(m2, s[i + 2]); m3 = fmaxf(m3, s[i + 3]); }
           mt = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
         }
-      }
-      if constexpr (SIG) {                             // (a wait gave up: only the barrier's count is kept)
-        named_barrier_sync(1 + q4, 64);
-        continue;
       }
       // the row's maximum over all 128 columns: exchange with the thread that holds the other half of the row
       bars->xmax[j & 1][half][r] = mt;
@@ -450,17 +388,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     bars->xmax[n_tiles & 1][half][r] = l;      // the parity buffer the last tile left alone
     named_barrier_sync(1 + q4, 64);
     l += bars->xmax[n_tiles & 1][half ^ 1][r];
-    float lse_shift = 0.f;     // log2 of the factor the sink adds to the denominator's scale
-    float inv = SIG ? 1.f : l > 0.f ? 1.f / l : 0.f;
-    if (VAR && !SIG && var.sinks != nullptr) {
-      // the sink joins the denominator only: softmax over [scores, sink] with the sink's value column dropped
-      const float sink2 = var.sinks[h] * 1.4426950408889634f;
-      const float m_fin = fmaxf(m_used, sink2);
-      const float a = m_used > -INFINITY ? fast_exp2(m_used - m_fin) : 0.f;
-      const float l_fin = l * a + fast_exp2(sink2 - m_fin);
-      inv = a / l_fin;
-      lse_shift = m_fin + log2f(l_fin);
-    }
+    const float inv = l > 0.f ? 1.f / l : 0.f;
     if (ok) {
       tc_fence_after();
       const int row = q0 + r;
@@ -501,9 +429,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
         }
       }
       if (half == 0 && row < S && lse != nullptr) {
-        float v = l > 0.f ? (m_used + log2f(l)) * 0.6931471805599453f : -INFINITY;
-        if (VAR && var.sinks != nullptr) v = lse_shift * 0.6931471805599453f;
-        lse[(static_cast<long long>(b) * Hq + h) * S + row] = v;
+        lse[(static_cast<long long>(b) * Hq + h) * S + row] = l > 0.f ? (m_used + log2f(l)) * 0.6931471805599453f : -INFINITY;
       }
     }
   }
@@ -516,18 +442,17 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
   }
 }
 
-template <int DK, int DV, bool CAUSAL, bool PT, bool VAR, bool SIG = false>
+template <int DK, int DV, bool CAUSAL, bool PT>
 static int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tq2, const CUtensorMap& tk2, void* out,
                   float* lse, int B, int S, int T, int Hq, int Hkv, long long osb, long long oss, long long osh, float scale_log2,
-                  const Variant& var, const Parts& parts, int* err, cudaStream_t stream) {
+                  const Parts& parts, int* err, cudaStream_t stream) {
   static_assert(PT || Cfg<DK, DV>::P_BYTES > 0, "P has no shared memory here");
-  static_assert(!SIG || (PT && VAR), "sigmoid weights run the tensor-memory form of the variants");
-  auto kern = flash_fwd_kernel<DK, DV, CAUSAL, PT, VAR, SIG>;
+  auto kern = flash_fwd_kernel<DK, DV, CAUSAL, PT>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<DK, DV>::SMEM);
   if (e != cudaSuccess) return static_cast<int>(e);
   dim3 grid((S + BM - 1) / BM, Hq, B);
   kern<<<grid, THREADS, Cfg<DK, DV>::SMEM, stream>>>(tq, tk, tv, tq2, tk2, reinterpret_cast<__nv_bfloat16*>(out), lse, S, T, Hq, Hkv,
-                                                      osb, oss, osh, scale_log2, var, parts, err);
+                                                      osb, oss, osh, scale_log2, parts, err);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -541,7 +466,7 @@ static int make_qkv_map(CUtensorMap* m, const void* base, int B, int L, int H, i
   return make_tmap_nd(m, base, 4, dims, strides, box, 2, true);
 }
 
-static int g_variant = 1;     // 0: P through shared memory, 1: P in tensor memory (default)
+static int g_variant = 1;     // 0: P through shared memory, one query tile a CTA, 1: P in tensor memory, two (default)
 
 }  // namespace attnfwd
 }  // namespace dewb
@@ -585,24 +510,11 @@ static int flash_fwd_any(const void* q, const void* k, const void* v, void* out,
   const Variant var{window, softcap, sinks, q_seg, k_seg, chunk, keep, gain, sig, first};
   const Parts parts{D / 64, D, nullptr, 0};
   const bool any = window > 0 || chunk > 0 || softcap > 0.f || sinks != nullptr || q_seg != nullptr || gain != nullptr || sig != nullptr || first != nullptr;
-#define DEWB_FLASH_GO(DD, CC, PP, VV) launch<DD, DD, CC, PP, VV>(tq, tk, tv, tq, tk, out, lse, B, S, T, Hq, Hkv, o_sb, o_ss, o_sh, scale_log2, var, parts, err, stream)
-  const bool pt = g_variant != 0;
-  if (sig != nullptr) {
-#define DEWB_FLASH_SIG(DD) launch<DD, DD, true, true, true, true>(tq, tk, tv, tq, tk, out, lse, B, S, T, Hq, Hkv, o_sb, o_ss, o_sh, scale_log2, var, parts, err, stream)
-    return D == 128 ? DEWB_FLASH_SIG(128) : DEWB_FLASH_SIG(64);
-#undef DEWB_FLASH_SIG
-  }
-  if (any) {
-    // the variants run the tensor-memory form only
-    if (D == 128) return causal ? DEWB_FLASH_GO(128, true, true, true) : DEWB_FLASH_GO(128, false, true, true);
-    return causal ? DEWB_FLASH_GO(64, true, true, true) : DEWB_FLASH_GO(64, false, true, true);
-  }
-  if (D == 128) {
-    if (causal) return pt ? DEWB_FLASH_GO(128, true, true, false) : DEWB_FLASH_GO(128, true, false, false);
-    return pt ? DEWB_FLASH_GO(128, false, true, false) : DEWB_FLASH_GO(128, false, false, false);
-  }
-  if (causal) return pt ? DEWB_FLASH_GO(64, true, true, false) : DEWB_FLASH_GO(64, true, false, false);
-  return pt ? DEWB_FLASH_GO(64, false, true, false) : DEWB_FLASH_GO(64, false, false, false);
+  // the form with P in shared memory serves the plain kernels only
+  if (g_variant != 0 || any) return dewb::attnpair::run(tq, tk, tv, out, lse, B, S, T, Hq, Hkv, D, o_sb, o_ss, o_sh, scale_log2, causal, var, err, stream);
+#define DEWB_FLASH_GO(DD, CC) launch<DD, DD, CC, false>(tq, tk, tv, tq, tk, out, lse, B, S, T, Hq, Hkv, o_sb, o_ss, o_sh, scale_log2, parts, err, stream)
+  if (D == 128) return causal ? DEWB_FLASH_GO(128, true) : DEWB_FLASH_GO(128, false);
+  return causal ? DEWB_FLASH_GO(64, true) : DEWB_FLASH_GO(64, false);
 #undef DEWB_FLASH_GO
 }
 
@@ -661,11 +573,10 @@ extern "C" int dewb_flash_fwd_parts(const void* q, const void* k, const void* k2
   if ((r = make_qkv_map(&tk2, k2, B, T, 1, db, k2_sb, k2_ss, k2_ss))) return 2500 + r;
   if ((r = make_qkv_map(&tv, v, B, T, H, dv, v_sb, v_ss, v_sh))) return 3000 + r;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
-  const Variant var{0, 0.f, nullptr, nullptr, nullptr, 0, 0, nullptr, nullptr, nullptr};
   const Parts parts{first, dv, static_cast<const __nv_bfloat16*>(gate), gate_stride};
   const long long oss = static_cast<long long>(H) * dv, osb = oss * S;
-#define DEWB_PARTS_GO(KK, VV) launch<KK, VV, true, true, false>(tq, tk, tv, tq2, tk2, out, nullptr, B, S, T, H, H, osb, oss, dv, \
-    scale * 1.4426950408889634f, var, parts, err, stream)
+#define DEWB_PARTS_GO(KK, VV) launch<KK, VV, true, true>(tq, tk, tv, tq2, tk2, out, nullptr, B, S, T, H, H, osb, oss, dv, \
+    scale * 1.4426950408889634f, parts, err, stream)
   if (sub == 2) return dv <= 64 ? DEWB_PARTS_GO(128, 64) : DEWB_PARTS_GO(128, 128);
   return dv <= 64 ? DEWB_PARTS_GO(192, 64) : DEWB_PARTS_GO(192, 128);
 #undef DEWB_PARTS_GO

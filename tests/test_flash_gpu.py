@@ -34,3 +34,29 @@ def test_flash_packed_documents_of_uneven_work(S, docs, seed):
     L.check_status()
     assert all(torch.equal(out, ops.attention(q, k, v, segment_ids=seg, kernel="sm100_flash")) for _ in range(5))
     assert rel_err(out, ops.attention_reference(q.float(), k.float(), v.float(), segment_ids=seg)) < 6e-3
+
+
+def truth(q, k, v, causal, scale):
+    """Attention in 64 bits, the causal mask aligned at the last query and key; -> output, log-sum-exp (natural), with a graph where the operands have one."""
+    S, T, rep = q.shape[1], k.shape[1], q.shape[2] // k.shape[2]
+    s = torch.einsum("bshd,bthd->bhst", q, k.repeat_interleave(rep, 2)) * scale
+    if causal:
+        s = s.masked_fill(~torch.ones(S, T, dtype=torch.bool, device=q.device).tril(T - S), float("-inf"))
+    return torch.einsum("bhst,bthd->bshd", torch.softmax(s, -1), v.repeat_interleave(rep, 2)), torch.logsumexp(s, -1)
+
+
+# query tiles alone (no more than there are SMs), two heads of a key head, and neighbouring rows (odd numbers of heads a key head, odd numbers of tiles); more items than
+# CTAs; lengths that end inside a tile; more keys than queries
+@pytest.mark.parametrize("B,S,T,Hq,Hkv,D,causal", [(1, 128, 128, 1, 1, 128, True), (1, 8, 8, 2, 1, 64, True), (2, 200, 200, 4, 2, 128, False), (2, 640, 640, 30, 30, 64, True),
+                                                   (1, 1152, 1152, 17, 17, 128, True), (3, 384, 384, 32, 8, 64, False), (1, 2048, 2048, 12, 4, 128, True),
+                                                   (1, 128, 640, 160, 80, 64, True), (2, 264, 1000, 40, 8, 128, True)])
+def test_flash_forward_pairs_of_tiles(B, S, T, Hq, Hkv, D, causal):
+    """The probabilities are rounded to bf16 (2^-9 each, independent) and so is the result; the log-sum-exp is made of fp32 sums of fp32 products of bf16 operands."""
+    from dew_b200.ops.flash import flash_fwd
+    g = torch.Generator(device=DEV).manual_seed(S + Hq)
+    q, k, v = (torch.randn(B, n, h, D, generator=g, device=DEV).bfloat16() for n, h in ((S, Hq), (T, Hkv), (T, Hkv)))
+    out, lse = flash_fwd(q, k, v, causal, D ** -0.5)
+    L.check_status()
+    want, want_lse = truth(q.double(), k.double(), v.double(), causal, D ** -0.5)
+    assert rel_err(out, want) < 2.0 ** -8
+    assert float((lse.double() - want_lse).abs().max()) < 1e-5 * max(1.0, float(want_lse.abs().max()))

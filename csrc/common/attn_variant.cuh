@@ -33,27 +33,8 @@ struct Variant {
 // tanh to fp32 accuracy relative to 1 (scores under a cap are fp32 quantities): 1 - 2 / (1 + e^2x)
 __device__ __forceinline__ float soft_tanh(float x) { return 1.f - __fdividef(2.f, 1.f + exp2f(x * 2.8853900817779268f)); }
 
-// First key tile (of `bn` keys) that a query tile starting at row q0 can see; `off` = T - S (bottom-right alignment).
-__device__ __forceinline__ int first_key_tile(const Variant& v, int b, int q0, int S, int T, int bn, int n_tiles) {
-  const int off = T - S;
-  int lo = 0;
-  if (v.window > 0) lo = max(0, (q0 + off - v.window + 1) / bn);
-  if (v.chunk > 0) lo = max(lo, (q0 + off) / v.chunk * v.chunk / bn);
-  if (v.first != nullptr) lo = max(lo, v.first[q0 / bn]);
-  if (v.q_seg != nullptr && v.k_seg != nullptr) {
-    const int first = v.q_seg[static_cast<long long>(b) * S + min(q0, S - 1)];
-    const int* ks = v.k_seg + static_cast<long long>(b) * T;
-    // id 0 marks padding, which may follow the last document: a tile that ends in padding is never skipped
-    while (lo < n_tiles) {
-      const int last = ks[min(lo * bn + bn - 1, T - 1)];
-      if (last == 0 || last >= first) break;
-      ++lo;
-    }
-  }
-  return min(lo, n_tiles);
-}
-
-// The same, found by a whole warp: 32 tiles of packed documents a turn.
+// First key tile (of `bn` keys) that a query tile starting at row q0 can see (bottom-right alignment); a whole warp asks, and looks through packed documents 32 tiles a
+// turn.  Id 0 marks padding, which may follow the last document: a tile that ends in padding is never skipped.
 __device__ __forceinline__ int first_key_tile_of_warp(const Variant& v, int b, int q0, int S, int T, int bn, int n_tiles, int lane) {
   const int off = T - S;
   int lo = 0;

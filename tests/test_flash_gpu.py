@@ -60,3 +60,22 @@ def test_flash_forward_pairs_of_tiles(B, S, T, Hq, Hkv, D, causal):
     want, want_lse = truth(q.double(), k.double(), v.double(), causal, D ** -0.5)
     assert rel_err(out, want) < 2.0 ** -8
     assert float((lse.double() - want_lse).abs().max()) < 1e-5 * max(1.0, float(want_lse.abs().max()))
+
+
+@pytest.mark.parametrize("B,S,Hq,Hkv,D,causal", [(1, 64, 1, 1, 128, True), (1, 192, 4, 1, 64, False), (1, 192, 2, 2, 128, True), (2, 640, 30, 15, 64, True), (1, 1152, 18, 6, 128, True),
+                                                 (2, 256, 96, 32, 128, False)])
+def test_flash_backward_tiles(B, S, Hq, Hkv, D, causal):
+    """Lengths that end in the middle of a tile of queries (their statistics are half there), more query tiles than CTAs, several heads a key head.  Weights and their
+    gradients are rounded to bf16 (2^-9 each) in front of the products, the results once more."""
+    from dew_b200.ops.flash import flash_bwd, flash_fwd
+    g = torch.Generator(device=DEV).manual_seed(S + Hq)
+    q, k, v, do = (torch.randn(B, S, h, D, generator=g, device=DEV).bfloat16() for h in (Hq, Hkv, Hkv, Hq))
+    out, lse = flash_fwd(q, k, v, causal, D ** -0.5)
+    got = flash_bwd(do, q, k, v, out, lse, causal, D ** -0.5)
+    again = flash_bwd(do, q, k, v, out, lse, causal, D ** -0.5)
+    L.check_status()
+    leaves = [x.double().requires_grad_() for x in (q, k, v)]
+    want = torch.autograd.grad(truth(*leaves, causal, D ** -0.5)[0], leaves, do.double())
+    for a, b, w in zip(got, again, want):
+        assert torch.equal(a, b)
+        assert rel_err(a, w) < 2.0 ** -7

@@ -18,11 +18,12 @@
 //                        and stores G as it stands on entry to each chunk (the gradient of that chunk's exit state).
 //
 // A scan is one chain of products and of the elementwise steps between them, on B * H of the SMs, and nothing in it is near the rate of any unit; what counts is what
-// stands in the chain.  Warp roles: warps 0..7 hold the state (thread = TMEM lane = value index, half of the keys each, half of a chunk's tokens in the steps over
-// tokens), one warp fetches (2-stage ring of per-chunk operand tiles), one issues the products, uniformly, and in the forward scan four write O, whose accumulators
-// are double, beside the chain.  What leaves for memory (Vn, the states) leaves behind the arrival that the next product waits for, and the backward's products that
-// need no state are issued before the state is there.  Measured for 2 x 16 heads of 8192 tokens, with four warps for all of it and now: forward 660 -> 400 us,
-// backward 344 -> 275 us.  Every wait is bounded; a timed-out wait records a status code, raises
+// stands in the chain.  Warp roles: warps 0..15 hold the state (thread = TMEM lane = value index, a quarter of the keys each, a quarter of a chunk's tokens in the steps
+// over tokens) and keep it as an operand in tensor memory; two warps fetch, what the start of a chunk needs apart from the rest; one issues the products, uniformly; in
+// the forward scan four write O, whose accumulators are double, beside the chain; what the backward reads (Vn, the states and their gradients) leaves as whole tiles
+// through shared memory, sent by one thread.  The backward's products that need no state are issued before the state is there.  Measured for 2 x 16 heads of 8192
+// tokens: with eight warps, the state's operand in shared memory, two stages of everything and stores from registers the forward walk took 400 us with the output and
+// 400 with what the backward reads, the reverse walk 275; now 279, 228 and 223.  Every wait is bounded; a timed-out wait records a status code, raises
 // the CTA's abort flag, and all roles leave through the common exit that frees the tensor memory.
 //
 // Replaces the reference's fla-style kernels KktSolve / RecomputeWU / ChunkFwdH / ChunkFwdO / ChunkBwdDhu
@@ -256,69 +257,104 @@ gdn_prepare_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 // ------------------------------------------------------------------------------------------------------------------
 // scans
 
-constexpr int STATE_WARPS = 8, OUT_WARPS = 4;          // of the forward scan: state, output, TMA, products; the backward has no output warps
-constexpr int FWD_THREADS = 32 * (STATE_WARPS + OUT_WARPS + 2), BWD_THREADS = 32 * (STATE_WARPS + 2);
-constexpr int HALF = HD / 2;                           // keys of the state that one thread holds
+constexpr int STATE_WARPS = 16, OUT_WARPS = 4;
+constexpr int KEYS = HD * 4 / STATE_WARPS;             // of the state, held by one thread (32)
+constexpr int TOKENS = CH * 4 / STATE_WARPS;           // of a chunk, in its steps over tokens (16)
 constexpr int T16 = CH * HD * 2;                       // 16 KiB: a [64 x 128] bf16 tile (two 64-column sub-tiles)
 constexpr int T8 = CH * CH * 2;                        // 8 KiB: P
-constexpr int STAGE = 4 * T16 + T8;                    // 72 KiB of tiles per chunk
-constexpr int OFF_STATE = 2 * STAGE;                   // [128 x 128] bf16 state tile (32 KiB)
-constexpr int OFF_VN = OFF_STATE + 2 * T16;            // two [128 x 64] bf16 tiles (16 KiB each)
-constexpr int OFF_G = OFF_VN + 2 * T16;                // g of the two stages
-constexpr int OFF_BARS = OFF_G + 2 * CH * 4;
-constexpr int OFF_W = OFF_BARS + 256;                  // a warp's own copy of its tokens' decays: one exponential a token and warp, read back as broadcasts
-constexpr int SCAN_SMEM = OFF_W + (STATE_WARPS * 32 + OUT_WARPS * CH) * 4;
 
-struct ScanBars {
-  uint64_t in_full[2], in_empty[2], s_ready, acc_full, vn_ready, ds_full, o_full[2];
+// Backward: what the start of a chunk needs (dO, Qg, K, P, g) in two slots that are free early in the chunk, W in three.  With `SEND` the chunks' exit-state gradients and
+// dVn leave as bf16 tiles that one thread sends to memory; without, the state gradients in fp32 by the threads that hold them.
+template <bool SEND>
+struct Bwd {
+  static constexpr int A = 2, W = 3;
+  static constexpr int A_SLOT = 3 * T16 + T8;
+  static constexpr int OFF_A = 0, OFF_WT = A * A_SLOT, OFF_DVN = OFF_WT + W * T16;      // DVN: -dVn^T [128 x 64] as an operand
+  static constexpr int OFF_OUT = OFF_DVN + T16, OFF_ST = OFF_OUT + (SEND ? T16 : 0);     // dVn [64 x 128] and the state gradient [key][value] on their way to memory
+  static constexpr int OFF_G = OFF_ST + (SEND ? 2 * T16 : 0), OFF_BARS = OFF_G + A * CH * 4, OFF_W = OFF_BARS + 256;      // OFF_W: a warp's own copy of its tokens' decays
+  static constexpr int SMEM = OFF_W + STATE_WARPS * TOKENS * 4;
+  static constexpr int SEND_WARP = STATE_WARPS, TMA_WARP = STATE_WARPS + 1, TMA2_WARP = TMA_WARP + 1, MMA_WARP = TMA_WARP + 2, THREADS = 32 * (MMA_WARP + 1);
+  static_assert(SMEM <= 232448, "scan kernels exceed the shared memory of an SM");
+};
+
+struct BwdBars {
+  uint64_t a_full[2], a_empty[2], w_full[3], w_empty[3];
+  uint64_t s_ready, acc_full, vn_ready, ds_full, tile_ready, state_sent, vn_sent;
   uint32_t tmem_base;
   int abort_flag, poisoned;
 };
-static_assert(sizeof(ScanBars) <= 256, "ScanBars must fit its slot");
-static_assert(SCAN_SMEM <= 232448, "scan kernels exceed the shared memory of an SM");
+static_assert(sizeof(BwdBars) <= 256, "BwdBars must fit its slot");
+
+// Forward: W, U and g in three slots, Q in three, K and P in as many as there is room for.  A chunk's share arrives some 2.3 us after its slot is free, and what the start
+// of a chunk needs is free early in the one it was for, so a third slot there covers what two stages of everything did not: the walk waited for its tiles for two of
+// every five cycles.  With `OUT` the output is written (by four warps); without, what the backward reads: the states in front of the chunks and Vn, as tiles that one
+// thread sends to memory, since 48 scattered stores a thread and chunk stood in the chain for half of its time.
+template <bool OUT>
+struct Fwd {
+  static constexpr int AB = 3, C = OUT ? 2 : 3;                        // slots
+  static constexpr int A_SLOT = 2 * T16, C_SLOT = T16 + (OUT ? T8 : 0);
+  static constexpr int OFF_A = 0, OFF_Q = AB * A_SLOT, OFF_C = OFF_Q + (OUT ? AB * T16 : 0), OFF_VD = OFF_C + C * C_SLOT;
+  static constexpr int OFF_VN = OFF_VD + T16;                          // OUT: Vn^T [128 x 64] as an operand; else Vn [64 x 128] on its way to memory
+  static constexpr int OFF_ST = OFF_VN + T16;                          // the state [128 x 128] on its way to memory
+  static constexpr int OFF_G = OFF_ST + (OUT ? 0 : 2 * T16);
+  static constexpr int OFF_BARS = OFF_G + AB * CH * 4, OFF_W = OFF_BARS + 256;
+  static constexpr int SMEM = OFF_W + (STATE_WARPS * TOKENS + (OUT ? OUT_WARPS * CH : 0)) * 4;
+  static constexpr int EXTRA = OUT ? OUT_WARPS : 1;                    // output warps, or the one that sends tiles off
+  static constexpr int TMA_WARP = STATE_WARPS + EXTRA, TMA2_WARP = TMA_WARP + 1, MMA_WARP = TMA_WARP + 2, THREADS = 32 * (MMA_WARP + 1);
+  static_assert(SMEM <= 232448, "scan kernels exceed the shared memory of an SM");
+};
+
+struct FwdBars {
+  uint64_t a_full[3], a_empty[3], q_full[3], q_empty[3], c_full[3], c_empty[3];
+  uint64_t s_ready, acc_full, vn_ready, ds_full, o_full[2], o_read[2], tile_ready, state_sent, vn_sent;
+  uint32_t tmem_base;
+  int abort_flag, poisoned;
+};
+static_assert(sizeof(FwdBars) <= 256, "FwdBars must fit its slot");
 
 __device__ __forceinline__ uint4 pack8(const float* v) {
   return make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
 }
 
-// Writes this thread's half row (64 values) of the transposed state as bf16 into the K-major operand tile.
-__device__ __forceinline__ void write_state_row(uint8_t* tile, int v, int half, const float (&S)[HALF]) {
+// Writes this thread's part of a row of the transposed state as bf16 to the tensor-memory operand (two keys a 32-bit column).
+__device__ __forceinline__ void write_state_row(uint32_t operand, const float (&S)[KEYS]) {
+  uint32_t w[KEYS / 2];
 #pragma unroll
-  for (int c16 = 0; c16 < 8; ++c16) *reinterpret_cast<uint4*>(tile + half * (HD * 128) + swz(v, c16)) = pack8(S + c16 * 8);
+  for (int d = 0; d < KEYS / 2; ++d) w[d] = pack_bf16(S[2 * d], S[2 * d + 1]);
+  tmem_st_32x32b_x16(operand, w);
+  tmem_st_wait();
 }
 
-// This thread's half row of a state [key][value] in memory, or zeros.
-__device__ __forceinline__ void read_state(float (&S)[HALF], const float* states, int x, int v, int half) {
+// This thread's part of a row of a state [key][value] in memory, or zeros.
+__device__ __forceinline__ void read_state(float (&S)[KEYS], const float* states, int x, int v, int part) {
   if (states == nullptr) {
 #pragma unroll
-    for (int d = 0; d < HALF; ++d) S[d] = 0.f;
+    for (int d = 0; d < KEYS; ++d) S[d] = 0.f;
   } else {
-    const float* src = states + (static_cast<long long>(x) * HD + half * HALF) * HD + v;
+    const float* src = states + (static_cast<long long>(x) * HD + part * KEYS) * HD + v;
 #pragma unroll
-    for (int d = 0; d < HALF; ++d) S[d] = src[d * HD];
+    for (int d = 0; d < KEYS; ++d) S[d] = src[d * HD];
   }
 }
 
 struct ScanCommon {
   uint8_t* smem;
-  ScanBars* bars;
   uint32_t tmem;
   volatile int* abort_flag;
 };
 
-// Common prologue: status check, barriers, tensor memory.  Returns false if the CTA must leave at once.
-__device__ __forceinline__ bool scan_prologue(uint8_t* smem, int* err, ScanCommon& sc, int readers, int alloc_warp) {
+// Common prologue: status check, barriers (`init`, by one thread), tensor memory.  Returns false if the CTA must leave at once.
+template <typename Bars, typename Init>
+__device__ __forceinline__ bool scan_prologue(uint8_t* smem, Bars* bars, int* err, ScanCommon& sc, int alloc_warp, Init init) {
   if ((smem_u32(smem) & 1023u) != 0) {
     if (threadIdx.x == 0) atomicCAS(err, 0, ERR_BAD_ARG);
     return false;
   }
-  ScanBars* bars = reinterpret_cast<ScanBars*>(smem + OFF_BARS);
   if (threadIdx.x == 0) bars->poisoned = *reinterpret_cast<volatile int*>(err);
   __syncthreads();
   if (bars->poisoned != 0) return false;
-  const int warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 2; ++i) { mbar_init(&bars->in_full[i], 1); mbar_init(&bars->in_empty[i], readers); mbar_init(&bars->o_full[i], 1); }
+    init();
     mbar_init(&bars->s_ready, STATE_WARPS);
     mbar_init(&bars->acc_full, 1);
     mbar_init(&bars->vn_ready, STATE_WARPS);
@@ -327,12 +363,11 @@ __device__ __forceinline__ bool scan_prologue(uint8_t* smem, int* err, ScanCommo
     fence_barrier_init();
     fence_proxy_async();
   }
-  if (warp == alloc_warp) { tmem_alloc(&bars->tmem_base, 512); tmem_relinquish(); }
+  if ((threadIdx.x >> 5) == alloc_warp) { tmem_alloc(&bars->tmem_base, 512); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   sc.smem = smem;
-  sc.bars = bars;
   sc.tmem = bars->tmem_base;
   sc.abort_flag = &bars->abort_flag;
   return true;
@@ -358,112 +393,146 @@ __device__ __forceinline__ bool math_wait(uint64_t* bar, uint32_t parity, const 
   return true;
 }
 
-// Stage tile offsets of the forward scan: W, U, Q, K, P.  Of the backward scan: dO, Qg, K, W, P.
-constexpr int F_W = 0, F_U = T16, F_Q = 2 * T16, F_K = 3 * T16, F_P = 4 * T16;
-constexpr int B_DO = 0, B_QG = T16, B_K = 2 * T16, B_W = 3 * T16, B_P = 4 * T16;
-
-__global__ void __launch_bounds__(FWD_THREADS, 1)
+template <bool OUT>
+__global__ void __launch_bounds__(Fwd<OUT>::THREADS, 1)
 gdn_scan_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                     const __grid_constant__ CUtensorMap tw, const __grid_constant__ CUtensorMap tu,
-                    const __grid_constant__ CUtensorMap tp, const float* __restrict__ gc,
-                    const float* __restrict__ initial, __nv_bfloat16* __restrict__ out, float* __restrict__ final_state,
-                    __nv_bfloat16* __restrict__ states, __nv_bfloat16* __restrict__ vn_out, int T, int H, int rep, int Tp,
-                    int N, float scale, int* __restrict__ err) {
+                    const __grid_constant__ CUtensorMap tp, const __grid_constant__ CUtensorMap tstates, const __grid_constant__ CUtensorMap tvn,
+                    const float* __restrict__ gc, const float* __restrict__ initial, __nv_bfloat16* __restrict__ out, float* __restrict__ final_state,
+                    __nv_bfloat16* __restrict__ states, __nv_bfloat16* __restrict__ vn_out, int T, int H, int rep, int Tp, int N, float scale, int* __restrict__ err) {
+  using F = Fwd<OUT>;
   extern __shared__ __align__(1024) uint8_t smem[];
-  constexpr int TMA_WARP = STATE_WARPS + OUT_WARPS, MMA_WARP = TMA_WARP + 1;
+  FwdBars* bars = reinterpret_cast<FwdBars*>(smem + F::OFF_BARS);
   ScanCommon sc;
-  if (!scan_prologue(smem, err, sc, STATE_WARPS + OUT_WARPS, MMA_WARP)) return;
-  ScanBars* bars = sc.bars;
+  if (!scan_prologue(smem, bars, err, sc, F::MMA_WARP, [&]() {
+        for (int i = 0; i < 3; ++i) {
+          mbar_init(&bars->a_full[i], 1); mbar_init(&bars->a_empty[i], STATE_WARPS + (OUT ? OUT_WARPS : 0) + 1);
+          mbar_init(&bars->q_full[i], 1); mbar_init(&bars->q_empty[i], 1);
+          mbar_init(&bars->c_full[i], 1); mbar_init(&bars->c_empty[i], 1);
+        }
+        for (int i = 0; i < 2; ++i) { mbar_init(&bars->o_full[i], 1); mbar_init(&bars->o_read[i], OUT_WARPS); }
+        mbar_init(&bars->tile_ready, STATE_WARPS);
+        mbar_init(&bars->state_sent, 1);
+        mbar_init(&bars->vn_sent, 1);
+      })) return;
   const uint32_t tmem = sc.tmem;
   volatile int* abort_flag = sc.abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int x = blockIdx.x, b = x / H, h = x % H;
-  uint8_t* sState = smem + OFF_STATE;
-  uint8_t* sVn = smem + OFF_VN;
-  uint8_t* sVd = smem + OFF_VN + T16;
-  float* sG = reinterpret_cast<float*>(smem + OFF_G);
-  constexpr int TM_ACC1 = 0, TM_O1 = 64, TM_O2 = 192, TM_DS = 384;       // O1 and O2 by the parity of the chunk, 64 columns apart
+  uint8_t* sVn = smem + F::OFF_VN;
+  uint8_t* sVd = smem + F::OFF_VD;
+  float* sG = reinterpret_cast<float*>(smem + F::OFF_G);
+  constexpr int TM_ACC1 = 0, TM_O1 = 64, TM_O2 = 192, TM_ST = 320, TM_DS = 384;       // O1 and O2 by the parity of the chunk, 64 columns apart; ST: the state as an operand
   const int v = tid & 127;                               // value index == TMEM lane == row of the transposed state
   const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
 
-  if (warp == TMA_WARP) {
+  if (warp == F::TMA_WARP) {
+    // W, U, g and Q
     if (lane == 0) {
-      tma_prefetch_desc(&tq); tma_prefetch_desc(&tk); tma_prefetch_desc(&tw); tma_prefetch_desc(&tu); tma_prefetch_desc(&tp);
+      tma_prefetch_desc(&tq); tma_prefetch_desc(&tw); tma_prefetch_desc(&tu);
       for (int n = 0; n < N; ++n) {
-        const int s = n & 1; const uint32_t ph = (n >> 1) & 1;
-        if (!mbar_wait(&bars->in_empty[s], ph ^ 1, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_EMPTY); break; }
-        uint8_t* st = smem + s * STAGE;
-        uint64_t* bar = &bars->in_full[s];
-        mbar_expect_tx(bar, STAGE + CH * 4);
+        const int s = n % F::AB; const uint32_t ph = (n / F::AB) & 1;
         const int row = x * Tp + n * CH;
+        if (!mbar_wait(&bars->a_empty[s], ph ^ 1, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_EMPTY); break; }
+        uint8_t* st = smem + F::OFF_A + s * F::A_SLOT;
+        mbar_expect_tx(&bars->a_full[s], F::A_SLOT + CH * 4);
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
-          tma_load_2d(st + F_W + t * (CH * 128), &tw, bar, t * 64, row);
-          tma_load_2d(st + F_U + t * (CH * 128), &tu, bar, t * 64, row);
-          tma_load_4d(st + F_Q + t * (CH * 128), &tq, bar, t * 64, h / rep, n * CH, b);
-          tma_load_4d(st + F_K + t * (CH * 128), &tk, bar, t * 64, h / rep, n * CH, b);
+          tma_load_2d(st + t * (CH * 128), &tw, &bars->a_full[s], t * 64, row);
+          tma_load_2d(st + T16 + t * (CH * 128), &tu, &bars->a_full[s], t * 64, row);
         }
-        tma_load_2d(st + F_P, &tp, bar, 0, row);
-        bulk_load_1d(sG + s * CH, gc + static_cast<long long>(x) * Tp + n * CH, CH * 4, bar);
+        bulk_load_1d(sG + s * CH, gc + static_cast<long long>(x) * Tp + n * CH, CH * 4, &bars->a_full[s]);
+        if (OUT) {
+          if (!mbar_wait(&bars->q_empty[s], ph ^ 1, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_EMPTY); break; }
+          mbar_expect_tx(&bars->q_full[s], T16);
+#pragma unroll
+          for (int t = 0; t < 2; ++t) tma_load_4d(smem + F::OFF_Q + s * T16 + t * (CH * 128), &tq, &bars->q_full[s], t * 64, h / rep, n * CH, b);
+        }
       }
     }
-  } else if (warp == MMA_WARP) {
+  } else if (warp == F::TMA2_WARP) {
+    // K and P
+    if (lane == 0) {
+      tma_prefetch_desc(&tk); tma_prefetch_desc(&tp);
+      for (int n = 0; n < N; ++n) {
+        const int s = n % F::C; const uint32_t ph = (n / F::C) & 1;
+        if (!mbar_wait(&bars->c_empty[s], ph ^ 1, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_EMPTY); break; }
+        uint8_t* st = smem + F::OFF_C + s * F::C_SLOT;
+        mbar_expect_tx(&bars->c_full[s], F::C_SLOT);
+#pragma unroll
+        for (int t = 0; t < 2; ++t) tma_load_4d(st + t * (CH * 128), &tk, &bars->c_full[s], t * 64, h / rep, n * CH, b);
+        if (OUT) tma_load_2d(st + T16, &tp, &bars->c_full[s], 0, x * Tp + n * CH);
+      }
+    }
+  } else if (warp == F::MMA_WARP) {
     constexpr uint32_t idesc_n64 = make_idesc(128, 64, 1, 1, 0, 0);
     constexpr uint32_t idesc_ds = make_idesc(128, 128, 1, 1, 0, 1);
-    const uint32_t sa = smem_u32(sState), vna = smem_u32(sVn), vda = smem_u32(sVd);
+    const uint32_t vna = smem_u32(sVn), vda = smem_u32(sVd);
     for (int n = 0; n < N; ++n) {
-      const int s = n & 1; const uint32_t ph = (n >> 1) & 1;
-      const uint32_t st = smem_u32(smem + s * STAGE);
-      if (!math_wait(&bars->in_full[s], ph, sc, err, ERR_WAIT_FULL)) break;
+      const int s = n & 1, sa = n % F::AB, sk = n % F::C; const uint32_t pa = (n / F::AB) & 1, pk = (n / F::C) & 1;
+      const uint32_t wa = smem_u32(smem + F::OFF_A + sa * F::A_SLOT), qa = smem_u32(smem + F::OFF_Q + sa * T16), ka = smem_u32(smem + F::OFF_C + sk * F::C_SLOT);
+      if (!math_wait(&bars->a_full[sa], pa, sc, err, ERR_WAIT_FULL)) break;
       if (!math_wait(&bars->s_ready, n & 1, sc, err, ERR_WAIT_OTHER)) break;
       tc_fence_after();
       if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < HD / 16; ++kk) {
-          const uint32_t aoff = (kk >> 2) * (HD * 128) + (kk & 3) * 32, boff = (kk >> 2) * (CH * 128) + (kk & 3) * 32;
-          umma_bf16_ss(tmem + TM_ACC1, make_sdesc_sw128(sa + aoff, 16, 1024), make_sdesc_sw128(st + F_W + boff, 16, 1024),
-                       idesc_n64, kk > 0 ? 1u : 0u);
+          const uint32_t boff = (kk >> 2) * (CH * 128) + (kk & 3) * 32;
+          umma_bf16_ts(tmem + TM_ACC1, tmem + TM_ST + kk * 8, make_sdesc_sw128(wa + boff, 16, 1024), idesc_n64, kk > 0 ? 1u : 0u);
         }
         umma_commit(&bars->acc_full);
-#pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
-          const uint32_t aoff = (kk >> 2) * (HD * 128) + (kk & 3) * 32, boff = (kk >> 2) * (CH * 128) + (kk & 3) * 32;
-          umma_bf16_ss(tmem + TM_O1 + s * 64, make_sdesc_sw128(sa + aoff, 16, 1024), make_sdesc_sw128(st + F_Q + boff, 16, 1024),
-                       idesc_n64, kk > 0 ? 1u : 0u);
-        }
+        umma_commit(&bars->a_empty[sa]);
       }
       __syncwarp();
+      if (OUT) {
+        if (!math_wait(&bars->q_full[sa], pa, sc, err, ERR_WAIT_FULL)) break;
+        if (n > 1 && !math_wait(&bars->o_read[s], ((n >> 1) - 1) & 1, sc, err, ERR_WAIT_TMEM_EMPTY)) break;
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+          for (int kk = 0; kk < HD / 16; ++kk) {
+            const uint32_t boff = (kk >> 2) * (CH * 128) + (kk & 3) * 32;
+            umma_bf16_ts(tmem + TM_O1 + s * 64, tmem + TM_ST + kk * 8, make_sdesc_sw128(qa + boff, 16, 1024), idesc_n64, kk > 0 ? 1u : 0u);
+          }
+          umma_commit(&bars->q_empty[sa]);
+        }
+        __syncwarp();
+      }
+      if (!math_wait(&bars->c_full[sk], pk, sc, err, ERR_WAIT_FULL)) break;
       if (!math_wait(&bars->vn_ready, n & 1, sc, err, ERR_WAIT_OTHER)) break;
       tc_fence_after();
       if (elect_one()) {
-        // the state's product first: the chain waits for it (and for all before it, so that O1 is done with the state tile)
+        // the state's product first: the chain waits for it (and for all before it, so that O1 is done with the state)
 #pragma unroll
         for (int kk = 0; kk < CH / 16; ++kk) {
-          umma_bf16_ss(tmem + TM_DS, make_sdesc_sw128(vda + kk * 32, 16, 1024),
-                       make_sdesc_sw128(st + F_K + kk * 2048, CH * 128, 1024), idesc_ds, kk > 0 ? 1u : 0u);
+          umma_bf16_ss(tmem + TM_DS, make_sdesc_sw128(vda + kk * 32, 16, 1024), make_sdesc_sw128(ka + kk * 2048, CH * 128, 1024), idesc_ds, kk > 0 ? 1u : 0u);
         }
         umma_commit(&bars->ds_full);
+        if (OUT) {
 #pragma unroll
-        for (int kk = 0; kk < CH / 16; ++kk) {
-          umma_bf16_ss(tmem + TM_O2 + s * 64, make_sdesc_sw128(vna + kk * 32, 16, 1024), make_sdesc_sw128(st + F_P + kk * 32, 16, 1024),
-                       idesc_n64, kk > 0 ? 1u : 0u);
+          for (int kk = 0; kk < CH / 16; ++kk) {
+            umma_bf16_ss(tmem + TM_O2 + s * 64, make_sdesc_sw128(vna + kk * 32, 16, 1024), make_sdesc_sw128(ka + T16 + kk * 32, 16, 1024),
+                         idesc_n64, kk > 0 ? 1u : 0u);
+          }
+          umma_commit(&bars->o_full[s]);                 // Vn's tile is rewritten only after the next acc_full, which comes behind this product
         }
-        umma_commit(&bars->o_full[s]);                   // Vn's tile is rewritten only after the next acc_full, which comes behind this product
+        umma_commit(&bars->c_empty[sk]);
       }
       __syncwarp();
     }
   } else if (warp >= STATE_WARPS) {
-    float* w = reinterpret_cast<float*>(smem + OFF_W) + STATE_WARPS * 32 + (warp - STATE_WARPS) * CH;
-    for (int n = 0; n < N; ++n) {
-      const int s = n & 1; const uint32_t ph = (n >> 1) & 1;
-      const float* gs = sG + s * CH;
-      if (!math_wait(&bars->in_full[s], ph, sc, err, ERR_WAIT_FULL)) break;
-      w[lane] = scale * __expf(gs[lane]);
-      w[lane + 32] = scale * __expf(gs[lane + 32]);
-      __syncwarp();
-      if (!math_wait(&bars->o_full[s], ph, sc, err, ERR_WAIT_TMEM_FULL)) break;
-      tc_fence_after();
-      if (out != nullptr) {
+    if constexpr (OUT) {
+      float* w = reinterpret_cast<float*>(smem + F::OFF_W) + STATE_WARPS * TOKENS + (warp - STATE_WARPS) * CH;
+      for (int n = 0; n < N; ++n) {
+        const int s = n & 1, sa = n % F::AB;
+        const float* gs = sG + sa * CH;
+        if (!math_wait(&bars->a_full[sa], (n / F::AB) & 1, sc, err, ERR_WAIT_FULL)) break;
+        w[lane] = scale * __expf(gs[lane]);
+        w[lane + 32] = scale * __expf(gs[lane + 32]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->a_empty[sa]);
+        if (!math_wait(&bars->o_full[s], (n >> 1) & 1, sc, err, ERR_WAIT_TMEM_FULL)) break;
+        tc_fence_after();
         // O^T row
         __nv_bfloat16* orow = out + ((static_cast<long long>(b) * T + n * CH) * H + h) * HD + v;
 #pragma unroll
@@ -476,158 +545,206 @@ gdn_scan_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
           for (int ii = 0; ii < 16; ++ii) {
             const int i = q * 16 + ii;
             const float o = w[i] * __uint_as_float(o1[ii]) + __uint_as_float(o2[ii]);
-            if (n * CH + i < T) orow[static_cast<long long>(i) * H * HD] = __float2bfloat16(o);
+            if (out != nullptr && n * CH + i < T) orow[static_cast<long long>(i) * H * HD] = __float2bfloat16(o);
           }
         }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->o_read[s]);
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->in_empty[s]);
+    } else if (lane == 0) {
+      // the tiles on their way to memory
+      for (int n = 0; n < N; ++n) {
+        if (!mbar_wait(&bars->tile_ready, n & 1, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_OTHER); break; }
+#pragma unroll
+        for (int t = 0; t < 2; ++t) tma_store_2d(&tstates, smem + F::OFF_ST + t * (HD * 128), t * 64, (x * N + n) * HD);
+        tma_store_commit();
+        tma_store_wait_read<0>();
+        mbar_arrive(&bars->state_sent);
+        if (!mbar_wait(&bars->vn_ready, n & 1, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_OTHER); break; }
+#pragma unroll
+        for (int t = 0; t < 2; ++t) tma_store_2d(&tvn, smem + F::OFF_VN + t * (CH * 128), t * 64, x * Tp + n * CH);
+        tma_store_commit();
+        tma_store_wait_read<0>();
+        mbar_arrive(&bars->vn_sent);
+      }
+      tma_store_wait<0>();
     }
   } else {
-    const int half = warp >> 2, j0 = half * 32;          // this thread's keys 64 half .., and its tokens of a chunk
-    float* w = reinterpret_cast<float*>(smem + OFF_W) + warp * 32;
-    float S[HALF];
-    read_state(S, initial, x, v, half);
-    write_state_row(sState, v, half, S);
-    fence_proxy_async();
-    tc_fence_before();
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&bars->s_ready);
+    const int part = warp >> 2, j0 = part * TOKENS;      // this thread's keys KEYS part .., and its tokens of a chunk
+    float* w = reinterpret_cast<float*>(smem + F::OFF_W) + warp * TOKENS;
+    const uint32_t operand = tmem + lane_addr + TM_ST + part * (KEYS / 2);
+    uint8_t* srow = smem + F::OFF_ST + (part >> 1) * (HD * 128);
+    float S[KEYS];
+    // the state as the operand of the next products, then (not OUT) as a row of the tile that goes to memory
+    auto deliver = [&](bool last) {
+      write_state_row(operand, S);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars->s_ready);
+      if (!OUT && !last) {
+#pragma unroll
+        for (int c = 0; c < KEYS / 8; ++c) *reinterpret_cast<uint4*>(srow + swz(v, (part & 1) * 4 + c)) = pack8(S + c * 8);
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->tile_ready);
+      }
+    };
+    read_state(S, initial, x, v, part);
+    deliver(false);
     bool ok = true;
     for (int n = 0; n < N && ok; ++n) {
-      const int s = n & 1; const uint32_t ph = (n >> 1) & 1;
-      const uint8_t* st = smem + s * STAGE;
-      const float* gs = sG + s * CH;
-      if (!math_wait(&bars->in_full[s], ph, sc, err, ERR_WAIT_FULL)) { ok = false; break; }
+      const int sa = n % F::AB;
+      const uint8_t* st = smem + F::OFF_A + sa * F::A_SLOT;
+      const float* gs = sG + sa * CH;
+      if (!math_wait(&bars->a_full[sa], (n / F::AB) & 1, sc, err, ERR_WAIT_FULL)) { ok = false; break; }
       const float gl = gs[CH - 1];
       // Vn^T row: U[j][v] - acc1[j]; the copy for the state update carries e^{g_L - g_j}.  U and the decays are read while the product runs.
-      const uint8_t* ucol = st + F_U + (v >> 6) * (CH * 128) + (v & 7) * 2;
+      const uint8_t* ucol = st + T16 + (v >> 6) * (CH * 128) + (v & 7) * 2;
       const int uc16 = (v & 63) >> 3;
-      uint32_t u[16];                                    // U, then Vn
+      uint32_t u[TOKENS / 2];                            // U, then Vn
 #pragma unroll
-      for (int jj = 0; jj < 16; ++jj)
+      for (int jj = 0; jj < TOKENS / 2; ++jj)
         u[jj] = *reinterpret_cast<const uint16_t*>(ucol + swz(j0 + 2 * jj, uc16)) |
                 static_cast<uint32_t>(*reinterpret_cast<const uint16_t*>(ucol + swz(j0 + 2 * jj + 1, uc16))) << 16;
-      w[lane] = __expf(gl - gs[j0 + lane]);
+      if (lane < TOKENS) w[lane] = __expf(gl - gs[j0 + lane]);
       __syncwarp();
+      if (lane == 0) mbar_arrive(&bars->a_empty[sa]);
+      if (!OUT && n > 0 && !math_wait(&bars->vn_sent, (n - 1) & 1, sc, err, ERR_WAIT_OTHER)) { ok = false; break; }
       if (!math_wait(&bars->acc_full, n & 1, sc, err, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        uint32_t a[16];
-        tmem_ld_32x32b_x16(tmem + lane_addr + TM_ACC1 + j0 + q * 16, a);
+      {
+        uint32_t a[TOKENS];
+        tmem_ld_32x32b_x16(tmem + lane_addr + TM_ACC1 + j0, a);
         tmem_ld_wait();
 #pragma unroll
-        for (int j8 = 0; j8 < 2; ++j8) {
+        for (int j8 = 0; j8 < TOKENS / 8; ++j8) {
           float vn[8], vd[8];
 #pragma unroll
           for (int jj = 0; jj < 8; ++jj) {
-            const uint32_t pair = u[q * 8 + j8 * 4 + (jj >> 1)];
+            const uint32_t pair = u[j8 * 4 + (jj >> 1)];
             vn[jj] = ((jj & 1) ? bf16_hi(pair) : bf16_lo(pair)) - __uint_as_float(a[j8 * 8 + jj]);
-            vd[jj] = vn[jj] * w[q * 16 + j8 * 8 + jj];
+            vd[jj] = vn[jj] * w[j8 * 8 + jj];
           }
           const uint4 packed = pack8(vn);
-          u[q * 8 + j8 * 4] = packed.x; u[q * 8 + j8 * 4 + 1] = packed.y; u[q * 8 + j8 * 4 + 2] = packed.z; u[q * 8 + j8 * 4 + 3] = packed.w;
-          *reinterpret_cast<uint4*>(sVd + swz(v, half * 4 + q * 2 + j8)) = pack8(vd);
-          *reinterpret_cast<uint4*>(sVn + swz(v, half * 4 + q * 2 + j8)) = packed;
+          u[j8 * 4] = packed.x; u[j8 * 4 + 1] = packed.y; u[j8 * 4 + 2] = packed.z; u[j8 * 4 + 3] = packed.w;
+          *reinterpret_cast<uint4*>(sVd + swz(v, part * (TOKENS / 8) + j8)) = pack8(vd);
+          if (OUT) *reinterpret_cast<uint4*>(sVn + swz(v, part * (TOKENS / 8) + j8)) = packed;
         }
+      }
+      if (!OUT) {
+        uint8_t* ncol = sVn + (v >> 6) * (CH * 128) + (v & 7) * 2;
+#pragma unroll
+        for (int jj = 0; jj < TOKENS; ++jj) *reinterpret_cast<uint16_t*>(ncol + swz(j0 + jj, uc16)) = static_cast<uint16_t>(u[jj >> 1] >> (jj & 1) * 16);
       }
       fence_proxy_async();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars->vn_ready);
-      if (vn_out != nullptr) {
+      if (OUT && vn_out != nullptr) {
         uint16_t* dst = reinterpret_cast<uint16_t*>(vn_out) + (static_cast<long long>(x) * Tp + n * CH + j0) * HD + v;
 #pragma unroll
-        for (int jj = 0; jj < 32; ++jj) dst[jj * HD] = static_cast<uint16_t>(u[jj >> 1] >> (jj & 1) * 16);
+        for (int jj = 0; jj < TOKENS; ++jj) dst[jj * HD] = static_cast<uint16_t>(u[jj >> 1] >> (jj & 1) * 16);
       }
-      if (states != nullptr) {
-        // the state on entry to this chunk, as the operand tile holds it (row v = 128 bf16)
-        uint4* dst = reinterpret_cast<uint4*>(states + ((static_cast<long long>(x) * N + n) * HD + v) * HD + half * HALF);
+      if (OUT && states != nullptr) {
+        // the state on entry to this chunk, as the operand holds it (row v = 128 bf16)
+        uint4* dst = reinterpret_cast<uint4*>(states + ((static_cast<long long>(x) * N + n) * HD + v) * HD + part * KEYS);
 #pragma unroll
-        for (int c16 = 0; c16 < 8; ++c16) dst[c16] = pack8(S + c16 * 8);
+        for (int c16 = 0; c16 < KEYS / 8; ++c16) dst[c16] = pack8(S + c16 * 8);
       }
+      if (!OUT && !math_wait(&bars->state_sent, n & 1, sc, err, ERR_WAIT_OTHER)) { ok = false; break; }
       if (!math_wait(&bars->ds_full, n & 1, sc, err, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       // S^T <- e^{g_L} S^T + dS
       const float dl = __expf(gl);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        uint32_t d[16];
-        tmem_ld_32x32b_x16(tmem + lane_addr + TM_DS + half * HALF + q * 16, d);
+      {
+        uint32_t d[KEYS];
+        tmem_ld_32x32b_x32(tmem + lane_addr + TM_DS + part * KEYS, d);
         tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 16; ++i) S[q * 16 + i] = fmaf(S[q * 16 + i], dl, __uint_as_float(d[i]));
+        for (int i = 0; i < KEYS; ++i) S[i] = fmaf(S[i], dl, __uint_as_float(d[i]));
       }
-      write_state_row(sState, v, half, S);
-      fence_proxy_async();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) { mbar_arrive(&bars->s_ready); mbar_arrive(&bars->in_empty[s]); }
+      deliver(n + 1 == N);
     }
     if (ok && final_state != nullptr) {
-      float* dst = final_state + (static_cast<long long>(x) * HD + half * HALF) * HD + v;
+      float* dst = final_state + (static_cast<long long>(x) * HD + part * KEYS) * HD + v;
 #pragma unroll
-      for (int d = 0; d < HALF; ++d) dst[d * HD] = S[d];
+      for (int d = 0; d < KEYS; ++d) dst[d * HD] = S[d];
     }
   }
-  scan_epilogue(sc, MMA_WARP);
+  scan_epilogue(sc, F::MMA_WARP);
 }
 
-__global__ void __launch_bounds__(BWD_THREADS, 1)
+template <bool SEND>
+__global__ void __launch_bounds__(Bwd<SEND>::THREADS, 1)
 gdn_scan_bwd_kernel(const __grid_constant__ CUtensorMap tdo, const __grid_constant__ CUtensorMap tk,
                     const __grid_constant__ CUtensorMap tw, const __grid_constant__ CUtensorMap tqg,
-                    const __grid_constant__ CUtensorMap tp, const float* __restrict__ gc,
-                    const float* __restrict__ d_final, float* __restrict__ dstates, __nv_bfloat16* __restrict__ dstates_bf16,
-                    __nv_bfloat16* __restrict__ dvn_out, float* __restrict__ d_initial, int T, int H, int rep, int Tp, int N,
-                    int* __restrict__ err) {
+                    const __grid_constant__ CUtensorMap tp, const __grid_constant__ CUtensorMap tstates, const __grid_constant__ CUtensorMap tvn,
+                    const float* __restrict__ gc, const float* __restrict__ d_final, float* __restrict__ dstates, __nv_bfloat16* __restrict__ dstates_bf16,
+                    __nv_bfloat16* __restrict__ dvn_out, float* __restrict__ d_initial, int T, int H, int rep,
+                    int Tp, int N, int* __restrict__ err) {
+  using F = Bwd<SEND>;
   extern __shared__ __align__(1024) uint8_t smem[];
-  constexpr int TMA_WARP = STATE_WARPS, MMA_WARP = TMA_WARP + 1;
+  BwdBars* bars = reinterpret_cast<BwdBars*>(smem + F::OFF_BARS);
   ScanCommon sc;
-  if (!scan_prologue(smem, err, sc, STATE_WARPS, MMA_WARP)) return;
-  ScanBars* bars = sc.bars;
+  if (!scan_prologue(smem, bars, err, sc, F::MMA_WARP, [&]() {
+        for (int i = 0; i < F::A; ++i) { mbar_init(&bars->a_full[i], 1); mbar_init(&bars->a_empty[i], STATE_WARPS + 1); }
+        for (int i = 0; i < F::W; ++i) { mbar_init(&bars->w_full[i], 1); mbar_init(&bars->w_empty[i], 1); }
+        mbar_init(&bars->tile_ready, STATE_WARPS);
+        mbar_init(&bars->state_sent, 1);
+        mbar_init(&bars->vn_sent, 1);
+      })) return;
   const uint32_t tmem = sc.tmem;
   volatile int* abort_flag = sc.abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int x = blockIdx.x, b = x / H, h = x % H;
-  uint8_t* sState = smem + OFF_STATE;                    // G^T as bf16
-  uint8_t* sDvn = smem + OFF_VN;                         // -dVn^T as bf16
-  float* sG = reinterpret_cast<float*>(smem + OFF_G);
-  constexpr int TM_A = 0, TM_B = 128, TM_DD = 256;       // A and DD by the parity of the step, 64 and 128 columns apart
+  uint8_t* sDvn = smem + F::OFF_DVN;                     // -dVn^T as bf16
+  float* sG = reinterpret_cast<float*>(smem + F::OFF_G);
+  constexpr int TM_A = 0, TM_B = 128, TM_ST = 192, TM_DD = 256;       // A and DD by the parity of the step, 64 and 128 columns apart; ST: G^T as an operand
+  constexpr int B_DO = 0, B_QG = T16, B_K = 2 * T16, B_P = 3 * T16;   // in a slot
 
-  if (warp == TMA_WARP) {
+  if (warp == F::TMA_WARP) {
     if (lane == 0) {
-      tma_prefetch_desc(&tdo); tma_prefetch_desc(&tk); tma_prefetch_desc(&tw); tma_prefetch_desc(&tqg); tma_prefetch_desc(&tp);
+      tma_prefetch_desc(&tdo); tma_prefetch_desc(&tk); tma_prefetch_desc(&tqg); tma_prefetch_desc(&tp);
       for (int it = 0; it < N; ++it) {
         const int n = N - 1 - it;
         const int s = it & 1; const uint32_t ph = (it >> 1) & 1;
-        if (!mbar_wait(&bars->in_empty[s], ph ^ 1, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_EMPTY); break; }
-        uint8_t* st = smem + s * STAGE;
-        uint64_t* bar = &bars->in_full[s];
-        mbar_expect_tx(bar, STAGE + CH * 4);
+        if (!mbar_wait(&bars->a_empty[s], ph ^ 1, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_EMPTY); break; }
+        uint8_t* st = smem + F::OFF_A + s * F::A_SLOT;
+        uint64_t* bar = &bars->a_full[s];
+        mbar_expect_tx(bar, F::A_SLOT + CH * 4);
         const int row = x * Tp + n * CH;
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
+          tma_load_4d(st + B_K + t * (CH * 128), &tk, bar, t * 64, h / rep, n * CH, b);
           tma_load_4d(st + B_DO + t * (CH * 128), &tdo, bar, t * 64, h, n * CH, b);
           tma_load_2d(st + B_QG + t * (CH * 128), &tqg, bar, t * 64, row);
-          tma_load_4d(st + B_K + t * (CH * 128), &tk, bar, t * 64, h / rep, n * CH, b);
-          tma_load_2d(st + B_W + t * (CH * 128), &tw, bar, t * 64, row);
         }
         tma_load_2d(st + B_P, &tp, bar, 0, row);
         bulk_load_1d(sG + s * CH, gc + static_cast<long long>(x) * Tp + n * CH, CH * 4, bar);
       }
     }
-  } else if (warp == MMA_WARP) {
+  } else if (warp == F::TMA2_WARP) {
+    if (lane == 0) {
+      tma_prefetch_desc(&tw);
+      for (int it = 0; it < N; ++it) {
+        const int s = it % F::W; const uint32_t ph = (it / F::W) & 1;
+        if (!mbar_wait(&bars->w_empty[s], ph ^ 1, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_EMPTY); break; }
+        mbar_expect_tx(&bars->w_full[s], T16);
+#pragma unroll
+        for (int t = 0; t < 2; ++t) tma_load_2d(smem + F::OFF_WT + s * T16 + t * (CH * 128), &tw, &bars->w_full[s], t * 64, x * Tp + (N - 1 - it) * CH);
+      }
+    }
+  } else if (warp == F::MMA_WARP) {
     constexpr uint32_t idesc_a = make_idesc(128, 64, 1, 1, 1, 1);      // dO^T P: both operands MN-major
     constexpr uint32_t idesc_b = make_idesc(128, 64, 1, 1, 0, 0);      // G^T K^T: both K-major
     constexpr uint32_t idesc_dq = make_idesc(128, 128, 1, 1, 1, 1);    // dO^T Qg
     constexpr uint32_t idesc_dw = make_idesc(128, 128, 1, 1, 0, 1);    // (-dVn^T) W
-    const uint32_t sa = smem_u32(sState), dva = smem_u32(sDvn);
+    const uint32_t dva = smem_u32(sDvn);
     for (int it = 0; it < N; ++it) {
-      const int s = it & 1; const uint32_t ph = (it >> 1) & 1;
-      const uint32_t st = smem_u32(smem + s * STAGE);
-      if (!math_wait(&bars->in_full[s], ph, sc, err, ERR_WAIT_FULL)) break;
+      const int s = it & 1, sw = it % F::W; const uint32_t ph = (it >> 1) & 1;
+      const uint32_t st = smem_u32(smem + F::OFF_A + s * F::A_SLOT), wa = smem_u32(smem + F::OFF_WT + sw * T16);
+      if (!math_wait(&bars->a_full[s], ph, sc, err, ERR_WAIT_FULL)) break;
       tc_fence_after();
       if (elect_one()) {
         // what needs no state, into the half of the accumulators that the step before last has left
@@ -648,111 +765,150 @@ gdn_scan_bwd_kernel(const __grid_constant__ CUtensorMap tdo, const __grid_consta
       if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < HD / 16; ++kk) {
-          const uint32_t aoff = (kk >> 2) * (HD * 128) + (kk & 3) * 32, boff = (kk >> 2) * (CH * 128) + (kk & 3) * 32;
-          umma_bf16_ss(tmem + TM_B, make_sdesc_sw128(sa + aoff, 16, 1024), make_sdesc_sw128(st + B_K + boff, 16, 1024),
-                       idesc_b, kk > 0 ? 1u : 0u);
+          const uint32_t boff = (kk >> 2) * (CH * 128) + (kk & 3) * 32;
+          umma_bf16_ts(tmem + TM_B, tmem + TM_ST + kk * 8, make_sdesc_sw128(st + B_K + boff, 16, 1024), idesc_b, kk > 0 ? 1u : 0u);
         }
         umma_commit(&bars->acc_full);
+        umma_commit(&bars->a_empty[s]);
       }
       __syncwarp();
+      if (!math_wait(&bars->w_full[sw], (it / F::W) & 1, sc, err, ERR_WAIT_FULL)) break;
       if (!math_wait(&bars->vn_ready, it & 1, sc, err, ERR_WAIT_OTHER)) break;
       tc_fence_after();
       if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < CH / 16; ++kk) {
           umma_bf16_ss(tmem + TM_DD + s * 128, make_sdesc_sw128(dva + kk * 32, 16, 1024),
-                       make_sdesc_sw128(st + B_W + kk * 2048, CH * 128, 1024), idesc_dw, 1u);
+                       make_sdesc_sw128(wa + kk * 2048, CH * 128, 1024), idesc_dw, 1u);
         }
         umma_commit(&bars->ds_full);
+        umma_commit(&bars->w_empty[sw]);
       }
       __syncwarp();
     }
+  } else if (warp == F::SEND_WARP) {
+    if (SEND && lane == 0) {
+      for (int it = 0; it < N; ++it) {
+        const int n = N - 1 - it;
+        if (!mbar_wait(&bars->tile_ready, it & 1, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_OTHER); break; }
+#pragma unroll
+        for (int t = 0; t < 2; ++t) tma_store_2d(&tstates, smem + F::OFF_ST + t * (HD * 128), t * 64, (x * N + n) * HD);
+        tma_store_commit();
+        tma_store_wait_read<0>();
+        mbar_arrive(&bars->state_sent);
+        if (!mbar_wait(&bars->vn_ready, it & 1, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_OTHER); break; }
+#pragma unroll
+        for (int t = 0; t < 2; ++t) tma_store_2d(&tvn, smem + F::OFF_OUT + t * (CH * 128), t * 64, x * Tp + n * CH);
+        tma_store_commit();
+        tma_store_wait_read<0>();
+        mbar_arrive(&bars->vn_sent);
+      }
+      tma_store_wait<0>();
+    }
   } else {
-    const int v = tid & 127, half = warp >> 2, j0 = half * 32;      // as in the forward scan
-    float* w = reinterpret_cast<float*>(smem + OFF_W) + warp * 32;
+    const int v = tid & 127, part = warp >> 2, j0 = part * TOKENS;      // as in the forward scan
+    float* w = reinterpret_cast<float*>(smem + F::OFF_W) + warp * TOKENS;
     const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    float G[HALF];
-    read_state(G, d_final, x, v, half);
-    write_state_row(sState, v, half, G);
-    fence_proxy_async();
-    tc_fence_before();
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&bars->s_ready);
+    const uint32_t operand = tmem + lane_addr + TM_ST + part * (KEYS / 2);
+    const int c16 = (v & 63) >> 3;
+    uint8_t* gcol = smem + F::OFF_ST + (v >> 6) * (HD * 128) + (v & 7) * 2;            // this value's column of both tiles
+    uint8_t* ncol = smem + F::OFF_OUT + (v >> 6) * (CH * 128) + (v & 7) * 2;
+    float G[KEYS];
+    // the state gradient as the operand of the next products, then as it stands on entry to the next chunk of the walk (that chunk's exit state's gradient), for memory
+    auto deliver = [&](int n) {
+      write_state_row(operand, G);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars->s_ready);
+      if (n < 0) return;
+      if (SEND) {
+#pragma unroll
+        for (int d = 0; d < KEYS; d += 2) {
+          const uint32_t pair = pack_bf16(G[d], G[d + 1]);
+          *reinterpret_cast<uint16_t*>(gcol + swz(part * KEYS + d, c16)) = static_cast<uint16_t>(pair);
+          *reinterpret_cast<uint16_t*>(gcol + swz(part * KEYS + d + 1, c16)) = static_cast<uint16_t>(pair >> 16);
+        }
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->tile_ready);
+      } else {
+        // [Dk, Dv] with the value index contiguous
+        const long long cell = ((static_cast<long long>(x) * N + n) * HD + part * KEYS) * HD + v;
+        if (dstates != nullptr) {
+#pragma unroll
+          for (int d = 0; d < KEYS; ++d) dstates[cell + d * HD] = G[d];
+        }
+        if (dstates_bf16 != nullptr) {
+#pragma unroll
+          for (int d = 0; d < KEYS; ++d) dstates_bf16[cell + d * HD] = __float2bfloat16(G[d]);
+        }
+      }
+    };
+    read_state(G, d_final, x, v, part);
+    deliver(N - 1);
     bool ok = true;
     for (int it = 0; it < N && ok; ++it) {
       const int n = N - 1 - it;
       const int s = it & 1; const uint32_t ph = (it >> 1) & 1;
       const float* gs = sG + s * CH;
-      const long long cell = ((static_cast<long long>(x) * N + n) * HD + half * HALF) * HD + v;
-      if (dstates != nullptr) {
-        // the gradient of this chunk's exit state, [Dk, Dv] with the value index contiguous
-#pragma unroll
-        for (int d = 0; d < HALF; ++d) dstates[cell + d * HD] = G[d];
-      }
-      if (dstates_bf16 != nullptr) {
-#pragma unroll
-        for (int d = 0; d < HALF; ++d) dstates_bf16[cell + d * HD] = __float2bfloat16(G[d]);
-      }
-      if (!math_wait(&bars->in_full[s], ph, sc, err, ERR_WAIT_FULL)) { ok = false; break; }
+      if (!math_wait(&bars->a_full[s], ph, sc, err, ERR_WAIT_FULL)) { ok = false; break; }
       const float gl = gs[CH - 1];
-      w[lane] = __expf(gl - gs[j0 + lane]);
+      if (lane < TOKENS) w[lane] = __expf(gl - gs[j0 + lane]);
       __syncwarp();
+      if (lane == 0) mbar_arrive(&bars->a_empty[s]);
+      if (SEND && it > 0 && !math_wait(&bars->vn_sent, (it - 1) & 1, sc, err, ERR_WAIT_OTHER)) { ok = false; break; }
       if (!math_wait(&bars->acc_full, it & 1, sc, err, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
-      uint4 packed[4];                                   // -dVn
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        uint32_t a[16], bb[16];
-        tmem_ld_32x32b_x16(tmem + lane_addr + TM_A + s * 64 + j0 + q * 16, a);
-        tmem_ld_32x32b_x16(tmem + lane_addr + TM_B + j0 + q * 16, bb);
+      {
+        uint32_t a[TOKENS], bb[TOKENS];
+        tmem_ld_32x32b_x16(tmem + lane_addr + TM_A + s * 64 + j0, a);
+        tmem_ld_32x32b_x16(tmem + lane_addr + TM_B + j0, bb);
         tmem_ld_wait();
 #pragma unroll
-        for (int j8 = 0; j8 < 2; ++j8) {
+        for (int j8 = 0; j8 < TOKENS / 8; ++j8) {
           float nv[8];
 #pragma unroll
-          for (int jj = 0; jj < 8; ++jj) nv[jj] = -(__uint_as_float(a[j8 * 8 + jj]) + w[q * 16 + j8 * 8 + jj] * __uint_as_float(bb[j8 * 8 + jj]));
-          packed[q * 2 + j8] = pack8(nv);
-          *reinterpret_cast<uint4*>(sDvn + swz(v, half * 4 + q * 2 + j8)) = packed[q * 2 + j8];
+          for (int jj = 0; jj < 8; ++jj) nv[jj] = -(__uint_as_float(a[j8 * 8 + jj]) + w[j8 * 8 + jj] * __uint_as_float(bb[j8 * 8 + jj]));
+          const uint4 packed = pack8(nv);                // -dVn
+          *reinterpret_cast<uint4*>(sDvn + swz(v, part * (TOKENS / 8) + j8)) = packed;
+          if (SEND) {
+            const uint32_t pairs[4] = {packed.x ^ 0x80008000u, packed.y ^ 0x80008000u, packed.z ^ 0x80008000u, packed.w ^ 0x80008000u};      // the sign of both
+#pragma unroll
+            for (int j2 = 0; j2 < 4; ++j2) {
+              *reinterpret_cast<uint16_t*>(ncol + swz(j0 + j8 * 8 + 2 * j2, c16)) = static_cast<uint16_t>(pairs[j2]);
+              *reinterpret_cast<uint16_t*>(ncol + swz(j0 + j8 * 8 + 2 * j2 + 1, c16)) = static_cast<uint16_t>(pairs[j2] >> 16);
+            }
+          } else if (dvn_out != nullptr) {
+            __nv_bfloat16* dst = dvn_out + (static_cast<long long>(x) * Tp + n * CH + j0 + j8 * 8) * HD + v;
+#pragma unroll
+            for (int jj = 0; jj < 8; ++jj) dst[jj * HD] = __float2bfloat16(-nv[jj]);
+          }
         }
       }
       fence_proxy_async();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars->vn_ready);
-      if (dvn_out != nullptr) {
-        uint16_t* dst = reinterpret_cast<uint16_t*>(dvn_out) + (static_cast<long long>(x) * Tp + n * CH + j0) * HD + v;
-#pragma unroll
-        for (int j2 = 0; j2 < 16; ++j2) {
-          const uint4 p = packed[j2 >> 2];
-          const uint32_t pair = ((j2 & 3) == 0 ? p.x : (j2 & 3) == 1 ? p.y : (j2 & 3) == 2 ? p.z : p.w) ^ 0x80008000u;      // the sign of both
-          dst[2 * j2 * HD] = static_cast<uint16_t>(pair);
-          dst[(2 * j2 + 1) * HD] = static_cast<uint16_t>(pair >> 16);
-        }
-      }
+      if (SEND && !math_wait(&bars->state_sent, it & 1, sc, err, ERR_WAIT_OTHER)) { ok = false; break; }
       if (!math_wait(&bars->ds_full, it & 1, sc, err, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       const float dl = __expf(gl);
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        uint32_t d[32];
-        tmem_ld_32x32b_x32(tmem + lane_addr + TM_DD + s * 128 + half * HALF + q * 32, d);
+      {
+        uint32_t d[KEYS];
+        tmem_ld_32x32b_x32(tmem + lane_addr + TM_DD + s * 128 + part * KEYS, d);
         tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 32; ++i) G[q * 32 + i] = fmaf(G[q * 32 + i], dl, __uint_as_float(d[i]));
+        for (int i = 0; i < KEYS; ++i) G[i] = fmaf(G[i], dl, __uint_as_float(d[i]));
       }
-      write_state_row(sState, v, half, G);
-      fence_proxy_async();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) { mbar_arrive(&bars->s_ready); mbar_arrive(&bars->in_empty[s]); }
+      deliver(n - 1);
     }
     if (ok && d_initial != nullptr) {
-      float* dst = d_initial + (static_cast<long long>(x) * HD + half * HALF) * HD + v;
+      float* dst = d_initial + (static_cast<long long>(x) * HD + part * KEYS) * HD + v;
 #pragma unroll
-      for (int d = 0; d < HALF; ++d) dst[d * HD] = G[d];
+      for (int d = 0; d < KEYS; ++d) dst[d * HD] = G[d];
     }
   }
-  scan_epilogue(sc, MMA_WARP);
+  scan_epilogue(sc, F::MMA_WARP);
 }
 
 // A [B, T, H, 128] bf16 tensor with element strides (sb, st, sh), tiled [rows x 64 columns].
@@ -815,11 +971,19 @@ extern "C" int dewb_gdn_scan_fwd(const void* q, const void* k, const float* gc, 
   if ((r = dewb::make_tmap_2d(&tw, W, rows, HD, HD, CH, 64, 2, true))) return 3000 + r;
   if ((r = dewb::make_tmap_2d(&tu, U, rows, HD, HD, CH, 64, 2, true))) return 4000 + r;
   if ((r = dewb::make_tmap_2d(&tp, P, rows, CH, CH, CH, 64, 2, true))) return 5000 + r;
-  cudaError_t e = cudaFuncSetAttribute(gdn_scan_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM);
+  // What the backward reads and nothing else, or any other selection, by the threads that hold it.
+  const bool send = out == nullptr && states != nullptr && vn_out != nullptr;
+  CUtensorMap ts = tu, tv = tu;                                            // (not read where nothing is sent)
+  if (send) {
+    if ((r = dewb::make_tmap_2d(&ts, states, static_cast<uint64_t>(B) * H * N * HD, HD, HD, HD, 64, 2, true))) return 6000 + r;
+    if ((r = dewb::make_tmap_2d(&tv, vn_out, rows, HD, HD, CH, 64, 2, true))) return 7000 + r;
+  }
+  auto fn = send ? gdn_scan_fwd_kernel<false> : gdn_scan_fwd_kernel<true>;
+  const int smem = send ? Fwd<false>::SMEM : Fwd<true>::SMEM, threads = send ? Fwd<false>::THREADS : Fwd<true>::THREADS;
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return static_cast<int>(e);
-  gdn_scan_fwd_kernel<<<B * H, FWD_THREADS, SCAN_SMEM, reinterpret_cast<cudaStream_t>(stream_ptr)>>>(
-      tq, tk, tw, tu, tp, gc, initial, reinterpret_cast<__nv_bfloat16*>(out), final_state,
-      reinterpret_cast<__nv_bfloat16*>(states), reinterpret_cast<__nv_bfloat16*>(vn_out), T, H, rep, Tp, N, scale, err);
+  fn<<<B * H, threads, smem, reinterpret_cast<cudaStream_t>(stream_ptr)>>>(tq, tk, tw, tu, tp, ts, tv, gc, initial, reinterpret_cast<__nv_bfloat16*>(out), final_state,
+                                                                           reinterpret_cast<__nv_bfloat16*>(states), reinterpret_cast<__nv_bfloat16*>(vn_out), T, H, rep, Tp, N, scale, err);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -843,10 +1007,18 @@ extern "C" int dewb_gdn_scan_bwd(const void* d_out, const void* k, const float* 
   if ((r = dewb::make_tmap_2d(&tw, W, rows, HD, HD, CH, 64, 2, true))) return 3000 + r;
   if ((r = dewb::make_tmap_2d(&tqg, Qg, rows, HD, HD, CH, 64, 2, true))) return 4000 + r;
   if ((r = dewb::make_tmap_2d(&tp, P, rows, CH, CH, CH, 64, 2, true))) return 5000 + r;
-  cudaError_t e = cudaFuncSetAttribute(gdn_scan_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM);
+  // What the local kernels read and nothing else, or any other selection, by the threads that hold it.
+  const bool send = dstates == nullptr && dstates_bf16 != nullptr && dvn_out != nullptr;
+  CUtensorMap ts = tw, tv = tw;                                            // (not read where nothing is sent)
+  if (send) {
+    if ((r = dewb::make_tmap_2d(&ts, dstates_bf16, static_cast<uint64_t>(B) * H * N * HD, HD, HD, HD, 64, 2, true))) return 6000 + r;
+    if ((r = dewb::make_tmap_2d(&tv, dvn_out, rows, HD, HD, CH, 64, 2, true))) return 7000 + r;
+  }
+  auto fn = send ? gdn_scan_bwd_kernel<true> : gdn_scan_bwd_kernel<false>;
+  const int smem = send ? Bwd<true>::SMEM : Bwd<false>::SMEM;
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return static_cast<int>(e);
-  gdn_scan_bwd_kernel<<<B * H, BWD_THREADS, SCAN_SMEM, reinterpret_cast<cudaStream_t>(stream_ptr)>>>(
-      tdo, tk, tw, tqg, tp, gc, d_final, dstates, reinterpret_cast<__nv_bfloat16*>(dstates_bf16),
-      reinterpret_cast<__nv_bfloat16*>(dvn_out), d_initial, T, H, rep, Tp, N, err);
+  fn<<<B * H, Bwd<true>::THREADS, smem, reinterpret_cast<cudaStream_t>(stream_ptr)>>>(tdo, tk, tw, tqg, tp, ts, tv, gc, d_final, dstates, reinterpret_cast<__nv_bfloat16*>(dstates_bf16),
+                                                                                      reinterpret_cast<__nv_bfloat16*>(dvn_out), d_initial, T, H, rep, Tp, N, err);
   return static_cast<int>(cudaGetLastError());
 }

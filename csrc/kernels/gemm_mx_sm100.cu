@@ -40,6 +40,7 @@ constexpr int ACC_COLS = BN;
 constexpr int SF_BASE = 2 * ACC_COLS;   // 384
 constexpr int SF_SLOT = 16;             // columns per stage: A at +0 (4 columns), B at +4 (6 columns)
 constexpr int TMEM_COLS = 512;
+constexpr int AHEAD = 4;                // stages whose scales a stager has on their way
 constexpr int THREADS = 320;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
 
@@ -173,23 +174,26 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      int stage = 0; uint32_t phase = 0;
-      int acc = 0; uint32_t acc_phase = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        int m0, n0, b_row0;
-        if (!tile_of(t, m0, n0, b_row0)) continue;
-        if (!mbar_wait(&sh->tmem_empty[acc], acc_phase ^ 1, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_TMEM_EMPTY); ok = false; break; }
+    // The whole warp runs this loop and waits together; one elected lane issues (see mbar_wait_warp).
+    int stage = 0; uint32_t phase = 0;
+    int acc = 0; uint32_t acc_phase = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      int m0, n0, b_row0;
+      if (!tile_of(t, m0, n0, b_row0)) continue;
+      if (!mbar_wait_warp(&sh->tmem_empty[acc], acc_phase ^ 1, abort_flag)) { if (lane == 0) atomicCAS(err, 0, ERR_WAIT_TMEM_EMPTY); break; }
+      const uint32_t d_tmem = tmem_base + acc * ACC_COLS;
+      for (int k = 0; k < k_iters; ++k) {
+        // two lanes wait at the same time: for the stage's operands and for its scales
+        bool got = true;
+        if (lane == 0) got = mbar_wait(&sh->full[stage], phase, abort_flag);
+        else if (lane == 1) got = mbar_wait(&sh->sf_full[stage], phase, abort_flag);
+        if (!__all_sync(0xffffffffu, got)) { if (lane == 0) atomicCAS(err, 0, ERR_WAIT_FULL); ok = false; break; }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * ACC_COLS;
-        for (int k = 0; k < k_iters; ++k) {
-          if (!mbar_wait(&sh->full[stage], phase, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_FULL); ok = false; break; }
-          if (!mbar_wait(&sh->sf_full[stage], phase, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_FULL); ok = false; break; }
-          tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * STAGE_BYTES);
-          const uint32_t sb = sa + A_BYTES;
-          const uint32_t sfa = tmem_base + SF_BASE + stage * SF_SLOT, sfb = sfa + 4;
+        const uint32_t sa = smem_u32(smem + stage * STAGE_BYTES);
+        const uint32_t sb = sa + A_BYTES;
+        const uint32_t sfa = tmem_base + SF_BASE + stage * SF_SLOT, sfb = sfa + 4;
+        if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) {          // 32 fp8 elements = 32 bytes per product
             const uint64_t da = make_sdesc_sw128(sa + kk * 32, 16, 1024);
@@ -197,12 +201,12 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
             umma_mxf8_ss(d_tmem, da, db, make_idesc_mx(BM, BN, kk), sfa, sfb, (k > 0 || kk > 0) ? 1u : 0u);
           }
           umma_commit(&sh->empty[stage]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+          if (k == k_iters - 1) umma_commit(&sh->tmem_full[acc]);
         }
-        if (!ok) break;
-        umma_commit(&sh->tmem_full[acc]);
-        if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
+      if (++acc == 2) { acc = 0; acc_phase ^= 1; }
     }
   } else if (warp < 6) {
     // ------------------------------------------------------------------ epilogue (warps 2..5)
@@ -250,29 +254,56 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
     // ------------------------------------------------------------------ scale stagers (warps 6..9): warp w fills lane quarter w & 3
     const int q = warp & 3;
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
+    // The words of the next AHEAD stages are on their way while one is staged: a stage's products take 400 cycles, and loads that were waited for one stage after another
+    // took longer than that (the four products of a 64-expert layer's step, 8192 tokens, 2048 x 1408, top 6: 1375 us, with the issue out of one lane of a divergent warp; 1124 now).
+    int t = blockIdx.x, k = 0;                       // the next stage to load
+    const uint32_t *pa = nullptr, *pb = nullptr;
+    auto begin_tile = [&]() -> bool {
+      for (; t < num_tiles; t += gridDim.x) {
+        int m0, n0, b_row0;
+        if (!tile_of(t, m0, n0, b_row0)) continue;
+        pa = ga.sfa + m0 + lane;
+        pb = ga.sfb + b_row0 + n0 + lane;
+        k = 0;
+        return true;
+      }
+      return false;
+    };
+    bool more = begin_tile() && k_iters > 0;
+    uint32_t words[AHEAD][10];
+    bool loaded[AHEAD];
+    auto load = [&](uint32_t (&w)[10]) -> bool {
+      if (!more) return false;
+      const uint32_t *a = pa + static_cast<long long>(k) * ga.sfa_rows, *b = pb + static_cast<long long>(k) * ga.sfb_rows;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) w[i] = __ldg(a + i * 32);
+#pragma unroll
+      for (int i = 0; i < 6; ++i) w[4 + i] = __ldg(b + i * 32);
+      if (++k == k_iters) { t += gridDim.x; more = begin_tile(); }
+      return true;
+    };
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) loaded[u] = load(words[u]);
     int stage = 0; uint32_t phase = 0;
     bool ok = true;
-    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-      int m0, n0, b_row0;
-      if (!tile_of(t, m0, n0, b_row0)) continue;
-      for (int k = 0; k < k_iters; ++k) {
+    while (ok && loaded[0]) {
+#pragma unroll
+      for (int u = 0; u < AHEAD; ++u) {
+        if (!ok || !loaded[u]) { ok = false; continue; }
         // the slot is free once the products of its previous use have completed (the same event that frees the operands)
         const bool got = mbar_wait(&sh->empty[stage], phase ^ 1, abort_flag);
-        if (!__all_sync(0xffffffffu, got)) { atomicCAS(err, 0, ERR_WAIT_EMPTY); ok = false; break; }
+        if (!__all_sync(0xffffffffu, got)) { atomicCAS(err, 0, ERR_WAIT_EMPTY); ok = false; continue; }
         tc_fence_after();
-        const uint32_t* pa = ga.sfa + static_cast<long long>(k) * ga.sfa_rows + m0 + lane;
-        const uint32_t* pb = ga.sfb + static_cast<long long>(k) * ga.sfb_rows + b_row0 + n0 + lane;
-        const uint32_t a0 = pa[0], a1 = pa[32], a2 = pa[64], a3 = pa[96];
-        const uint32_t b0 = pb[0], b1 = pb[32], b2 = pb[64], b3 = pb[96], b4 = pb[128], b5 = pb[160];
         const uint32_t base = tmem_base + lane_addr + SF_BASE + stage * SF_SLOT;
-        tmem_st_32x32b_x4(base, a0, a1, a2, a3);
-        tmem_st_32x32b_x4(base + 4, b0, b1, b2, b3);
-        tmem_st_32x32b_x2(base + 8, b4, b5);
+        tmem_st_32x32b_x4(base, words[u][0], words[u][1], words[u][2], words[u][3]);
+        tmem_st_32x32b_x4(base + 4, words[u][4], words[u][5], words[u][6], words[u][7]);
+        tmem_st_32x32b_x2(base + 8, words[u][8], words[u][9]);
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh->sf_full[stage]);
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        loaded[u] = load(words[u]);
       }
     }
   }

@@ -48,3 +48,19 @@ def test_zero_pads_touches_the_pads_alone():
     for o, c, e in zip(offsets, counts, offsets[1:]):
         live[o + c:e] = False
     assert torch.equal((rows != 0).all(1).cpu(), live) and torch.equal((rows == 0).all(1).cpu(), ~live)
+
+
+# reductions of one stage, of as many as the scales are fetched ahead, of one more, and past the ring; tiles with rows and columns to spare, more tiles than CTAs
+@pytest.mark.parametrize("M,N,K", [(1, 192, 128), (130, 200, 512), (128, 384, 640), (300, 64, 768), (2048, 2112, 896)])
+def test_block_scaled_product_by_stages(M, N, K):
+    """Against the same numbers in 64 bits: fp32 sums rounded to bf16 once."""
+    from dew_b200.ops import mx
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    a, b = (torch.randn(n, K, generator=g, device="cuda").mul(torch.rand(n, 1, generator=g, device="cuda") * 4).bfloat16() for n in (M, N))
+    aq, sa = mx.quantize_mx(a, sf_rows=-(-M // 128) * 128)
+    bq, sb = mx.quantize_mx(b, sf_rows=N + mx.TILE_N)
+    out = mx.gemm_mx(aq, sa, bq, sb)
+    L.check_status()
+    full = [mx.dequantize_mx(q, mx.unpack_scales(s, q.shape[0], K)).double() for q, s in ((aq, sa), (bq, sb))]
+    want = full[0] @ full[1].t()
+    assert float((out.double() - want).norm() / want.norm()) < 2.0 ** -8

@@ -787,6 +787,18 @@ def linear_cross_entropy_reference(h, weight, targets, ignore_index=-100, z_loss
     return loss.sum(), live.sum()
 
 
+def _scaled(x, scale, dtype):
+    """``(x * scale).to(dtype)``, in one pass where a bf16 result of fp32 values leaves no graph behind."""
+    if not (dtype == torch.bfloat16 and x.is_cuda and scale.dtype == torch.float32 and scale.numel() == 1 and scale.device == x.device and x.is_contiguous()
+            and x.data_ptr() % 16 == 0 and L.unrecorded(x, scale)):
+        return (x * scale).to(dtype)
+    out = torch.empty_like(x, dtype=dtype)
+    L.ensure_device(x)
+    L.check(L.load().dewb_scale_cast(L.ptr(x), L.ptr(scale), L.ptr(out), c_ll(x.numel()), L.stream_ptr()), "scale_cast")
+    L.count_launches()
+    return out
+
+
 class _LinearCE(torch.autograd.Function):
     """Token-chunked head: per chunk, logits = h W^T (tcgen05 GEMM), a row kernel reduces the loss and overwrites
     the logits with their gradient, and two more GEMMs produce dH and accumulate dW - all inside forward, so the
@@ -803,7 +815,7 @@ class _LinearCE(torch.autograd.Function):
         main = getattr(weight, "main_grad", None)
         dw = None
         if need_grad and weight.requires_grad and main is None:
-            dw = torch.zeros((V, d), dtype=torch.float32, device=h.device)
+            dw = (torch.empty if T else torch.zeros)((V, d), dtype=torch.float32, device=h.device)      # (the first chunk's product writes all of it)
         acc = main if main is not None else dw
         losses = torch.empty(T, dtype=torch.float32, device=h.device)
         tg = targets.to(torch.int64).contiguous()
@@ -822,7 +834,7 @@ class _LinearCE(torch.autograd.Function):
                 gemm(lg, weight, b_mn=True, out=dh[s:e])                       # dH = dlogits @ W
                 if acc is not None:
                     gemm(lg, h[s:e], a_mn=True, b_mn=True, out=acc,
-                         accumulate=grad_accumulates(weight) if main is not None else True)    # dW += dlogits^T @ h
+                         accumulate=grad_accumulates(weight) if main is not None else s > 0)    # dW += dlogits^T @ h
         ctx.save_for_backward(dh, dw)
         ctx.used_main = main is not None
         ctx.w_dtype = weight.dtype
@@ -835,7 +847,7 @@ class _LinearCE(torch.autograd.Function):
         gh = (dh * gloss.to(dh.dtype)) if dh is not None else None
         gw = None
         if dw is not None:
-            gw = (dw * gloss).to(ctx.w_dtype)
+            gw = _scaled(dw, gloss, ctx.w_dtype)
         return gh, gw, None, None, None, None, None
 
 

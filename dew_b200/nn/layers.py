@@ -59,7 +59,7 @@ class Embedding(nn.Module):
             self.weight.normal_(0.0, self.init_std, generator=generator)
 
     def forward(self, ids):
-        return F.embedding(ids, self.weight)
+        return ops.embedding(ids, self.weight)
 
 
 class RMSNorm(nn.Module):

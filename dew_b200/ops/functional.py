@@ -365,6 +365,41 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     return _Linear.apply(x, weight, bias)
 
 
+class _Embedding(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, ids, weight):
+        ctx.save_for_backward(ids)
+        ctx.rows = weight.shape[0]
+        return F.embedding(ids, weight)
+
+    @staticmethod
+    def backward(ctx, dy):
+        ids, = ctx.saved_tensors
+        T, d = ids.numel(), dy.shape[-1]
+        if T > L.load().dewb_embed_grad_most() or not L.unrecorded(dy):      # (what is differentiated again keeps its graph)
+            return None, torch.ops.aten.embedding_dense_backward(dy, ids, ctx.rows, -1, False)
+        dy, ids = dy.contiguous(), ids.contiguous()
+        if dy.data_ptr() % 16:
+            dy = dy.clone()
+        dw = torch.empty(ctx.rows, d, dtype=torch.bfloat16, device=dy.device)
+        scratch = torch.empty(3 * T, dtype=torch.int32, device=dy.device)
+        L.ensure_device(dy)
+        L.check(L.load().dewb_embed_grad(L.ptr(dy), L.ptr(ids), L.ptr(dw), L.ptr(scratch), c_int(T), c_int(d), c_ll(ctx.rows), L.stream_ptr()), "embed_grad")
+        L.count_launches(3)
+        return None, dw
+
+
+def embedding(ids: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    """Rows of ``weight`` by ``ids``; a bf16 table's gradient comes from the kernels where plain autograd records the lookup of up to 16384 tokens, and there is enough to
+    sum: below two million values the library's backward takes less time to issue than this one's node and launches (2048 tokens of 128 features: 60 us against 140, with
+    some 60 us of work either way)."""
+    if (ids.numel() * weight.shape[-1] >= 1 << 21 and weight.is_cuda and weight.requires_grad and weight.dtype == torch.bfloat16 and weight.dim() == 2 and weight.shape[1] % 8 == 0 and weight.shape[1] > 0
+            and ids.dtype == torch.int64 and ids.device == weight.device and type(weight) in (torch.Tensor, torch.nn.Parameter) and torch.is_grad_enabled()
+            and L.plain_autograd() and L.use_cuda(weight) and hasattr(L.load(), "dewb_embed_grad")):
+        return _Embedding.apply(ids, weight)
+    return F.embedding(ids, weight)
+
+
 # ---------------------------------------------------------------------------------------------------------------
 # RMSNorm family
 

@@ -123,7 +123,12 @@ def unrecorded(*tensors: Optional[torch.Tensor]) -> bool:
         for t in tensors:
             if t is not None and t.requires_grad:
                 return False
-    return (torch.autograd.forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active() and torch._C._get_tracing_state() is None)
+    return plain_autograd()
+
+
+def plain_autograd() -> bool:
+    """Neither forward-mode differentiation, nor a functorch transform, nor a trace is under way."""
+    return torch.autograd.forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active() and torch._C._get_tracing_state() is None
 
 
 _TLS = threading.local()

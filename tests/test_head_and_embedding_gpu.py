@@ -10,6 +10,47 @@ pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not torch.cuda.is_available(),
 DEV = "cuda"
 
 
+def embedding_gradient(dy, ids, V):
+    dw = torch.empty(V, dy.shape[1], dtype=torch.bfloat16, device=DEV)
+    scratch = torch.empty(3 * ids.numel(), dtype=torch.int32, device=DEV)
+    L.ensure_device(dy)
+    L.check(L.load().dewb_embed_grad(L.ptr(dy), L.ptr(ids), L.ptr(dw), L.ptr(scratch), functional.c_int(ids.numel()), functional.c_int(dy.shape[1]), functional.c_ll(V),
+                                     L.stream_ptr()), "embed_grad")
+    return dw
+
+
+# slices of the count of one token to sixteen; runs of one token, of a handful, of all; widths of one piece, past a block's columns, of both
+@pytest.mark.parametrize("T,V,d", [(1, 1, 8), (3, 2, 1032), (255, 300, 64), (1024, 1, 128), (1025, 7, 8), (4096, 50000, 256), (16384, 256, 16), (0, 5, 8)])
+def test_embedding_gradient(T, V, d):
+    """The tokens' rows are summed in fp32 in their order and rounded to bf16 once."""
+    g = torch.Generator(device=DEV).manual_seed(T)
+    ids, dy = torch.randint(0, V, (T,), generator=g, device=DEV), torch.randn(T, d, generator=g, device=DEV).bfloat16()
+    got = embedding_gradient(dy, ids, V)
+    want = torch.zeros(V, d, dtype=torch.float64, device=DEV).index_add_(0, ids, dy.double())
+    size = torch.zeros(V, d, dtype=torch.float64, device=DEV).index_add_(0, ids, dy.double().abs())
+    assert bool(((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + T * 2.0 ** -24 * size).all())
+    assert torch.equal(got, embedding_gradient(dy, ids, V))
+
+
+def test_embedding_lookup_keeps_its_gradients():
+    """Through the lookup itself: by size to either backward, under second derivatives, and for tables that the kernels do not take."""
+    g = torch.Generator(device=DEV).manual_seed(0)
+    ids = torch.randint(0, 100, (4, 1024), generator=g, device=DEV)
+    for width, dtype in ((512, torch.bfloat16), (64, torch.bfloat16), (513, torch.bfloat16), (512, torch.float32)):
+        table = torch.randn(100, width, generator=g, device=DEV).to(dtype).requires_grad_()
+        up = torch.randn(4, 1024, width, generator=g, device=DEV).to(dtype)
+        out = ops.embedding(ids, table)
+        assert torch.equal(out, table.detach()[ids])
+        want = torch.zeros(100, width, dtype=torch.float64, device=DEV).index_add_(0, ids.reshape(-1), up.double().reshape(-1, width))
+        got, = torch.autograd.grad(out, table, up)
+        assert got.dtype == dtype and float((got.double() - want).norm() / want.norm()) < 2.0 ** -8
+    table = torch.randn(100, 512, generator=g, device=DEV).bfloat16().requires_grad_()
+    up = torch.randn(4, 1024, 512, generator=g, device=DEV).bfloat16().requires_grad_()
+    first, = torch.autograd.grad(ops.embedding(ids, table), table, up, create_graph=True)
+    second, = torch.autograd.grad(first.float().square().sum(), up)
+    assert second.shape == up.shape and float(second.abs().sum()) > 0
+
+
 @pytest.mark.parametrize("n", [1, 7, 8, 9, 8 * 256 + 5, 1 << 20])
 def test_scaled_cast(n):
     """The bits of the product and the conversion one after the other."""

@@ -791,6 +791,11 @@ class CausalTransformer(nn.Module):
         if self.engrams is not None and (cache is not None or tokens is None or getattr(self, "tp", None) is not None):
             raise NotImplementedError("n-gram memories read the token ids behind each position: they run on whole sequences given as tokens, without "
                                       "a KV cache and without tensor parallelism")
+        if cache is not None and self.engrams is None and segment_ids is None and h.shape[1] == 1:
+            from . import decode_step
+            done = decode_step.run(self, h, cos, sin, positions, cache)
+            if done is not None:
+                return self._finish(*done)
         for layer in self.layers:
             if self.engrams is not None and str(layer.index) in self.engrams:
                 h = h if branch is None else h + branch               # the memory's gate reads the stream as the layer will see it

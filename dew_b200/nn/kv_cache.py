@@ -443,6 +443,17 @@ class KVStore:
 
     MIN_TILES = 4            # fewest 64-key tiles one CTA of the balanced decode kernel takes (bounds the parts a row is cut into)
 
+    def _row_arrivals(self, n: int, device) -> torch.Tensor:
+        """Zeros that the decode kernel counts up and leaves at zero again."""
+        if getattr(self, "_arrivals", None) is None or self._arrivals.numel() < n:
+            self._arrivals = torch.zeros(n, dtype=torch.int32, device=device)
+        return self._arrivals
+
+    def _decode_ctas(self, device) -> int:
+        if getattr(self, "_ctas", None) is None:
+            self._ctas = 2 * torch.cuda.get_device_properties(device).multi_processor_count
+        return self._ctas
+
     def _fused_decode(self, lib, layer: int, q, q_row_stride: int, lens32, R: int, Hq: int, D: int, window, sinks32, out,
                       scale: Optional[float] = None, kv_heads: Optional[int] = None, table: Optional[torch.Tensor] = None,
                       visible: P.Visible = P.PLAIN) -> None:
@@ -462,20 +473,17 @@ class KVStore:
         scale = 1.0 / math.sqrt(D) if scale is None else scale
         kv_heads = self.kv_heads if kv_heads is None else kv_heads
         pm, pl, pa = self._partials(n, D, q.device)
-        if getattr(self, "_arrivals", None) is None or self._arrivals.numel() < R * kv_heads:
-            self._arrivals = torch.zeros(R * kv_heads, dtype=torch.int32, device=q.device)
+        arrivals = self._row_arrivals(R * kv_heads, q.device)
         at = lambda t: 0 if t is None else t.data_ptr()
         if persist:
-            if getattr(self, "_ctas", None) is None:
-                self._ctas = 2 * torch.cuda.get_device_properties(q.device).multi_processor_count
             L.check(lib.dewb_paged_decode_persist(at(q), at(self.k[layer]), at(self.v[layer]), self.pages * self.page_size, at(self.page_table if table is None else table),
-                                                  at(lens32), at(pm), at(pl), at(pa), at(self._arrivals), at(sinks32), at(out), R, Hq, kv_heads, self.page_size,
+                                                  at(lens32), at(pm), at(pl), at(pa), at(arrivals), at(sinks32), at(out), R, Hq, kv_heads, self.page_size,
                                                   self.max_pages, splits, min_tiles, scale, window or 0, visible.keep, visible.chunk or 0, visible.softcap,
-                                                  at(visible.gain), at(visible.sigmoid), q_row_stride, self._ctas, at(L.status(q.device)), L.stream()),
+                                                  at(visible.gain), at(visible.sigmoid), q_row_stride, self._decode_ctas(q.device), at(L.status(q.device)), L.stream()),
                     "paged_decode_persist")
         else:
             common = (L.ptr(q), L.ptr(self.k[layer]), L.ptr(self.v[layer]), ctypes.c_longlong(self.pages * self.page_size),
-                      L.ptr(self.page_table if table is None else table), L.ptr(lens32), L.ptr(pm), L.ptr(pl), L.ptr(pa), L.ptr(self._arrivals), L.ptr(sinks32),
+                      L.ptr(self.page_table if table is None else table), L.ptr(lens32), L.ptr(pm), L.ptr(pl), L.ptr(pa), L.ptr(arrivals), L.ptr(sinks32),
                       L.ptr(out), ctypes.c_int(R), ctypes.c_int(Hq), ctypes.c_int(kv_heads), ctypes.c_int(self.page_size),
                       ctypes.c_int(self.max_pages), ctypes.c_int(splits))
             L.check(lib.dewb_paged_decode_fused(*common, ctypes.c_int(share), ctypes.c_float(scale),

@@ -95,6 +95,17 @@ def _few_rows(M: int, N: int, K: int) -> bool:
     return N <= (12288 if pair else 4096) and N * K <= (6 << 20 if pair else 2 << 20) and (K >= 256 or N <= (4096 if pair else 2048))
 
 
+def few_row_products_declared() -> bool:
+    """Whether products of few rows that ``_few_rows`` takes go to its kernel, whatever the environment says of others."""
+    return (_GEMM.declared.get(("rows",)) == "sm100_rows" and _GEMM.declared.get(("decode",)) != "sm100_skinny" and not _GEMM.forced_by_environment()
+            and hasattr(L.load(), "dewb_gemm_rows_bf16"))
+
+
+def count_few_row_products(n: int) -> None:
+    """Enters ``n`` products that a larger call has made into the routes."""
+    _GEMM._record("sm100_rows", {}, None, ("rows",), n)
+
+
 def _skinny_built() -> bool:
     try:
         return hasattr(L.load(), "dewb_gemm_skinny_bf16")

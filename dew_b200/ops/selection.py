@@ -78,12 +78,12 @@ class Op:
     def explain(self, case: Dict[str, Any]) -> Dict[str, List[str]]:
         return {k.name: k.refusals(case) for k in self.kernels}
 
-    def _record(self, chosen: str, refused: Dict[str, List[str]], forced: Optional[str], cell: Optional[Tuple]) -> None:
+    def _record(self, chosen: str, refused: Dict[str, List[str]], forced: Optional[str], cell: Optional[Tuple], calls: int = 1) -> None:
         """Route bookkeeping: how often each kernel took a call and, when an earlier kernel in the order refused, why."""
         row = self.routes.setdefault(chosen, {"calls": 0, "forced": 0, "declared_cell": 0, "after_refusals": {}})
-        row["calls"] += 1
-        row["forced"] += 1 if forced else 0
-        row["declared_cell"] += 1 if (cell is not None and cell in self.declared) else 0
+        row["calls"] += calls
+        row["forced"] += calls if forced else 0
+        row["declared_cell"] += calls if (cell is not None and cell in self.declared) else 0
         for name, why in refused.items():
             for w in why:
                 key = f"{name}: {w.split(':')[0]}"

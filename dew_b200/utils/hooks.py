@@ -29,8 +29,18 @@ def _watched(module) -> bool:
     return False
 
 
+def nobody_watches_all() -> bool:
+    """No hook that all modules have, in either direction."""
+    return not (_all._global_forward_hooks or _all._global_forward_pre_hooks or _all._global_backward_hooks or _all._global_backward_pre_hooks)
+
+
+def runs_alone_by_itself(module) -> bool:
+    """``runs_alone`` but for the hooks of all modules."""
+    own = module.__dict__
+    return not ("forward" in own or own["_forward_hooks"] or own["_forward_pre_hooks"] or own["_backward_hooks"] or own["_backward_pre_hooks"])
+
+
 def runs_alone(module) -> bool:
     """Whether calling ``module`` is running its class's ``forward`` and nothing else: no hook of its own or of all modules, in either direction, and no ``forward``
     set on the instance."""
-    return not ("forward" in module.__dict__ or module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks
-                or _all._global_forward_hooks or _all._global_forward_pre_hooks or _all._global_backward_hooks or _all._global_backward_pre_hooks)
+    return runs_alone_by_itself(module) and nobody_watches_all()

@@ -659,7 +659,7 @@ __global__ void swiglu_bwd_kernel(const bf16* __restrict__ dy, const bf16* __res
 // RoPE (rotate-half convention) applied in place to the first `rot_heads` heads of a packed
 // [tokens, heads, D] tensor; positions[t] indexes cos/sin [table_rows, D/2] (fp32). sign = -1 gives the backward.
 __global__ void rope_kernel(bf16* __restrict__ x, const float* __restrict__ cosb, const float* __restrict__ sinb,
-                            const int* __restrict__ positions, long long tokens, int heads, int rot_heads, int D,
+                            const int* __restrict__ positions, long long tokens, int per_row, int heads, int rot_heads, int D,
                             int table_rows, float sign) {
   const int half = D >> 1;
   const int hv = half >> 3;  // uint4 vectors per half
@@ -670,7 +670,7 @@ __global__ void rope_kernel(bf16* __restrict__ x, const float* __restrict__ cosb
     const long long th = i / hv;
     const int h = static_cast<int>(th % rot_heads);
     const long long t = th / rot_heads;
-    int pos = positions != nullptr ? positions[t] : static_cast<int>(t);
+    int pos = positions != nullptr ? positions[t] : static_cast<int>(per_row > 0 ? t % per_row : t);
     pos = min(max(pos, 0), table_rows - 1);     // a position past the tables reads their last row, never outside them
     bf16* base = x + (t * heads + h) * D;
     uint4* p1 = reinterpret_cast<uint4*>(base) + c;
@@ -1017,7 +1017,17 @@ extern "C" int dewb_rope(void* x, const float* cosb, const float* sinb, const in
   if (D % 16 != 0 || table_rows <= 0) return -3;
   if (tokens <= 0 || rot_heads <= 0) return 0;
   rope_kernel<<<grid_for(tokens * rot_heads * (D >> 4), 256), 256, 0, STREAM(stream)>>>(
-      (bf16*)x, cosb, sinb, positions, tokens, heads, rot_heads, D, table_rows, sign);
+      (bf16*)x, cosb, sinb, positions, tokens, 0, heads, rot_heads, D, table_rows, sign);
+  return LAST_ERR();
+}
+
+// The same for rows of `per_row` tokens, each from position 0 on.
+extern "C" int dewb_rope_rows(void* x, const float* cosb, const float* sinb, long long tokens, int per_row, int heads, int rot_heads, int D, int table_rows, float sign,
+                              void* stream) {
+  if (D % 16 != 0 || table_rows <= 0 || per_row <= 0) return -3;
+  if (tokens <= 0) return 0;
+  rope_kernel<<<grid_for(tokens * rot_heads * (D >> 4), 256), 256, 0, STREAM(stream)>>>(
+      (bf16*)x, cosb, sinb, nullptr, tokens, per_row, heads, rot_heads, D, table_rows, sign);
   return LAST_ERR();
 }
 

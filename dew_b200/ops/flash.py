@@ -12,8 +12,9 @@ c_ll, c_int, c_float = ctypes.c_longlong, ctypes.c_int, ctypes.c_float
 
 def _strides(t):
     """(batch, sequence, head) element strides of a [B, L, H, D] tensor with unit stride along D."""
-    assert t.stride(3) == 1
-    return c_ll(t.stride(0)), c_ll(t.stride(1)), c_ll(t.stride(2))
+    s = t.stride()
+    assert s[3] == 1
+    return s[:3]
 
 
 class Variants:
@@ -47,11 +48,10 @@ def flash_fwd(q, k, v, causal: bool, scale: float, need_lse: bool = True, var: V
     T, Hkv = k.shape[1], k.shape[2]
     out = torch.empty((B, S, Hq, D), dtype=q.dtype, device=q.device)
     lse = torch.empty((B, Hq, S), dtype=torch.float32, device=q.device) if need_lse else None
-    rc = L.load().dewb_flash_fwd_var(L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(out), L.ptr(lse), c_int(B), c_int(S), c_int(T),
-                                     c_int(Hq), c_int(Hkv), c_int(D), *_strides(q), *_strides(k), *_strides(v),
-                                     *_strides(out), c_float(scale), c_int(int(causal)), c_int(var.window), c_int(var.keep), c_int(var.chunk), c_float(var.softcap),
-                                     L.ptr(var.sinks), L.ptr(var.segments), L.ptr(var.segments), L.ptr(var.gain), L.ptr(var.sigmoid), L.ptr(L.status(q.device)),
-                                     L.stream_ptr())
+    at = L.at
+    rc = L.load().dewb_flash_fwd_var(at(q), at(k), at(v), at(out), at(lse), B, S, T, Hq, Hkv, D, *_strides(q), *_strides(k), *_strides(v), *_strides(out), scale, int(causal),
+                                     var.window, var.keep, var.chunk, var.softcap, at(var.sinks), at(var.segments), at(var.segments), at(var.gain), at(var.sigmoid),
+                                     at(L.status(q.device)), L.stream())
     L.check(rc, "flash_fwd")
     L.count_launches()
     return out, lse
@@ -93,15 +93,10 @@ def flash_bwd(do, q, k, v, out, lse, causal: bool, scale: float, grads=None, var
     delta = torch.empty((2, B, Hq, S), dtype=torch.float32, device=q.device)     # delta, then lse in log2 units
     if do.stride(3) != 1 or any(st % 8 for st in do.stride()[:3]):
         do = do.contiguous()
-    st = []
-    for t in (q, k, v, out, do, dq, dk, dv):
-        assert t.stride(3) == 1
-        st += [t.stride(0), t.stride(1), t.stride(2)]
-    strides = (c_ll * 24)(*st)
-    rc = L.load().dewb_flash_bwd_var(L.ptr(do), L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(out), L.ptr(lse), L.ptr(delta), L.ptr(dq),
-                                     L.ptr(dk), L.ptr(dv), c_int(B), c_int(S), c_int(T), c_int(Hq), c_int(Hkv), c_int(D),
-                                     strides, c_float(scale), c_int(int(causal)), c_int(var.window), c_float(var.softcap),
-                                     L.ptr(var.segments), L.ptr(var.segments), L.ptr(L.status(q.device)), L.stream_ptr())
+    strides = (c_ll * 24)(*(s for t in (q, k, v, out, do, dq, dk, dv) for s in _strides(t)))
+    at = L.at
+    rc = L.load().dewb_flash_bwd_var(at(do), at(q), at(k), at(v), at(out), at(lse), at(delta), at(dq), at(dk), at(dv), B, S, T, Hq, Hkv, D, strides, scale, int(causal), var.window,
+                                     var.softcap, at(var.segments), at(var.segments), at(L.status(q.device)), L.stream())
     L.check(rc, "flash_bwd")
     L.count_launches(3)
     if want_delta:
@@ -140,18 +135,25 @@ def flash_sm100(q, k, v, causal: bool, scale: float, window=None, softcap: float
     return flash_fwd(q, k, v, causal, scale, need_lse=False, var=var)[0]
 
 
+def _rotate(x, cos, sin, pos, heads: int, sign: float) -> None:
+    """The first ``heads`` heads of ``x [B, S, H, D]`` in place, at ``pos`` (int32 ``[B S]``) or each row from position 0 on."""
+    B, S, H, D = x.shape
+    lib = L.load()
+    if pos is None:
+        rc = lib.dewb_rope_rows(x.data_ptr(), cos.data_ptr(), sin.data_ptr(), B * S, S, H, heads, D, cos.shape[0], sign, L.stream()) if B * S else 0
+    else:
+        rc = lib.dewb_rope(x.data_ptr(), cos.data_ptr(), sin.data_ptr(), pos.data_ptr(), B * S, H, heads, D, cos.shape[0], sign, L.stream())
+    L.check(rc, "rope")
+    L.count_launches()
+
+
 def _packed(qkv, cos, sin, positions, Hq: int, Hkv: int, causal: bool, scale: float, need_lse: bool):
     """Rotates ``qkv`` in place (not where ``cos`` is None) and attends; -> out, lse, the positions the rotation took."""
-    B, S, H, D = qkv.shape
     pos = None
     if cos is not None:
         if positions is not None:
             pos = positions.reshape(-1).to(torch.int32).contiguous()
-        elif B > 1:
-            pos = torch.arange(S, device=qkv.device, dtype=torch.int32).repeat(B)
-        L.check(L.load().dewb_rope(L.ptr(qkv), L.ptr(cos), L.ptr(sin), L.ptr(pos), c_ll(B * S), c_int(H), c_int(Hq + Hkv),
-                                   c_int(D), c_int(cos.shape[0]), c_float(1.0), L.stream_ptr()), "rope")
-        L.count_launches()      # written through the raw pointer: autograd neither sees nor needs to see the change
+        _rotate(qkv, cos, sin, pos, Hq + Hkv, 1.0)      # written through the raw pointer: autograd neither sees nor needs to see the change
     out, lse = flash_fwd(qkv[:, :, :Hq], qkv[:, :, Hq:Hq + Hkv], qkv[:, :, Hq + Hkv:], causal, scale, need_lse)
     return out, lse, pos
 
@@ -174,14 +176,11 @@ class _PackedRopeFlash(torch.autograd.Function):
     def backward(ctx, do):
         qkv, out, lse, cos, sin, pos = ctx.saved_tensors
         Hq, Hkv, causal, scale = ctx.meta
-        B, S, H, D = qkv.shape
         q, k, v = qkv[:, :, :Hq], qkv[:, :, Hq:Hq + Hkv], qkv[:, :, Hq + Hkv:]
         dqkv = torch.empty_like(qkv)
         flash_bwd(do, q, k, v, out, lse, causal, scale, grads=(dqkv[:, :, :Hq], dqkv[:, :, Hq:Hq + Hkv], dqkv[:, :, Hq + Hkv:]))
         if cos is not None:
-            L.check(L.load().dewb_rope(L.ptr(dqkv), L.ptr(cos), L.ptr(sin), L.ptr(pos), c_ll(B * S), c_int(H), c_int(Hq + Hkv),
-                                       c_int(D), c_int(cos.shape[0]), c_float(-1.0), L.stream_ptr()), "rope_bwd")
-            L.count_launches()
+            _rotate(dqkv, cos, sin, pos, Hq + Hkv, -1.0)
         return dqkv, None, None, None, None, None, None, None
 
 

@@ -506,11 +506,13 @@ class _RMSNorm(torch.autograd.Function):
         dres = dh.reshape(-1, d).contiguous() if (ctx.mode == 1 and dh is not None) else None
         dx = torch.empty_like(xin)
         dz = torch.empty_like(xin) if ctx.mode == 2 else None
-        dw = torch.empty(d, dtype=torch.float32, device=xin.device)
+        # the kernel's sums are rounded as it writes them, where the weights are bf16
+        half = ctx.w_dtype == torch.bfloat16
+        dw = torch.empty(d, dtype=torch.bfloat16 if half else torch.float32, device=xin.device)
         scratch = _bwd_scratch(rows, d, xin.device)
-        L.check(lib.dewb_rmsnorm_bwd(L.ptr(dy2), L.ptr(xin), L.ptr(wb), L.ptr(rstd), L.ptr(dres), L.ptr(z), L.ptr(dx),
-                                     L.ptr(dz), L.ptr(scratch), L.ptr(dw), L.ptr(None), c_int(0), c_ll(rows), c_int(d),
-                                     L.stream_ptr()), "rmsnorm_bwd")
+        at = L.at
+        L.check(lib.dewb_rmsnorm_bwd(at(dy2), at(xin), at(wb), at(rstd), at(dres), at(z), at(dx), at(dz), at(scratch), 0 if half else at(dw), at(dw) if half else 0, 0, rows, d,
+                                     L.stream()), "rmsnorm_bwd")
         L.count_launches(2)
         dxr = dx.reshape(ctx.shape)
         dwr = dw.to(ctx.w_dtype)
@@ -580,9 +582,7 @@ class _PackedSwiGLU(torch.autograd.Function):
         rows = g2.shape[0]
         dy2 = dy.reshape(-1, Fh).contiguous()
         dgu = torch.empty_like(g2)
-        L.check(lib.dewb_swiglu_bwd(L.ptr(dy2), L.ptr(g2), ctypes.c_void_p(g2.data_ptr() + Fh * 2), L.ptr(dgu),
-                                    ctypes.c_void_p(dgu.data_ptr() + Fh * 2), c_ll(rows), c_int(Fh), c_ll(F2),
-                                    L.stream_ptr()), "swiglu_bwd")
+        L.check(lib.dewb_swiglu_bwd(dy2.data_ptr(), g2.data_ptr(), g2.data_ptr() + Fh * 2, dgu.data_ptr(), dgu.data_ptr() + Fh * 2, rows, Fh, F2, L.stream()), "swiglu_bwd")
         L.count_launches()
         return dgu.reshape(ctx.shape)
 
@@ -871,10 +871,8 @@ class _LinearCE(torch.autograd.Function):
             n = e - s
             lg = logits[:n]
             gemm(h[s:e], weight, out=lg)
-            L.check(lib.dewb_ce_rows(L.ptr(lg), ctypes.c_void_p(tg.data_ptr() + s * 8),
-                                     ctypes.c_void_p(losses.data_ptr() + s * 4), L.ptr(None), c_ll(n), c_int(V),
-                                     c_ll(lg.stride(0)), c_int(ignore_index), c_float(1.0), c_float(z_loss),
-                                     c_float(softcap), c_int(int(need_grad)), L.stream_ptr()), "ce_rows")
+            L.check(lib.dewb_ce_rows(lg.data_ptr(), tg.data_ptr() + s * 8, losses.data_ptr() + s * 4, 0, n, V, lg.stride(0), ignore_index, 1.0, z_loss, softcap,
+                                     int(need_grad), L.stream()), "ce_rows")
             L.count_launches()
             if need_grad:
                 gemm(lg, weight, b_mn=True, out=dh[s:e])                       # dH = dlogits @ W

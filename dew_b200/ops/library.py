@@ -62,6 +62,12 @@ _SIGNATURES = {
     "dewb_gemm_rows_bf16": "pppp" + "iii" + "lll" + "p",
     "dewb_swiglu_fwd": "ppp" + "lil" + "p",
     "dewb_rope": "pppp" + "liiiif" + "p",
+    "dewb_rope_rows": "ppp" + "liiiiif" + "p",
+    "dewb_rmsnorm_bwd": "pppppppppppi" + "li" + "p",
+    "dewb_swiglu_bwd": "ppppp" + "lil" + "p",
+    "dewb_ce_rows": "pppp" + "lil" + "ifffi" + "p",
+    "dewb_flash_fwd_var": "ppppp" + "iiiiii" + "l" * 12 + "f" + "iiiif" + "ppppp" + "pp",
+    "dewb_flash_bwd_var": "pppppppppp" + "iiiiii" + "p" + "f" + "ii" + "f" + "pppp",
     "dewb_rope_append": "pppp" + "iiiii" + "ppp" + "ii" + "p",
     "dewb_paged_decode_persist": "ppp" + "l" + "pppppppp" + "iiiiiii" + "f" + "iii" + "f" + "pp" + "l" + "i" + "pp",
 }
@@ -156,6 +162,11 @@ def stream_ptr() -> ctypes.c_void_p:
 
 def ptr(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
     return ctypes.c_void_p(0 if t is None else t.data_ptr())
+
+
+def at(t: Optional[torch.Tensor]) -> int:
+    """A tensor's address for a declared launcher."""
+    return 0 if t is None else t.data_ptr()
 
 
 def status(device: Optional[torch.device] = None) -> torch.Tensor:

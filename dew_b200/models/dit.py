@@ -11,9 +11,11 @@ from typing import Any, Mapping, Optional, Sequence
 
 import torch
 import torch.nn as nn
+import torch.nn.functional as F
 
 from ..nn.dit import ConditioningEmbed, ModulatedBlock, PatchEmbedding, PatchSequenceOutput
 from ..ops.ada import sincos_grid
+from ..utils.hooks import runs_alone
 from ..utils.registry import register
 
 
@@ -42,6 +44,9 @@ class SimpleDiT(nn.Module):
         tokens = self.embed(x.to(dt))
         tokens = tokens + sincos_grid(gh, gw, self.emb_features, tokens.device, dt)[None]
         c = self.conditioning(temb, conditions.get("text"), conditions.get("label"), duration, conditions.get("guidance"))
+        # the blocks and the output share one silu(c), where nobody sees what they are given
+        active = F.silu(c)
+        given = lambda m: (active,) if type(m) in (ModulatedBlock, PatchSequenceOutput) and runs_alone(m) else ()
         routed = None
         for i, block in enumerate(self.blocks):
             if train and self.routes:
@@ -53,12 +58,12 @@ class SimpleDiT(nn.Module):
                         kept_idx = perm[:, :keep].sort(1).values
                         routed = (tokens, kept_idx, int(end))
                         tokens = torch.gather(tokens, 1, kept_idx[..., None].expand(-1, -1, tokens.shape[-1]))
-            tokens = block(tokens, c)
+            tokens = block(tokens, c, *given(block))
             if routed is not None and i == routed[2]:
                 full, kept_idx, _ = routed
                 tokens = full.scatter(1, kept_idx[..., None].expand(-1, -1, tokens.shape[-1]), tokens)
                 routed = None
-        return self.output(tokens, c, (gh, gw))
+        return self.output(tokens, c, (gh, gw), *given(self.output))
 
     def model_flops(self, tokens: int, batch: int = 1) -> float:
         d, L = self.emb_features, self.num_layers

@@ -70,11 +70,11 @@ class ConditioningEmbed(nn.Module):
 
     def forward(self, t, context=None, labels=None, duration=None, guidance=None):
         dt = self.t1.weight.dtype
-        c = self.t2(F.silu(self.t1(sinusoidal(t, self.features, scale=self.time_scale).to(dt))))
+        c = self.t2(F.silu(self.t1(sinusoidal(t, self.features, scale=self.time_scale, dtype=dt))))
         if self.g1 is not None and guidance is not None:
-            c = c + self.g2(F.silu(self.g1(sinusoidal(guidance, self.features, scale=self.time_scale).to(dt))))
+            c = c + self.g2(F.silu(self.g1(sinusoidal(guidance, self.features, scale=self.time_scale, dtype=dt))))
         if self.d1 is not None and duration is not None:
-            c = c + self.d1(sinusoidal(duration, self.features, scale=self.time_scale).to(dt))
+            c = c + self.d1(sinusoidal(duration, self.features, scale=self.time_scale, dtype=dt))
         if self.text is not None and context is not None:
             pooled = context.mean(1) if context.dim() == 3 else context
             c = c + self.text(pooled.to(dt))
@@ -103,8 +103,9 @@ class ModulatedBlock(nn.Module):
         self.ada_proj = Linear(features, 6 * features, bias=True, zero_init=True, axes=("embed", "modulation"), dtype=dtype, device=device)
         self.adaln_silu = adaln_silu
 
-    def forward(self, x, c):
-        m = self.ada_proj(F.silu(c) if self.adaln_silu else c)
+    def forward(self, x, c, active=None):
+        """``active``: ``silu(c)``, where the caller has it."""
+        m = self.ada_proj((F.silu(c) if active is None else active) if self.adaln_silu else c)
         s1, sc1, g1, s2, sc2, g2 = m.chunk(6, -1)
         if not (_bare(self.norm1) and _bare(self.norm2)):
             x = x + g1.unsqueeze(1) * self.attn(modulate(self.norm1(x), s1, sc1))
@@ -124,8 +125,9 @@ class PatchSequenceOutput(nn.Module):
         self.ada_proj = Linear(features, 2 * features, bias=True, zero_init=True, dtype=dtype, device=device)
         self.out = Linear(features, patch_size * patch_size * out_channels, bias=True, zero_init=True, dtype=dtype, device=device)
 
-    def forward(self, x, c, grid):
-        shift, scale = self.ada_proj(F.silu(c)).chunk(2, -1)
+    def forward(self, x, c, grid, active=None):
+        """``active``: ``silu(c)``, where the caller has it."""
+        shift, scale = self.ada_proj(F.silu(c) if active is None else active).chunk(2, -1)
         x = self.out(ada.ada_norm(x, shift, scale, self.norm.eps) if _bare(self.norm) else modulate(self.norm(x), shift, scale)).float()
         B = x.shape[0]
         gh, gw = grid

@@ -11,6 +11,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import ops
+from ..ops import ada
 
 
 def declare(param: nn.Parameter, axes: Sequence[Optional[str]], kind: str = "kernel") -> nn.Parameter:
@@ -120,12 +121,15 @@ def reset_all(module: nn.Module, seed: int, prefix: str = "") -> None:
             fn()
 
 
-def sinusoidal(t: torch.Tensor, dim: int, max_period: float = 10000.0, scale: float = 1.0) -> torch.Tensor:
+def sinusoidal(t: torch.Tensor, dim: int, max_period: float = 10000.0, scale: float = 1.0, dtype: torch.dtype = torch.float32) -> torch.Tensor:
     """Fourier features of a scalar per row: ``[B] -> [B, dim]``."""
+    made = ada.time_features(t, dim, max_period, scale, dtype)
+    if made is not None:
+        return made
     half = dim // 2
     freqs = torch.exp(-math.log(max_period) * torch.arange(half, device=t.device, dtype=torch.float32) / half)
     args = t.float()[:, None] * scale * freqs[None]
     emb = torch.cat([args.cos(), args.sin()], -1)
     if dim % 2:
         emb = F.pad(emb, (0, 1))
-    return emb
+    return emb.to(dtype)

@@ -6,6 +6,7 @@ way on a GPU in bf16, the plain expressions elsewhere.  Parity: ``modulate`` and
 from __future__ import annotations
 
 import ctypes
+import math
 from typing import Optional, Tuple
 
 import torch
@@ -134,6 +135,17 @@ def gated_add(x: torch.Tensor, branch: torch.Tensor, gate: torch.Tensor) -> torc
     if _usable(x, branch, gate):
         return _run(x, branch, gate, None, None, 0.0)
     return x + gate.unsqueeze(1) * branch
+
+
+def time_features(t: torch.Tensor, dim: int, max_period: float, scale: float, dtype: torch.dtype) -> Optional[torch.Tensor]:
+    """``nn.layers.sinusoidal`` by one kernel, where a row of fp32 times on a GPU leaves no trace in autograd; None elsewhere."""
+    if not (t.is_cuda and t.dtype == torch.float32 and t.dim() == 1 and t.is_contiguous() and dim >= 2 and t.numel() * dim < 1 << 30 and dtype in (torch.float32, torch.bfloat16)
+            and L.unrecorded(t) and L.use_cuda(t) and hasattr(L.load(), "dewb_time_features")):
+        return None
+    out = torch.empty(t.shape[0], dim, dtype=dtype, device=t.device)
+    L.check(L.load().dewb_time_features(t.data_ptr(), out.data_ptr(), int(dtype == torch.bfloat16), t.shape[0], dim, -math.log(max_period), scale, L.stream()), "time_features")
+    L.count_launches()
+    return out
 
 
 def sincos_grid(h: int, w: int, dim: int, device, dtype) -> torch.Tensor:

@@ -61,6 +61,7 @@ _SIGNATURES = {
     "dewb_ada_fwd": "ppppp" + "l" + "ppp" + "lii" + "f" + "p",
     "dewb_gemm_rows_bf16": "pppp" + "iii" + "lll" + "p",
     "dewb_swiglu_fwd": "ppp" + "lil" + "p",
+    "dewb_time_features": "pp" + "iii" + "ff" + "p",
     "dewb_rope": "pppp" + "liiiif" + "p",
     "dewb_rope_rows": "ppp" + "liiiiif" + "p",
     "dewb_rmsnorm_bwd": "pppppppppppi" + "li" + "p",

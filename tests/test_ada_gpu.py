@@ -1,4 +1,6 @@
 """Modulated norms and gated residuals, forward and every gradient, against the plain expressions in 64 bits."""
+import math
+
 import pytest
 import torch
 import torch.nn.functional as F
@@ -70,3 +72,36 @@ def test_position_table_and_a_hooked_norm():
         hooked = block(x, c)
         handle.remove()
         assert seen == [1] and rel_err(hooked, plain) < 2e-2
+
+
+@pytest.mark.parametrize("B,d,dtype", [(1, 2, torch.float32), (3, 7, torch.float32), (5, 256, torch.bfloat16), (64, 1153, torch.bfloat16), (0, 8, torch.bfloat16)])
+def test_time_features(B, d, dtype):
+    """Against 64 bits: an angle of up to 1000 turns on its fp32 roundings (the product with the frequency, and the frequency: some 2^-23 of it each), the rest on one
+    rounding of the result; and a time that is differentiated keeps its graph."""
+    from dew_b200.nn.layers import sinusoidal
+    t = torch.rand(B, generator=torch.Generator(device=DEV).manual_seed(d), device=DEV) * 1000
+    got = sinusoidal(t, d, scale=16.0 if d < 8 else 1.0, dtype=dtype)
+    assert got.shape == (B, d) and got.dtype == dtype
+    half = d // 2
+    angle = t.double()[:, None] * (16.0 if d < 8 else 1.0) * torch.exp(-math.log(10000.0) * torch.arange(half, device=DEV, dtype=torch.float64) / half)
+    want = torch.cat([angle.cos(), angle.sin(), angle.new_zeros(B, d % 2)], -1)
+    bound = torch.cat([angle, angle, angle.new_zeros(B, d % 2)], -1) * 2.0 ** -20 + (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -22)
+    assert bool(((got.double() - want).abs() <= bound).all())
+    leaf = t.clone().requires_grad_()
+    assert B == 0 or float(torch.autograd.grad(sinusoidal(leaf, d, dtype=dtype).float().sum(), leaf)[0].abs().sum()) > 0
+
+
+def test_blocks_share_the_activation_of_their_condition():
+    """The same outputs whether the blocks make it themselves (somebody looks at them) or are given it."""
+    from dew_b200.models import SimpleDiT
+    torch.manual_seed(0)
+    model = SimpleDiT(patch_size=2, emb_features=128, num_layers=3, num_heads=2, input_channels=4, output_channels=4, num_classes=10, dtype=torch.bfloat16, device=DEV)
+    for p in model.parameters():
+        torch.nn.init.normal_(p, std=0.05)
+    x, t, label = torch.randn(2, 8, 8, 4, device=DEV), torch.rand(2, device=DEV), torch.tensor([1, 7], device=DEV)
+    shared = model(x, t, {"label": label})
+    hooks = [m.register_forward_hook(lambda *a: None) for m in (*model.blocks, model.output)]
+    own = model(x, t, {"label": label})
+    for h in hooks:
+        h.remove()
+    assert torch.equal(shared, own)

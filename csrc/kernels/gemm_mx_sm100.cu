@@ -229,16 +229,7 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
         if (row < M && col < N) {
           __nv_bfloat16* out = D + static_cast<long long>(row) * ldd + col;
           if (col + 32 <= N && ((reinterpret_cast<uintptr_t>(out) & 15) == 0)) {
-            uint4* o4 = reinterpret_cast<uint4*>(out);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              uint4 pk;
-              pk.x = pack_bf16(__uint_as_float(r[j * 8 + 0]), __uint_as_float(r[j * 8 + 1]));
-              pk.y = pack_bf16(__uint_as_float(r[j * 8 + 2]), __uint_as_float(r[j * 8 + 3]));
-              pk.z = pack_bf16(__uint_as_float(r[j * 8 + 4]), __uint_as_float(r[j * 8 + 5]));
-              pk.w = pack_bf16(__uint_as_float(r[j * 8 + 6]), __uint_as_float(r[j * 8 + 7]));
-              o4[j] = pk;
-            }
+            store_row_32<false>(out, r, 1.f);
           } else {
 #pragma unroll
             for (int i = 0; i < 32; ++i) if (col + i < N) out[i] = __float2bfloat16(__uint_as_float(r[i]));

@@ -283,22 +283,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           if (EPI == EPI_BF16 || EPI == EPI_BF16_ACC) {
             __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(Dptr) + ti.d_off + static_cast<long long>(row) * ldd + col;
             if (full && ((reinterpret_cast<uintptr_t>(out) & 15) == 0)) {
-              uint4* o4 = reinterpret_cast<uint4*>(out);
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                float v[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = al * __uint_as_float(r[j * 8 + i]);
-                if (EPI == EPI_BF16_ACC) {
-                  const uint4 old = o4[j];
-                  v[0] += bf16_lo(old.x); v[1] += bf16_hi(old.x); v[2] += bf16_lo(old.y); v[3] += bf16_hi(old.y);
-                  v[4] += bf16_lo(old.z); v[5] += bf16_hi(old.z); v[6] += bf16_lo(old.w); v[7] += bf16_hi(old.w);
-                }
-                uint4 pk;
-                pk.x = pack_bf16(v[0], v[1]); pk.y = pack_bf16(v[2], v[3]);
-                pk.z = pack_bf16(v[4], v[5]); pk.w = pack_bf16(v[6], v[7]);
-                o4[j] = pk;
-              }
+              store_row_32<EPI == EPI_BF16_ACC>(out, r, al);
             } else {
 #pragma unroll
               for (int i = 0; i < 32; ++i) {
@@ -312,14 +297,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           } else {
             float* out = reinterpret_cast<float*>(Dptr) + ti.d_off + static_cast<long long>(row) * ldd + col;
             if (full && ((reinterpret_cast<uintptr_t>(out) & 15) == 0)) {
-              float4* o4 = reinterpret_cast<float4*>(out);
-#pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                float4 v = make_float4(al * __uint_as_float(r[j * 4 + 0]), al * __uint_as_float(r[j * 4 + 1]),
-                                       al * __uint_as_float(r[j * 4 + 2]), al * __uint_as_float(r[j * 4 + 3]));
-                if (EPI == EPI_F32_ACC) { const float4 o = o4[j]; v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w; }
-                o4[j] = v;
-              }
+              store_row_32<EPI == EPI_F32_ACC>(out, r, al);
             } else {
 #pragma unroll
               for (int i = 0; i < 32; ++i) {

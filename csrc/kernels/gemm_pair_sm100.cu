@@ -65,6 +65,39 @@ __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int
   n_blk = r / gsize;
 }
 
+// Several products of one shape side by side (GROUPED): product g reduces over [offsets[g], offsets[g + 1]) (experts' weight gradients), or over `per` indices each
+// where there are no offsets (the parts of a split reduction), and writes D + g * stride.  A pair fetches two thirds of the operand bytes that two lone CTAs do, which
+// short reductions waited for beside their stores: 64 groups of 768 rows into 2816 x 2048 took lone CTAs 471 us and take pairs 424, 16 groups of 128 rows into
+// 512 x 256 13.3 either way; the twelve split weight gradients of a diffusion transformer's step (768 x 768
+// to 3072 over 16384) 684 and 600.  A group without rows is cleared in wide stores (one among 16 of
+// 640 x 1408: 77 us in single values, 32 now).
+struct Groups {
+  const int* offsets;
+  int per, count;
+  long long stride;
+};
+
+struct Tile {
+  int m_blk, n_blk, k0, k_iters;
+  long long d_off;
+};
+
+template <bool GROUPED>
+__device__ __forceinline__ Tile tile_of(int t, int tiles_m, int tiles_n, int group_m, int K, const Groups& gr) {
+  Tile ti;
+  ti.k0 = 0; ti.k_iters = (K + BK - 1) / BK; ti.d_off = 0;
+  if constexpr (GROUPED) {
+    const int per = tiles_m * tiles_n, g = t / per;
+    t -= g * per;
+    ti.k0 = gr.offsets != nullptr ? gr.offsets[g] : g * gr.per;
+    const int end = gr.offsets != nullptr ? gr.offsets[g + 1] : min(K, ti.k0 + gr.per);
+    ti.k_iters = (end - ti.k0 + BK - 1) / BK;
+    ti.d_off = g * gr.stride;
+  }
+  tile_coords(t, tiles_m, tiles_n, group_m, ti.m_blk, ti.n_blk);
+  return ti;
+}
+
 template <int EPI>
 __device__ __forceinline__ void store_chunk(const uint32_t (&r_in)[32], void* Dptr, int row, int col, int N, long long ldd,
                                             float alpha_in, const __nv_bfloat16* __restrict__ bias) {
@@ -106,11 +139,11 @@ __device__ __forceinline__ void store_chunk(const uint32_t (&r_in)[32], void* Dp
   }
 }
 
-template <bool A_MN, bool B_MN, int EPI>
+template <bool A_MN, bool B_MN, int EPI, bool GROUPED>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                  void* __restrict__ Dptr, int M, int N, int K, long long ldd, float alpha, int group_m,
-                 const __nv_bfloat16* __restrict__ bias,
+                 const __nv_bfloat16* __restrict__ bias, const Groups groups,
                  int* __restrict__ err) {
   extern __shared__ uint8_t smem_raw[];
   // 1024-byte alignment: required by the 128-byte swizzle atoms the descriptors assume. The dynamic shared memory
@@ -127,8 +160,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   const int num_pairs = gridDim.x >> 1;
   const int tiles_m = (M + PAIR_M - 1) / PAIR_M;
   const int tiles_n = (N + BN - 1) / BN;
-  const int num_tiles = tiles_m * tiles_n;
-  const int k_iters = (K + BK - 1) / BK;
+  const int num_tiles = tiles_m * tiles_n * (GROUPED ? groups.count : 1);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&sh->full[s], 1); mbar_init(&sh->empty[s], 1); }
@@ -162,17 +194,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       long long issued = 0;
       bool ok = true;
       for (int t = pair; t < num_tiles && ok; t += num_pairs) {
-        int m_blk, n_blk;
-        tile_coords(t, tiles_m, tiles_n, group_m, m_blk, n_blk);
-        const int m0 = m_blk * PAIR_M + static_cast<int>(rank) * BM;
-        const int n0 = n_blk * BN + static_cast<int>(rank) * HALF_N;
-        for (int k = 0; k < k_iters; ++k) {
+        const Tile ti = tile_of<GROUPED>(t, tiles_m, tiles_n, group_m, K, groups);
+        const int m0 = ti.m_blk * PAIR_M + static_cast<int>(rank) * BM;
+        const int n0 = ti.n_blk * BN + static_cast<int>(rank) * HALF_N;
+        for (int k = 0; k < ti.k_iters; ++k) {
           if (!mbar_wait(&sh->empty[stage], phase ^ 1, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_EMPTY); ok = false; break; }
           uint8_t* sa = smem + stage * STAGE_BYTES;
           uint8_t* sb = sa + A_BYTES;
           if (rank == leader) mbar_expect_tx(&sh->full[stage], 2 * STAGE_BYTES);     // both CTAs' bytes
           const uint32_t full_bar = map_to_cta(smem_u32(&sh->full[stage]), leader);
-          const int k0 = k * BK;
+          const int k0 = ti.k0 + k * BK;
           if (!A_MN) {
             tma_load_2d_pair(sa, &tma_a, full_bar, k0, m0);
           } else {
@@ -211,6 +242,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       int acc = 0; uint32_t acc_phase = 0;
       bool ok = true;
       for (int t = pair; t < num_tiles && ok; t += num_pairs) {
+        const int k_iters = tile_of<GROUPED>(t, tiles_m, tiles_n, group_m, K, groups).k_iters;
+        if (k_iters <= 0) continue;
         if (!mbar_wait_warp(&sh->tmem_empty[acc], acc_phase ^ 1, abort_flag)) { if (lane == 0) atomicCAS(err, 0, ERR_WAIT_TMEM_EMPTY); break; }
         const uint32_t d_tmem = tmem_base + acc * ACC_COLS;
         for (int k = 0; k < k_iters; ++k) {
@@ -247,10 +280,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     int acc = 0; uint32_t acc_phase = 0;
     bool ok = true;
     for (int t = pair; t < num_tiles && ok; t += num_pairs) {
-      int m_blk, n_blk;
-      tile_coords(t, tiles_m, tiles_n, group_m, m_blk, n_blk);
-      const int row = m_blk * PAIR_M + static_cast<int>(rank) * BM + q * 32 + lane;
-      const int n0 = n_blk * BN;
+      const Tile ti = tile_of<GROUPED>(t, tiles_m, tiles_n, group_m, K, groups);
+      const int row = ti.m_blk * PAIR_M + static_cast<int>(rank) * BM + q * 32 + lane;
+      const int n0 = ti.n_blk * BN;
+      constexpr bool F32 = EPI == EPI_F32 || EPI == EPI_F32_ACC;
+      void* D = F32 ? static_cast<void*>(static_cast<float*>(Dptr) + ti.d_off) : static_cast<void*>(static_cast<__nv_bfloat16*>(Dptr) + ti.d_off);
+      if (GROUPED && ti.k_iters <= 0) {
+        // nothing to reduce over: the product is zero (nothing to add when accumulating)
+        if ((EPI == EPI_BF16 || EPI == EPI_F32) && row < M) {
+          const uint32_t zero[32] = {};
+          for (int c = n0 + first * 32; c < min(N, n0 + first * 32 + BN / 2); c += 32) store_chunk<EPI>(zero, D, row, c, N, ldd, 1.f, nullptr);
+        }
+        continue;
+      }
       if (!mbar_wait(&sh->tmem_full[acc], acc_phase, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_TMEM_FULL); ok = false; break; }
       tc_fence_after();
       const uint32_t taddr = tmem_base + acc * ACC_COLS + (static_cast<uint32_t>(q * 32) << 16);
@@ -261,8 +303,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         tmem_ld_32x32b_x32(taddr + c * 32 + 32, r1);
         tmem_ld_wait();
         const int col = n0 + c * 32;
-        if (row < M && col < N) store_chunk<EPI>(r0, Dptr, row, col, N, ldd, alpha, bias);
-        if (row < M && col + 32 < N) store_chunk<EPI>(r1, Dptr, row, col + 32, N, ldd, alpha, bias);
+        if (row < M && col < N) store_chunk<EPI>(r0, D, row, col, N, ldd, alpha, bias);
+        if (row < M && col + 32 < N) store_chunk<EPI>(r1, D, row, col + 32, N, ldd, alpha, bias);
       }
       tc_fence_before();
       __syncwarp();
@@ -284,10 +326,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   }
 }
 
-template <bool A_MN, bool B_MN, int EPI>
+template <bool A_MN, bool B_MN, int EPI, bool GROUPED = false>
 static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, void* D, int M, int N, int K, long long ldd,
-                      float alpha, int* err, int max_pairs, cudaStream_t stream, const __nv_bfloat16* bias = nullptr) {
-  auto kern = gemm_pair_kernel<A_MN, B_MN, EPI>;
+                      float alpha, int* err, int max_pairs, cudaStream_t stream, const __nv_bfloat16* bias = nullptr, const Groups& groups = {nullptr, 0, 1, 0}) {
+  auto kern = gemm_pair_kernel<A_MN, B_MN, EPI, GROUPED>;
   static int resident[64] = {};          // co-resident clusters of this instantiation per device (0 = not asked yet)
   int dev = 0;
   cudaGetDevice(&dev);
@@ -314,7 +356,7 @@ static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, void* D, int
   }
   int pairs = resident[dev];
   if (max_pairs > 0 && max_pairs < pairs) pairs = max_pairs;
-  const int tiles = ((M + PAIR_M - 1) / PAIR_M) * ((N + BN - 1) / BN);
+  const int tiles = ((M + PAIR_M - 1) / PAIR_M) * ((N + BN - 1) / BN) * groups.count;
   if (tiles < pairs) pairs = tiles;
   cfg.gridDim = dim3(static_cast<unsigned>(2 * pairs), 1, 1);
   // Measured on the layer shapes (gate|up forward, 8192 / 16384 x 28672 x 4096): 16 row blocks per group are 5 % faster than 4
@@ -328,8 +370,18 @@ static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, void* D, int
   if (group_m <= 0) {
     group_m = K <= 8192 ? 16 : 8;
   }
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb, D, M, N, K, ldd, alpha, group_m, bias, err);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb, D, M, N, K, ldd, alpha, group_m, bias, groups, err);
   return static_cast<int>(e);
+}
+
+static int operand_maps(CUtensorMap* ta, CUtensorMap* tb, const void* A, const void* B, int M, int N, int K, long long lda, long long ldb, int a_mn, int b_mn) {
+  int r;
+  if (!a_mn) r = make_tmap_2d(ta, A, M, K, lda, BM, BK, 2, true);
+  else       r = make_tmap_2d(ta, A, K, M, lda, BK, 64, 2, true);
+  if (r) return 1000 + r;
+  if (!b_mn) r = make_tmap_2d(tb, B, N, K, ldb, HALF_N, BK, 2, true);
+  else       r = make_tmap_2d(tb, B, K, N, ldb, BK, 64, 2, true);
+  return r ? 2000 + r : 0;
 }
 
 template <bool A_MN, bool B_MN>
@@ -342,6 +394,30 @@ static int launch_epi(int epi, const CUtensorMap& ta, const CUtensorMap& tb, voi
     case EPI_BF16_ACC: return launch_one<A_MN, B_MN, EPI_BF16_ACC>(ta, tb, D, M, N, K, ldd, alpha, err, max_pairs, stream, bias);
   }
   return -2;
+}
+
+// part [splits, M, N] fp32 -> D [M, N] (row stride ldd): the sum over the splits as bf16 (epi 0) or fp32 (1), or added to what is there in fp32 (2) or bf16 (3)
+__global__ void __launch_bounds__(256)
+split_sum_kernel(const float* __restrict__ part, void* __restrict__ D, int M, int N, long long ldd, int splits, float alpha, int epi, const int* __restrict__ err) {
+  if (*reinterpret_cast<const volatile int*>(err) != 0) return;
+  const long long total = static_cast<long long>(M) * N, at = (blockIdx.x * 256ll + threadIdx.x) * 4;
+  if (at >= total) return;
+  float4 s = *reinterpret_cast<const float4*>(part + at);
+  for (int k = 1; k < splits; ++k) {
+    const float4 v = *reinterpret_cast<const float4*>(part + k * total + at);
+    s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+  }
+  s.x *= alpha; s.y *= alpha; s.z *= alpha; s.w *= alpha;
+  const long long to = at / N * ldd + at % N;
+  if (epi == EPI_F32 || epi == EPI_F32_ACC) {
+    float4* d = reinterpret_cast<float4*>(reinterpret_cast<float*>(D) + to);
+    if (epi == EPI_F32_ACC) { const float4 o = *d; s.x += o.x; s.y += o.y; s.z += o.z; s.w += o.w; }
+    *d = s;
+  } else {
+    uint2* d = reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(D) + to);
+    if (epi == EPI_BF16_ACC) { const uint2 o = *d; s.x += bf16_lo(o.x); s.y += bf16_hi(o.x); s.z += bf16_lo(o.y); s.w += bf16_hi(o.y); }
+    *d = make_uint2(pack_bf16(s.x, s.y), pack_bf16(s.z, s.w));
+  }
 }
 
 }  // namespace gemm_pair
@@ -362,13 +438,8 @@ extern "C" int dewb_gemm_pair_bf16(const void* A, const void* B, void* D, int M,
   if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return -3;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
   CUtensorMap ta, tb;
-  int r;
-  if (!a_mn) r = make_tmap_2d(&ta, A, M, K, lda, BM, BK, 2, true);
-  else       r = make_tmap_2d(&ta, A, K, M, lda, BK, 64, 2, true);
-  if (r) return 1000 + r;
-  if (!b_mn) r = make_tmap_2d(&tb, B, N, K, ldb, HALF_N, BK, 2, true);
-  else       r = make_tmap_2d(&tb, B, K, N, ldb, BK, 64, 2, true);
-  if (r) return 2000 + r;
+  const int r = operand_maps(&ta, &tb, A, B, M, N, K, lda, ldb, a_mn, b_mn);
+  if (r) return r;
   const int max_pairs = max_ctas > 0 ? (max_ctas / 2 > 0 ? max_ctas / 2 : 1) : 0;
   const __nv_bfloat16* bias = g_pair_bias;
   if (!a_mn && !b_mn) return launch_epi<false, false>(epi, ta, tb, D, M, N, K, ldd, alpha, err, max_pairs, stream, bias);
@@ -385,4 +456,55 @@ extern "C" int dewb_gemm_pair_bf16_bias(const void* A, const void* B, void* D, c
   const int rc = dewb_gemm_pair_bf16(A, B, D, M, N, K, lda, ldb, ldd, a_mn, b_mn, epi, alpha, err, max_ctas, stream_ptr);
   g_pair_bias = nullptr;
   return rc;
+}
+
+// The same product with its reduction in `splits` parts of `per` (a multiple of 64; splits * per >= K, every part with something in it): scratch holds
+// splits * M * N floats.  N and ldd multiples of 4, D and scratch 16-byte aligned.
+extern "C" int dewb_gemm_bf16_split(const void* A, const void* B, void* D, float* scratch, int M, int N, int K, int splits, int per, long long lda, long long ldb,
+                                    long long ldd, int a_mn, int b_mn, int epi, float alpha, int* err, void* stream_ptr) {
+  using namespace dewb;
+  using namespace dewb::gemm_pair;
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || (N % 4) || (ldd % 4) ||
+      (reinterpret_cast<uintptr_t>(D) & 15) || (reinterpret_cast<uintptr_t>(scratch) & 15) || splits < 1 || per % BK || per <= 0 ||
+      static_cast<long long>(splits) * per < K || static_cast<long long>(splits - 1) * per >= K || epi < 0 || epi > 3)
+    return -3;
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
+  CUtensorMap ta, tb;
+  int r = operand_maps(&ta, &tb, A, B, M, N, K, lda, ldb, a_mn, b_mn);
+  if (r) return r;
+  const Groups gr{nullptr, per, splits, static_cast<long long>(M) * N};
+  if (!a_mn && !b_mn) r = launch_one<false, false, EPI_F32, true>(ta, tb, scratch, M, N, K, N, 1.f, err, 0, stream, nullptr, gr);
+  else if (!a_mn) r = launch_one<false, true, EPI_F32, true>(ta, tb, scratch, M, N, K, N, 1.f, err, 0, stream, nullptr, gr);
+  else if (!b_mn) r = launch_one<true, false, EPI_F32, true>(ta, tb, scratch, M, N, K, N, 1.f, err, 0, stream, nullptr, gr);
+  else r = launch_one<true, true, EPI_F32, true>(ta, tb, scratch, M, N, K, N, 1.f, err, 0, stream, nullptr, gr);
+  if (r) return r;
+  const long long total = static_cast<long long>(M) * N;
+  split_sum_kernel<<<static_cast<unsigned>((total / 4 + 255) / 256), 256, 0, stream>>>(scratch, D, M, N, ldd, splits, alpha, epi, err);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// Grouped reduction (mixture-of-experts weight gradient): for every group g,
+//   D_g[M, N] (+)= A[rows of g, M]^T * B[rows of g, N]   with A stored [R, M] and B stored [R, N] (R = all rows),
+//   rows of g = [group_offsets[g], group_offsets[g + 1]) (multiples of 64; padding rows are zero)
+//   D stacks the groups: D_g = D + g * d_group_stride, row stride ldd.
+extern "C" int dewb_tgmm_bf16(const void* A, const void* B, void* D, const int* group_offsets, int R, int M, int N,
+                              int groups, long long lda, long long ldb, long long ldd, long long d_group_stride, int epi,
+                              float alpha, int* err, void* stream_ptr) {
+  using namespace dewb;
+  using namespace dewb::gemm_pair;
+  if (R <= 0 || M <= 0 || N <= 0 || groups <= 0) return 0;
+  if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return -3;
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
+  CUtensorMap ta, tb;
+  const int r = operand_maps(&ta, &tb, A, B, M, N, R, lda, ldb, 1, 1);
+  if (r) return r;
+  const Groups gr{group_offsets, 0, groups, d_group_stride};
+  switch (epi) {
+    case EPI_BF16: return launch_one<true, true, EPI_BF16, true>(ta, tb, D, M, N, R, ldd, alpha, err, 0, stream, nullptr, gr);
+    case EPI_F32: return launch_one<true, true, EPI_F32, true>(ta, tb, D, M, N, R, ldd, alpha, err, 0, stream, nullptr, gr);
+    case EPI_F32_ACC: return launch_one<true, true, EPI_F32_ACC, true>(ta, tb, D, M, N, R, ldd, alpha, err, 0, stream, nullptr, gr);
+    case EPI_BF16_ACC: return launch_one<true, true, EPI_BF16_ACC, true>(ta, tb, D, M, N, R, ldd, alpha, err, 0, stream, nullptr, gr);
+  }
+  return -2;
 }

@@ -6,9 +6,6 @@
 //   warps 2..9  epilogue       : tcgen05.ld the finished accumulator, convert, store; overlaps the next tile's MMAs.  Two warps share a quarter of the rows
 //                                and take half of the columns each
 //
-// Weight gradients whose outputs have few tiles (768 x 2304 of 16384 tokens: 54) split the reduction: every split's partial product goes to fp32 scratch and a
-// small kernel adds them in order.
-//
 // Operand layouts. "K-major" means the reduction index is contiguous in global memory; "MN-major" means the
 // M (for A) or N (for B) index is contiguous. The three combinations cover a linear layer's forward
 // (x[M,K], W[N,K]), its input gradient (dY[M,N'] K-major, W[N',K'] MN-major) and its weight gradient (both
@@ -52,28 +49,18 @@ struct Shared {
 //   mode 1  grouped rows      D[rows of g] = A[rows of g] * B_g^T   (forward and input gradient); B stacks the
 //           groups along its row dimension, `b_rows_per_group` rows each; `tile_group[m_tile]` names the group of
 //           each 128-row tile (< 0: the tile holds no rows)
-//   mode 2  grouped reduction D_g = A[rows of g]^T-style product over the rows of g (weight gradient); the reduction
-//           runs over rows [group_offsets[g], group_offsets[g+1]) and D stacks the groups, `d_group_stride` apart
-//   mode 3  split reduction   D_g = the product over reduction indices [g, g + 1) * `b_rows_per_group` (a multiple of BK); D stacks the
-//           splits, `d_group_stride` apart
 struct GroupArgs {
   const int* tile_group;
-  const int* group_offsets;
   int mode;
   int b_rows_per_group;
-  int groups;
-  long long d_group_stride;
   const float* row_scale;   // fp8: per-row scale of A (length M), or null
   const float* col_scale;   // fp8: per-row scale of the stacked B operand (indexed by B's row), or null
   const __nv_bfloat16* bias; // one value per output column added after the scale (dense mode), or null
 };
 
 struct Tile {
-  int m0, n0;        // output tile origin (within the group for mode 2)
+  int m0, n0;        // output tile origin
   int b_row0;        // row offset added to B's stacked-row coordinate (mode 1)
-  int k_begin;       // first reduction index
-  int k_iters;       // reduction steps of BK
-  long long d_off;   // element offset of the group's output (mode 2)
   bool skip;         // nothing to compute and nothing to store
 };
 
@@ -88,26 +75,15 @@ __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int
   n_blk = r / gsize;
 }
 
-__device__ __forceinline__ Tile decode_tile(int t, int tiles_m, int tiles_n, int K, const GroupArgs& ga, int bk = BK) {
+__device__ __forceinline__ Tile decode_tile(int t, int tiles_m, int tiles_n, const GroupArgs& ga) {
   Tile ti;
   int m_blk, n_blk;
-  ti.b_row0 = 0; ti.k_begin = 0; ti.k_iters = (K + bk - 1) / bk; ti.d_off = 0; ti.skip = false;
-  if (ga.mode >= 2) {
-    const int per = tiles_m * tiles_n;
-    const int g = t / per;
-    tile_coords(t - g * per, tiles_m, tiles_n, m_blk, n_blk);
-    const int r0 = ga.mode == 3 ? g * ga.b_rows_per_group : ga.group_offsets[g];
-    const int r1 = ga.mode == 3 ? min(K, r0 + ga.b_rows_per_group) : ga.group_offsets[g + 1];
-    ti.k_begin = r0;
-    ti.k_iters = (r1 - r0 + BK - 1) / BK;
-    ti.d_off = static_cast<long long>(g) * ga.d_group_stride;
-  } else {
-    tile_coords(t, tiles_m, tiles_n, m_blk, n_blk);
-    if (ga.mode == 1) {
-      const int g = ga.tile_group[m_blk];
-      ti.skip = g < 0;
-      ti.b_row0 = (g < 0 ? 0 : g) * ga.b_rows_per_group;
-    }
+  ti.b_row0 = 0; ti.skip = false;
+  tile_coords(t, tiles_m, tiles_n, m_blk, n_blk);
+  if (ga.mode == 1) {
+    const int g = ga.tile_group[m_blk];
+    ti.skip = g < 0;
+    ti.b_row0 = (g < 0 ? 0 : g) * ga.b_rows_per_group;
   }
   ti.m0 = m_blk * BM;
   ti.n0 = n_blk * BN;
@@ -138,7 +114,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   const int lane = threadIdx.x & 31;
   const int tiles_m = (M + BM - 1) / BM;
   const int tiles_n = (N + BN - 1) / BN;
-  const int num_tiles = tiles_m * tiles_n * (ga.mode >= 2 ? ga.groups : 1);
+  const int num_tiles = tiles_m * tiles_n;
+  const int k_iters = (K + (FP8 ? 2 * BK : BK) - 1) / (FP8 ? 2 * BK : BK);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&sh->full[s], 1); mbar_init(&sh->empty[s], 1); }
@@ -165,15 +142,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       long long issued = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        const Tile ti = decode_tile(t, tiles_m, tiles_n, K, ga, FP8 ? 2 * BK : BK);
-        if (ti.skip || ti.k_iters == 0) continue;
+        const Tile ti = decode_tile(t, tiles_m, tiles_n, ga);
+        if (ti.skip) continue;
         const int m0 = ti.m0, n0 = ti.n0;
-        for (int k = 0; k < ti.k_iters; ++k) {
+        for (int k = 0; k < k_iters; ++k) {
           if (!mbar_wait(&sh->empty[stage], phase ^ 1, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_EMPTY); ok = false; break; }
           uint8_t* sa = smem + stage * STAGE_BYTES;
           uint8_t* sb = sa + A_BYTES;
           mbar_expect_tx(&sh->full[stage], STAGE_BYTES);
-          const int k0 = ti.k_begin + k * (FP8 ? 2 * BK : BK);
+          const int k0 = k * (FP8 ? 2 * BK : BK);
           if (!A_MN) {
             tma_load_2d(sa, &tma_a, &sh->full[stage], k0, m0);
           } else {
@@ -208,9 +185,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       int acc = 0; uint32_t acc_phase = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        const Tile ti = decode_tile(t, tiles_m, tiles_n, K, ga, FP8 ? 2 * BK : BK);
-        if (ti.skip || ti.k_iters == 0) continue;
-        const int k_iters = ti.k_iters;
+        const Tile ti = decode_tile(t, tiles_m, tiles_n, ga);
+        if (ti.skip) continue;
         if (!mbar_wait(&sh->tmem_empty[acc], acc_phase ^ 1, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_TMEM_EMPTY); ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * ACC_COLS;
@@ -241,20 +217,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     int acc = 0; uint32_t acc_phase = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-      const Tile ti = decode_tile(t, tiles_m, tiles_n, K, ga, FP8 ? 2 * BK : BK);
+      const Tile ti = decode_tile(t, tiles_m, tiles_n, ga);
       if (ti.skip) continue;
       const int row = ti.m0 + q * 32 + lane;
       const int n0 = ti.n0;
-      if (ti.k_iters == 0) {
-        // an empty group: its product is zero (nothing to add when accumulating)
-        if ((EPI == EPI_BF16 || EPI == EPI_F32) && row < M) {
-          for (int c = first * 32; c < first * 32 + BN / 2 && n0 + c < N; ++c) {
-            if (EPI == EPI_BF16) reinterpret_cast<__nv_bfloat16*>(Dptr)[ti.d_off + static_cast<long long>(row) * ldd + n0 + c] = __float2bfloat16(0.f);
-            else reinterpret_cast<float*>(Dptr)[ti.d_off + static_cast<long long>(row) * ldd + n0 + c] = 0.f;
-          }
-        }
-        continue;
-      }
       if (!mbar_wait(&sh->tmem_full[acc], acc_phase, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_TMEM_FULL); ok = false; break; }
       tc_fence_after();
       const uint32_t taddr = tmem_base + acc * ACC_COLS + (static_cast<uint32_t>(q * 32) << 16);
@@ -281,7 +247,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         if (row < M && col < N) {
           const bool full = (col + 32 <= N);
           if (EPI == EPI_BF16 || EPI == EPI_BF16_ACC) {
-            __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(Dptr) + ti.d_off + static_cast<long long>(row) * ldd + col;
+            __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(Dptr) + static_cast<long long>(row) * ldd + col;
             if (full && ((reinterpret_cast<uintptr_t>(out) & 15) == 0)) {
               store_row_32<EPI == EPI_BF16_ACC>(out, r, al);
             } else {
@@ -295,7 +261,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
               }
             }
           } else {
-            float* out = reinterpret_cast<float*>(Dptr) + ti.d_off + static_cast<long long>(row) * ldd + col;
+            float* out = reinterpret_cast<float*>(Dptr) + static_cast<long long>(row) * ldd + col;
             if (full && ((reinterpret_cast<uintptr_t>(out) & 15) == 0)) {
               store_row_32<EPI == EPI_F32_ACC>(out, r, al);
             } else {
@@ -339,7 +305,7 @@ static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, void* D, int
     if (e != cudaSuccess) return static_cast<int>(e);
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * (ga.mode >= 2 ? ga.groups : 1);
+  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
   const int grid = tiles < sms ? tiles : sms;
   kern<<<grid, THREADS, SMEM_BYTES, stream>>>(ta, tb, D, M, N, K, ldd, alpha, ga, err);
   return static_cast<int>(cudaGetLastError());
@@ -374,30 +340,6 @@ static int dispatch(int a_mn, int b_mn, int epi, const CUtensorMap& ta, const CU
   if (!a_mn && b_mn) return launch_epi<false, true>(epi, ta, tb, D, M, N, K, ldd, alpha, ga, err, sms, stream);
   if (a_mn && !b_mn) return launch_epi<true, false>(epi, ta, tb, D, M, N, K, ldd, alpha, ga, err, sms, stream);
   return launch_epi<true, true>(epi, ta, tb, D, M, N, K, ldd, alpha, ga, err, sms, stream);
-}
-
-// part [splits, M, N] fp32 -> D [M, N] (row stride ldd): the sum over the splits as bf16 (epi 0) or fp32 (1), or added to what is there in fp32 (2) or bf16 (3)
-__global__ void __launch_bounds__(256)
-split_sum_kernel(const float* __restrict__ part, void* __restrict__ D, int M, int N, long long ldd, int splits, float alpha, int epi, const int* __restrict__ err) {
-  if (*reinterpret_cast<const volatile int*>(err) != 0) return;
-  const long long total = static_cast<long long>(M) * N, at = (blockIdx.x * 256ll + threadIdx.x) * 4;
-  if (at >= total) return;
-  float4 s = *reinterpret_cast<const float4*>(part + at);
-  for (int k = 1; k < splits; ++k) {
-    const float4 v = *reinterpret_cast<const float4*>(part + k * total + at);
-    s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
-  }
-  s.x *= alpha; s.y *= alpha; s.z *= alpha; s.w *= alpha;
-  const long long to = at / N * ldd + at % N;
-  if (epi == EPI_F32 || epi == EPI_F32_ACC) {
-    float4* d = reinterpret_cast<float4*>(reinterpret_cast<float*>(D) + to);
-    if (epi == EPI_F32_ACC) { const float4 o = *d; s.x += o.x; s.y += o.y; s.z += o.z; s.w += o.w; }
-    *d = s;
-  } else {
-    uint2* d = reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(D) + to);
-    if (epi == EPI_BF16_ACC) { const uint2 o = *d; s.x += bf16_lo(o.x); s.y += bf16_hi(o.x); s.z += bf16_lo(o.y); s.w += bf16_hi(o.y); }
-    *d = make_uint2(pack_bf16(s.x, s.y), pack_bf16(s.z, s.w));
-  }
 }
 
 }  // namespace gemm
@@ -444,7 +386,7 @@ extern "C" int dewb_gemm_bf16(const void* A, const void* B, void* D, int M, int 
   if (r) return 2000 + r;
   int sms = sm_count();
   if (max_ctas > 0 && max_ctas < sms) sms = max_ctas;
-  GroupArgs ga{nullptr, nullptr, 0, 0, 1, 0, nullptr, nullptr, g_dense_bias};
+  GroupArgs ga{nullptr, 0, 0, nullptr, nullptr, g_dense_bias};
   return dispatch(a_mn, b_mn, epi, ta, tb, D, M, N, K, ldd, alpha, ga, err, sms, stream);
 }
 
@@ -456,33 +398,6 @@ extern "C" int dewb_gemm_bf16_bias(const void* A, const void* B, void* D, const 
   const int rc = dewb_gemm_bf16(A, B, D, M, N, K, lda, ldb, ldd, a_mn, b_mn, epi, alpha, err, max_ctas, stream_ptr);
   g_dense_bias = nullptr;
   return rc;
-}
-
-// The same product with its reduction in `splits` parts of `per` (a multiple of 64; splits * per >= K, every part with something in it): scratch holds
-// splits * M * N floats.  N and ldd multiples of 4, D and scratch 16-byte aligned.
-extern "C" int dewb_gemm_bf16_split(const void* A, const void* B, void* D, float* scratch, int M, int N, int K, int splits, int per, long long lda, long long ldb,
-                                    long long ldd, int a_mn, int b_mn, int epi, float alpha, int* err, void* stream_ptr) {
-  using namespace dewb;
-  using namespace dewb::gemm;
-  if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || (N % 4) || (ldd % 4) ||
-      (reinterpret_cast<uintptr_t>(D) & 15) || (reinterpret_cast<uintptr_t>(scratch) & 15) || splits < 1 || per % BK || per <= 0 ||
-      static_cast<long long>(splits) * per < K || static_cast<long long>(splits - 1) * per >= K || epi < 0 || epi > 3)
-    return -3;
-  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
-  CUtensorMap ta, tb;
-  int r;
-  if (!a_mn) r = make_tmap_2d(&ta, A, M, K, lda, BM, BK, 2, true);
-  else       r = make_tmap_2d(&ta, A, K, M, lda, BK, 64, 2, true);
-  if (r) return 1000 + r;
-  if (!b_mn) r = make_tmap_2d(&tb, B, N, K, ldb, BN, BK, 2, true);
-  else       r = make_tmap_2d(&tb, B, K, N, ldb, BK, 64, 2, true);
-  if (r) return 2000 + r;
-  GroupArgs ga{nullptr, nullptr, 3, per, splits, static_cast<long long>(M) * N, nullptr, nullptr, nullptr};
-  if ((r = dispatch(a_mn, b_mn, EPI_F32, ta, tb, scratch, M, N, K, N, 1.f, ga, err, sm_count(), stream))) return r;
-  const long long total = static_cast<long long>(M) * N;
-  split_sum_kernel<<<static_cast<unsigned>((total / 4 + 255) / 256), 256, 0, stream>>>(scratch, D, M, N, ldd, splits, alpha, epi, err);
-  return static_cast<int>(cudaGetLastError());
 }
 
 // Grouped rows (mixture-of-experts forward and input gradient):
@@ -505,29 +420,8 @@ extern "C" int dewb_gmm_bf16(const void* A, const void* B, void* D, const int* t
   if (!b_mn) r = make_tmap_2d(&tb, B, static_cast<uint64_t>(groups) * N, K, ldb, BN, BK, 2, true);
   else       r = make_tmap_2d(&tb, B, static_cast<uint64_t>(groups) * K, N, ldb, BK, 64, 2, true);
   if (r) return 2000 + r;
-  GroupArgs ga{tile_group, nullptr, 1, b_mn ? K : N, groups, 0, nullptr, nullptr, nullptr};
+  GroupArgs ga{tile_group, 1, b_mn ? K : N, nullptr, nullptr, nullptr};
   return dispatch(0, b_mn, epi, ta, tb, D, M, N, K, ldd, alpha, ga, err, sm_count(), stream);
-}
-
-// Grouped reduction (mixture-of-experts weight gradient): for every group g,
-//   D_g[M, N] (+)= A[rows of g, M]^T * B[rows of g, N]   with A stored [R, M] and B stored [R, N] (R = all rows),
-//   rows of g = [group_offsets[g], group_offsets[g + 1]) (multiples of 64; padding rows are zero)
-//   D stacks the groups: D_g = D + g * d_group_stride, row stride ldd.
-extern "C" int dewb_tgmm_bf16(const void* A, const void* B, void* D, const int* group_offsets, int R, int M, int N,
-                              int groups, long long lda, long long ldb, long long ldd, long long d_group_stride, int epi,
-                              float alpha, int* err, void* stream_ptr) {
-  using namespace dewb;
-  using namespace dewb::gemm;
-  if (R <= 0 || M <= 0 || N <= 0 || groups <= 0) return 0;
-  if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return -3;
-  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
-  CUtensorMap ta, tb;
-  int r = make_tmap_2d(&ta, A, R, M, lda, BK, 64, 2, true);
-  if (r) return 1000 + r;
-  r = make_tmap_2d(&tb, B, R, N, ldb, BK, 64, 2, true);
-  if (r) return 2000 + r;
-  GroupArgs ga{nullptr, group_offsets, 2, 0, groups, d_group_stride, nullptr, nullptr, nullptr};
-  return dispatch(1, 1, epi, ta, tb, D, M, N, R, ldd, alpha, ga, err, sm_count(), stream);
 }
 
 // Row-wise scaled fp8 (e4m3) GEMM, dense or grouped rows: D[M,N] (bf16) = (A_q * a_scale[row]) * (B_q * b_scale[row of B])^T.
@@ -546,6 +440,6 @@ extern "C" int dewb_gemm_fp8(const void* A, const void* B, void* D, const float*
   if (r) return 1000 + r;
   r = make_tmap_2d(&tb, B, static_cast<uint64_t>(groups) * N, K, ldb, BN, 2 * BK, 1, true);
   if (r) return 2000 + r;
-  GroupArgs ga{tile_group, nullptr, tile_group != nullptr ? 1 : 0, N, groups, 0, a_scale, b_scale, nullptr};
+  GroupArgs ga{tile_group, tile_group != nullptr ? 1 : 0, N, a_scale, b_scale, nullptr};
   return launch_fp8(ta, tb, D, M, N, K, ldd, 1.f, ga, err, sm_count(), stream);
 }

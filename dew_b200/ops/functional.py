@@ -154,17 +154,18 @@ _SKINNY_PDL = int(os.environ.get("DEWB_SKINNY_PDL", "1"))
 
 
 def reduction_splits(M: int, N: int, K: int, sms: int = 148) -> int:
-    """Parts the reduction of a product with few output tiles is cut into: the fewest that come close to the shortest last wave of (tile, part) pairs, each at least
-    1024 long (a part costs its fp32 partial product, written and read once).  1: no cut - one wave or more of tiles, a short reduction, or nothing to gain."""
-    tiles = -(-M // 128) * -(-N // 256)
-    if tiles * 2 > sms:
+    """Parts the reduction of a product with few output tiles is cut into: the fewest that come close to the shortest last wave of (256 x 256 tile, part) items over
+    the pairs of SMs, each at least 1024 long (a part costs its fp32 partial product, written and read once).  1: no cut - half a wave or more of a lone CTA's tiles
+    of 128 x 256, a short reduction, or nothing to gain."""
+    if -(-M // 128) * -(-N // 256) * 2 > sms:
         return 1
-    best, least = 1, 1.0
+    tiles, pairs = -(-M // 256) * -(-N // 256), sms // 2
+    best, least = 1, float(-(-tiles // pairs))
     for s in range(2, min(8, K // 1024) + 1):
         per = -(-K // s // 64) * 64
         if (s - 1) * per >= K:
             continue
-        wave = -(-tiles * s // sms) / s
+        wave = -(-tiles * s // pairs) / s
         if wave < 0.85 * least:
             best, least = s, wave
     return best

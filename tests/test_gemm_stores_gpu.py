@@ -43,3 +43,29 @@ def test_block_scaled_rows_of_any_alignment(N):
     # (the tensor cores keep fewer bits of a sum than fp32 where operands are 8 bits wide: 2^-13 of the largest term is beyond what they drop)
     bound = 256 * 2.0 ** -22 * (da.abs() @ db.abs().T) + 2.0 ** -8 * exact.abs()
     assert bool(((got.double() - exact).abs() <= bound).all())
+
+
+# groups of no rows (first, among others, last), of one reduction step and of several; outputs of one pair's tile and past it, on both sides of half a tile
+@pytest.mark.parametrize("dtype,acc", [(torch.bfloat16, False), (torch.bfloat16, True), (torch.float32, False), (torch.float32, True)])
+@pytest.mark.parametrize("M,N", [(64, 72), (128, 256), (136, 264), (384, 520)])
+def test_grouped_reductions(M, N, dtype, acc):
+    from dew_b200.ops import grouped
+    rows = [0, 128, 64, 0, 0, 704, 128, 0]
+    offsets = [sum(rows[:i]) for i in range(len(rows) + 1)]
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    dy, x = (torch.randn(offsets[-1] + 128, n, generator=g, device=DEV).bfloat16() for n in (M, N))      # rows behind the last group belong to none
+    out = torch.randn(len(rows), M, N, generator=g, device=DEV).to(dtype)
+    held = out.double()
+
+    class Layout:
+        pass
+    layout = Layout()
+    layout.offsets = torch.tensor(offsets, dtype=torch.int32, device=DEV)
+    grouped.tgmm(dy, x, layout, len(rows), out=out, accumulate=acc)
+    L.check_status()
+    for i, (a, b) in enumerate(zip(offsets, offsets[1:])):
+        exact = dy[a:b].double().T @ x[a:b].double() + (held[i] if acc else 0)
+        size = dy[a:b].double().abs().T @ x[a:b].double().abs()
+        # fp32 sums of (b - a) exact products in some order, and one rounding of the result
+        bound = (b - a) * 2.0 ** -24 * size + (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -23) * exact.abs()
+        assert bool(((out[i].double() - exact).abs() <= bound).all()), i

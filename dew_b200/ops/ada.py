@@ -46,7 +46,7 @@ def _forward(x, branch, gate, shift, scale, eps):
     h = x if branch is None else torch.empty_like(x)
     y = torch.empty_like(x) if norm else None
     stats = torch.empty(B * n, 2, dtype=torch.float32, device=x.device) if norm else None
-    at = lambda t: 0 if t is None else t.data_ptr()
+    at = L.at
     L.check(L.load().dewb_ada_fwd(at(x), at(branch), at(shift), at(scale), at(gate), (gate if shift is None else shift).stride(0), 0 if branch is None else at(h), at(y), at(stats),
                                   B * n, n, d, eps, L.stream()), "ada_fwd")
     L.count_launches()
@@ -94,15 +94,16 @@ class _Ada(torch.autograd.Function):
         dy, dh = (None if t is None else _rows(t.to(h.dtype)) for t in (dy, dh))
         B, n, d = h.shape
         lib = L.load()
-        slab = lib.dewb_ada_slab(c_int(B), c_int(n))
+        slab = lib.dewb_ada_slab(B, n)
         sets = 2 * norm + (branch is not None)
         L.ensure_device(h)
         part = torch.empty(B, -(-n // slab), sets, d, dtype=torch.float32, device=h.device)
         dmod = torch.empty(B, sets, d, dtype=h.dtype, device=h.device)
         dx = torch.empty_like(h) if norm else dh
         dbranch = None if branch is None else torch.empty_like(h)
-        L.check(lib.dewb_ada_bwd(L.ptr(dy), L.ptr(dh), L.ptr(h), L.ptr(branch), L.ptr(scale), L.ptr(gate), c_ll((gate if scale is None else scale).stride(0)), L.ptr(stats), L.ptr(dx),
-                                 L.ptr(dbranch), L.ptr(part), L.ptr(dmod), c_int(B), c_int(n), c_int(d), c_int(slab), L.stream_ptr()), "ada_bwd")
+        at = L.at
+        L.check(lib.dewb_ada_bwd(at(dy), at(dh), at(h), at(branch), at(scale), at(gate), (gate if scale is None else scale).stride(0), at(stats), at(dx), at(dbranch), at(part),
+                                 at(dmod), B, n, d, slab, L.stream()), "ada_bwd")
         L.count_launches(2)
         return dx, dbranch, None if branch is None else dmod[:, 2 * norm], dmod[:, 0] if norm else None, dmod[:, 1] if norm else None, None
 

@@ -208,6 +208,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     if fresh:
         out = torch.empty((M, N), dtype=out_dtype, device=a.device)
         accumulate = False
+    if kernel is None and cell is None and not _TUNE and not _GEMM.forced_by_environment() and _tensor_core_operands(a, b, out):
+        # both tensor-core kernels take these operands and the size alone says which: nothing about the call needs looking up.  The pair kernel is 5-15 % faster on
+        # the layer shapes; the single-CTA kernel keeps the very wide head.
+        paired = tiles >= 148 and LARGE_GEMM == "sm100_pair" and N <= 32768 and _pair_built()
+        which = "sm100_pair" if paired else "sm100_tcgen05"
+        _GEMM._record(which, {}, which if tiles >= 148 else None, None)
+        return _gemm_tensor_cores(which, a, b, out, M, N, K, a_mn, b_mn, accumulate, alpha, max_ctas, bias)
     case = dict(dtype=a.dtype if a.dtype == b.dtype else None, lda=a.stride(0), ldb=b.stride(0), ldd=out.stride(0),
                 aligned=(a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0),
                 inner_contig=(a.stride(1) == 1 and b.stride(1) == 1 and out.stride(1) == 1), M=M, N=N, K=K, plain=plain, k_major=plain and fresh,
@@ -238,34 +245,37 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         L.check(rc, which)
         L.count_launches()
         return out
-    epi = {(torch.bfloat16, False): 0, (torch.float32, False): 1, (torch.float32, True): 2,
-           (torch.bfloat16, True): 3}[(out.dtype, bool(accumulate))]
-    lib = L.load()
+    return _gemm_tensor_cores(which, a, b, out, M, N, K, a_mn, b_mn, accumulate, alpha, max_ctas, bias)
+
+
+def _tensor_core_operands(a, b, out) -> bool:
+    """What the tensor-core kernels require of their operands (the requirements of ``_GEMM`` in one look)."""
+    (lda, ia), (ldb, ib), (ldd, io) = a.stride(), b.stride(), out.stride()
+    return (a.dtype == b.dtype == torch.bfloat16 and out.dtype in (torch.bfloat16, torch.float32) and ia == ib == io == 1 and (lda | ldb | ldd) % 8 == 0
+            and (a.data_ptr() | b.data_ptr() | out.data_ptr()) % 16 == 0)
+
+
+def _gemm_tensor_cores(which, a, b, out, M, N, K, a_mn, b_mn, accumulate, alpha, max_ctas, bias):
+    epi = {(torch.bfloat16, False): 0, (torch.float32, False): 1, (torch.float32, True): 2, (torch.bfloat16, True): 3}[(out.dtype, bool(accumulate))]
+    lib, at = L.load(), L.at
+    lda, ldb, ldd = a.stride(0), b.stride(0), out.stride(0)
+    launches = 1
     if bias is not None:
         bb = bias.to(torch.bfloat16).contiguous()                 # referenced until the launch is enqueued
         fn = lib.dewb_gemm_pair_bf16_bias if which == "sm100_pair" else lib.dewb_gemm_bf16_bias
-        rc = fn(L.ptr(a), L.ptr(b), L.ptr(out), L.ptr(bb), c_int(M), c_int(N), c_int(K), c_ll(a.stride(0)),
-                c_ll(b.stride(0)), c_ll(out.stride(0)), c_int(int(a_mn)), c_int(int(b_mn)), c_int(epi),
-                c_float(alpha), L.ptr(L.status(a.device)), c_int(max_ctas), L.stream_ptr())
-        L.check(rc, which)
-        L.count_launches()
-        return out
-    if which == "sm100_tcgen05" and max_ctas == 0:
-        splits = reduction_splits(M, N, K)
-        if splits > 1 and N % 4 == 0 and hasattr(lib, "dewb_gemm_bf16_split"):
+        rc = fn(at(a), at(b), at(out), at(bb), M, N, K, lda, ldb, ldd, int(a_mn), int(b_mn), epi, alpha, at(L.status(a.device)), max_ctas, L.stream())
+    else:
+        splits = reduction_splits(M, N, K) if which == "sm100_tcgen05" and max_ctas == 0 and N % 4 == 0 and hasattr(lib, "dewb_gemm_bf16_split") else 1
+        if splits > 1:
             scratch = torch.empty(splits, M, N, dtype=torch.float32, device=a.device)
-            rc = lib.dewb_gemm_bf16_split(L.ptr(a), L.ptr(b), L.ptr(out), L.ptr(scratch), c_int(M), c_int(N), c_int(K), c_int(splits), c_int(-(-K // splits // 64) * 64),
-                                          c_ll(a.stride(0)), c_ll(b.stride(0)), c_ll(out.stride(0)), c_int(int(a_mn)), c_int(int(b_mn)), c_int(epi), c_float(alpha),
-                                          L.ptr(L.status(a.device)), L.stream_ptr())
-            L.check(rc, which)
-            L.count_launches(2)
-            return out
-    fn = lib.dewb_gemm_pair_bf16 if which == "sm100_pair" else lib.dewb_gemm_bf16
-    rc = fn(L.ptr(a), L.ptr(b), L.ptr(out), c_int(M), c_int(N), c_int(K), c_ll(a.stride(0)),
-            c_ll(b.stride(0)), c_ll(out.stride(0)), c_int(int(a_mn)), c_int(int(b_mn)), c_int(epi),
-            c_float(alpha), L.ptr(L.status(a.device)), c_int(max_ctas), L.stream_ptr())
+            rc = lib.dewb_gemm_bf16_split(at(a), at(b), at(out), at(scratch), M, N, K, splits, -(-K // splits // 64) * 64, lda, ldb, ldd, int(a_mn), int(b_mn), epi, alpha,
+                                          at(L.status(a.device)), L.stream())
+            launches = 2
+        else:
+            fn = lib.dewb_gemm_pair_bf16 if which == "sm100_pair" else lib.dewb_gemm_bf16
+            rc = fn(at(a), at(b), at(out), M, N, K, lda, ldb, ldd, int(a_mn), int(b_mn), epi, alpha, at(L.status(a.device)), max_ctas, L.stream())
     L.check(rc, which)
-    L.count_launches()
+    L.count_launches(launches)
     return out
 
 
@@ -323,9 +333,9 @@ def _column_sums(dy):
             and hasattr(L.load(), "dewb_colsum_bf16")):
         return dy.sum(0)
     lib = L.load()
-    part = torch.empty(lib.dewb_colsum_slabs(c_ll(rows), c_int(d)), d, dtype=torch.float32, device=dy.device)
+    part = torch.empty(lib.dewb_colsum_slabs(rows, d), d, dtype=torch.float32, device=dy.device)
     out = torch.empty(d, dtype=torch.bfloat16, device=dy.device)
-    L.check(lib.dewb_colsum_bf16(L.ptr(dy), L.ptr(part), L.ptr(out), c_ll(rows), c_int(d), c_ll(dy.stride(0)), L.stream_ptr()), "colsum_bf16")
+    L.check(lib.dewb_colsum_bf16(dy.data_ptr(), part.data_ptr(), out.data_ptr(), rows, d, dy.stride(0), L.stream_ptr()), "colsum_bf16")
     L.count_launches(2)
     return out
 

@@ -69,6 +69,15 @@ _SIGNATURES = {
     "dewb_ce_rows": "pppp" + "lil" + "ifffi" + "p",
     "dewb_flash_fwd_var": "ppppp" + "iiiiii" + "l" * 12 + "f" + "iiiif" + "ppppp" + "pp",
     "dewb_flash_bwd_var": "pppppppppp" + "iiiiii" + "p" + "f" + "ii" + "f" + "pppp",
+    "dewb_gemm_bf16": "ppp" + "iii" + "lll" + "iii" + "f" + "pip",
+    "dewb_gemm_pair_bf16": "ppp" + "iii" + "lll" + "iii" + "f" + "pip",
+    "dewb_gemm_bf16_bias": "pppp" + "iii" + "lll" + "iii" + "f" + "pip",
+    "dewb_gemm_pair_bf16_bias": "pppp" + "iii" + "lll" + "iii" + "f" + "pip",
+    "dewb_gemm_bf16_split": "pppp" + "iiiii" + "lll" + "iii" + "f" + "pp",
+    "dewb_colsum_slabs": "li",
+    "dewb_colsum_bf16": "ppp" + "lil" + "p",
+    "dewb_ada_slab": "ii",
+    "dewb_ada_bwd": "pppppp" + "l" + "ppppp" + "iiii" + "p",
     "dewb_rope_append": "pppp" + "iiiii" + "ppp" + "ii" + "p",
     "dewb_paged_decode_persist": "ppp" + "l" + "pppppppp" + "iiiiiii" + "f" + "iii" + "f" + "pp" + "l" + "i" + "pp",
 }

@@ -211,7 +211,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     if kernel is None and cell is None and not _TUNE and not _GEMM.forced_by_environment() and _tensor_core_operands(a, b, out):
         # both tensor-core kernels take these operands and the size alone says which: nothing about the call needs looking up.  The pair kernel is 5-15 % faster on
         # the layer shapes; the single-CTA kernel keeps the very wide head.
-        paired = tiles >= 148 and LARGE_GEMM == "sm100_pair" and N <= 32768 and _pair_built()
+        # Below 148 tiles the same where the reduction is long and not split: the pair's smaller operand traffic shows from some 2048 on (2048 x 2048 over 512 14.4 us
+        # either way, over 2048 24.6 and 22.5, over 8192 64 and 55, over 32768 200 and 176; 1152 x 2304 over 768 14.4 and 16.4).
+        paired = LARGE_GEMM == "sm100_pair" and N <= 32768 and _pair_built() and (
+            tiles >= 148 or K >= 2048 and max_ctas == 0 and (N % 4 != 0 or reduction_splits(M, N, K) == 1))
         which = "sm100_pair" if paired else "sm100_tcgen05"
         _GEMM._record(which, {}, which if tiles >= 148 else None, None)
         return _gemm_tensor_cores(which, a, b, out, M, N, K, a_mn, b_mn, accumulate, alpha, max_ctas, bias)

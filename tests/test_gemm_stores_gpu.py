@@ -69,3 +69,13 @@ def test_grouped_reductions(M, N, dtype, acc):
         # fp32 sums of (b - a) exact products in some order, and one rounding of the result
         bound = (b - a) * 2.0 ** -24 * size + (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -23) * exact.abs()
         assert bool(((out[i].double() - exact).abs() <= bound).all()), i
+
+
+# less than a wave of tiles: reductions on both sides of the line where pairs take them, outputs within one tile's rows, past them, and not of whole pieces
+@pytest.mark.parametrize("M,N,K", [(2048, 2048, 2040), (2048, 2048, 2048), (1096, 2312, 2056), (200, 16392, 4096), (128, 16384, 2304), (130, 9992, 2304)])
+def test_pairs_below_a_wave(M, N, K):
+    g = torch.Generator(device=DEV).manual_seed(K)
+    A, B = (torch.randn(n, K, generator=g, device=DEV).bfloat16() for n in (M, N))
+    got = ops.gemm(A, B, out_dtype=torch.float32)
+    L.check_status()
+    assert torch.equal(got, ops.gemm(A, B, out_dtype=torch.float32, kernel="sm100_tcgen05", max_ctas=148))       # either kernel's sums are in the same order

@@ -782,13 +782,14 @@ static int run_states(const Call& k, const Walk<Out>& forward, const Walk<Out>* 
 // A quarter of the columns a CTA while that leaves every SM no more than two of them, else half (two more resident CTAs hide what a step's chain waits for, and a
 // step of half the columns scales and splits half as often as two of a quarter).  In fp32, all of them where that alone makes one wave of two CTAs an SM: halves would
 // make two waves, each of which scales and splits what the other does.  Both walks of 2 x 4096 tokens and 64 heads (256 CTAs): 278 us by quarters, 243 by halves, 226
-// whole; of 4 x 2048 and 32 heads 141, 126, 117; but one walk of 128 CTAs, less than a CTA an SM, 121, 88, 103.
+// whole; of 4 x 2048 and 32 heads 141, 126, 117; but one walk of 128 CTAs, less than a CTA an SM, 121, 88, 103.  Where few SMs have two the others wait for them:
+// 4096 tokens of 80 heads (160 CTAs) 218 us by halves and 223 whole, 2048 of 96 (192) 123 and 115; hence the line at five quarters of the SMs.
 template <int TERMS, typename Out>
 static int walk(const Call& k, const Walk<Out>& forward, const Walk<Out>* reverse, cudaStream_t stream) {
   const int rows = k.B * k.H * (reverse == nullptr ? 1 : 2);
   if (rows * 4 <= 2 * SMS) return run_states<4, TERMS, Out>(k, forward, reverse, stream);
   if constexpr (TERMS == 3)
-    if (rows > SMS && rows <= 2 * SMS) return run_states<16, TERMS, Out>(k, forward, reverse, stream);
+    if (rows * 4 > 5 * SMS && rows <= 2 * SMS) return run_states<16, TERMS, Out>(k, forward, reverse, stream);
   return run_states<8, TERMS, Out>(k, forward, reverse, stream);
 }
 

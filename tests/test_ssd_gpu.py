@@ -48,8 +48,8 @@ def test_ssd_forward_and_gradients(B, T, H, G, with_state):
         assert rel_err(a, b) < limit[n], (n, rel_err(a, b))
 
 
-# either side of the lines between a CTA's quarter, half and all of a state's columns: 148 and 296 rows of one walk, the same of both
-@pytest.mark.parametrize("B,H", [(1, 74), (1, 75), (1, 148), (1, 149), (2, 148), (3, 99)])
+# either side of the lines between a CTA's quarter, half and all of a state's columns: 74, 185 and 296 rows of one walk, the same of both
+@pytest.mark.parametrize("B,H", [(1, 37), (1, 74), (1, 92), (1, 93), (1, 185), (1, 186), (2, 148), (3, 99)])
 def test_ssd_walks_by_quarters_halves_and_whole_states(B, H):
     test_ssd_forward_and_gradients(B, 130, H, 1, True)
 

@@ -363,6 +363,15 @@ __device__ __forceinline__ void ld_global_32(const void* p, uint32_t* w) {
   asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "l"(p) : "memory");
 }
+// 32 bytes to a 16-byte boundary.
+__device__ __forceinline__ void st_global_32_any(void* p, const uint32_t* w) {
+  if ((reinterpret_cast<uintptr_t>(p) & 31) == 0) {
+    st_global_32(p, w);
+  } else {
+    reinterpret_cast<uint4*>(p)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    reinterpret_cast<uint4*>(p)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+  }
+}
 // 32 fp32 values times `by` to (ADD: added to what is at) `out`, as bf16 or fp32; `out` on a 16-byte boundary.
 template <bool ADD>
 __device__ __forceinline__ void store_row_32(__nv_bfloat16* out, const uint32_t (&r)[32], float by) {

@@ -140,13 +140,11 @@ __device__ __forceinline__ void write_quarter(uint32_t addr, bool any, float sca
   }
   if (real) {
 #pragma unroll
-    for (int q = 0; q < D / 32; ++q) {
-      uint4 pk;
-      pk.x = pack_bf16(__uint_as_float(v[q * 8 + 0]) * scale, __uint_as_float(v[q * 8 + 1]) * scale);
-      pk.y = pack_bf16(__uint_as_float(v[q * 8 + 2]) * scale, __uint_as_float(v[q * 8 + 3]) * scale);
-      pk.z = pack_bf16(__uint_as_float(v[q * 8 + 4]) * scale, __uint_as_float(v[q * 8 + 5]) * scale);
-      pk.w = pack_bf16(__uint_as_float(v[q * 8 + 6]) * scale, __uint_as_float(v[q * 8 + 7]) * scale);
-      reinterpret_cast<uint4*>(to)[q] = pk;
+    for (int q = 0; q < D / 64; ++q) {
+      uint32_t w[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) w[i] = pack_bf16(__uint_as_float(v[q * 16 + 2 * i]) * scale, __uint_as_float(v[q * 16 + 2 * i + 1]) * scale);
+      st_global_32_any(to + q * 16, w);
     }
   }
   __syncwarp();

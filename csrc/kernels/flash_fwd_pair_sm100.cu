@@ -503,18 +503,7 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
 #pragma unroll
           for (int x = 0; x < 32; ++x) v[x] = 0;
         }
-        if (row < S) {
-          uint4* o4 = reinterpret_cast<uint4*>(orow + c * 32);
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            uint4 pk;
-            pk.x = pack_bf16(__uint_as_float(v[q * 8]) * inv, __uint_as_float(v[q * 8 + 1]) * inv);
-            pk.y = pack_bf16(__uint_as_float(v[q * 8 + 2]) * inv, __uint_as_float(v[q * 8 + 3]) * inv);
-            pk.z = pack_bf16(__uint_as_float(v[q * 8 + 4]) * inv, __uint_as_float(v[q * 8 + 5]) * inv);
-            pk.w = pack_bf16(__uint_as_float(v[q * 8 + 6]) * inv, __uint_as_float(v[q * 8 + 7]) * inv);
-            o4[q] = pk;
-          }
-        }
+        if (row < S) store_row_32<false>(orow + c * 32, v, inv);
         __syncwarp();
       }
       if (row < S && lse != nullptr) {

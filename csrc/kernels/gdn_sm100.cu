@@ -171,31 +171,31 @@ gdn_prepare_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
       tmem_ld_32x32b_x32(from, va);
       tmem_ld_wait();
       // P row: scale * (q_i . k_j) * e^{g_i - g_j} for j <= i;  A row: beta_i * (k_i . k_j) * e^{g_i - g_j} for j < i
-      uint4* prow = reinterpret_cast<uint4*>(P + row * CH + j0);
 #pragma unroll
-      for (int j8 = 0; j8 < 4; ++j8) {
-        float p[8];
+      for (int j16 = 0; j16 < 2; ++j16) {
+        float p[16];
 #pragma unroll
-        for (int jj = 0; jj < 8; ++jj) {
-          const int at = j8 * 8 + jj, j = j0 + at;
+        for (int jj = 0; jj < 16; ++jj) {
+          const int at = j16 * 16 + jj, j = j0 + at;
           const float decay = j <= il ? __expf(gi - tail->g[c * 64 + j]) : 0.f;
           p[jj] = j <= il ? scale * __uint_as_float(vp[at]) * decay : 0.f;
           a[at] = j < il ? bi * __uint_as_float(va[at]) * decay : 0.f;
         }
-        uint4 pk;
-        pk.x = pack_bf16(p[0], p[1]); pk.y = pack_bf16(p[2], p[3]); pk.z = pack_bf16(p[4], p[5]); pk.w = pack_bf16(p[6], p[7]);
-        prow[j8] = pk;
+        uint32_t w[8];
+#pragma unroll
+        for (int x = 0; x < 8; ++x) w[x] = pack_bf16(p[2 * x], p[2 * x + 1]);
+        st_global_32_any(P + row * CH + j0 + j16 * 16, w);
       }
       if (Qg != nullptr) {
         const float m = scale * tail->eg[i];
-        uint4* qrow = reinterpret_cast<uint4*>(Qg + row * HD + part * 64);
 #pragma unroll
-        for (int c16 = 0; c16 < 8; ++c16) {
-          const uint4 in = *reinterpret_cast<const uint4*>(sQ + part * (PT * 128) + swz(i, c16));
-          uint4 o;
-          o.x = pack_bf16(bf16_lo(in.x) * m, bf16_hi(in.x) * m); o.y = pack_bf16(bf16_lo(in.y) * m, bf16_hi(in.y) * m);
-          o.z = pack_bf16(bf16_lo(in.z) * m, bf16_hi(in.z) * m); o.w = pack_bf16(bf16_lo(in.w) * m, bf16_hi(in.w) * m);
-          qrow[c16] = o;
+        for (int c32 = 0; c32 < 4; ++c32) {
+          const uint4 a = *reinterpret_cast<const uint4*>(sQ + part * (PT * 128) + swz(i, 2 * c32)), b = *reinterpret_cast<const uint4*>(sQ + part * (PT * 128) + swz(i, 2 * c32 + 1));
+          const uint32_t in[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+          uint32_t w[8];
+#pragma unroll
+          for (int x = 0; x < 8; ++x) w[x] = pack_bf16(bf16_lo(in[x]) * m, bf16_hi(in[x]) * m);
+          st_global_32_any(Qg + row * HD + part * 64 + c32 * 16, w);
         }
       }
     }

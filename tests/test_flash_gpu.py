@@ -79,3 +79,22 @@ def test_flash_backward_tiles(B, S, Hq, Hkv, D, causal):
     for a, b, w in zip(got, again, want):
         assert torch.equal(a, b)
         assert rel_err(a, w) < 2.0 ** -7
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("gap", [0, 8, 16, 24])
+def test_flash_gradients_into_rows_of_any_alignment(D, gap):
+    """Rows that start on a 16-byte boundary only, all of them or every second one, get the same bits, and what lies between them is left alone."""
+    from dew_b200.ops.flash import flash_bwd, flash_fwd
+    g = torch.Generator(device=DEV).manual_seed(gap)
+    B, S, Hq, Hkv = 1, 192, 4, 2
+    q, k, v, do = (torch.randn(B, S, h, D, generator=g, device=DEV).bfloat16() for h in (Hq, Hkv, Hkv, Hq))
+    out, lse = flash_fwd(q, k, v, True, D ** -0.5)
+    want = flash_bwd(do, q, k, v, out, lse, True, D ** -0.5)
+    wide = [torch.full((B, S, h, D + gap), 7.0, device=DEV, dtype=torch.bfloat16) for h in (Hq, Hkv, Hkv)]
+    first = gap // 2 // 8 * 8
+    flash_bwd(do, q, k, v, out, lse, True, D ** -0.5, grads=[w[..., first:first + D] for w in wide])
+    L.check_status()
+    for a, w in zip(want, wide):
+        assert torch.equal(w[..., first:first + D], a)
+        assert bool((w[..., :first] == 7).all()) and bool((w[..., first + D:] == 7).all())

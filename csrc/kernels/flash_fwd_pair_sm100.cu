@@ -46,7 +46,7 @@ struct Cfg {
   static constexpr int KV_TILE = BN * D * 2;
   static constexpr int QSTAGES = D == 128 ? 1 : 2;   // pairs of query tiles
   static constexpr int RING = D == 128 ? 5 : 8;      // keys and values alike
-  static constexpr int SMEM = QSTAGES * 2 * Q_TILE + RING * KV_TILE + 1024;
+  static constexpr int SMEM = QSTAGES * 2 * Q_TILE + RING * KV_TILE + 2048;
   static constexpr int TM_S = 0, TM_O = 256, TM_COLS = 512;      // 128 columns a tile each
 };
 
@@ -57,14 +57,16 @@ struct Bars {
   uint32_t tmem_base;
   int abort_flag;
   int poisoned;
+  float2 half[BM];                                   // SPLIT: maximum and sum of tile 1's rows
 };
-static_assert(sizeof(Bars) <= 1024 && Cfg<128>::SMEM <= 232448 && Cfg<64>::SMEM <= 232448, "over the 227 KB a CTA may use");
+static_assert(sizeof(Bars) <= 2048 && Cfg<128>::SMEM <= 232448 && Cfg<64>::SMEM <= 232448, "over the 227 KB a CTA may use");
 
 // What a launch is about, and how its query tiles are paired.
-enum : int { SINGLE = 0, HEADS = 1, ROWS = 2 };
+enum : int { SINGLE = 0, HEADS = 1, ROWS = 2, SPLIT = 3 };
 struct Shape {
   int B, S, T, Hq, Hkv;
-  int pairing;                     // HEADS: the same rows of two neighbouring query heads of a key head; ROWS: two neighbouring tiles of a head; SINGLE: tile 1 empty
+  int pairing;                     // HEADS: the same rows of two neighbouring query heads of a key head; ROWS: two neighbouring tiles of a head; SINGLE: tile 1 empty;
+                                   // SPLIT: both the same rows, tile 0 against the first, third, ... of their key tiles, tile 1 against the others (one item a CTA)
   int items;
 };
 
@@ -75,7 +77,7 @@ struct Item {
   int q0[2], h[2], lo[2], hi[2], keep[2];
 };
 
-template <bool CAUSAL, bool VAR>
+template <bool CAUSAL, bool VAR, bool HALVES>
 __device__ __forceinline__ Item make_item(int index, const Shape& s, const Variant& var, int lane) {
   Item w;
   const int heads = s.pairing == HEADS ? s.Hq / 2 : s.Hq;
@@ -101,6 +103,11 @@ __device__ __forceinline__ Item make_item(int index, const Shape& s, const Varia
     if (qt >= tiles || (s.pairing == SINGLE && i == 1)) w.q0[i] = s.S;
     int lo = 0;
     if (hi > 0) lo = VAR ? attn::first_key_tile_of_warp(var, w.b, w.q0[i], s.S, s.T, BN, hi, lane) : var.first != nullptr ? min(var.first[qt], hi) : 0;
+    if constexpr (HALVES) {
+      const int n = max(hi - lo, 0);
+      hi = i == 0 ? (n > 0 ? lo + ((n - 1) & ~1) + 1 : 0) : n > 1 ? lo + (n & ~1) : 0;
+      lo += i;
+    }
     w.keep[i] = VAR ? min(lo, (var.keep + BN - 1) / BN) : 0;
     if (lo >= hi) {                                  // (kept tiles are before lo: a tile whose window is empty has none to add)
       hi = w.keep[i] > 0 ? min(w.keep[i], hi) : 0;
@@ -135,7 +142,7 @@ __device__ __forceinline__ int item_index(int turn) {
   return turn * g + ((turn & 1) ? g - 1 - c : c);
 }
 
-template <int D, bool CAUSAL, bool VAR, bool SIG>
+template <int D, bool CAUSAL, bool VAR, bool SIG, bool HALVES>
 __global__ void __launch_bounds__(THREADS, 1)
 flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
                       __nv_bfloat16* __restrict__ out, float* __restrict__ lse, Shape shape, long long o_stride_b, long long o_stride_s, long long o_stride_h,
@@ -187,7 +194,7 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
       const int index = item_index(turn);
       if (turn * static_cast<int>(gridDim.x) >= shape.items) break;
       if (index >= shape.items) continue;
-      const Item w = make_item<CAUSAL, VAR>(index, shape, var, lane);
+      const Item w = make_item<CAUSAL, VAR, HALVES>(index, shape, var, lane);
       if (empty(w)) continue;
       const int qs = items % C::QSTAGES;
       if (!mbar_wait_warp(&bars->q_empty[qs], ((items / C::QSTAGES) & 1) ^ 1, abort_flag)) { if (lane == 0) atomicCAS(err, 0, ERR_WAIT_EMPTY); break; }
@@ -212,6 +219,13 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
           for (int t = 0; t < C::SUB; ++t) tma_load_4d(sQ + (qs * 2 + i) * C::Q_TILE + t * (BM * 128), &tq, &bars->q_full[qs], t * 64, w.h[i], w.q0[i], w.b);
       }
       __syncwarp();
+      if constexpr (HALVES) {
+        // in the order in which the issuer takes them
+        const int end = w.to;
+        ok = fetch(&tk, w.from * BN) && (w.from + 1 >= end || fetch(&tk, (w.from + 1) * BN));
+        for (int j = w.from; ok && j < end; ++j) ok = fetch(&tv, j * BN) && (j + 2 >= end || fetch(&tk, (j + 2) * BN));
+        continue;
+      }
       const int end = walk_last(w);
       for (int j = walk_begin(w); ok; j = walk_next(w, j)) {
         ok = fetch(&tk, j * BN) && fetch(&tv, j * BN);
@@ -232,7 +246,7 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
         if (turn * static_cast<int>(gridDim.x) >= shape.items) return false;
         const int index = item_index(turn);
         if (index >= shape.items) continue;
-        w = make_item<CAUSAL, VAR>(index, shape, var, lane);
+        w = make_item<CAUSAL, VAR, HALVES>(index, shape, var, lane);
         if (!empty(w)) { ++turn; ++items; return true; }
       }
     };
@@ -262,6 +276,41 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
     };
     bool more = next_item();
     int j = 0, qs = 0, k_at = 0, v_at = 0;
+    auto product = [&](int i, bool fresh, bool last) -> bool {      // P V of the tile, with the values in slot v_at
+      if (!mbar_wait_warp(&bars->p_full[i], p_phase[i], abort_flag)) { if (lane == 0) atomicCAS(err, 0, ERR_WAIT_OTHER); return false; }
+      p_phase[i] ^= 1;
+      tc_fence_after();
+      const uint32_t va = smem_u32(sKV + v_at * C::KV_TILE), tp = tmem + C::TM_S + i * 128, to = tmem + C::TM_O + i * 128;
+      if (elect_one()) {
+#pragma unroll
+        for (int kk = 0; kk < BN / 16; ++kk)             // 16 keys of P = 8 packed 32-bit columns
+          umma_bf16_ts(to, tp + kk * 8, make_sdesc_sw128(va + kk * 2048, BN * 128, 1024), idesc_pv, kk > 0 || !fresh ? 1u : 0u);
+        if (last) umma_commit(&bars->o_full[i]);
+      }
+      __syncwarp();
+      return true;
+    };
+    if constexpr (HALVES) {
+      // One item: the tiles' scores are in front of each other's products, as with two tiles of rows.
+      const int end = w.to;
+      ok = more && await_queries(0);
+      for (int i = 0; ok && i < 2 && w.from + i < end; ++i) {
+        ok = take(k_at);
+        tc_fence_after();
+        if (ok) { scores(i, 0, k_at); commit(&bars->kv_empty[k_at]); }
+      }
+      for (int at = w.from; ok && at < end; ++at) {
+        const int i = (at - w.from) & 1;
+        ok = take(v_at) && product(i, at - w.from < 2, at + 2 >= end);
+        if (!ok) break;
+        commit(&bars->kv_empty[v_at]);
+        if (at + 2 >= end) continue;
+        ok = take(k_at);
+        tc_fence_after();
+        if (ok) { scores(i, 0, k_at); commit(&bars->kv_empty[k_at]); }
+      }
+      more = false;
+    }
     if (more) {
       j = walk_begin(w);
       qs = (items - 1) % C::QSTAGES;
@@ -288,20 +337,7 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
         j = walk_next(w, at);
       }
       auto values = [&](int i) -> bool {
-        if (!active(now, i, at)) return true;
-        if (!mbar_wait_warp(&bars->p_full[i], p_phase[i], abort_flag)) { if (lane == 0) atomicCAS(err, 0, ERR_WAIT_OTHER); return false; }
-        p_phase[i] ^= 1;
-        tc_fence_after();
-        const uint32_t va = smem_u32(sKV + v_at * C::KV_TILE), tp = tmem + C::TM_S + i * 128, to = tmem + C::TM_O + i * 128;
-        const uint32_t fresh = first_of(now, i, at) ? 0u : 1u;
-        if (elect_one()) {
-#pragma unroll
-          for (int kk = 0; kk < BN / 16; ++kk)             // 16 keys of P = 8 packed 32-bit columns
-            umma_bf16_ts(to, tp + kk * 8, make_sdesc_sw128(va + kk * 2048, BN * 128, 1024), idesc_pv, kk > 0 ? 1u : fresh);
-          if (at == last_of(now, i)) umma_commit(&bars->o_full[i]);
-        }
-        __syncwarp();
-        return true;
+        return !active(now, i, at) || product(i, first_of(now, i, at), at == last_of(now, i));
       };
       // At an item's end the other tile's products go first: the next item's queries may still be on their way.
       if (crosses) {
@@ -338,7 +374,7 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
       const int index = item_index(turn);
       if (turn * static_cast<int>(gridDim.x) >= shape.items) break;
       if (index >= shape.items) continue;
-      const Item w = make_item<CAUSAL, VAR>(index, shape, var, lane);
+      const Item w = make_item<CAUSAL, VAR, HALVES>(index, shape, var, lane);
       // (picked, not indexed: a row's tile is known when the kernel runs)
       const int q0 = i ? w.q0[1] : w.q0[0], h = i ? w.h[1] : w.h[0], b = w.b;
       const int lo = i ? w.lo[1] : w.lo[0], hi = i ? w.hi[1] : w.hi[0], kept = i ? w.keep[1] : w.keep[0];
@@ -473,13 +509,28 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->p_full[i]);
         if (j == hi - 1) break;
-        ++j;
+        j += HALVES ? 2 : 1;
         if (VAR && j >= kept && j < lo) j = lo;
       }
       // epilogue: O / l -> bf16, lse
       if (ok && any) {
         if (!__all_sync(0xffffffffu, mbar_wait(&bars->o_full[i], o_phase, abort_flag))) { atomicCAS(err, 0, ERR_WAIT_OTHER); ok = false; }
         o_phase ^= 1;
+      }
+      float own = 1.f, other = 0.f;                    // what the tiles' rows weigh in the result
+      if constexpr (HALVES) {
+        // (every warp passes here, whatever went wrong before)
+        if (i == 1) bars->half[r] = make_float2(m_used, l);
+        tc_fence_before();
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (i == 1) { if (ok) continue; break; }
+        const float2 o = bars->half[r];
+        // (the other half's products are complete: its warps waited for them before they came here)
+        const float m = fmaxf(m_used, o.x);
+        own = m_used > -INFINITY ? fast_exp2(m_used - m) : 0.f;
+        other = o.x > -INFINITY ? fast_exp2(o.x - m) : 0.f;
+        l = l * own + o.y * other;
+        m_used = m;
       }
       if (!ok) break;
       tc_fence_after();
@@ -502,6 +553,13 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
         else {
 #pragma unroll
           for (int x = 0; x < 32; ++x) v[x] = 0;
+        }
+        if constexpr (HALVES) {
+          uint32_t u[32];
+          tmem_ld_32x32b_x32(t_o + 128 + c * 32, u);       // (nothing of sense where the other half has no keys: its weight is 0 then)
+          tmem_ld_wait();
+#pragma unroll
+          for (int x = 0; x < 32; ++x) v[x] = __float_as_uint(own * __uint_as_float(v[x]) + (other > 0.f ? other * __uint_as_float(u[x]) : 0.f));
         }
         if (row < S) store_row_32<false>(orow + c * 32, v, inv);
         __syncwarp();
@@ -534,20 +592,26 @@ static int multiprocessors() {
   return n[dev];
 }
 
-template <int D, bool CAUSAL, bool VAR, bool SIG>
+template <int D, bool CAUSAL, bool VAR, bool SIG, bool HALVES = false>
 static int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, void* out, float* lse, Shape s, long long osb, long long oss, long long osh,
                   float scale_log2, const Variant& var, int* err, cudaStream_t stream) {
-  auto kern = flash_fwd_pair_kernel<D, CAUSAL, VAR, SIG>;
+  auto kern = flash_fwd_pair_kernel<D, CAUSAL, VAR, SIG, HALVES>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<D>::SMEM);
   if (e != cudaSuccess) return static_cast<int>(e);
   // Two tiles to a CTA wherever that leaves no SM without one; heads of one key head before neighbouring rows, since their key tiles are the same.
   const int tiles = (s.S + BM - 1) / BM, sms = multiprocessors();
   const long long singles = static_cast<long long>(tiles) * s.Hq * s.B;
-  s.pairing = singles <= sms ? SINGLE : (s.Hq / s.Hkv) % 2 == 0 ? HEADS : ROWS;
-  const long long items = s.pairing == SINGLE ? singles : s.pairing == HEADS ? singles / 2 : static_cast<long long>((tiles + 1) / 2) * s.Hq * s.B;
+  // Few tiles: both halves of a CTA on one tile's keys, a CTA an item.  With an empty second tile the first one's chain stood alone (11008 causal tokens of one
+  // head of 128, 86 tiles: 152 us, now 93; 3328 of 4 heads of 64, 104 tiles: 46 and 28).  Causal rows up to two tiles an SM: the longest items set the pace, and are half
+  // as long (1 x 2048, 12 heads of 128, 192 tiles: 40 us by pairs, 25; 1 x 1152, 32 heads, 288 tiles: 26.6 and 24.8); not for less than eight tiles a row, where setting
+  // an item up takes as long as its keys (3 x 640, 16 heads of 64, 240 tiles: 15.0 by pairs, 16.7).
+  if constexpr (!VAR && !SIG && !HALVES)
+    if (singles <= (CAUSAL && tiles >= 8 ? 2 : 1) * sms) return launch<D, CAUSAL, VAR, SIG, true>(tq, tk, tv, out, lse, s, osb, oss, osh, scale_log2, var, err, stream);
+  s.pairing = HALVES ? SPLIT : singles <= sms ? SINGLE : (s.Hq / s.Hkv) % 2 == 0 ? HEADS : ROWS;
+  const long long items = HALVES || s.pairing == SINGLE ? singles : s.pairing == HEADS ? singles / 2 : static_cast<long long>((tiles + 1) / 2) * s.Hq * s.B;
   if (items > 0x3fffffff) return -3;
   s.items = static_cast<int>(items);
-  kern<<<s.items < sms ? s.items : sms, THREADS, Cfg<D>::SMEM, stream>>>(tq, tk, tv, reinterpret_cast<__nv_bfloat16*>(out), lse, s, osb, oss, osh, scale_log2, var, err);
+  kern<<<HALVES || s.items < sms ? s.items : sms, THREADS, Cfg<D>::SMEM, stream>>>(tq, tk, tv, reinterpret_cast<__nv_bfloat16*>(out), lse, s, osb, oss, osh, scale_log2, var, err);
   return static_cast<int>(cudaGetLastError());
 }
 

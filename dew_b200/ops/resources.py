@@ -59,7 +59,7 @@ LAUNCHES: Dict[str, Launch] = {
     "gemm_pair_kernel": Launch(192, 6 * 32768 + 1280, 512),
     "gemm_mx_kernel": Launch(320, 5 * 40960 + 1280, 512),
     "flash_fwd_kernel": Launch(320, 229376 + 2560, 512),
-    "flash_fwd_pair_kernel": Launch(384, 229376 + 1024, 512),
+    "flash_fwd_pair_kernel": Launch(384, 229376 + 2048, 512),
     "flash_dq_kernel": Launch(640, 7 * 32768 + 256, 512),
     "flash_dkv_kernel": Launch(640, 2 * 32768 + 2 * (2 * 32768 + 1024) + 256, 512),
     "paged_decode_tma_kernel": Launch(128, 100 * 1024, 0),

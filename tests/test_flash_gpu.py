@@ -98,3 +98,28 @@ def test_flash_gradients_into_rows_of_any_alignment(D, gap):
     for a, w in zip(want, wide):
         assert torch.equal(w[..., first:first + D], a)
         assert bool((w[..., :first] == 7).all()) and bool((w[..., first + D:] == 7).all())
+
+
+# one key tile (the second half has none), two, an odd number; rows and keys that end inside a tile; keys before and behind the queries; rows that one half sees nothing
+# of, and rows that see nothing; a second wave of items; one row fewer and more than the line to pairs
+@pytest.mark.parametrize("B,S,T,Hq,Hkv,D,causal", [(1, 128, 128, 1, 1, 128, True), (1, 64, 384, 2, 2, 64, False), (2, 384, 640, 2, 1, 128, True), (1, 200, 333, 4, 2, 64, True),
+                                                   (1, 333, 200, 2, 2, 128, True), (1, 1100, 1100, 8, 8, 64, False), (1, 1024, 1024, 37, 37, 64, True), (1, 896, 896, 37, 37, 128, True),
+                                                   (1, 2000, 2000, 12, 4, 128, True)])
+@pytest.mark.parametrize("sinks", [False, True])
+def test_flash_halves_of_a_rows_keys(B, S, T, Hq, Hkv, D, causal, sinks):
+    from dew_b200.ops.flash import NONE, Variants, flash_fwd
+    g = torch.Generator(device=DEV).manual_seed(S + T)
+    q, k, v = (torch.randn(B, n, h, D, generator=g, device=DEV).bfloat16() for n, h in ((S, Hq), (T, Hkv), (T, Hkv)))
+    sink = torch.randn(Hq, generator=g, device=DEV)
+    out, lse = flash_fwd(q, k, v, causal, D ** -0.5, var=Variants(sinks=sink) if sinks else NONE)
+    L.check_status()
+    scores = torch.einsum("bshd,bthd->bhst", q.double(), k.double().repeat_interleave(Hq // Hkv, 2)) * D ** -0.5
+    if causal:
+        scores = scores.masked_fill(torch.ones(S, T, dtype=torch.bool, device=DEV).triu(T - S + 1), float("-inf"))
+    with_sink = torch.cat([scores, sink.double()[None, :, None, None].expand(B, Hq, S, 1)], -1) if sinks else scores
+    want_lse = torch.logsumexp(with_sink, -1)
+    weights = (scores - want_lse[..., None]).exp().nan_to_num(0.0)
+    # a rounding of the probabilities (2^-9) and one of the result
+    assert rel_err(out, torch.einsum("bhst,bthd->bshd", weights, v.double().repeat_interleave(Hq // Hkv, 2))) < 2.0 ** -8
+    seen = want_lse.isfinite()
+    assert float((lse.double() - want_lse)[seen].abs().max()) < 1e-5 * max(1.0, float(want_lse[seen].abs().max())) and bool((lse[~seen] == float("-inf")).all())

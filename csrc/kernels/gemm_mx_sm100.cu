@@ -184,11 +184,12 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
       if (!mbar_wait_warp(&sh->tmem_empty[acc], acc_phase ^ 1, abort_flag)) { if (lane == 0) atomicCAS(err, 0, ERR_WAIT_TMEM_EMPTY); break; }
       const uint32_t d_tmem = tmem_base + acc * ACC_COLS;
       for (int k = 0; k < k_iters; ++k) {
-        // two lanes wait at the same time: for the stage's operands and for its scales
-        bool got = true;
-        if (lane == 0) got = mbar_wait(&sh->full[stage], phase, abort_flag);
-        else if (lane == 1) got = mbar_wait(&sh->sf_full[stage], phase, abort_flag);
-        if (!__all_sync(0xffffffffu, got)) { if (lane == 0) atomicCAS(err, 0, ERR_WAIT_FULL); ok = false; break; }
+        // every lane waits for the stage's operands and for its scales: the lane that issues has to have seen both itself, since a vote orders no memory between lanes
+        if (!mbar_wait_warp(&sh->full[stage], phase, abort_flag) || !mbar_wait_warp(&sh->sf_full[stage], phase, abort_flag)) {
+          if (lane == 0) atomicCAS(err, 0, ERR_WAIT_FULL);
+          ok = false;
+          break;
+        }
         tc_fence_after();
         const uint32_t sa = smem_u32(smem + stage * STAGE_BYTES);
         const uint32_t sb = sa + A_BYTES;

@@ -22,7 +22,7 @@ def embedding_gradient(dy, ids, V):
 # slices of the count of one token to sixteen; runs of one token, of a handful, of all; widths of one piece, past a block's columns, of both
 @pytest.mark.parametrize("T,V,d", [(1, 1, 8), (3, 2, 1032), (255, 300, 64), (1024, 1, 128), (1025, 7, 8), (4096, 50000, 256), (16384, 256, 16), (0, 5, 8)])
 def test_embedding_gradient(T, V, d):
-    """The tokens' rows are summed in fp32 in their order and rounded to bf16 once."""
+    """The tokens' rows are summed in fp32 and rounded to bf16 once."""
     g = torch.Generator(device=DEV).manual_seed(T)
     ids, dy = torch.randint(0, V, (T,), generator=g, device=DEV), torch.randn(T, d, generator=g, device=DEV).bfloat16()
     got = embedding_gradient(dy, ids, V)
@@ -30,6 +30,45 @@ def test_embedding_gradient(T, V, d):
     size = torch.zeros(V, d, dtype=torch.float64, device=DEV).index_add_(0, ids, dy.double().abs())
     assert bool(((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + T * 2.0 ** -24 * size).all())
     assert torch.equal(got, embedding_gradient(dy, ids, V))
+
+
+# runs of as many tokens as one block takes, one more, up to and past the next multiples of it; at the front, behind others, at the end; columns short of and past a chunk
+@pytest.mark.parametrize("d", [8, 72, 1032])
+@pytest.mark.parametrize("runs", [[64], [65], [1, 64, 65, 1], [63, 66, 127, 2, 129], [30, 64, 64, 65, 300], [128, 128], [5] * 40 + [1000] + [3] * 20 + [70, 4096], [16384]])
+def test_embedding_gradient_of_long_runs(runs, d):
+    g = torch.Generator(device=DEV).manual_seed(len(runs) + d)
+    ids = torch.repeat_interleave(torch.arange(len(runs), device=DEV) * 3, torch.tensor(runs, device=DEV))
+    ids = ids[torch.randperm(len(ids), generator=g, device=DEV)].contiguous()
+    dy = torch.randn(len(ids), d, generator=g, device=DEV).bfloat16()
+    V = 3 * len(runs) + 1
+    got = embedding_gradient(dy, ids, V)
+    want, size = (torch.zeros(V, d, dtype=torch.float64, device=DEV).index_add_(0, ids, x) for x in (dy.double(), dy.double().abs()))
+    assert bool(((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + max(runs) * 2.0 ** -24 * size).all())
+    assert torch.equal(got, embedding_gradient(dy, ids, V))
+
+
+def test_padding_costs_no_more_than_tokens():
+    """Half of a batch of one id: as many rows read and fewer written as where the ids differ, so at most as long but for the launches (twice, as a bound; a run that was
+    summed by one block took nineteen times as long)."""
+    T, d, V = 8192, 2048, 32768
+    g = torch.Generator(device=DEV).manual_seed(0)
+    dy, ids = torch.randn(T, d, generator=g, device=DEV).bfloat16(), torch.randint(0, V, (T,), generator=g, device=DEV)
+    padded = ids.clone()
+    padded[T // 2:] = 0
+    took = {}
+    for name, which in (("differ", ids), ("padded", padded)):
+        times = []
+        for _ in range(7):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            torch.cuda._sleep(500000)                            # (the launches are enqueued by the time the first one starts)
+            a.record()
+            embedding_gradient(dy, which, V)
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        took[name] = sorted(times)[3]
+    assert took["padded"] < 2 * took["differ"], took
 
 
 def test_embedding_lookup_keeps_its_gradients():

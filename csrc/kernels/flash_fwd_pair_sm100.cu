@@ -1,6 +1,7 @@
 // Flash attention forward for sm_100a (bf16, causal or full, GQA, heads of 64 or 128): two query tiles a CTA against one stream of keys and values.
 //
-// Persistent, one CTA per SM, 12 warps; a work item is two query tiles of 128 rows that share a key head:
+// Persistent, one CTA per SM, 12 warps; a work item is two query tiles of 128 rows that share a key head, or, where tiles are few, the two halves of one tile's keys
+// (every second key tile each; the halves' outputs, maxima and sums are joined at the end, and a CTA has one item):
 //   warps 0..3  softmax of tile 0, one thread per query row (all 128 key columns: no reduction crosses threads)
 //   warps 4..7  softmax of tile 1
 //   warp 8      TMA producer : the item's queries, then its keys and values in the order they are used, into one ring
@@ -62,15 +63,16 @@ struct Bars {
 static_assert(sizeof(Bars) <= 2048 && Cfg<128>::SMEM <= 232448 && Cfg<64>::SMEM <= 232448, "over the 227 KB a CTA may use");
 
 // What a launch is about, and how its query tiles are paired.
-enum : int { SINGLE = 0, HEADS = 1, ROWS = 2, SPLIT = 3 };
+enum : int { HEADS = 0, ROWS = 1, SPLIT = 2 };
 struct Shape {
   int B, S, T, Hq, Hkv;
-  int pairing;                     // HEADS: the same rows of two neighbouring query heads of a key head; ROWS: two neighbouring tiles of a head; SINGLE: tile 1 empty;
+  int pairing;                     // HEADS: the same rows of two neighbouring query heads of a key head; ROWS: two neighbouring tiles of a head;
                                    // SPLIT: both the same rows, tile 0 against the first, third, ... of their key tiles, tile 1 against the others (one item a CTA)
   int items;
 };
 
-// One item: its tiles' rows, heads and key tiles [0, kept) and [lo, hi); an empty tile has hi = 0 and lo = NEVER.
+// One item: its tiles' rows, heads and key tiles [0, keep) and [lo, hi); an empty tile has hi = 0 and lo = NEVER.  SPLIT: the key tiles of its rows are counted, `to` of
+// them: the first keep[0] ones, then those from lo[0] on.
 struct Item {
   int b, hk, from, to;             // the walk is over the tiles of both: [0, kept) and [from, to)
   int kept;
@@ -91,6 +93,7 @@ __device__ __forceinline__ Item make_item(int index, const Shape& s, const Varia
   w.b = rest / heads;
   w.from = NEVER;
   w.to = w.kept = 0;
+  int first = 0;
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     const int qt = s.pairing == ROWS ? 2 * qi + i : qi;
@@ -99,14 +102,24 @@ __device__ __forceinline__ Item make_item(int index, const Shape& s, const Varia
     int hi = (s.T + BN - 1) / BN;
     // keys visible to this query tile: causal alignment is bottom-right (query i sees keys <= i + T - S)
     if (CAUSAL) hi = min(hi, (w.q0[i] + BM + (s.T - s.S) + BN - 1) / BN);
-    if (qt >= tiles || (s.pairing == SINGLE && i == 1)) hi = 0;
-    if (qt >= tiles || (s.pairing == SINGLE && i == 1)) w.q0[i] = s.S;
-    int lo = 0;
-    if (hi > 0) lo = VAR ? attn::first_key_tile_of_warp(var, w.b, w.q0[i], s.S, s.T, BN, hi, lane) : var.first != nullptr ? min(var.first[qt], hi) : 0;
+    if (qt >= tiles) {
+      hi = 0;
+      w.q0[i] = s.S;
+    }
+    if (i == 1 && (HALVES || s.pairing == HEADS)) {
+      first = min(first, max(hi, 0));                // (the same rows)
+    } else if (hi > 0) {
+      first = VAR ? attn::first_key_tile_of_warp(var, w.b, w.q0[i], s.S, s.T, BN, hi, lane) : var.first != nullptr ? min(var.first[qt], hi) : 0;
+    } else {
+      first = 0;
+    }
+    int lo = first;
     if constexpr (HALVES) {
-      const int n = max(hi - lo, 0);
-      hi = i == 0 ? (n > 0 ? lo + ((n - 1) & ~1) + 1 : 0) : n > 1 ? lo + (n & ~1) : 0;
-      lo += i;
+      w.lo[i] = lo;
+      w.keep[i] = VAR ? min(lo, (var.keep + BN - 1) / BN) : 0;
+      w.hi[i] = w.to = w.keep[i] + max(hi - lo, 0);
+      w.from = 0;
+      continue;
     }
     w.keep[i] = VAR ? min(lo, (var.keep + BN - 1) / BN) : 0;
     if (lo >= hi) {                                  // (kept tiles are before lo: a tile whose window is empty has none to add)
@@ -123,11 +136,14 @@ __device__ __forceinline__ Item make_item(int index, const Shape& s, const Varia
     w.hi[i] = hi;
   }
   w.hk = w.h[0] / (s.Hq / s.Hkv);
+  if constexpr (HALVES) return w;
   if (w.from < NEVER) w.to = max(w.to, w.kept);
   w.kept = min(w.kept, w.from);
   return w;
 }
 
+// (SPLIT) the key tile that is n-th of an item's
+__device__ __forceinline__ int nth_tile(const Item& w, int n) { return n < w.keep[0] ? n : w.lo[0] + n - w.keep[0]; }
 __device__ __forceinline__ bool active(const Item& w, int i, int j) { return j < w.hi[i] && (j >= w.lo[i] || j < w.keep[i]); }
 __device__ __forceinline__ bool first_of(const Item& w, int i, int j) { return j == (w.keep[i] > 0 ? 0 : w.lo[i]); }
 __device__ __forceinline__ int last_of(const Item& w, int i) { return w.hi[i] - 1; }
@@ -222,8 +238,8 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
       if constexpr (HALVES) {
         // in the order in which the issuer takes them
         const int end = w.to;
-        ok = fetch(&tk, w.from * BN) && (w.from + 1 >= end || fetch(&tk, (w.from + 1) * BN));
-        for (int j = w.from; ok && j < end; ++j) ok = fetch(&tv, j * BN) && (j + 2 >= end || fetch(&tk, (j + 2) * BN));
+        ok = fetch(&tk, nth_tile(w, 0) * BN) && (1 >= end || fetch(&tk, nth_tile(w, 1) * BN));
+        for (int n = 0; ok && n < end; ++n) ok = fetch(&tv, nth_tile(w, n) * BN) && (n + 2 >= end || fetch(&tk, nth_tile(w, n + 2) * BN));
         continue;
       }
       const int end = walk_last(w);
@@ -294,14 +310,14 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
       // One item: the tiles' scores are in front of each other's products, as with two tiles of rows.
       const int end = w.to;
       ok = more && await_queries(0);
-      for (int i = 0; ok && i < 2 && w.from + i < end; ++i) {
+      for (int i = 0; ok && i < 2 && i < end; ++i) {
         ok = take(k_at);
         tc_fence_after();
         if (ok) { scores(i, 0, k_at); commit(&bars->kv_empty[k_at]); }
       }
-      for (int at = w.from; ok && at < end; ++at) {
-        const int i = (at - w.from) & 1;
-        ok = take(v_at) && product(i, at - w.from < 2, at + 2 >= end);
+      for (int at = 0; ok && at < end; ++at) {
+        const int i = at & 1;
+        ok = take(v_at) && product(i, at < 2, at + 2 >= end);
         if (!ok) break;
         commit(&bars->kv_empty[v_at]);
         if (at + 2 >= end) continue;
@@ -386,8 +402,26 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
       float m_used = -INFINITY, l = 0.f;
       const float gained = VAR && var.gain != nullptr ? scale_log2 * var.gain[h] : scale_log2;
       const float sig2 = SIG ? var.sig[h] * LOG2E : 0.f;
-      const bool any = hi > 0;
-      for (int j = j_first; any && ok; ) {
+      const bool any = HALVES ? i < w.to : hi > 0;
+      const bool packed = VAR && var.q_seg != nullptr;
+      const int mine = packed ? var.q_seg[static_cast<long long>(b) * S + min(row, S - 1)] : 0;      // this row's document
+      for (int j = HALVES ? nth_tile(w, i) : j_first, n = i; any && ok; ) {
+        // which keys of the tile are of this row's document, bit l of word q for key 4 l + q: found once for each of the documents that the warp's rows are of, while the
+        // scores are made (T is a multiple of 4 here)
+        uint32_t same[4] = {0u, 0u, 0u, 0u};
+        if (packed) {
+          const int key = j * BN + lane * 4;
+          const int4 id = key < T ? *reinterpret_cast<const int4*>(var.k_seg + static_cast<long long>(b) * T + key) : make_int4(0, 0, 0, 0);
+          for (unsigned todo = 0xffffffffu; todo != 0; ) {
+            const int doc = __shfl_sync(0xffffffffu, mine, __ffs(todo) - 1);
+            const bool hit = mine == doc;
+            const uint32_t v[4] = {__ballot_sync(0xffffffffu, id.x == doc), __ballot_sync(0xffffffffu, id.y == doc), __ballot_sync(0xffffffffu, id.z == doc),
+                                   __ballot_sync(0xffffffffu, id.w == doc)};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) same[q] = hit ? v[q] : same[q];
+            todo &= ~__ballot_sync(0xffffffffu, hit);
+          }
+        }
         if (!__all_sync(0xffffffffu, mbar_wait(&bars->s_full[i], s_phase, abort_flag))) { atomicCAS(err, 0, ERR_WAIT_TMEM_FULL); ok = false; break; }
         s_phase ^= 1;
         tc_fence_after();
@@ -404,10 +438,10 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
         }
         const int k0 = j * BN;
         if (VAR && var.softcap > 0.f) {
-          // cap * tanh(score / cap), kept in the log2 domain
-          const float inv_cap = 1.f / (var.softcap * LOG2E), cap2 = var.softcap * LOG2E;
+          // cap * tanh(score / cap) = cap - 2 cap / (1 + e^(2 score / cap)), kept in the log2 domain; fp32 accurate relative to the cap
+          const float cap2 = var.softcap * LOG2E, twice = 2.f * LOG2E / cap2;
 #pragma unroll
-          for (int x = 0; x < BN; ++x) s[x] = cap2 * attn::soft_tanh(s[x] * inv_cap);
+          for (int x = 0; x < BN; ++x) s[x] = fmaf(-2.f * cap2, __fdividef(1.f, 1.f + fast_exp2(s[x] * twice)), cap2);
         }
         if (k0 + BN - 1 > warp_limit) {
           const int past = limit - k0;
@@ -424,25 +458,9 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
               for (int x = 0; x < BN; ++x) if (k0 + x < first && k0 + x >= var.keep) s[x] = -INFINITY;
             }
           }
-          if (var.q_seg != nullptr && k0 < T) {
-            const int mine = var.q_seg[static_cast<long long>(b) * S + min(row, S - 1)];
-            const int* ks = var.k_seg + static_cast<long long>(b) * T + k0;
-            // ids are non-decreasing: the whole tile matches iff its ends do
-            if (ks[0] != mine || ks[min(BN - 1, T - 1 - k0)] != mine) {
+          if (packed && (same[0] & same[1] & same[2] & same[3]) != 0xffffffffu) {
 #pragma unroll
-              for (int x = 0; x < BN; x += 4) {
-                if (k0 + x + 3 < T) {
-                  const int4 id = *reinterpret_cast<const int4*>(ks + x);
-                  if (id.x != mine) s[x] = -INFINITY;
-                  if (id.y != mine) s[x + 1] = -INFINITY;
-                  if (id.z != mine) s[x + 2] = -INFINITY;
-                  if (id.w != mine) s[x + 3] = -INFINITY;
-                } else {
-#pragma unroll
-                  for (int q = 0; q < 4; ++q) if (k0 + x + q < T && ks[x + q] != mine) s[x + q] = -INFINITY;
-                }
-              }
-            }
+            for (int x = 0; x < BN; ++x) if (!(same[x & 3] >> (x >> 2) & 1)) s[x] = -INFINITY;
           }
         }
         __syncwarp();                                  // the masks above branch by row; what follows takes whole warps
@@ -470,7 +488,7 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
           if (__any_sync(0xffffffffu, need)) {
             const float alpha = (need && m_used > -INFINITY) ? fast_exp2(m_used - m_new) : 1.f;
             if (need) { m_used = m_new; l *= alpha; }
-            if (j != j_first) {
+            if (HALVES ? n != i : j != j_first) {
 #pragma unroll
               for (int c = 0; c < D / 16; ++c) {
                 uint32_t v[16];
@@ -508,9 +526,15 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->p_full[i]);
-        if (j == hi - 1) break;
-        j += HALVES ? 2 : 1;
-        if (VAR && j >= kept && j < lo) j = lo;
+        if constexpr (HALVES) {
+          n += 2;
+          if (n >= w.to) break;
+          j = nth_tile(w, n);
+        } else {
+          if (j == hi - 1) break;
+          ++j;
+          if (VAR && j >= kept && j < lo) j = lo;
+        }
       }
       // epilogue: O / l -> bf16, lse
       if (ok && any) {
@@ -519,18 +543,22 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
       }
       float own = 1.f, other = 0.f;                    // what the tiles' rows weigh in the result
       if constexpr (HALVES) {
-        // (every warp passes here, whatever went wrong before)
-        if (i == 1) bars->half[r] = make_float2(m_used, l);
+        // (every warp passes here, whatever went wrong before; with one key tile there is nothing to join)
+        if (i == 1 && w.to > 1) bars->half[r] = make_float2(m_used, l);
         tc_fence_before();
-        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (w.to > 1) asm volatile("bar.sync 1, 256;" ::: "memory");
         if (i == 1) { if (ok) continue; break; }
-        const float2 o = bars->half[r];
+        const float2 o = w.to > 1 ? bars->half[r] : make_float2(-INFINITY, 0.f);
         // (the other half's products are complete: its warps waited for them before they came here)
-        const float m = fmaxf(m_used, o.x);
-        own = m_used > -INFINITY ? fast_exp2(m_used - m) : 0.f;
-        other = o.x > -INFINITY ? fast_exp2(o.x - m) : 0.f;
-        l = l * own + o.y * other;
-        m_used = m;
+        if constexpr (SIG) {
+          other = w.to > 1 ? 1.f : 0.f;
+        } else {
+          const float m = fmaxf(m_used, o.x);
+          own = m_used > -INFINITY ? fast_exp2(m_used - m) : 0.f;
+          other = o.x > -INFINITY ? fast_exp2(o.x - m) : 0.f;
+          l = l * own + o.y * other;
+          m_used = m;
+        }
       }
       if (!ok) break;
       tc_fence_after();
@@ -555,11 +583,13 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
           for (int x = 0; x < 32; ++x) v[x] = 0;
         }
         if constexpr (HALVES) {
-          uint32_t u[32];
-          tmem_ld_32x32b_x32(t_o + 128 + c * 32, u);       // (nothing of sense where the other half has no keys: its weight is 0 then)
-          tmem_ld_wait();
+          if (w.to > 1) {
+            uint32_t u[32];
+            tmem_ld_32x32b_x32(t_o + 128 + c * 32, u);
+            tmem_ld_wait();
 #pragma unroll
-          for (int x = 0; x < 32; ++x) v[x] = __float_as_uint(own * __uint_as_float(v[x]) + (other > 0.f ? other * __uint_as_float(u[x]) : 0.f));
+            for (int x = 0; x < 32; ++x) v[x] = __float_as_uint(own * __uint_as_float(v[x]) + (other > 0.f ? other * __uint_as_float(u[x]) : 0.f));
+          }
         }
         if (row < S) store_row_32<false>(orow + c * 32, v, inv);
         __syncwarp();
@@ -592,23 +622,43 @@ static int multiprocessors() {
   return n[dev];
 }
 
+// Few tiles: both halves of a CTA on one tile's keys, a CTA an item.  Up to a tile an SM always (pairs / halves, us: 11008 causal tokens of one head of 128, 86 tiles, 163 / 88;
+// 3328 tokens, 4 heads of 64, 104 tiles, 50 / 27, with a soft cap 127 / 65, packed documents 24 / 16).  Up to two tiles an SM where pairs of odd numbers of rows take a second
+// wave (6 x 384, 16 heads of 64, a window, 20.5 / 17.8; of one tile 2 x 128, 100 heads, 13.1 / 14.9), and where a row's keys are many: the longest items set the pace, and are half as long by halves, but setting an
+// item up takes as long as a few key tiles.  The lines, in key tiles that a row sees:
+//   causal 8 (5 up to four thirds of a tile an SM)   1 x 2048, 12 heads of 128, 37.5 / 23.8   1 x 1152, 32 heads, 26.6 / 24.8   2 x 768, 16 heads of 64, a window of 512, 20.5 / 17.2
+//                                                    3 x 640, 16 heads of 64, 14.3 / 16.5   1 x 896, 32 / 8 heads of 128, a window of 256, 17.2 / 22.7
+//   causal, soft caps and sigmoids 3                 2 x 384, 32 / 8 heads of 128, 22.9 / 21.3 and 18.4 / 18.6   8 x 512, 8 heads of 64, 27.2 / 24.4   1 x 256, 100 heads, 15.6 / 18.6
+//   not causal, chunks and documents 9               1 x 1152, 18 heads of 128, 28.7 / 20.7 and 33.0 / 23.1   1 x 1024, 32 / 8 heads, 27.4 / 28.7 and 31.5 / 31.1
+//   not causal, windows and soft caps 16             1 x 3200, 8 heads of 64, 60 / 37 and 140 / 123   1 x 1152, 18 heads of 128, 28.3 / 32.0 and 52 / 55
+//   not causal, else never                           1 x 3200, 8 heads of 64, 50 / 52   1 x 1152, 18 heads of 128, 25 / 30
+template <bool CAUSAL, bool VAR, bool SIG>
+static bool by_halves(const Shape& s, const Variant& var, int sms) {
+  const int tiles = (s.S + BM - 1) / BM;
+  const long long singles = static_cast<long long>(tiles) * s.Hq * s.B;
+  if (singles <= sms) return true;
+  if (singles > 2 * sms) return false;
+  if (tiles >= 3 && (s.Hq / s.Hkv) % 2 != 0 && static_cast<long long>((tiles + 1) / 2) * s.Hq * s.B > sms) return true;
+  int keys = (s.T + BN - 1) / BN;
+  if (!CAUSAL) return VAR && (var.chunk > 0 || var.q_seg != nullptr ? keys >= 9 : (var.window > 0 || var.softcap > 0.f) && keys >= 16);
+  if (VAR && var.window > 0) keys = min(keys, var.window / BN + 1);
+  if (VAR && var.chunk > 0) keys = min(keys, (var.chunk + BN - 1) / BN);
+  return keys >= (SIG || (VAR && var.softcap > 0.f) ? 3 : 3 * singles <= 4 * sms ? 5 : 8);
+}
+
 template <int D, bool CAUSAL, bool VAR, bool SIG, bool HALVES = false>
 static int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, void* out, float* lse, Shape s, long long osb, long long oss, long long osh,
                   float scale_log2, const Variant& var, int* err, cudaStream_t stream) {
   auto kern = flash_fwd_pair_kernel<D, CAUSAL, VAR, SIG, HALVES>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<D>::SMEM);
   if (e != cudaSuccess) return static_cast<int>(e);
-  // Two tiles to a CTA wherever that leaves no SM without one; heads of one key head before neighbouring rows, since their key tiles are the same.
   const int tiles = (s.S + BM - 1) / BM, sms = multiprocessors();
   const long long singles = static_cast<long long>(tiles) * s.Hq * s.B;
-  // Few tiles: both halves of a CTA on one tile's keys, a CTA an item.  With an empty second tile the first one's chain stood alone (11008 causal tokens of one
-  // head of 128, 86 tiles: 152 us, now 93; 3328 of 4 heads of 64, 104 tiles: 46 and 28).  Causal rows up to two tiles an SM: the longest items set the pace, and are half
-  // as long (1 x 2048, 12 heads of 128, 192 tiles: 40 us by pairs, 25; 1 x 1152, 32 heads, 288 tiles: 26.6 and 24.8); not for less than eight tiles a row, where setting
-  // an item up takes as long as its keys (3 x 640, 16 heads of 64, 240 tiles: 15.0 by pairs, 16.7).
-  if constexpr (!VAR && !SIG && !HALVES)
-    if (singles <= (CAUSAL && tiles >= 8 ? 2 : 1) * sms) return launch<D, CAUSAL, VAR, SIG, true>(tq, tk, tv, out, lse, s, osb, oss, osh, scale_log2, var, err, stream);
-  s.pairing = HALVES ? SPLIT : singles <= sms ? SINGLE : (s.Hq / s.Hkv) % 2 == 0 ? HEADS : ROWS;
-  const long long items = HALVES || s.pairing == SINGLE ? singles : s.pairing == HEADS ? singles / 2 : static_cast<long long>((tiles + 1) / 2) * s.Hq * s.B;
+  if constexpr (!HALVES)
+    if (by_halves<CAUSAL, VAR, SIG>(s, var, sms)) return launch<D, CAUSAL, VAR, SIG, true>(tq, tk, tv, out, lse, s, osb, oss, osh, scale_log2, var, err, stream);
+  // pairs: heads of one key head before neighbouring rows, since their key tiles are the same
+  s.pairing = HALVES ? SPLIT : (s.Hq / s.Hkv) % 2 == 0 ? HEADS : ROWS;
+  const long long items = HALVES ? singles : s.pairing == HEADS ? singles / 2 : static_cast<long long>((tiles + 1) / 2) * s.Hq * s.B;
   if (items > 0x3fffffff) return -3;
   s.items = static_cast<int>(items);
   kern<<<HALVES || s.items < sms ? s.items : sms, THREADS, Cfg<D>::SMEM, stream>>>(tq, tk, tv, reinterpret_cast<__nv_bfloat16*>(out), lse, s, osb, oss, osh, scale_log2, var, err);
@@ -618,7 +668,7 @@ static int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
 // Maps with boxes of 128 rows x 64 columns; the arguments have been checked.
 int run(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, void* out, float* lse, int B, int S, int T, int Hq, int Hkv, int D, long long osb, long long oss,
         long long osh, float scale_log2, int causal, const Variant& var, int* err, cudaStream_t stream) {
-  const Shape s{B, S, T, Hq, Hkv, SINGLE, 0};
+  const Shape s{B, S, T, Hq, Hkv, HEADS, 0};
   // what changes single scores takes kernels of its own; a first key tile and sinks do not
   const bool any = var.window > 0 || var.chunk > 0 || var.softcap > 0.f || var.q_seg != nullptr || var.gain != nullptr || !(scale_log2 > 0.f);
 #define DEWB_PAIR_GO(DD, CC, VV, SS) launch<DD, CC, VV, SS>(tq, tk, tv, out, lse, s, osb, oss, osh, scale_log2, var, err, stream)

@@ -123,3 +123,78 @@ def test_flash_halves_of_a_rows_keys(B, S, T, Hq, Hkv, D, causal, sinks):
     assert rel_err(out, torch.einsum("bhst,bthd->bshd", weights, v.double().repeat_interleave(Hq // Hkv, 2))) < 2.0 ** -8
     seen = want_lse.isfinite()
     assert float((lse.double() - want_lse)[seen].abs().max()) < 1e-5 * max(1.0, float(want_lse[seen].abs().max())) and bool((lse[~seen] == float("-inf")).all())
+
+
+# few tiles, where both halves of a CTA share a row's keys: one key tile, two, an odd number, and the lines up to two tiles an SM; kept first tiles, in the walk of one half or
+# of both, beside a window that starts in every place of a tile; documents that end inside a tile, of a few tokens, and padding behind the last
+@pytest.mark.parametrize("B,S,Hq,Hkv,D", [(1, 100, 2, 1, 64), (1, 256, 3, 3, 128), (2, 640, 4, 2, 64), (1, 1100, 5, 1, 128), (2, 768, 16, 16, 64), (6, 384, 16, 16, 64), (1, 896, 32, 8, 128),
+                                          (2, 128, 100, 100, 64)])
+@pytest.mark.parametrize("kind", ["window", "keep", "keep many", "chunk", "softcap", "gain", "sigmoid", "packed", "packed short", "packed and padded", "window and documents", "sinks and window"])
+@pytest.mark.parametrize("causal", [True, False])
+def test_flash_variants_of_few_tiles(B, S, Hq, Hkv, D, kind, causal):
+    from dew_b200.ops.flash import Variants, flash_fwd
+    if kind == "sigmoid" and not causal:
+        pytest.skip("sigmoid weights are causal")
+    if not causal and kind not in ("softcap", "packed", "window", "chunk"):
+        pytest.skip("the walk is the causal one's")
+    g = torch.Generator(device=DEV).manual_seed(S + Hq)
+    q, k, v = (torch.randn(B, S, h, D, generator=g, device=DEV).bfloat16() for h in (Hq, Hkv, Hkv))
+    at = torch.arange(S, device=DEV)
+    lengths = torch.tensor([37, 3, 130, 1, 200, 129, 64], device=DEV)
+    docs = {"packed": at // 300 + 1, "packed short": torch.repeat_interleave(torch.arange(1, 8, device=DEV), lengths).repeat(S // 564 + 1)[:S] + at // 564 * 7,
+            "packed and padded": torch.where(at < S - 90, at // 200 + 1, torch.zeros_like(at)), "window and documents": at // 250 + 1}
+    kw = dict(window=dict(window=77), keep=dict(window=70, keep=4), chunk=dict(chunk=96), softcap=dict(softcap=5.0), gain=dict(gain=torch.rand(Hq, generator=g, device=DEV) + 0.5),
+              sigmoid=dict(sigmoid=torch.randn(Hq, generator=g, device=DEV)), **{"keep many": dict(window=130, keep=300), "window and documents": dict(window=200),
+                                                                                 "sinks and window": dict(window=200, sinks=torch.randn(Hq, generator=g, device=DEV))}).get(kind, {})
+    if kind in docs:
+        if S % 4:
+            pytest.skip("rows of documents are on 16-byte boundaries")
+        kw["segments"] = docs[kind].to(torch.int32)[None].expand(B, S).contiguous()
+    out, lse = flash_fwd(q, k, v, causal, D ** -0.5, need_lse=kind != "sigmoid", var=Variants(**kw))
+    L.check_status()
+    scores = torch.einsum("bshd,bthd->bhst", q.double(), k.double().repeat_interleave(Hq // Hkv, 2)) * D ** -0.5
+    if "gain" in kw:
+        scores = scores * kw["gain"].double()[:, None, None]
+    if "softcap" in kw:
+        scores = kw["softcap"] * torch.tanh(scores / kw["softcap"])
+    seen = torch.ones(S, S, dtype=torch.bool, device=DEV)
+    if causal:
+        seen &= at[None] <= at[:, None]
+    if "window" in kw:
+        seen &= (at[None] > at[:, None] - kw["window"]) | (at[None] < kw.get("keep", 0))
+    if "chunk" in kw:
+        seen &= at[None] >= at[:, None] // kw["chunk"] * kw["chunk"]
+    if "segments" in kw:
+        seen = seen & (kw["segments"][0][None] == kw["segments"][0][:, None])
+    if kind == "sigmoid":
+        weights = torch.sigmoid(scores + kw["sigmoid"].double()[:, None, None]) * seen
+    else:
+        scores = scores.masked_fill(~seen, float("-inf"))
+        both = torch.cat([scores, kw["sinks"].double()[None, :, None, None].expand(B, Hq, S, 1)], -1) if "sinks" in kw else scores
+        want_lse = torch.logsumexp(both, -1)
+        weights = (scores - want_lse[..., None]).exp()
+        # fp32 sums of fp32 products of bf16 operands; a soft cap's tanh is good to 2^-22 of the cap
+        assert float((lse.double() - want_lse).abs().max()) < 1e-5 * max(1.0, float(want_lse.abs().max()))
+    # a rounding of the weights (2^-9) and one of the result
+    assert rel_err(out, torch.einsum("bhst,bthd->bshd", weights, v.double().repeat_interleave(Hq // Hkv, 2))) < 2.0 ** -8
+
+
+def test_variants_of_few_tiles_take_no_longer():
+    """Sixteen tiles with factors of the heads' scores, one multiplication a score, against the same without (1.07 times; 1.64 with half of a CTA idle)."""
+    from dew_b200.ops.flash import NONE, Variants, flash_fwd
+    q, k, v = (torch.randn(1, 2048, 1, 128, device=DEV).bfloat16() for _ in range(3))
+    took = []
+    for var in (NONE, Variants(gain=torch.ones(1, device=DEV))):
+        times = []
+        for _ in range(7):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            torch.cuda._sleep(1000000)                           # (the launches are enqueued by the time the first one starts)
+            a.record()
+            for _ in range(10):
+                flash_fwd(q, k, v, True, 128 ** -0.5, need_lse=False, var=var)
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        took.append(sorted(times)[3])
+    assert took[1] < 1.35 * took[0], took

@@ -171,6 +171,14 @@ def reduction_splits(M: int, N: int, K: int, sms: int = 148) -> int:
     return best
 
 
+def pairs_below_a_wave(M: int, N: int, K: int, sms: int = 148) -> bool:
+    """Whether an unsplit product with less than a wave of a lone CTA's tiles of 128 x 256 goes to pairs of CTAs (256 x 256): where their tiles are no second wave and the
+    reduction is long.  A pair fetches two thirds of the operands.  Lone CTAs / pairs, us: 2048 x 2048 over 2048 17.2 / 17.6, over 4096 26.8 / 27.2, over 8192 53.5 / 47.9;
+    512 x 8192 17.2 / 17.8, 30.3 / 28.7, 59.2 / 51.4; 128 x 16384 17.6 / 18.0, 36.9 / 33.0, 63.3 / 56.1.  A second wave: 1152 x 4096 over 4096 (144 tiles, 80 pairs') 28.0 / 45.3,
+    384 x 12288 35.2 / 46.5."""
+    return K >= 4096 and -(-M // 256) * -(-N // 256) <= sms // 2
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False,
          out: Optional[torch.Tensor] = None, out_dtype: torch.dtype = torch.bfloat16, accumulate: bool = False,
          alpha: float = 1.0, max_ctas: int = 0, kernel: Optional[str] = None, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -211,10 +219,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     if kernel is None and cell is None and not _TUNE and not _GEMM.forced_by_environment() and _tensor_core_operands(a, b, out):
         # both tensor-core kernels take these operands and the size alone says which: nothing about the call needs looking up.  The pair kernel is 5-15 % faster on
         # the layer shapes; the single-CTA kernel keeps the very wide head.
-        # Below 148 tiles the same where the reduction is long and not split: the pair's smaller operand traffic shows from some 2048 on (2048 x 2048 over 512 14.4 us
-        # either way, over 2048 24.6 and 22.5, over 8192 64 and 55, over 32768 200 and 176; 1152 x 2304 over 768 14.4 and 16.4).
         paired = LARGE_GEMM == "sm100_pair" and N <= 32768 and _pair_built() and (
-            tiles >= 148 or K >= 2048 and max_ctas == 0 and (N % 4 != 0 or reduction_splits(M, N, K) == 1))
+            tiles >= 148 or max_ctas == 0 and pairs_below_a_wave(M, N, K) and (N % 4 != 0 or reduction_splits(M, N, K) == 1))
         which = "sm100_pair" if paired else "sm100_tcgen05"
         _GEMM._record(which, {}, which if tiles >= 148 else None, None)
         return _gemm_tensor_cores(which, a, b, out, M, N, K, a_mn, b_mn, accumulate, alpha, max_ctas, bias)

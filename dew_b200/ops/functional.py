@@ -179,6 +179,11 @@ def pairs_below_a_wave(M: int, N: int, K: int, sms: int = 148) -> bool:
     return K >= 4096 and -(-M // 256) * -(-N // 256) <= sms // 2
 
 
+def _parts(M: int, N: int, K: int, max_ctas: int, bias) -> int:
+    """``reduction_splits`` where the product may be split: partial products are joined in whole vectors, and take no bias."""
+    return reduction_splits(M, N, K) if max_ctas == 0 and bias is None and N % 4 == 0 else 1
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False,
          out: Optional[torch.Tensor] = None, out_dtype: torch.dtype = torch.bfloat16, accumulate: bool = False,
          alpha: float = 1.0, max_ctas: int = 0, kernel: Optional[str] = None, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -220,7 +225,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         # both tensor-core kernels take these operands and the size alone says which: nothing about the call needs looking up.  The pair kernel is 5-15 % faster on
         # the layer shapes; the single-CTA kernel keeps the very wide head.
         paired = LARGE_GEMM == "sm100_pair" and N <= 32768 and _pair_built() and (
-            tiles >= 148 or max_ctas == 0 and pairs_below_a_wave(M, N, K) and (N % 4 != 0 or reduction_splits(M, N, K) == 1))
+            tiles >= 148 or max_ctas == 0 and pairs_below_a_wave(M, N, K) and _parts(M, N, K, max_ctas, bias) == 1)
         which = "sm100_pair" if paired else "sm100_tcgen05"
         _GEMM._record(which, {}, which if tiles >= 148 else None, None)
         return _gemm_tensor_cores(which, a, b, out, M, N, K, a_mn, b_mn, accumulate, alpha, max_ctas, bias)
@@ -274,7 +279,7 @@ def _gemm_tensor_cores(which, a, b, out, M, N, K, a_mn, b_mn, accumulate, alpha,
         fn = lib.dewb_gemm_pair_bf16_bias if which == "sm100_pair" else lib.dewb_gemm_bf16_bias
         rc = fn(at(a), at(b), at(out), at(bb), M, N, K, lda, ldb, ldd, int(a_mn), int(b_mn), epi, alpha, at(L.status(a.device)), max_ctas, L.stream())
     else:
-        splits = reduction_splits(M, N, K) if which == "sm100_tcgen05" and max_ctas == 0 and N % 4 == 0 and hasattr(lib, "dewb_gemm_bf16_split") else 1
+        splits = _parts(M, N, K, max_ctas, bias) if which == "sm100_tcgen05" else 1
         if splits > 1:
             scratch = torch.empty(splits, M, N, dtype=torch.float32, device=a.device)
             rc = lib.dewb_gemm_bf16_split(at(a), at(b), at(out), at(scratch), M, N, K, splits, -(-K // splits // 64) * 64, lda, ldb, ldd, int(a_mn), int(b_mn), epi, alpha,

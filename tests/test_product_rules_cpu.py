@@ -50,7 +50,9 @@ def product(M, N, K, **kw):
 
 @pytest.mark.parametrize("M,N,K,kw,kernel", [
     (2048, 2048, 64, {}, "dewb_gemm_bf16"), (2048, 2048, 8192, {}, "dewb_gemm_pair_bf16"), (1152, 4096, 4096, {}, "dewb_gemm_bf16"), (2048, 2560, 64, {}, "dewb_gemm_pair_bf16"),
-    (1152, 4096, 4096, dict(bias=True), "dewb_gemm_bf16_bias")])
+    # a bias is added by the kernel that makes the whole product: no parts, so the line for pairs is that of unsplit ones
+    (1024, 768, 3072, dict(bias=True), "dewb_gemm_bf16_bias"), (512, 3072, 12288, dict(bias=True), "dewb_gemm_pair_bf16_bias"), (1536, 1536, 16384, dict(bias=True), "dewb_gemm_pair_bf16_bias"),
+    (1152, 4096, 4096, dict(bias=True), "dewb_gemm_bf16_bias"), (1536, 1536, 16384, dict(max_ctas=100), "dewb_gemm_bf16")])
 def test_products_get_their_kernels(launched, M, N, K, kw, kernel):
     calls = launched()
     product(M, N, K, **kw)

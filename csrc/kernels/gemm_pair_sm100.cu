@@ -21,6 +21,7 @@
 // (src/dew/nn/kernels/templates/mosaic_sm100.py:1-220).
 #include "../common/ptx.cuh"
 #include "../common/tmap.h"
+#include "../common/reduction_ranges.cuh"
 #include <cstdlib>
 
 namespace dewb {
@@ -65,34 +66,26 @@ __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int
   n_blk = r / gsize;
 }
 
-// Several products of one shape side by side (GROUPED): product g reduces over [offsets[g], offsets[g + 1]) (experts' weight gradients), or over `per` indices each
-// where there are no offsets (the parts of a split reduction), and writes D + g * stride.  A pair fetches two thirds of the operand bytes that two lone CTAs do, which
-// short reductions waited for beside their stores: 64 groups of 768 rows into 2816 x 2048 took lone CTAs 471 us and take pairs 424, 16 groups of 128 rows into
-// 512 x 256 13.3 either way; the twelve split weight gradients of a diffusion transformer's step (768 x 768
-// to 3072 over 16384) 684 and 600.  A group without rows is cleared in wide stores (one among 16 of
-// 640 x 1408: 77 us in single values, 32 now).
-struct Groups {
-  const int* offsets;
-  int per, count;
-  long long stride;
-};
-
+// Several products side by side (GROUPED: Ranges).  A pair fetches two thirds of the operand bytes that two lone CTAs do, which shows where reductions are long (64 groups of
+// 768 rows into 2816 x 2048: lone CTAs 498 us, pairs 430; 8 of 4096 into 512 x 1024 33.8 and 30.3; the twelve split weight gradients of a diffusion transformer's step,
+// 768 x 768 to 3072 over 16384, 684 and 600).  Short ones over few tiles, and outputs of up to 128 rows, are left to lone CTAs (gemm_sm100.cu): 16 of 128 into 512 x 256 10.0
+// and 10.9.  A group without rows is cleared in wide stores (one among 16 of 640 x 1408: 77 us in single values, some 30 now).
 struct Tile {
   int m_blk, n_blk, k0, k_iters;
   long long d_off;
 };
 
 template <bool GROUPED>
-__device__ __forceinline__ Tile tile_of(int t, int tiles_m, int tiles_n, int group_m, int K, const Groups& gr) {
+__device__ __forceinline__ Tile tile_of(int t, int tiles_m, int tiles_n, int group_m, int K, const Ranges& gr) {
   Tile ti;
   ti.k0 = 0; ti.k_iters = (K + BK - 1) / BK; ti.d_off = 0;
   if constexpr (GROUPED) {
     const int per = tiles_m * tiles_n, g = t / per;
     t -= g * per;
-    ti.k0 = gr.offsets != nullptr ? gr.offsets[g] : g * gr.per;
-    const int end = gr.offsets != nullptr ? gr.offsets[g + 1] : min(K, ti.k0 + gr.per);
-    ti.k_iters = (end - ti.k0 + BK - 1) / BK;
-    ti.d_off = g * gr.stride;
+    const Range of = range_of(gr, g, K, BK);
+    ti.k0 = of.k0;
+    ti.k_iters = of.k_iters;
+    ti.d_off = of.d_off;
   }
   tile_coords(t, tiles_m, tiles_n, group_m, ti.m_blk, ti.n_blk);
   return ti;
@@ -143,7 +136,7 @@ template <bool A_MN, bool B_MN, int EPI, bool GROUPED>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                  void* __restrict__ Dptr, int M, int N, int K, long long ldd, float alpha, int group_m,
-                 const __nv_bfloat16* __restrict__ bias, const Groups groups,
+                 const __nv_bfloat16* __restrict__ bias, const Ranges groups,
                  int* __restrict__ err) {
   extern __shared__ uint8_t smem_raw[];
   // 1024-byte alignment: required by the 128-byte swizzle atoms the descriptors assume. The dynamic shared memory
@@ -328,7 +321,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 
 template <bool A_MN, bool B_MN, int EPI, bool GROUPED = false>
 static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, void* D, int M, int N, int K, long long ldd,
-                      float alpha, int* err, int max_pairs, cudaStream_t stream, const __nv_bfloat16* bias = nullptr, const Groups& groups = {nullptr, 0, 1, 0}) {
+                      float alpha, int* err, int max_pairs, cudaStream_t stream, const __nv_bfloat16* bias = nullptr, const Ranges& groups = {nullptr, 0, 1, 0}) {
   auto kern = gemm_pair_kernel<A_MN, B_MN, EPI, GROUPED>;
   static int resident[64] = {};          // co-resident clusters of this instantiation per device (0 = not asked yet)
   int dev = 0;
@@ -351,7 +344,7 @@ static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, void* D, int
     cfg.gridDim = dim3(static_cast<unsigned>(sms), 1, 1);
     int clusters = 0;
     e = cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg);
-    if (e != cudaSuccess || clusters <= 0) { cudaGetLastError(); return -6; }   // pairs cannot be placed: caller falls back
+    if (e != cudaSuccess || clusters <= 0) { cudaGetLastError(); return -6; }   // pairs cannot be placed: the caller takes lone CTAs
     resident[dev] = clusters;
   }
   int pairs = resident[dev];
@@ -420,6 +413,12 @@ split_sum_kernel(const float* __restrict__ part, void* __restrict__ D, int M, in
   }
 }
 
+int split_sum(const float* part, void* D, int M, int N, long long ldd, int splits, float alpha, int epi, const int* err, cudaStream_t stream) {
+  const long long total = static_cast<long long>(M) * N;
+  split_sum_kernel<<<static_cast<unsigned>((total / 4 + 255) / 256), 256, 0, stream>>>(part, D, M, N, ldd, splits, alpha, epi, err);
+  return static_cast<int>(cudaGetLastError());
+}
+
 }  // namespace gemm_pair
 }  // namespace dewb
 
@@ -473,15 +472,12 @@ extern "C" int dewb_gemm_bf16_split(const void* A, const void* B, void* D, float
   CUtensorMap ta, tb;
   int r = operand_maps(&ta, &tb, A, B, M, N, K, lda, ldb, a_mn, b_mn);
   if (r) return r;
-  const Groups gr{nullptr, per, splits, static_cast<long long>(M) * N};
+  const Ranges gr{nullptr, per, splits, static_cast<long long>(M) * N};
   if (!a_mn && !b_mn) r = launch_one<false, false, EPI_F32, true>(ta, tb, scratch, M, N, K, N, 1.f, err, 0, stream, nullptr, gr);
   else if (!a_mn) r = launch_one<false, true, EPI_F32, true>(ta, tb, scratch, M, N, K, N, 1.f, err, 0, stream, nullptr, gr);
   else if (!b_mn) r = launch_one<true, false, EPI_F32, true>(ta, tb, scratch, M, N, K, N, 1.f, err, 0, stream, nullptr, gr);
   else r = launch_one<true, true, EPI_F32, true>(ta, tb, scratch, M, N, K, N, 1.f, err, 0, stream, nullptr, gr);
-  if (r) return r;
-  const long long total = static_cast<long long>(M) * N;
-  split_sum_kernel<<<static_cast<unsigned>((total / 4 + 255) / 256), 256, 0, stream>>>(scratch, D, M, N, ldd, splits, alpha, epi, err);
-  return static_cast<int>(cudaGetLastError());
+  return r ? r : split_sum(scratch, D, M, N, ldd, splits, alpha, epi, err, stream);
 }
 
 // Grouped reduction (mixture-of-experts weight gradient): for every group g,
@@ -499,7 +495,7 @@ extern "C" int dewb_tgmm_bf16(const void* A, const void* B, void* D, const int* 
   CUtensorMap ta, tb;
   const int r = operand_maps(&ta, &tb, A, B, M, N, R, lda, ldb, 1, 1);
   if (r) return r;
-  const Groups gr{group_offsets, 0, groups, d_group_stride};
+  const Ranges gr{group_offsets, 0, groups, d_group_stride};
   switch (epi) {
     case EPI_BF16: return launch_one<true, true, EPI_BF16, true>(ta, tb, D, M, N, R, ldd, alpha, err, 0, stream, nullptr, gr);
     case EPI_F32: return launch_one<true, true, EPI_F32, true>(ta, tb, D, M, N, R, ldd, alpha, err, 0, stream, nullptr, gr);

@@ -6,6 +6,8 @@
 //   warps 2..9  epilogue       : tcgen05.ld the finished accumulator, convert, store; overlaps the next tile's MMAs.  Two warps share a quarter of the rows
 //                                and take half of the columns each
 //
+// RANGES: several products side by side, each over reduction indices of its own (the parts of a split reduction, experts' weight gradients); a small kernel adds the parts.
+//
 // Operand layouts. "K-major" means the reduction index is contiguous in global memory; "MN-major" means the
 // M (for A) or N (for B) index is contiguous. The three combinations cover a linear layer's forward
 // (x[M,K], W[N,K]), its input gradient (dY[M,N'] K-major, W[N',K'] MN-major) and its weight gradient (both
@@ -14,8 +16,12 @@
 // Replaces the reference's GEMM template for tcgen05 (src/dew/nn/kernels/gemm.py:84, templates/gemm/mosaic_gpu.py).
 #include "../common/ptx.cuh"
 #include "../common/tmap.h"
+#include "../common/reduction_ranges.cuh"
 
 namespace dewb {
+namespace gemm_pair {      // gemm_pair_sm100.cu
+int split_sum(const float* part, void* D, int M, int N, long long ldd, int splits, float alpha, int epi, const int* err, cudaStream_t stream);
+}
 namespace gemm {
 
 constexpr int BM = 128;
@@ -56,12 +62,14 @@ struct GroupArgs {
   const float* row_scale;   // fp8: per-row scale of A (length M), or null
   const float* col_scale;   // fp8: per-row scale of the stacked B operand (indexed by B's row), or null
   const __nv_bfloat16* bias; // one value per output column added after the scale (dense mode), or null
+  Ranges ranges;            // (RANGES)
 };
 
 struct Tile {
-  int m0, n0;        // output tile origin
+  int m0, n0;        // output tile origin (of its product)
   int b_row0;        // row offset added to B's stacked-row coordinate (mode 1)
   bool skip;         // nothing to compute and nothing to store
+  Range range;
 };
 
 __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int& m_blk, int& n_blk) {
@@ -75,10 +83,17 @@ __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int
   n_blk = r / gsize;
 }
 
-__device__ __forceinline__ Tile decode_tile(int t, int tiles_m, int tiles_n, const GroupArgs& ga) {
+template <bool RANGES>
+__device__ __forceinline__ Tile decode_tile(int t, int tiles_m, int tiles_n, int K, int step, const GroupArgs& ga) {
   Tile ti;
   int m_blk, n_blk;
   ti.b_row0 = 0; ti.skip = false;
+  ti.range = {0, (K + step - 1) / step, 0};
+  if constexpr (RANGES) {
+    const int per = tiles_m * tiles_n, g = t / per;
+    t -= g * per;
+    ti.range = range_of(ga.ranges, g, K, step);
+  }
   tile_coords(t, tiles_m, tiles_n, m_blk, n_blk);
   if (ga.mode == 1) {
     const int g = ga.tile_group[m_blk];
@@ -92,7 +107,7 @@ __device__ __forceinline__ Tile decode_tile(int t, int tiles_m, int tiles_n, con
 
 // FP8 = true: operands are e4m3 bytes (K-major only), 128 elements per 128-byte swizzle row, tcgen05 kind::f8f6f4
 // with K = 32 per instruction; the epilogue applies the row-wise scales of both operands.
-template <bool A_MN, bool B_MN, int EPI, bool FP8 = false>
+template <bool A_MN, bool B_MN, int EPI, bool FP8 = false, bool RANGES = false>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                  void* __restrict__ Dptr, int M, int N, int K, long long ldd, float alpha, const GroupArgs ga,
@@ -114,8 +129,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   const int lane = threadIdx.x & 31;
   const int tiles_m = (M + BM - 1) / BM;
   const int tiles_n = (N + BN - 1) / BN;
-  const int num_tiles = tiles_m * tiles_n;
-  const int k_iters = (K + (FP8 ? 2 * BK : BK) - 1) / (FP8 ? 2 * BK : BK);
+  const int num_tiles = tiles_m * tiles_n * (RANGES ? ga.ranges.count : 1);
+  constexpr int STEP = FP8 ? 2 * BK : BK;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&sh->full[s], 1); mbar_init(&sh->empty[s], 1); }
@@ -142,15 +157,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       long long issued = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        const Tile ti = decode_tile(t, tiles_m, tiles_n, ga);
+        const Tile ti = decode_tile<RANGES>(t, tiles_m, tiles_n, K, STEP, ga);
         if (ti.skip) continue;
         const int m0 = ti.m0, n0 = ti.n0;
-        for (int k = 0; k < k_iters; ++k) {
+        for (int k = 0; k < ti.range.k_iters; ++k) {
           if (!mbar_wait(&sh->empty[stage], phase ^ 1, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_EMPTY); ok = false; break; }
           uint8_t* sa = smem + stage * STAGE_BYTES;
           uint8_t* sb = sa + A_BYTES;
           mbar_expect_tx(&sh->full[stage], STAGE_BYTES);
-          const int k0 = k * (FP8 ? 2 * BK : BK);
+          const int k0 = ti.range.k0 + k * STEP;
           if (!A_MN) {
             tma_load_2d(sa, &tma_a, &sh->full[stage], k0, m0);
           } else {
@@ -185,8 +200,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       int acc = 0; uint32_t acc_phase = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        const Tile ti = decode_tile(t, tiles_m, tiles_n, ga);
-        if (ti.skip) continue;
+        const Tile ti = decode_tile<RANGES>(t, tiles_m, tiles_n, K, STEP, ga);
+        const int k_iters = ti.range.k_iters;
+        if (ti.skip || (RANGES && k_iters <= 0)) continue;
         if (!mbar_wait(&sh->tmem_empty[acc], acc_phase ^ 1, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_TMEM_EMPTY); ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * ACC_COLS;
@@ -217,18 +233,25 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     int acc = 0; uint32_t acc_phase = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-      const Tile ti = decode_tile(t, tiles_m, tiles_n, ga);
+      const Tile ti = decode_tile<RANGES>(t, tiles_m, tiles_n, K, STEP, ga);
       if (ti.skip) continue;
       const int row = ti.m0 + q * 32 + lane;
       const int n0 = ti.n0;
-      if (!mbar_wait(&sh->tmem_full[acc], acc_phase, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_TMEM_FULL); ok = false; break; }
+      const bool nothing = RANGES && ti.range.k_iters <= 0;      // to reduce over: the product is zero (nothing to add when accumulating)
+      if (nothing && (EPI == EPI_F32_ACC || EPI == EPI_BF16_ACC)) continue;
+      if (!nothing && !mbar_wait(&sh->tmem_full[acc], acc_phase, abort_flag)) { atomicCAS(err, 0, ERR_WAIT_TMEM_FULL); ok = false; break; }
       tc_fence_after();
       const uint32_t taddr = tmem_base + acc * ACC_COLS + (static_cast<uint32_t>(q * 32) << 16);
 #pragma unroll 1
       for (int c = first; c < first + BN / 64; ++c) {
         uint32_t r[32];
-        tmem_ld_32x32b_x32(taddr + c * 32, r);
-        tmem_ld_wait();
+        if (!nothing) {
+          tmem_ld_32x32b_x32(taddr + c * 32, r);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) r[i] = 0;
+        }
         const int col = n0 + c * 32;
         if (FP8 && row < M && col < N) {
           const float rs = ga.row_scale != nullptr ? ga.row_scale[row] : 1.f;
@@ -247,7 +270,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         if (row < M && col < N) {
           const bool full = (col + 32 <= N);
           if (EPI == EPI_BF16 || EPI == EPI_BF16_ACC) {
-            __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(Dptr) + static_cast<long long>(row) * ldd + col;
+            __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(Dptr) + ti.range.d_off + static_cast<long long>(row) * ldd + col;
             if (full && ((reinterpret_cast<uintptr_t>(out) & 15) == 0)) {
               store_row_32<EPI == EPI_BF16_ACC>(out, r, al);
             } else {
@@ -261,7 +284,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
               }
             }
           } else {
-            float* out = reinterpret_cast<float*>(Dptr) + static_cast<long long>(row) * ldd + col;
+            float* out = reinterpret_cast<float*>(Dptr) + ti.range.d_off + static_cast<long long>(row) * ldd + col;
             if (full && ((reinterpret_cast<uintptr_t>(out) & 15) == 0)) {
               store_row_32<EPI == EPI_F32_ACC>(out, r, al);
             } else {
@@ -277,6 +300,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           }
         }
       }
+      if (nothing) continue;
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&sh->tmem_empty[acc]);
@@ -293,10 +317,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   }
 }
 
-template <bool A_MN, bool B_MN, int EPI>
+template <bool A_MN, bool B_MN, int EPI, bool RANGES = false>
 static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, void* D, int M, int N, int K, long long ldd,
                       float alpha, const GroupArgs& ga, int* err, int sms, cudaStream_t stream) {
-  auto kern = gemm_bf16_kernel<A_MN, B_MN, EPI>;
+  auto kern = gemm_bf16_kernel<A_MN, B_MN, EPI, false, RANGES>;
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -305,7 +329,7 @@ static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, void* D, int
     if (e != cudaSuccess) return static_cast<int>(e);
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * (RANGES ? ga.ranges.count : 1);
   const int grid = tiles < sms ? tiles : sms;
   kern<<<grid, THREADS, SMEM_BYTES, stream>>>(ta, tb, D, M, N, K, ldd, alpha, ga, err);
   return static_cast<int>(cudaGetLastError());
@@ -340,6 +364,16 @@ static int dispatch(int a_mn, int b_mn, int epi, const CUtensorMap& ta, const CU
   if (!a_mn && b_mn) return launch_epi<false, true>(epi, ta, tb, D, M, N, K, ldd, alpha, ga, err, sms, stream);
   if (a_mn && !b_mn) return launch_epi<true, false>(epi, ta, tb, D, M, N, K, ldd, alpha, ga, err, sms, stream);
   return launch_epi<true, true>(epi, ta, tb, D, M, N, K, ldd, alpha, ga, err, sms, stream);
+}
+
+static int operand_maps(CUtensorMap* ta, CUtensorMap* tb, const void* A, const void* B, int M, int N, int K, long long lda, long long ldb, int a_mn, int b_mn) {
+  int r;
+  if (!a_mn) r = make_tmap_2d(ta, A, M, K, lda, BM, BK, 2, true);
+  else       r = make_tmap_2d(ta, A, K, M, lda, BK, 64, 2, true);
+  if (r) return 1000 + r;
+  if (!b_mn) r = make_tmap_2d(tb, B, N, K, ldb, BN, BK, 2, true);
+  else       r = make_tmap_2d(tb, B, K, N, ldb, BK, 64, 2, true);
+  return r ? 2000 + r : 0;
 }
 
 }  // namespace gemm
@@ -377,16 +411,11 @@ extern "C" int dewb_gemm_bf16(const void* A, const void* B, void* D, int M, int 
   if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return -3;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
   CUtensorMap ta, tb;
-  int r;
-  if (!a_mn) r = make_tmap_2d(&ta, A, M, K, lda, BM, BK, 2, true);
-  else       r = make_tmap_2d(&ta, A, K, M, lda, BK, 64, 2, true);
-  if (r) return 1000 + r;
-  if (!b_mn) r = make_tmap_2d(&tb, B, N, K, ldb, BN, BK, 2, true);
-  else       r = make_tmap_2d(&tb, B, K, N, ldb, BK, 64, 2, true);
-  if (r) return 2000 + r;
+  const int r = operand_maps(&ta, &tb, A, B, M, N, K, lda, ldb, a_mn, b_mn);
+  if (r) return r;
   int sms = sm_count();
   if (max_ctas > 0 && max_ctas < sms) sms = max_ctas;
-  GroupArgs ga{nullptr, 0, 0, nullptr, nullptr, g_dense_bias};
+  GroupArgs ga{nullptr, 0, 0, nullptr, nullptr, g_dense_bias, {}};
   return dispatch(a_mn, b_mn, epi, ta, tb, D, M, N, K, ldd, alpha, ga, err, sms, stream);
 }
 
@@ -420,8 +449,50 @@ extern "C" int dewb_gmm_bf16(const void* A, const void* B, void* D, const int* t
   if (!b_mn) r = make_tmap_2d(&tb, B, static_cast<uint64_t>(groups) * N, K, ldb, BN, BK, 2, true);
   else       r = make_tmap_2d(&tb, B, static_cast<uint64_t>(groups) * K, N, ldb, BK, 64, 2, true);
   if (r) return 2000 + r;
-  GroupArgs ga{tile_group, 1, b_mn ? K : N, nullptr, nullptr, nullptr};
+  GroupArgs ga{tile_group, 1, b_mn ? K : N, nullptr, nullptr, nullptr, {}};
   return dispatch(0, b_mn, epi, ta, tb, D, M, N, K, ldd, alpha, ga, err, sm_count(), stream);
+}
+
+// dewb_gemm_bf16_split and dewb_tgmm_bf16 (gemm_pair_sm100.cu) on lone CTAs, for the same operands: for outputs whose pairs' tiles would be half empty or too few.
+extern "C" int dewb_gemm_bf16_split_single(const void* A, const void* B, void* D, float* scratch, int M, int N, int K, int splits, int per, long long lda, long long ldb,
+                                           long long ldd, int a_mn, int b_mn, int epi, float alpha, int* err, void* stream_ptr) {
+  using namespace dewb;
+  using namespace dewb::gemm;
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || (N % 4) || (ldd % 4) ||
+      (reinterpret_cast<uintptr_t>(D) & 15) || (reinterpret_cast<uintptr_t>(scratch) & 15) || splits < 1 || per % BK || per <= 0 ||
+      static_cast<long long>(splits) * per < K || static_cast<long long>(splits - 1) * per >= K || epi < 0 || epi > 3)
+    return -3;
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
+  CUtensorMap ta, tb;
+  int r = operand_maps(&ta, &tb, A, B, M, N, K, lda, ldb, a_mn, b_mn);
+  if (r) return r;
+  const GroupArgs ga{nullptr, 0, 0, nullptr, nullptr, nullptr, {nullptr, per, splits, static_cast<long long>(M) * N}};
+  if (!a_mn && !b_mn) r = launch_one<false, false, EPI_F32, true>(ta, tb, scratch, M, N, K, N, 1.f, ga, err, sm_count(), stream);
+  else if (!a_mn) r = launch_one<false, true, EPI_F32, true>(ta, tb, scratch, M, N, K, N, 1.f, ga, err, sm_count(), stream);
+  else if (!b_mn) r = launch_one<true, false, EPI_F32, true>(ta, tb, scratch, M, N, K, N, 1.f, ga, err, sm_count(), stream);
+  else r = launch_one<true, true, EPI_F32, true>(ta, tb, scratch, M, N, K, N, 1.f, ga, err, sm_count(), stream);
+  return r ? r : gemm_pair::split_sum(scratch, D, M, N, ldd, splits, alpha, epi, err, stream);
+}
+
+extern "C" int dewb_tgmm_bf16_single(const void* A, const void* B, void* D, const int* group_offsets, int R, int M, int N, int groups, long long lda, long long ldb, long long ldd,
+                                     long long d_group_stride, int epi, float alpha, int* err, void* stream_ptr) {
+  using namespace dewb;
+  using namespace dewb::gemm;
+  if (R <= 0 || M <= 0 || N <= 0 || groups <= 0) return 0;
+  if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return -3;
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
+  CUtensorMap ta, tb;
+  const int r = operand_maps(&ta, &tb, A, B, M, N, R, lda, ldb, 1, 1);
+  if (r) return r;
+  const GroupArgs ga{nullptr, 0, 0, nullptr, nullptr, nullptr, {group_offsets, 0, groups, d_group_stride}};
+  switch (epi) {
+    case EPI_BF16: return launch_one<true, true, EPI_BF16, true>(ta, tb, D, M, N, R, ldd, alpha, ga, err, sm_count(), stream);
+    case EPI_F32: return launch_one<true, true, EPI_F32, true>(ta, tb, D, M, N, R, ldd, alpha, ga, err, sm_count(), stream);
+    case EPI_F32_ACC: return launch_one<true, true, EPI_F32_ACC, true>(ta, tb, D, M, N, R, ldd, alpha, ga, err, sm_count(), stream);
+    case EPI_BF16_ACC: return launch_one<true, true, EPI_BF16_ACC, true>(ta, tb, D, M, N, R, ldd, alpha, ga, err, sm_count(), stream);
+  }
+  return -2;
 }
 
 // Row-wise scaled fp8 (e4m3) GEMM, dense or grouped rows: D[M,N] (bf16) = (A_q * a_scale[row]) * (B_q * b_scale[row of B])^T.
@@ -440,6 +511,6 @@ extern "C" int dewb_gemm_fp8(const void* A, const void* B, void* D, const float*
   if (r) return 1000 + r;
   r = make_tmap_2d(&tb, B, static_cast<uint64_t>(groups) * N, K, ldb, BN, 2 * BK, 1, true);
   if (r) return 2000 + r;
-  GroupArgs ga{tile_group, tile_group != nullptr ? 1 : 0, N, a_scale, b_scale, nullptr};
+  GroupArgs ga{tile_group, tile_group != nullptr ? 1 : 0, N, a_scale, b_scale, nullptr, {}};
   return launch_fp8(ta, tb, D, M, N, K, ldd, 1.f, ga, err, sm_count(), stream);
 }

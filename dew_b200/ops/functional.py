@@ -153,19 +153,14 @@ if "DEWB_DECODE_GEMM" not in os.environ:
 _SKINNY_PDL = int(os.environ.get("DEWB_SKINNY_PDL", "1"))
 
 
-def reduction_splits(M: int, N: int, K: int, sms: int = 148) -> int:
-    """Parts the reduction of a product with few output tiles is cut into: the fewest that come close to the shortest last wave of (256 x 256 tile, part) items over
-    the pairs of SMs, each at least 1024 long (a part costs its fp32 partial product, written and read once).  1: no cut - half a wave or more of a lone CTA's tiles
-    of 128 x 256, a short reduction, or nothing to gain."""
-    if -(-M // 128) * -(-N // 256) * 2 > sms:
-        return 1
-    tiles, pairs = -(-M // 256) * -(-N // 256), sms // 2
-    best, least = 1, float(-(-tiles // pairs))
+def _fewest_parts(tiles: int, at_once: int, K: int) -> int:
+    """Parts of at least 1024 that the reductions of ``tiles`` output tiles are cut into, ``at_once`` (tile, part) items at a time: the fewest that come close to the
+    shortest last wave (a part costs its fp32 partial product, written and read once)."""
+    best, least = 1, float(-(-tiles // at_once))
     for s in range(2, min(8, K // 1024) + 1):
-        per = -(-K // s // 64) * 64
-        if (s - 1) * per >= K:
+        if (s - 1) * (-(-K // s // 64) * 64) >= K:
             continue
-        wave = -(-tiles * s // pairs) / s
+        wave = -(-tiles * s // at_once) / s
         if wave < 0.85 * least:
             best, least = s, wave
     return best
@@ -179,9 +174,32 @@ def pairs_below_a_wave(M: int, N: int, K: int, sms: int = 148) -> bool:
     return K >= 4096 and -(-M // 256) * -(-N // 256) <= sms // 2
 
 
-def _parts(M: int, N: int, K: int, max_ctas: int, bias) -> int:
-    """``reduction_splits`` where the product may be split: partial products are joined in whole vectors, and take no bias."""
-    return reduction_splits(M, N, K) if max_ctas == 0 and bias is None and N % 4 == 0 else 1
+def split_reduction(M: int, N: int, K: int, sms: int = 148) -> Tuple[int, bool]:
+    """Parts that the reduction of a product with few output tiles is cut into, and whether pairs of CTAs take them.  1: no cut - half a wave or more of a lone CTA's
+    tiles, a short reduction, or nothing that pairs gain by it.
+
+    Pairs where their waves are as short as those of lone CTAs and the parts longer than 2048; then they fetch less, before that their tiles are as fast at best (lone CTAs /
+    pairs, us: 1536 x 1536 over 16384, halves, 100 / 87, over 4096 29.1 / 30.0; 768 x 2304 over 16384, fifths, 59 / 53; 640 x 768 over 6144, sixths, 17.4 / 18.4).
+    Odd numbers of 128 rows leave a pair's tile half empty (384 x 6144 over 4096, halves and thirds, 29 / 33; 1152 x 768 over 8192, fifths and quarters, 24 / 27)."""
+    lone = -(-M // 128) * -(-N // 256)
+    if lone * 2 > sms:
+        return 1, False
+    pairs, at_once = -(-M // 256) * -(-N // 256), sms // 2
+    by_lone, by_pairs = _fewest_parts(lone, sms, K), _fewest_parts(pairs, at_once, K)
+    if by_pairs == 1:
+        return 1, False
+    shorter = -(-pairs * by_pairs // at_once) * by_lone > -(-lone * by_lone // sms) * by_pairs
+    return (by_lone, False) if shorter or K <= 2048 * by_pairs else (by_pairs, True)
+
+
+def reduction_splits(M: int, N: int, K: int, sms: int = 148) -> int:
+    """The parts of ``split_reduction``."""
+    return split_reduction(M, N, K, sms)[0]
+
+
+def _parts(M: int, N: int, K: int, max_ctas: int, bias) -> Tuple[int, bool]:
+    """``split_reduction`` where the product may be split: partial products are joined in whole vectors, and take no bias."""
+    return split_reduction(M, N, K) if max_ctas == 0 and bias is None and N % 4 == 0 else (1, False)
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False,
@@ -224,11 +242,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     if kernel is None and cell is None and not _TUNE and not _GEMM.forced_by_environment() and _tensor_core_operands(a, b, out):
         # both tensor-core kernels take these operands and the size alone says which: nothing about the call needs looking up.  The pair kernel is 5-15 % faster on
         # the layer shapes; the single-CTA kernel keeps the very wide head.
-        paired = LARGE_GEMM == "sm100_pair" and N <= 32768 and _pair_built() and (
-            tiles >= 148 or max_ctas == 0 and pairs_below_a_wave(M, N, K) and _parts(M, N, K, max_ctas, bias) == 1)
+        parts = _parts(M, N, K, max_ctas, bias) if tiles < 148 else (1, False)
+        paired = LARGE_GEMM == "sm100_pair" and N <= 32768 and _pair_built() and (tiles >= 148 or max_ctas == 0 and parts[0] == 1 and pairs_below_a_wave(M, N, K))
         which = "sm100_pair" if paired else "sm100_tcgen05"
         _GEMM._record(which, {}, which if tiles >= 148 else None, None)
-        return _gemm_tensor_cores(which, a, b, out, M, N, K, a_mn, b_mn, accumulate, alpha, max_ctas, bias)
+        return _gemm_tensor_cores(which, a, b, out, M, N, K, a_mn, b_mn, accumulate, alpha, max_ctas, bias, parts)
     case = dict(dtype=a.dtype if a.dtype == b.dtype else None, lda=a.stride(0), ldb=b.stride(0), ldd=out.stride(0),
                 aligned=(a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0),
                 inner_contig=(a.stride(1) == 1 and b.stride(1) == 1 and out.stride(1) == 1), M=M, N=N, K=K, plain=plain, k_major=plain and fresh,
@@ -259,7 +277,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         L.check(rc, which)
         L.count_launches()
         return out
-    return _gemm_tensor_cores(which, a, b, out, M, N, K, a_mn, b_mn, accumulate, alpha, max_ctas, bias)
+    return _gemm_tensor_cores(which, a, b, out, M, N, K, a_mn, b_mn, accumulate, alpha, max_ctas, bias,
+                              _parts(M, N, K, max_ctas, bias) if which == "sm100_tcgen05" else (1, False))
 
 
 def _tensor_core_operands(a, b, out) -> bool:
@@ -269,27 +288,22 @@ def _tensor_core_operands(a, b, out) -> bool:
             and (a.data_ptr() | b.data_ptr() | out.data_ptr()) % 16 == 0)
 
 
-def _gemm_tensor_cores(which, a, b, out, M, N, K, a_mn, b_mn, accumulate, alpha, max_ctas, bias):
+def _gemm_tensor_cores(which, a, b, out, M, N, K, a_mn, b_mn, accumulate, alpha, max_ctas, bias, parts=(1, False)):
     epi = {(torch.bfloat16, False): 0, (torch.float32, False): 1, (torch.float32, True): 2, (torch.bfloat16, True): 3}[(out.dtype, bool(accumulate))]
     lib, at = L.load(), L.at
-    lda, ldb, ldd = a.stride(0), b.stride(0), out.stride(0)
-    launches = 1
-    if bias is not None:
+    splits, paired = parts if parts[0] > 1 else (1, which == "sm100_pair")
+    strides, rest = (a.stride(0), b.stride(0), out.stride(0)), (int(a_mn), int(b_mn), epi, alpha, at(L.status(a.device)))
+    if splits > 1:
+        scratch = torch.empty(splits, M, N, dtype=torch.float32, device=a.device)
+        fns, args = (lib.dewb_gemm_bf16_split, lib.dewb_gemm_bf16_split_single), (at(a), at(b), at(out), at(scratch), M, N, K, splits, -(-K // splits // 64) * 64, *strides, *rest)
+    elif bias is not None:
         bb = bias.to(torch.bfloat16).contiguous()                 # referenced until the launch is enqueued
-        fn = lib.dewb_gemm_pair_bf16_bias if which == "sm100_pair" else lib.dewb_gemm_bf16_bias
-        rc = fn(at(a), at(b), at(out), at(bb), M, N, K, lda, ldb, ldd, int(a_mn), int(b_mn), epi, alpha, at(L.status(a.device)), max_ctas, L.stream())
+        fns, args = (lib.dewb_gemm_pair_bf16_bias, lib.dewb_gemm_bf16_bias), (at(a), at(b), at(out), at(bb), M, N, K, *strides, *rest, max_ctas)
     else:
-        splits = _parts(M, N, K, max_ctas, bias) if which == "sm100_tcgen05" else 1
-        if splits > 1:
-            scratch = torch.empty(splits, M, N, dtype=torch.float32, device=a.device)
-            rc = lib.dewb_gemm_bf16_split(at(a), at(b), at(out), at(scratch), M, N, K, splits, -(-K // splits // 64) * 64, lda, ldb, ldd, int(a_mn), int(b_mn), epi, alpha,
-                                          at(L.status(a.device)), L.stream())
-            launches = 2
-        else:
-            fn = lib.dewb_gemm_pair_bf16 if which == "sm100_pair" else lib.dewb_gemm_bf16
-            rc = fn(at(a), at(b), at(out), M, N, K, lda, ldb, ldd, int(a_mn), int(b_mn), epi, alpha, at(L.status(a.device)), max_ctas, L.stream())
+        fns, args = (lib.dewb_gemm_pair_bf16, lib.dewb_gemm_bf16), (at(a), at(b), at(out), M, N, K, *strides, *rest, max_ctas)
+    rc = fns[0 if paired else 1](*args, L.stream())
     L.check(rc, which)
-    L.count_launches(launches)
+    L.count_launches(2 if splits > 1 else 1)
     return out
 
 

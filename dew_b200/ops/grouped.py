@@ -104,6 +104,13 @@ def gmm_forward(x, w, layout: GroupLayout, transpose_w: bool = False, out=None):
     return out
 
 
+def pairs_reduce(rows: int, M: int, N: int, groups: int, sms: int = 148) -> bool:
+    """Whether pairs of CTAs take ``groups`` products ``[M, N]`` over ``rows`` in all: long reductions, for which they fetch less, and many tiles, of which a pair stores one while
+    it works on the next (lone CTAs / pairs, us: 64 of 768 into 2816 x 2048 498 / 430, of 128 rows 285 / 271; 8 of 2048 into 640 x 2048 52 / 44; but 16 of 128 into 512 x 256
+    10.0 / 10.9, 64 of 128 into 512 x 512 16.0 / 16.4).  Up to 128 rows leave half of a pair's tile empty (64 of 128 into 128 x 768 9.6 / 12.3, of 1024 28.9 / 28.1)."""
+    return rows // groups >= (512 if M > 128 else 1024) or groups * -(-M // 128) * -(-N // 256) > 4 * sms
+
+
 def tgmm(dy, x, layout: GroupLayout, groups: int, out: Optional[torch.Tensor] = None, accumulate: bool = False):
     """Per-group ``dW[g] = dy[rows of g]^T @ x[rows of g]`` -> ``[G, N, K]`` (fp32 when accumulating into ``out``)."""
     if not L.use_cuda(dy, x) or x.dtype != torch.bfloat16:
@@ -118,9 +125,9 @@ def tgmm(dy, x, layout: GroupLayout, groups: int, out: Optional[torch.Tensor] = 
         out = torch.empty((groups, N, K), dtype=torch.bfloat16, device=dy.device)
         accumulate = False
     epi = {(torch.bfloat16, False): 0, (torch.float32, False): 1, (torch.float32, True): 2, (torch.bfloat16, True): 3}[(out.dtype, accumulate)]
-    rc = L.load().dewb_tgmm_bf16(L.ptr(dy), L.ptr(x), L.ptr(out), L.ptr(layout.offsets), c_int(R), c_int(N), c_int(K),
-                                 c_int(groups), c_ll(dy.stride(0)), c_ll(x.stride(0)), c_ll(out.stride(1)),
-                                 c_ll(out.stride(0)), c_int(epi), c_float(1.0), L.ptr(L.status(dy.device)), L.stream_ptr())
+    lib, args = L.load(), (L.ptr(dy), L.ptr(x), L.ptr(out), L.ptr(layout.offsets), c_int(R), c_int(N), c_int(K), c_int(groups), c_ll(dy.stride(0)), c_ll(x.stride(0)),
+                           c_ll(out.stride(1)), c_ll(out.stride(0)), c_int(epi), c_float(1.0), L.ptr(L.status(dy.device)), L.stream_ptr())
+    rc = (lib.dewb_tgmm_bf16 if pairs_reduce(R, N, K, groups) else lib.dewb_tgmm_bf16_single)(*args)
     L.check(rc, "tgmm_bf16")
     L.count_launches()
     return out

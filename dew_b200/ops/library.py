@@ -74,6 +74,7 @@ _SIGNATURES = {
     "dewb_gemm_bf16_bias": "pppp" + "iii" + "lll" + "iii" + "f" + "pip",
     "dewb_gemm_pair_bf16_bias": "pppp" + "iii" + "lll" + "iii" + "f" + "pip",
     "dewb_gemm_bf16_split": "pppp" + "iiiii" + "lll" + "iii" + "f" + "pp",
+    "dewb_gemm_bf16_split_single": "pppp" + "iiiii" + "lll" + "iii" + "f" + "pp",
     "dewb_colsum_slabs": "li",
     "dewb_colsum_bf16": "ppp" + "lil" + "p",
     "dewb_ada_slab": "ii",

@@ -79,3 +79,25 @@ def test_pairs_below_a_wave(M, N, K):
     got = ops.gemm(A, B, out_dtype=torch.float32)
     L.check_status()
     assert torch.equal(got, ops.gemm(A, B, out_dtype=torch.float32, kernel="sm100_tcgen05", max_ctas=148))       # either kernel's sums are in the same order
+
+
+# the same groups and parts by either kind of CTAs: outputs within one tile's rows and past them, rows and columns to spare
+@pytest.mark.parametrize("paired", [False, True])
+@pytest.mark.parametrize("dtype,acc", [(torch.bfloat16, False), (torch.bfloat16, True), (torch.float32, False), (torch.float32, True)])
+@pytest.mark.parametrize("M,N", [(72, 264), (384, 520)])
+def test_reductions_by_either_kind(M, N, dtype, acc, paired, monkeypatch):
+    from dew_b200.ops import functional, grouped
+    monkeypatch.setattr(grouped, "pairs_reduce", lambda *a: paired)
+    test_grouped_reductions(M, N, dtype, acc)
+    g = torch.Generator(device=DEV).manual_seed(M)
+    for K, parts in ((2056, 2), (4096, 3)):
+        monkeypatch.setattr(functional, "split_reduction", lambda *a: (parts, paired))
+        A, B = torch.randn(K, M, generator=g, device=DEV).bfloat16(), torch.randn(N, K, generator=g, device=DEV).bfloat16()
+        held = torch.randn(M, N, generator=g, device=DEV).to(dtype)
+        out = held.clone()
+        ops.gemm(A, B, a_mn=True, out=out, accumulate=acc, kernel="sm100_tcgen05")
+        L.check_status()
+        exact = A.double().T @ B.double().T + (held.double() if acc else 0)
+        # fp32 sums of K exact products in some order, and one rounding of the result
+        bound = K * 2.0 ** -24 * (A.double().abs().T @ B.double().abs().T) + (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -23) * exact.abs()
+        assert bool(((out.double() - exact).abs() <= bound).all())

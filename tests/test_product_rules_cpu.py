@@ -1,8 +1,11 @@
 """Which kernel a product of a size gets: the rules themselves, and where they lead, on the CPU."""
+import random
+
 import pytest
 import torch
 
 from dew_b200.ops import functional as Fn
+from dew_b200.ops import grouped
 from dew_b200.ops import library as L
 
 SMS = 148
@@ -15,6 +18,25 @@ pair_tiles = lambda M, N: up(M, 256) * up(N, 256)
 @pytest.mark.parametrize("M,N,K", [(1152, 4096, 4096), (1025, 4096, 14336), (640, 7168, 4096), (384, 12288, 4096), (300, 12288, 4096), (384, 11264, 8192), (128, 19200, 4096), (128, 32768, 8192)])
 def test_pairs_make_no_second_wave(M, N, K):
     assert lone_tiles(M, N) <= SMS < 2 * pair_tiles(M, N) and not Fn.pairs_below_a_wave(M, N, K)
+
+
+def test_rules_over_the_sizes():
+    rng = random.Random(0)
+    for _ in range(4000):
+        M, N, K = (int(2 ** rng.uniform(*r)) for r in ((0, 13), (3, 15), (6, 16)))
+        if Fn.pairs_below_a_wave(M, N, K):
+            assert pair_tiles(M, N) <= SMS // 2 and K >= 4096
+        parts, paired = Fn.split_reduction(M, N, K)
+        assert parts == Fn.reduction_splits(M, N, K) and 1 <= parts <= 8
+        if parts == 1:
+            assert not paired
+            continue
+        per = up(up(K, parts), 64) * 64
+        assert 2 * lone_tiles(M, N) <= SMS and (parts - 1) * per < K <= parts * per and K >= 1024 * parts
+        if paired:                                                        # no longer waves than lone CTAs would have, whatever these split
+            assert K > 2048 * parts
+            least = min(up(lone_tiles(M, N) * s, SMS) / s for s in range(1, 9) if s <= max(1, K // 1024))
+            assert up(pair_tiles(M, N) * parts, SMS // 2) / parts <= least / 0.85
 
 
 class Launchers:
@@ -50,6 +72,7 @@ def product(M, N, K, **kw):
 
 @pytest.mark.parametrize("M,N,K,kw,kernel", [
     (2048, 2048, 64, {}, "dewb_gemm_bf16"), (2048, 2048, 8192, {}, "dewb_gemm_pair_bf16"), (1152, 4096, 4096, {}, "dewb_gemm_bf16"), (2048, 2560, 64, {}, "dewb_gemm_pair_bf16"),
+    (1536, 1536, 16384, {}, "dewb_gemm_bf16_split"), (384, 6144, 4096, {}, "dewb_gemm_bf16_split_single"), (1024, 768, 2048, {}, "dewb_gemm_bf16_split_single"),
     # a bias is added by the kernel that makes the whole product: no parts, so the line for pairs is that of unsplit ones
     (1024, 768, 3072, dict(bias=True), "dewb_gemm_bf16_bias"), (512, 3072, 12288, dict(bias=True), "dewb_gemm_pair_bf16_bias"), (1536, 1536, 16384, dict(bias=True), "dewb_gemm_pair_bf16_bias"),
     (1152, 4096, 4096, dict(bias=True), "dewb_gemm_bf16_bias"), (1536, 1536, 16384, dict(max_ctas=100), "dewb_gemm_bf16")])
@@ -57,3 +80,12 @@ def test_products_get_their_kernels(launched, M, N, K, kw, kernel):
     calls = launched()
     product(M, N, K, **kw)
     assert [c for c in calls if "gemm" in c] == [kernel]
+
+
+def test_grouped_reductions_get_their_kernels(launched):
+    layout = grouped.group_layout(torch.arange(8).repeat_interleave(512), 8)
+    calls = launched()
+    for M, N in ((256, 1024), (128, 256)):
+        grouped.tgmm(torch.empty(layout.rows, M, dtype=torch.bfloat16), torch.empty(layout.rows, N, dtype=torch.bfloat16), layout, 8)
+    assert calls == ["dewb_tgmm_bf16", "dewb_tgmm_bf16_single"]
+    assert not grouped.pairs_reduce(16 * 128, 512, 256, 16) and grouped.pairs_reduce(64 * 128, 2816, 2048, 64) and not grouped.pairs_reduce(64 * 128, 128, 768, 64)

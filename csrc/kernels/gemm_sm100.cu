@@ -453,7 +453,8 @@ extern "C" int dewb_gmm_bf16(const void* A, const void* B, void* D, const int* t
   return dispatch(0, b_mn, epi, ta, tb, D, M, N, K, ldd, alpha, ga, err, sm_count(), stream);
 }
 
-// dewb_gemm_bf16_split and dewb_tgmm_bf16 (gemm_pair_sm100.cu) on lone CTAs, for the same operands: for outputs whose pairs' tiles would be half empty or too few.
+// dewb_gemm_bf16_split and dewb_tgmm_bf16 (gemm_pair_sm100.cu) on lone CTAs, for the same operands: for outputs whose pairs' tiles would be half empty or too few, and where pairs
+// cannot be placed.
 extern "C" int dewb_gemm_bf16_split_single(const void* A, const void* B, void* D, float* scratch, int M, int N, int K, int splits, int per, long long lda, long long ldb,
                                            long long ldd, int a_mn, int b_mn, int epi, float alpha, int* err, void* stream_ptr) {
   using namespace dewb;

@@ -301,7 +301,9 @@ def _gemm_tensor_cores(which, a, b, out, M, N, K, a_mn, b_mn, accumulate, alpha,
         fns, args = (lib.dewb_gemm_pair_bf16_bias, lib.dewb_gemm_bf16_bias), (at(a), at(b), at(out), at(bb), M, N, K, *strides, *rest, max_ctas)
     else:
         fns, args = (lib.dewb_gemm_pair_bf16, lib.dewb_gemm_bf16), (at(a), at(b), at(out), M, N, K, *strides, *rest, max_ctas)
-    rc = fns[0 if paired else 1](*args, L.stream())
+    rc = fns[0](*args, L.stream()) if paired else L.NO_PAIRS
+    if rc == L.NO_PAIRS:
+        rc = fns[1](*args, L.stream())
     L.check(rc, which)
     L.count_launches(2 if splits > 1 else 1)
     return out

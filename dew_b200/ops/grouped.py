@@ -127,7 +127,9 @@ def tgmm(dy, x, layout: GroupLayout, groups: int, out: Optional[torch.Tensor] = 
     epi = {(torch.bfloat16, False): 0, (torch.float32, False): 1, (torch.float32, True): 2, (torch.bfloat16, True): 3}[(out.dtype, accumulate)]
     lib, args = L.load(), (L.ptr(dy), L.ptr(x), L.ptr(out), L.ptr(layout.offsets), c_int(R), c_int(N), c_int(K), c_int(groups), c_ll(dy.stride(0)), c_ll(x.stride(0)),
                            c_ll(out.stride(1)), c_ll(out.stride(0)), c_int(epi), c_float(1.0), L.ptr(L.status(dy.device)), L.stream_ptr())
-    rc = (lib.dewb_tgmm_bf16 if pairs_reduce(R, N, K, groups) else lib.dewb_tgmm_bf16_single)(*args)
+    rc = lib.dewb_tgmm_bf16(*args) if pairs_reduce(R, N, K, groups) else L.NO_PAIRS
+    if rc == L.NO_PAIRS:
+        rc = lib.dewb_tgmm_bf16_single(*args)
     L.check(rc, "tgmm_bf16")
     L.count_launches()
     return out

@@ -197,6 +197,9 @@ def check_status(device: Optional[torch.device] = None) -> None:
         raise KernelError(f"device kernel reported: {ERROR_NAMES.get(code, code)}")
 
 
+NO_PAIRS = -6          # of the products' launchers: clusters of two CTAs cannot be placed on this device (lone CTAs then take the product)
+
+
 def check(rc: int, what: str) -> None:
     if rc != 0:
         raise KernelError(f"{what}: launcher returned {rc}")

@@ -40,22 +40,22 @@ def test_rules_over_the_sizes():
 
 
 class Launchers:
-    """Stands in for the library: notes what is launched."""
+    """Stands in for the library: notes what is launched, and says that pairs cannot be placed where ``pairs`` is false."""
 
-    def __init__(self):
-        self.calls = []
+    def __init__(self, pairs):
+        self.pairs, self.calls = pairs, []
 
     def __getattr__(self, name):
         def launch(*args):
             self.calls.append(name)
-            return 0
+            return 0 if self.pairs or name not in ("dewb_gemm_pair_bf16", "dewb_gemm_pair_bf16_bias", "dewb_gemm_bf16_split", "dewb_tgmm_bf16") else -6
         return launch
 
 
 @pytest.fixture
 def launched(monkeypatch):
-    def made():
-        lib = Launchers()
+    def made(pairs=True):
+        lib = Launchers(pairs)
         monkeypatch.setattr(L, "load", lambda *a: lib)
         monkeypatch.setattr(L, "use_cuda", lambda *a: True)
         monkeypatch.setattr(L, "stream", lambda *a: 0)
@@ -82,10 +82,18 @@ def test_products_get_their_kernels(launched, M, N, K, kw, kernel):
     assert [c for c in calls if "gemm" in c] == [kernel]
 
 
+@pytest.mark.parametrize("M,N,K,kw,kernel", [(2048, 2560, 64, {}, "dewb_gemm_bf16"), (2048, 2560, 64, dict(bias=True), "dewb_gemm_bf16_bias"), (1536, 1536, 16384, {}, "dewb_gemm_bf16_split_single")])
+def test_lone_ctas_where_pairs_cannot_be_placed(launched, M, N, K, kw, kernel):
+    calls = launched(pairs=False)
+    product(M, N, K, **kw)
+    assert [c for c in calls if "gemm" in c][-1] == kernel
+
+
 def test_grouped_reductions_get_their_kernels(launched):
     layout = grouped.group_layout(torch.arange(8).repeat_interleave(512), 8)
-    calls = launched()
-    for M, N in ((256, 1024), (128, 256)):
-        grouped.tgmm(torch.empty(layout.rows, M, dtype=torch.bfloat16), torch.empty(layout.rows, N, dtype=torch.bfloat16), layout, 8)
-    assert calls == ["dewb_tgmm_bf16", "dewb_tgmm_bf16_single"]
+    for pairs in (True, False):
+        calls = launched(pairs)
+        for M, N in ((256, 1024), (128, 256)):
+            grouped.tgmm(torch.empty(layout.rows, M, dtype=torch.bfloat16), torch.empty(layout.rows, N, dtype=torch.bfloat16), layout, 8)
+        assert calls == (["dewb_tgmm_bf16"] if pairs else ["dewb_tgmm_bf16", "dewb_tgmm_bf16_single"]) + ["dewb_tgmm_bf16_single"]
     assert not grouped.pairs_reduce(16 * 128, 512, 256, 16) and grouped.pairs_reduce(64 * 128, 2816, 2048, 64) and not grouped.pairs_reduce(64 * 128, 128, 768, 64)

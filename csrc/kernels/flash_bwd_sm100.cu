@@ -30,7 +30,15 @@ constexpr int SOFTMAX_REGS = 104, ISSUE_REGS = 64;
 static_assert(4 * SOFTMAX_REGS + ISSUE_REGS <= 5 * 96, "an increase past what the block was launched with never ends");
 constexpr float LOG2E = 1.4426950408889634f;
 using attn::Variant;
-using attn::soft_tanh;
+
+// A capped score is cap * tanh(x), x = score / cap.  With e = e^(-2 |x|) and u = 1 / (1 + e) the tangent is (1 - e) u with the sign of x, and its derivative 4 e u^2: one exponential
+// and one reciprocal for both, and a derivative that is as good where it is small (with 1 - tanh^2 of a second pair in dK / dV the backward of 8192 tokens, 4 heads of 128 over
+// one, took 1273 us, 995 now).  `twice`: 2 log2(e) x / score.
+__device__ __forceinline__ float capped(uint32_t score, float twice, float& slope) {
+  const float x = __uint_as_float(score) * twice, e = fast_exp2(-fabsf(x)), u = __fdividef(1.f, 1.f + e);
+  slope = 4.f * e * u * u;
+  return copysignf((1.f - e) * u, x);
+}
 
 // ---------------------------------------------------------------------------------------------------------------
 // delta[b,h,s] = sum_d dO * O.  Bound by the read of dO and O.  A block takes ROWS consecutive positions of one head; D / 8 lanes share a row with one 16-byte
@@ -404,10 +412,9 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
         for (int i = 0; i < COLS; i += 2) {
           float x0, x1, f0 = 1.f, f1 = 1.f;           // f: d(capped score) / d(score)
           if (VAR && var.softcap > 0.f) {
-            const float cap2 = var.softcap * LOG2E, inv_cap2 = 1.f / cap2;
-            const float t0 = soft_tanh(__uint_as_float(v[i]) * scale_log2 * inv_cap2), t1 = soft_tanh(__uint_as_float(v[i + 1]) * scale_log2 * inv_cap2);
-            x0 = cap2 * t0 + nlse; x1 = cap2 * t1 + nlse;
-            f0 = 1.f - t0 * t0; f1 = 1.f - t1 * t1;
+            const float cap2 = var.softcap * LOG2E, twice = 2.f * scale / var.softcap * LOG2E;
+            x0 = fmaf(cap2, capped(v[i], twice, f0), nlse);
+            x1 = fmaf(cap2, capped(v[i + 1], twice, f1), nlse);
           } else {
             unpair(fma2(pair_of(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), factor, shift), x0, x1);
           }
@@ -720,10 +727,14 @@ flash_dkv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
       for (int i = 0; i < COLS; i += 4) {
         const float4 l4 = lse4[i >> 2];
         if (VAR && var.softcap > 0.f) {
-          const float cap2 = var.softcap * LOG2E, inv_cap2 = 1.f / cap2;
+          const float cap2 = var.softcap * LOG2E, twice = 2.f * scale / var.softcap * LOG2E;
           const float l[4] = {l4.x, l4.y, l4.z, l4.w};
 #pragma unroll
-          for (int q = 0; q < 4; ++q) p[i + q] = cap2 * soft_tanh(__uint_as_float(v[i + q]) * scale_log2 * inv_cap2) + l[q];
+          for (int q = 0; q < 4; ++q) {
+            float slope;
+            p[i + q] = fmaf(cap2, capped(v[i + q], twice, slope), l[q]);
+            v[i + q] = __float_as_uint(slope);
+          }
         } else {
           unpair(fma2(pair_of(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), factor, pair_of(l4.x, l4.y)), p[i], p[i + 1]);
           unpair(fma2(pair_of(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3])), factor, pair_of(l4.z, l4.w)), p[i + 2], p[i + 3]);
@@ -764,12 +775,8 @@ flash_dkv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
       for (int i = 0; i < COLS; i += 2) pk[i >> 1] = pack_bf16(p[i], p[i + 1]);
       if (VAR && var.softcap > 0.f) {
         // from here on the weight times d(capped score) / d(score)
-        const float cap2 = var.softcap * LOG2E, inv_cap2 = 1.f / cap2;
 #pragma unroll
-        for (int i = 0; i < COLS; ++i) {
-          const float t = soft_tanh(__uint_as_float(v[i]) * scale_log2 * inv_cap2);
-          p[i] *= 1.f - t * t;
-        }
+        for (int i = 0; i < COLS; ++i) p[i] *= __uint_as_float(v[i]);
       }
       if (C::P_APART) {
         // the product before has read its P^T

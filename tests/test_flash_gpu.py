@@ -198,3 +198,27 @@ def test_variants_of_few_tiles_take_no_longer():
             times.append(a.elapsed_time(b))
         took.append(sorted(times)[3])
     assert took[1] < 1.35 * took[0], took
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_flash_backward_of_saturated_caps(D):
+    """Scores of seven to nine caps, whose capped values have derivatives of 1e-6 and less: these hold to fp32 relative to themselves, not to 1; then a rounding of the scores'
+    gradients to bf16 (2^-9), and one of the results."""
+    from dew_b200.ops.flash import Variants, flash_bwd, flash_fwd
+    g = torch.Generator(device=DEV).manual_seed(D)
+    S = 256
+    q, k = torch.zeros(1, S, 2, D, device=DEV), torch.zeros(1, S, 1, D, device=DEV)
+    q[..., 0] = 8
+    k[..., 0] = (torch.randint(0, 2, (1, S, 1), generator=g, device=DEV) * 2 - 1) * (7 + 2 * torch.rand(1, S, 1, generator=g, device=DEV)) / 8 * D ** 0.5
+    q, k = q.bfloat16(), k.bfloat16()
+    v, do = (torch.randn(1, S, h, D, generator=g, device=DEV).bfloat16() for h in (1, 2))
+    var = Variants(softcap=1.0)
+    out, lse = flash_fwd(q, k, v, True, D ** -0.5, var=var)
+    _, dk, _ = flash_bwd(do, q, k, v, out, lse, True, D ** -0.5, var=var)
+    L.check_status()
+    leaves = [x.double().requires_grad_() for x in (q, k, v)]
+    scores = torch.tanh(torch.einsum("bshd,bthd->bhst", leaves[0], leaves[1].repeat_interleave(2, 2)) * D ** -0.5)
+    scores = scores.masked_fill(~torch.ones(S, S, dtype=torch.bool, device=DEV).tril(), float("-inf"))
+    want, = torch.autograd.grad(torch.einsum("bhst,bthd->bshd", torch.softmax(scores, -1), leaves[2].repeat_interleave(2, 2)), leaves[1:2], do.double())
+    # (of the keys' gradient: the queries' is a sum over keys that nearly cancels where the derivatives are alike)
+    assert rel_err(dk[..., 0], want[..., 0]) < 2.0 ** -7

@@ -44,9 +44,15 @@ class SimpleDiT(nn.Module):
         tokens = self.embed(x.to(dt))
         tokens = tokens + sincos_grid(gh, gw, self.emb_features, tokens.device, dt)[None]
         c = self.conditioning(temb, conditions.get("text"), conditions.get("label"), duration, conditions.get("guidance"))
-        # the blocks and the output share one silu(c), where nobody sees what they are given
-        active = F.silu(c)
-        given = lambda m: (active,) if type(m) in (ModulatedBlock, PatchSequenceOutput) and runs_alone(m) else ()
+        # the blocks and the output share one silu(c), where nobody sees what they are given; made for the first that takes it
+        active = []
+
+        def given(m):
+            if type(m) not in (ModulatedBlock, PatchSequenceOutput) or not runs_alone(m) or not getattr(m, "adaln_silu", True):
+                return ()
+            if not active:
+                active.append(F.silu(c))
+            return active
         routed = None
         for i, block in enumerate(self.blocks):
             if train and self.routes:

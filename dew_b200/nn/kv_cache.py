@@ -184,7 +184,7 @@ class KVStore:
         self.page_table = default_page_table(rows, self.max_pages, device) if spec.pages is None else \
             torch.zeros(rows, self.max_pages, dtype=torch.int32, device=device)
         self.lengths = torch.zeros(rows, dtype=torch.int32, device=device)
-        self.dtype, self.device = dtype, torch.device(device)
+        self.dtype, self.device = dtype, self.lengths.device               # (with the index that "cuda" leaves out)
         self.row_ids: Optional[torch.Tensor] = None      # rows of the store addressed by the batch rows of a call
         self._scratch = None
         self.chunk_span: Optional[Tuple[int, int]] = None      # (first position, one past the last) of the prefill chunk in flight, when the caller knows

@@ -3,7 +3,7 @@ import pytest
 import torch
 
 from dew_b200.models import CausalTransformer, decode_step
-from dew_b200.nn.kv_cache import KVCache
+from dew_b200.nn.kv_cache import KVCache, KVStore
 from dew_b200.sampling.text import RowBatch
 
 DEV = "cuda"
@@ -65,6 +65,18 @@ def test_same_bits_as_the_layers(rows, kw, monkeypatch):
     assert taken.n == 3
     assert all(torch.equal(a, b) for a, b in zip(one, by_layers))
     assert torch.equal(keys, batch.store.k) and torch.equal(values, batch.store.v)
+
+
+@pytest.mark.gpu
+def test_a_store_knows_its_device(monkeypatch):
+    """Asked for on "cuda", it is on the current device, as the rows are."""
+    model = decoder(DEV)
+    batch, lengths = rows_of(model, 1)
+    batch.store = KVStore(KVCache(page_size=64), len(model.layers), 1, 400, 2, 128, torch.bfloat16, "cuda")
+    assert batch.store.device == lengths.device
+    taken = Taken(monkeypatch)
+    batch.forward(torch.zeros(1, 1, dtype=torch.long, device=DEV), torch.zeros(1, 1, dtype=torch.long, device=DEV))
+    assert taken.n == 1
 
 
 @pytest.mark.gpu

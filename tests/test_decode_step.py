@@ -80,12 +80,10 @@ def test_a_store_knows_its_device(monkeypatch):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("kw", [dict(qk_norm=True), dict(mlp_activation="gelu_tanh"), dict(attn_bias=True), dict(residual_multiplier=0.5), dict(sandwich_norm=True)])
+@pytest.mark.parametrize("kw", [dict(qk_norm=True), dict(mlp_activation="gelu_tanh"), dict(attn_bias=True), dict(qkv_bias=True), dict(residual_multiplier=0.5), dict(sandwich_norm=True),
+                                dict(attn_softcap=30.0), dict(query_scale=0.2), dict(attn_out_gate=True)])
 def test_other_layers_go_their_own_way(kw, monkeypatch):
-    try:
-        model = decoder(DEV, **kw)
-    except TypeError:
-        pytest.skip(f"no option {sorted(kw)}")
+    model = decoder(DEV, **kw)
     batch, lengths = rows_of(model, 1)
     taken = Taken(monkeypatch)
     batch.forward(torch.zeros(1, 1, dtype=torch.long, device=DEV), lengths[:, None])

@@ -55,8 +55,8 @@ def occupancy(registers: int, launch: Launch, static_smem: int = 0) -> Occupancy
 
 # launch shapes of the tensor-core kernels (threads, dynamic shared memory, tensor-memory columns), as their launchers set them
 LAUNCHES: Dict[str, Launch] = {
-    "gemm_bf16_kernel": Launch(192, 4 * 49152 + 1280, 512),
-    "gemm_pair_kernel": Launch(192, 6 * 32768 + 1280, 512),
+    "gemm_bf16_kernel": Launch(320, 4 * 49152 + 1280, 512),
+    "gemm_pair_kernel": Launch(320, 6 * 32768 + 1280, 512),
     "gemm_mx_kernel": Launch(320, 5 * 40960 + 1280, 512),
     "flash_fwd_kernel": Launch(320, 229376 + 2560, 512),
     "flash_fwd_pair_kernel": Launch(384, 229376 + 2048, 512),

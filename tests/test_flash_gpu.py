@@ -129,14 +129,10 @@ def test_flash_halves_of_a_rows_keys(B, S, T, Hq, Hkv, D, causal, sinks):
 # of both, beside a window that starts in every place of a tile; documents that end inside a tile, of a few tokens, and padding behind the last
 @pytest.mark.parametrize("B,S,Hq,Hkv,D", [(1, 100, 2, 1, 64), (1, 256, 3, 3, 128), (2, 640, 4, 2, 64), (1, 1100, 5, 1, 128), (2, 768, 16, 16, 64), (6, 384, 16, 16, 64), (1, 896, 32, 8, 128),
                                           (2, 128, 100, 100, 64)])
-@pytest.mark.parametrize("kind", ["window", "keep", "keep many", "chunk", "softcap", "gain", "sigmoid", "packed", "packed short", "packed and padded", "window and documents", "sinks and window"])
-@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("kind,causal", [(kind, True) for kind in ("window", "keep", "keep many", "chunk", "softcap", "gain", "sigmoid", "packed", "packed short", "packed and padded",
+                                                                  "window and documents", "sinks and window")] + [(kind, False) for kind in ("window", "chunk", "softcap", "packed")])
 def test_flash_variants_of_few_tiles(B, S, Hq, Hkv, D, kind, causal):
     from dew_b200.ops.flash import Variants, flash_fwd
-    if kind == "sigmoid" and not causal:
-        pytest.skip("sigmoid weights are causal")
-    if not causal and kind not in ("softcap", "packed", "window", "chunk"):
-        pytest.skip("the walk is the causal one's")
     g = torch.Generator(device=DEV).manual_seed(S + Hq)
     q, k, v = (torch.randn(B, S, h, D, generator=g, device=DEV).bfloat16() for h in (Hq, Hkv, Hkv))
     at = torch.arange(S, device=DEV)
@@ -147,8 +143,6 @@ def test_flash_variants_of_few_tiles(B, S, Hq, Hkv, D, kind, causal):
               sigmoid=dict(sigmoid=torch.randn(Hq, generator=g, device=DEV)), **{"keep many": dict(window=130, keep=300), "window and documents": dict(window=200),
                                                                                  "sinks and window": dict(window=200, sinks=torch.randn(Hq, generator=g, device=DEV))}).get(kind, {})
     if kind in docs:
-        if S % 4:
-            pytest.skip("rows of documents are on 16-byte boundaries")
         kw["segments"] = docs[kind].to(torch.int32)[None].expand(B, S).contiguous()
     out, lse = flash_fwd(q, k, v, causal, D ** -0.5, need_lse=kind != "sigmoid", var=Variants(**kw))
     L.check_status()
@@ -177,6 +171,13 @@ def test_flash_variants_of_few_tiles(B, S, Hq, Hkv, D, kind, causal):
         assert float((lse.double() - want_lse).abs().max()) < 1e-5 * max(1.0, float(want_lse.abs().max()))
     # a rounding of the weights (2^-9) and one of the result
     assert rel_err(out, torch.einsum("bhst,bthd->bshd", weights, v.double().repeat_interleave(Hq // Hkv, 2))) < 2.0 ** -8
+
+
+# more items than CTAs, of neighbouring rows (which start at different key tiles) and of two heads: kept first tiles in front of a window, in the walk of one tile or of both
+@pytest.mark.parametrize("B,S,Hq,Hkv,D", [(2, 1280, 17, 17, 64), (2, 1152, 24, 4, 128), (1, 2176, 22, 2, 64)])
+@pytest.mark.parametrize("kind", ["window", "keep", "keep many", "chunk", "softcap", "sigmoid", "packed", "packed short", "packed and padded", "window and documents"])
+def test_flash_variants_of_several_items_a_cta(B, S, Hq, Hkv, D, kind):
+    test_flash_variants_of_few_tiles(B, S, Hq, Hkv, D, kind, True)
 
 
 def test_variants_of_few_tiles_take_no_longer():

@@ -7,6 +7,7 @@ path, which is also the numerics oracle the GPU tests compare against.
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 import os
 from typing import Optional, Tuple
@@ -174,6 +175,7 @@ def pairs_below_a_wave(M: int, N: int, K: int, sms: int = 148) -> bool:
     return K >= 4096 and -(-M // 256) * -(-N // 256) <= sms // 2
 
 
+@functools.lru_cache(maxsize=4096)          # (asked for every product of a few tiles: 7 us to work out, while the host sets the pace of small models)
 def split_reduction(M: int, N: int, K: int, sms: int = 148) -> Tuple[int, bool]:
     """Parts that the reduction of a product with few output tiles is cut into, and whether pairs of CTAs take them.  1: no cut - half a wave or more of a lone CTA's
     tiles, a short reduction, or nothing that pairs gain by it.
@@ -182,7 +184,7 @@ def split_reduction(M: int, N: int, K: int, sms: int = 148) -> Tuple[int, bool]:
     pairs, us: 1536 x 1536 over 16384, halves, 100 / 87, over 4096 29.1 / 30.0; 768 x 2304 over 16384, fifths, 59 / 53; 640 x 768 over 6144, sixths, 17.4 / 18.4).
     Odd numbers of 128 rows leave a pair's tile half empty (384 x 6144 over 4096, halves and thirds, 29 / 33; 1152 x 768 over 8192, fifths and quarters, 24 / 27)."""
     lone = -(-M // 128) * -(-N // 256)
-    if lone * 2 > sms:
+    if lone * 2 > sms or K < 2048:
         return 1, False
     pairs, at_once = -(-M // 256) * -(-N // 256), sms // 2
     by_lone, by_pairs = _fewest_parts(lone, sms, K), _fewest_parts(pairs, at_once, K)
@@ -242,8 +244,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     if kernel is None and cell is None and not _TUNE and not _GEMM.forced_by_environment() and _tensor_core_operands(a, b, out):
         # both tensor-core kernels take these operands and the size alone says which: nothing about the call needs looking up.  The pair kernel is 5-15 % faster on
         # the layer shapes; the single-CTA kernel keeps the very wide head.
-        parts = _parts(M, N, K, max_ctas, bias) if tiles < 148 else (1, False)
-        paired = LARGE_GEMM == "sm100_pair" and N <= 32768 and _pair_built() and (tiles >= 148 or max_ctas == 0 and parts[0] == 1 and pairs_below_a_wave(M, N, K))
+        parts = _parts(M, N, K, max_ctas, bias) if tiles <= 74 else (1, False)
+        paired = (tiles >= 148 or K >= 4096 and max_ctas == 0 and parts[0] == 1 and pairs_below_a_wave(M, N, K)) and LARGE_GEMM == "sm100_pair" and N <= 32768 and _pair_built()
         which = "sm100_pair" if paired else "sm100_tcgen05"
         _GEMM._record(which, {}, which if tiles >= 148 else None, None)
         return _gemm_tensor_cores(which, a, b, out, M, N, K, a_mn, b_mn, accumulate, alpha, max_ctas, bias, parts)
@@ -291,21 +293,24 @@ def _tensor_core_operands(a, b, out) -> bool:
 def _gemm_tensor_cores(which, a, b, out, M, N, K, a_mn, b_mn, accumulate, alpha, max_ctas, bias, parts=(1, False)):
     epi = {(torch.bfloat16, False): 0, (torch.float32, False): 1, (torch.float32, True): 2, (torch.bfloat16, True): 3}[(out.dtype, bool(accumulate))]
     lib, at = L.load(), L.at
-    splits, paired = parts if parts[0] > 1 else (1, which == "sm100_pair")
-    strides, rest = (a.stride(0), b.stride(0), out.stride(0)), (int(a_mn), int(b_mn), epi, alpha, at(L.status(a.device)))
+    lda, ldb, ldd = a.stride(0), b.stride(0), out.stride(0)
+    splits, launches = parts[0], 1
     if splits > 1:
         scratch = torch.empty(splits, M, N, dtype=torch.float32, device=a.device)
-        fns, args = (lib.dewb_gemm_bf16_split, lib.dewb_gemm_bf16_split_single), (at(a), at(b), at(out), at(scratch), M, N, K, splits, -(-K // splits // 64) * 64, *strides, *rest)
+        fn = lib.dewb_gemm_bf16_split if parts[1] else lib.dewb_gemm_bf16_split_single
+        rc = fn(at(a), at(b), at(out), at(scratch), M, N, K, splits, -(-K // splits // 64) * 64, lda, ldb, ldd, int(a_mn), int(b_mn), epi, alpha, at(L.status(a.device)), L.stream())
+        launches = 2
     elif bias is not None:
         bb = bias.to(torch.bfloat16).contiguous()                 # referenced until the launch is enqueued
-        fns, args = (lib.dewb_gemm_pair_bf16_bias, lib.dewb_gemm_bf16_bias), (at(a), at(b), at(out), at(bb), M, N, K, *strides, *rest, max_ctas)
+        fn = lib.dewb_gemm_pair_bf16_bias if which == "sm100_pair" else lib.dewb_gemm_bf16_bias
+        rc = fn(at(a), at(b), at(out), at(bb), M, N, K, lda, ldb, ldd, int(a_mn), int(b_mn), epi, alpha, at(L.status(a.device)), max_ctas, L.stream())
     else:
-        fns, args = (lib.dewb_gemm_pair_bf16, lib.dewb_gemm_bf16), (at(a), at(b), at(out), M, N, K, *strides, *rest, max_ctas)
-    rc = fns[0](*args, L.stream()) if paired else L.NO_PAIRS
+        fn = lib.dewb_gemm_pair_bf16 if which == "sm100_pair" else lib.dewb_gemm_bf16
+        rc = fn(at(a), at(b), at(out), M, N, K, lda, ldb, ldd, int(a_mn), int(b_mn), epi, alpha, at(L.status(a.device)), max_ctas, L.stream())
     if rc == L.NO_PAIRS:
-        rc = fns[1](*args, L.stream())
+        return _gemm_tensor_cores("sm100_tcgen05", a, b, out, M, N, K, a_mn, b_mn, accumulate, alpha, max_ctas, bias, (splits, False))
     L.check(rc, which)
-    L.count_launches(2 if splits > 1 else 1)
+    L.count_launches(launches)
     return out
 
 

@@ -247,7 +247,7 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
     const int q = warp & 3;
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
     // The words of the next AHEAD stages are on their way while one is staged: a stage's products take 400 cycles, and loads that were waited for one stage after another
-    // took longer than that (the four products of a 64-expert layer's step, 8192 tokens, 2048 x 1408, top 6: 1375 us, with the issue out of one lane of a divergent warp; 1124 now).
+    // took longer than that (the four products of a 64-expert layer's step, 8192 tokens, 2048 x 1408, top 6: 1375 us, with the issue out of one lane of a divergent warp; 1000 now).
     int t = blockIdx.x, k = 0;                       // the next stage to load
     const uint32_t *pa = nullptr, *pb = nullptr;
     auto begin_tile = [&]() -> bool {
